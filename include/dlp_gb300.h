@@ -149,9 +149,9 @@ typedef struct dlp_config {
                               thread block with block barriers; bit 1: passes
                               over mid-size frontiers run on a sub-grid with its
                               own barrier; bit 2: within the one-block mode,
-                              frontiers of at most 64 loaded rows run on 8 warps
-                              with a named barrier. Default 7 (all); same
-                              results. */
+                              only the warps that hold rows of the frontier run,
+                              with a named barrier (otherwise all warps of the
+                              block). Default 7 (all); same results. */
   int solo_entry;        /* one-block mode for total frontiers of at most this
                             many vertices; 0 = 512, at most 1024 (autotuned) */
   int subgrid_entry;     /* sub-grid mode for total frontiers of at most this
@@ -304,8 +304,8 @@ int dlp_engine_steps(const dlp_engine *e);
 int dlp_engine_debug(dlp_engine *e, int *out4);
 int dlp_engine_elapsed_ms(dlp_engine *e, int first_step, int last_step, float *ms);
 /* Propagation passes the engine's launches have run so far, by mode, and the
- * device time they took: [0] one block (including [1]), [1] the 8-warp team
- * (passes only; its time is counted in [0]), [2] the 16-block sub-grid,
+ * device time they took: [0] one block (including [1]), [1] those of
+ * them run by at most 16 warps (passes only; their time is counted in [0]), [2] the 16-block sub-grid,
  * [3] the full grid. Diagnostics of where a workload's propagation time goes;
  * cumulative since the engine was made. */
 int dlp_engine_pass_modes(dlp_engine *e, unsigned long long *passes4, double *seconds4);

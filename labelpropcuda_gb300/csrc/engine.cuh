@@ -49,6 +49,7 @@ struct EngineCtl {
   // overwrite a value a slow block has yet to read.
   int solo_k[2];
   int solo_passes[2];
+  int solo_full[2];     // a one-block stint ended for lack of room
   // Stop requests, written by thread 0 of block 0 and read by every block at
   // the top of a pass: (launch tag << 32) | the pass at which to stop. A read
   // at the top of pass k takes only a request naming pass k, so a request
@@ -60,7 +61,7 @@ struct EngineCtl {
   unsigned long long slice_stop;  // the launch's time slice ran out
   unsigned long long t_launch;  // global timer at the start of the launch (thread 0 of block 0)
   // Propagation passes run so far by mode, and the device time they took
-  // (global timer): 0 one block, 1 of which the 8-warp team, 2 sub-grid,
+  // (global timer): 0 one block, 1 of which by at most 16 warps, 2 sub-grid,
   // 3 full grid. Written by thread 0 of block 0 only, once per launch.
   unsigned long long mode_passes[4];
   unsigned long long mode_ns[4];
@@ -72,7 +73,7 @@ struct EngineArgs {
   int ng_new;   // the first ng_new of them start a batch; the rest continue one
   EngineCtl *ectl;
   unsigned long long timeout_ns;
-  int solo;  // bit 0: one-block passes; bit 1: sub-grid passes; bit 2: team passes
+  int solo;  // bit 0: one-block passes; bit 1: sub-grid passes; bit 2: one-block passes by the warps that hold rows only
   int fast_div;    // 1: the reference's fast-math division (dlp_config.arithmetic), else IEEE
   int solo_entry;  // total frontier at most this: one-block passes (<= kSoloEntryMax)
   int sub_entry;   // total frontier at most this: sub-grid passes (<= kSubLive)
