@@ -146,16 +146,17 @@ typedef struct dlp_config {
   int blocks_per_sm;     /* persistent grid occupancy; 0 = from the occupancy query */
   double wait_timeout_s; /* limit for any device-side wait; <= 0: 2 s */
   int small_frontier_solo; /* bit 0: passes over small frontiers run on one
-                              thread block with block barriers; bit 1: passes
-                              over mid-size frontiers run on a sub-grid with its
-                              own barrier; bit 2: within the one-block mode,
+                              thread block with block barriers; bit 1: accepted
+                              and without effect (mid-size frontiers run on the
+                              full grid, which is faster than a part of it);
+                              bit 2: within the one-block mode,
                               only the warps that hold rows of the frontier run,
                               with a named barrier (otherwise all warps of the
                               block). Default 7 (all); same results. */
   int solo_entry;        /* one-block mode for total frontiers of at most this
                             many vertices; 0 = 512, at most 1024 (autotuned) */
-  int subgrid_entry;     /* sub-grid mode for total frontiers of at most this
-                            many; 0 = 2048, at most 4096 (autotuned) */
+  int subgrid_entry;     /* in [0, 4096]; accepted and without effect (see
+                            small_frontier_solo, bit 1) */
   int arithmetic;        /* enum dlp_arithmetic: the division of the label
                             updates (default DLP_ARITH_IEEE) */
 } dlp_config;
@@ -305,8 +306,8 @@ int dlp_engine_debug(dlp_engine *e, int *out4);
 int dlp_engine_elapsed_ms(dlp_engine *e, int first_step, int last_step, float *ms);
 /* Propagation passes the engine's launches have run so far, by mode, and the
  * device time they took: [0] one block (including [1]), [1] those of
- * them run by at most 16 warps (passes only; their time is counted in [0]), [2] the 16-block sub-grid,
- * [3] the full grid. Diagnostics of where a workload's propagation time goes;
+ * them run by at most 16 warps (passes only; their time is counted in [0]), [2] always 0 (the
+ * sub-grid mode of earlier versions), [3] the full grid. Diagnostics of where a workload's propagation time goes;
  * cumulative since the engine was made. */
 int dlp_engine_pass_modes(dlp_engine *e, unsigned long long *passes4, double *seconds4);
 int dlp_session_pass_modes(dlp_session *s, unsigned long long *passes4, double *seconds4);

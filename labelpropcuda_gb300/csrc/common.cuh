@@ -135,6 +135,78 @@ __device__ __forceinline__ bool grid_sync(GridBarrier *bar, int *err, uint64_t t
   return grid_sync_n(bar, gridDim.x * gridDim.y * gridDim.z, err, timeout_ns);
 }
 
+// Barrier over all blocks of a cooperative launch, in one hop: every block adds
+// one word to a counter and one thread of it polls that counter, so an arrival
+// is seen after one addition and one load instead of two dependent atomics, a
+// release and a poll. The word is 64 bits of fields that the addition sums over
+// the blocks (arrivals, rows, blocks that moved a label, that want to stop,
+// that failed), which saves the loads that would follow the barrier. Four
+// counters take turns: block 0 clears the one used two generations ago, which
+// every block has read before it arrived at this one, and which is added to
+// again two generations on.
+//
+// Measured on 152 blocks of 1,024 threads, full-grid passes of replays: 5.1 us
+// a pass at 5,000 vertices, 7.5 to 8.0 at 50,000 and 16.2 at 500,000, against
+// 7.1 to 7.2, 9.4 to 10.1 and 17.7 to 18 with GridBarrier. (A word per block
+// polled by all blocks, 152 words each, gave 5.3 to 8.1 and 8 to 11 us: the
+// polls of 760 warps queue up in the L2 slices that hold the words.)
+//
+// The counters start at zero in every launch. Every wait has a time limit; a
+// block that runs out records DLP_ERR_TIMEOUT and leaves, and so do the blocks
+// that then wait for it.
+constexpr int kSumBlocks = 255;  // blocks at most
+constexpr unsigned long long kSumArrival = 1ull << 56, kSumError = 1ull << 48, kSumStop = 1ull << 40,
+                             kSumMoved = 1ull << 32;  // the low 32 bits sum a count
+
+struct SumBarrier {
+  struct {
+    unsigned long long v;
+    unsigned long long pad[15];
+  } word[4];
+};
+
+struct SumState {  // in shared memory, one per block
+  unsigned gen;    // barriers passed
+  unsigned long long sum;
+};
+
+// All threads of all blocks call. mine() is evaluated by thread 0 after the
+// block's own barrier; `sum` receives the fields summed over the blocks. False
+// when a block sent kSumError or a wait ran out.
+template <class Mine>
+__device__ __forceinline__ bool sum_sync(SumBarrier *bar, SumState &f, int *err, uint64_t timeout_ns, Mine mine,
+                                         unsigned long long &sum) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned gen = f.gen;
+    unsigned long long *word = &bar->word[gen & 3].v;
+    const unsigned long long add = kSumArrival | mine();
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(add) : "memory");
+    const unsigned long long want = static_cast<unsigned long long>(gridDim.x) << 56;
+    unsigned long long v;
+    uint64_t t0 = 0;
+    for (unsigned spins = 1;; ++spins) {
+      asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
+      if (v >= want) break;
+      if ((spins & 63u) == 0) {
+        const uint64_t now = global_timer_ns();
+        if (t0 == 0) t0 = now;
+        if (now - t0 > timeout_ns) {
+          atomicCAS(err, 0, DLP_ERR_TIMEOUT);
+          v = kSumError;
+          break;
+        }
+      }
+    }
+    if (blockIdx.x == 0) bar->word[(gen + 2) & 3].v = 0;
+    f.gen = gen + 1;
+    f.sum = v;
+  }
+  __syncthreads();
+  sum = f.sum;
+  return (sum & (0xffull * kSumError)) == 0;
+}
+
 // Appends the set lanes' values to list[*count ...] with one atomic per warp.
 // Must be called by all lanes of the warp (convergent).
 __device__ __forceinline__ void warp_append(bool pred, int value, int *list, int *count) {

@@ -377,7 +377,7 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
   GraphRec *recs = e->recs_dev + (p ? e->max_graphs : 0);
   DLP_CUDA_TRY(cudaMemcpyAsync(recs, rh, sizeof(GraphRec) * total, cudaMemcpyHostToDevice, e->stream));
   DLP_CUDA_TRY(cudaEventRecord(e->recs_free[p], e->stream));
-  dlp::engine::launch_zero_counters(recs, count, e->stream);
+  dlp::engine::launch_zero_counters(recs, count, e->ectl, e->stream);
   DLP_CUDA_TRY(cudaGetLastError());
   // every step_sliced call reads back which batches ended, budget or not
   const bool sliced = opts.resume || opts.pass_budget > 0 || opts.slice_ns > 0;
@@ -390,7 +390,6 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
   args.solo = e->cfg.small_frontier_solo < 0 ? 7 : e->cfg.small_frontier_solo;
   args.fast_div = e->cfg.arithmetic == DLP_ARITH_REFERENCE_FAST_MATH ? 1 : 0;
   args.solo_entry = e->cfg.solo_entry > 0 ? e->cfg.solo_entry : dlp::engine::kSoloEntryDefault;
-  args.sub_entry = e->cfg.subgrid_entry > 0 ? e->cfg.subgrid_entry : dlp::engine::kSubEntryDefault;
   args.pass_budget = opts.pass_budget;
   args.slice_ns = opts.slice_ns;
   args.tag = e->steps + 1;
@@ -623,7 +622,7 @@ int dlp_engine_create(const dlp_config *cfg_in, int max_graphs, size_t memory_bu
       per_sm <= 0)
     return bail(dlp::fail(DLP_ERR_CUDA, "occupancy query failed for the engine kernel"));
   if (cfg.blocks_per_sm > 0) per_sm = std::min(per_sm, cfg.blocks_per_sm);
-  e->grid = sms * per_sm;
+  e->grid = std::min(sms * per_sm, dlp::kSumBlocks);
   int st = DLP_OK;
   if ((st = dalloc(&e->ectl, 1, e->owned, e->owned_bytes)) ||
       (st = dalloc(&e->ctl_all, max_graphs, e->owned, e->owned_bytes)) ||

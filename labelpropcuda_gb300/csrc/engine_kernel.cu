@@ -78,6 +78,16 @@ __device__ __forceinline__ GV view(const EngineArgs &e, int g) {
   return GV{r.st, r.ba, static_cast<unsigned>(r.ba.seq) + 1u, r.st.ctl->stamp_base + 1u};
 }
 
+// ------------------------------------------------------- launch barrier ----
+__shared__ SumState s_bar;
+__shared__ int s_bad;  // this block found invalid input
+
+// All blocks of the launch; false when the launch has to end.
+__device__ __forceinline__ bool launch_sync(const EngineArgs &e) {
+  unsigned long long sum;
+  return sum_sync(&e.ectl->bar, s_bar, &e.ectl->err, e.timeout_ns, [] { return s_bad ? kSumError : 0ull; }, sum);
+}
+
 // ----------------------------------------------------------- warp helpers --
 // Reserves one slot per predicated lane in the list whose counter is `count`;
 // lanes of one warp may target different counters (different graphs).
@@ -285,7 +295,10 @@ __device__ void phase_a(const EngineArgs &e, const Ctx &c, int *pref) {
     const GraphRec &r = e.recs[g];
     r.st.ctl->touched_count[r.ba.seq & 1] = 0;
   }
-  if (bad) atomicCAS(&e.ectl->err, 0, DLP_ERR_INVALID_ARGUMENT);
+  if (bad) {
+    atomicCAS(&e.ectl->err, 0, DLP_ERR_INVALID_ARGUMENT);
+    s_bad = 1;
+  }
 }
 
 // ---------------------------------------------------------------- phase B ---
@@ -580,7 +593,7 @@ __device__ bool phase_d_sv(const EngineArgs &e, const Ctx &c, int *pref) {
       }
       if (changed) *flag = 1;
     });
-    if (!grid_sync(&e.ectl->bar, &e.ectl->err, e.timeout_ns)) return false;
+    if (!launch_sync(e)) return false;
     total = flat_build(pref, ng, [&](int g) { return active(g) && hook_count(view(e, g)) > 0 ? e.recs[g].ba.I : 0; });
     for (int item = c.gtid; item < total; item += c.nthreads) {
       const int g = locate(pref, ng, item);
@@ -594,7 +607,7 @@ __device__ bool phase_d_sv(const EngineArgs &e, const Ctx &c, int *pref) {
       }
       s.par[i] = p;
     }
-    if (!grid_sync(&e.ectl->bar, &e.ectl->err, e.timeout_ns)) return false;
+    if (!launch_sync(e)) return false;
   }
   return true;
 }
@@ -1446,53 +1459,16 @@ __device__ __forceinline__ void pass_sizes(const EngineArgs &e, int k, int *pref
   tw = pref2[ng];
 }
 
-// Sub-grid mode: mid-size frontiers are run by the first kSubBlocks blocks
-// with their own (cheaper) barrier while the other blocks wait at the next
-// grid barrier; the passes are those of the full grid.
-constexpr int kSubBlocks = 16;
-static_assert(kSubEntryMax <= kSubLive, "the sub-grid mode leaves above kSubLive");
-
-template <int G>
-__device__ bool sub_passes(const EngineArgs &e, int k0, int slot, int solo_from, int *pref, int *pref2) {
-  const int lane = threadIdx.x & 31;
-  const int warp0 = blockIdx.x * (kBlock / 32), nwarps = kSubBlocks * (kBlock / 32);
-  const int t0 = blockIdx.x * kBlock + threadIdx.x, nthreads = kSubBlocks * kBlock;
-  const uint64_t start = global_timer_ns();
-  int k = k0;
-  for (;; ++k) {
-    int tn, tw;
-    pass_sizes(e, k, pref, pref2, tn, tw);
-    const bool stop = ld_relaxed_u64(&e.ectl->sub_stop) == stop_code(e, k);
-    if (tn + tw == 0 || tn + tw > kSubLive || stop || (e.pass_budget > 0 && k >= e.pass_budget)) break;
-    // a frontier the one-block mode can take goes back to it (cheaper passes),
-    // unless that mode recently could not hold its working set
-    if (k > k0 && (e.solo & 1) && tn + tw <= e.solo_entry && k >= solo_from) break;
-    run_pass<G>(e, k, pref, tn, pref2, tw, lane, warp0 + (threadIdx.x >> 5), nwarps, t0, nthreads);
-    if (t0 == 0 && ((k - k0) & 31) == 31 && global_timer_ns() - start > 100000000ull)
-      e.ectl->sub_stop = stop_code(e, k + 1);
-    if (t0 == 0 && ((k - k0) & 7) == 7 && slice_over(e)) {
-      e.ectl->sub_stop = stop_code(e, k + 1);
-      e.ectl->slice_stop = stop_code(e, k + 1);
-    }
-    if (!grid_sync_n(&e.ectl->sub_bar, kSubBlocks, &e.ectl->err, e.timeout_ns)) return false;
-  }
-  if (t0 == 0) {
-    e.ectl->solo_k[slot] = k;
-    e.ectl->solo_passes[slot] = k - k0;
-  }
-  return true;
-}
-
 // The propagation passes of the launch; k_end is the first pass not run (the
 // graphs whose frontier is live at k_end continue in a later launch).
 template <int G>
 __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2, int &k_end) {
-  int no_small_at = -1;  // a pass the small modes declined goes to the full grid
+  int no_small_at = -1;  // a pass the one-block mode declined goes to the full grid
   int solo_from = 0;     // the one-block mode declined: not tried again before this pass
   int stint_no = 0;
   int k = 0;
   // thread 0 of block 0: passes and device time per mode in this launch
-  unsigned long long mp[3] = {0, 0, 0}, mns[3] = {0, 0, 0};  // one block, sub-grid, full grid
+  unsigned long long mp[2] = {0, 0}, mns[2] = {0, 0};  // one block, full grid
   for (;; ++k) {
     int tn, tw;
     pass_sizes(e, k, pref, pref2, tn, tw);
@@ -1501,47 +1477,39 @@ __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2
     if (ld_relaxed_u64(&e.ectl->slice_stop) == stop_code(e, k)) break;
     if (c.gtid == 0) e.ectl->where_pass = k;
     const bool solo_ok = (e.solo & 1) && tn + tw <= e.solo_entry && k != no_small_at && k >= solo_from;
-    const bool sub_ok = !solo_ok && (e.solo & 2) && gridDim.x > 2 * kSubBlocks && tn + tw <= e.sub_entry &&
-                        k != no_small_at;
-    if (solo_ok || sub_ok) {
+    if (solo_ok) {
       const uint64_t ts = c.gtid == 0 ? global_timer_ns() : 0;
-      if (solo_ok) {
-        if (blockIdx.x == 0) solo_passes(e, k, stint_no & 1);
-      } else if (blockIdx.x < kSubBlocks) {
-        if (!sub_passes<G>(e, k, stint_no & 1, solo_from, pref, pref2)) return false;
-      }
-      if (!grid_sync(&e.ectl->bar, &e.ectl->err, e.timeout_ns)) return false;
+      if (blockIdx.x == 0) solo_passes(e, k, stint_no & 1);
+      if (!launch_sync(e)) return false;
       const int done = ld_relaxed_i32(&e.ectl->solo_passes[stint_no & 1]);
       const int kk = ld_relaxed_i32(&e.ectl->solo_k[stint_no & 1]);
       ++stint_no;
       if (c.gtid == 0) {
-        mp[solo_ok ? 0 : 1] += done;
-        mns[solo_ok ? 0 : 1] += global_timer_ns() - ts;
+        mp[0] += done;
+        mns[0] += global_timer_ns() - ts;
       }
       if (done == 0) no_small_at = k;
       // A stint that ran out of room soon would run out again: a load costs
       // several passes, so the frontier stays with the grid for a while.
-      if (solo_ok && done < 256 && ld_relaxed_i32(&e.ectl->solo_full[(stint_no - 1) & 1])) solo_from = kk + 256;
+      if (done < 256 && ld_relaxed_i32(&e.ectl->solo_full[(stint_no - 1) & 1])) solo_from = kk + 256;
       k = kk - 1;  // the loop increment resumes at pass kk
       continue;
     }
     const uint64_t tp = c.gtid == 0 ? global_timer_ns() : 0;
     run_pass<G>(e, k, pref, tn, pref2, tw, c.lane, c.gwarp, c.nwarps, c.gtid, c.nthreads);
     if (c.gtid == 0 && slice_over(e)) e.ectl->slice_stop = stop_code(e, k + 1);
-    if (!grid_sync(&e.ectl->bar, &e.ectl->err, e.timeout_ns)) return false;
+    if (!launch_sync(e)) return false;
     if (c.gtid == 0) {
-      ++mp[2];
-      mns[2] += global_timer_ns() - tp;
+      ++mp[1];
+      mns[1] += global_timer_ns() - tp;
     }
   }
   k_end = k;
   if (c.gtid == 0) {
     e.ectl->mode_passes[0] += mp[0];
     e.ectl->mode_ns[0] += mns[0];
-    e.ectl->mode_passes[2] += mp[1];
-    e.ectl->mode_ns[2] += mns[1];
-    e.ectl->mode_passes[3] += mp[2];
-    e.ectl->mode_ns[3] += mns[2];
+    e.ectl->mode_passes[3] += mp[1];
+    e.ectl->mode_ns[3] += mns[1];
   }
   return true;
 }
@@ -1619,10 +1587,12 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) engine_kernel(const __g
   const Ctx c = make_ctx();
   __shared__ int pref[kMaxGraphs + 1];
   __shared__ int pref2[kMaxGraphs + 1];
-  GridBarrier *bar = &e.ectl->bar;
-  int *err = &e.ectl->err;
-  const uint64_t to = e.timeout_ns;
-  if (ld_relaxed_i32(err) != 0) return;
+  if (ld_relaxed_i32(&e.ectl->err) != 0) return;
+  if (threadIdx.x == 0) {
+    s_bar.gen = 0;
+    s_bad = 0;
+  }
+  __syncthreads();
 
   // block 0 records the last phase it reached (read back after a timeout)
   auto at = [&](int phase) {
@@ -1632,31 +1602,31 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) engine_kernel(const __g
   if (e.ng_new > 0) {  // a launch that only continues batches starts at phase G
     at(1);
     phase_a(e, c, pref);
-    if (!grid_sync(bar, err, to)) return;
+    if (!launch_sync(e)) return;
     at(2);
     phase_b(e, c, pref);
-    if (!grid_sync(bar, err, to)) return;
+    if (!launch_sync(e)) return;
     at(3);
     phase_c(e, c, pref);
-    if (!grid_sync(bar, err, to)) return;
+    if (!launch_sync(e)) return;
     at(4);
     phase_d_frontier(e, c, pref);
     if (!phase_d_sv(e, c, pref)) return;
     at(5);
-    if (!grid_sync(bar, err, to)) return;
+    if (!launch_sync(e)) return;
     at(6);
     phase_e(e, c, pref);
-    if (!grid_sync(bar, err, to)) return;
+    if (!launch_sync(e)) return;
     at(7);
     phase_f(e, c, pref);
-    if (!grid_sync(bar, err, to)) return;
+    if (!launch_sync(e)) return;
   }
   at(8);
   int k_end = 0;
   if (!phase_g<G>(e, c, pref, pref2, k_end)) return;
   at(9);
   phase_h(e, c, pref, k_end);
-  if (!grid_sync(bar, err, to)) return;
+  if (!launch_sync(e)) return;
   at(10);
 
   // per-graph statistics and the state the next batch starts from
@@ -1715,15 +1685,20 @@ template __global__ void engine_kernel<8>(const __grid_constant__ EngineArgs);
 template __global__ void engine_kernel<16>(const __grid_constant__ EngineArgs);
 template __global__ void engine_kernel<32>(const __grid_constant__ EngineArgs);
 
-// One block per graph that starts a batch: its counters back to zero.
-__global__ void zero_counters_kernel(const GraphRec *recs) {
+// One block per graph that starts a batch: its counters back to zero; block 0
+// also clears the launch's barrier.
+__global__ void zero_counters_kernel(const GraphRec *recs, int ng_new, EngineCtl *ectl) {
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < 4) ectl->bar.word[threadIdx.x].v = 0;
+  }
+  if (blockIdx.x >= ng_new) return;
   int *p = reinterpret_cast<int *>(recs[blockIdx.x].st.bc);
   constexpr int kWords = static_cast<int>(sizeof(BatchCounters) / sizeof(int));
   for (int i = threadIdx.x; i < kWords; i += blockDim.x) p[i] = 0;
 }
 
-void launch_zero_counters(const GraphRec *recs, int ng_new, cudaStream_t stream) {
-  if (ng_new > 0) zero_counters_kernel<<<ng_new, 128, 0, stream>>>(recs);
+void launch_zero_counters(const GraphRec *recs, int ng_new, EngineCtl *ectl, cudaStream_t stream) {
+  zero_counters_kernel<<<ng_new > 0 ? ng_new : 1, 128, 0, stream>>>(recs, ng_new, ectl);
 }
 
 size_t engine_dynamic_smem() { return sizeof(SoloCache); }
