@@ -133,7 +133,8 @@ struct dlp_engine {
   size_t used = 0;
   int lanes = 8;
   int grid = 0;
-  size_t smem = 0;
+  size_t smem = 0;      // dynamic shared memory of a launch over frontier lists
+  size_t smem_all = 0;  // all there is: launches with owned passes
   const void *kernel = nullptr;
   cudaStream_t stream = nullptr;
   std::vector<void *> owned;
@@ -156,6 +157,8 @@ struct dlp_engine {
   bool ev_made = false;
   int2 *progress_dev = nullptr;     // per launch position: {finished, passes}
   int2 *progress_host = nullptr;    // pinned copy
+  unsigned char *marks = nullptr;   // two planes of frontier marks (owned passes), all zero between stints
+  unsigned mark_plane = 0;          // bytes of a plane
   int inflight = 0;                 // graphs whose batch continues in a later step
   std::vector<int> last_finished;   // graphs whose batch ended in the last sliced step
 
@@ -168,6 +171,7 @@ struct dlp_engine {
         delete g;
       }
     for (void *p : owned) cudaFree(p);
+    cudaFree(marks);
     if (progress_host) cudaFreeHost(progress_host);
     for (int i = 0; i < 2; ++i) {
       if (recs_host[i]) cudaFreeHost(recs_host[i]);
@@ -236,6 +240,30 @@ int grow_graph_scratch(dlp_engine *e, GraphSlot *g, int E, int D) {
     g->keep_cap = cap;
   }
   return DLP_OK;
+}
+
+// A graph's vertices among those of a launch: whole tiles.
+size_t owned_room(int n) { return (static_cast<size_t>(n) + 63) & ~static_cast<size_t>(63); }
+
+// Mark planes for a launch over all resident graphs, as far as a grid can own
+// their vertices; sized when graphs are added, so that steps allocate nothing.
+// Without them (no memory, or a larger launch) passes run over frontier lists.
+void grow_marks(dlp_engine *e) {
+  size_t want = 0;
+  for (GraphSlot *g : e->graphs)
+    if (g) want += owned_room(g->n);
+  want = std::min<size_t>(want, dlp::engine::owned_limit(e->grid));
+  if (want <= e->mark_plane || cudaStreamSynchronize(e->stream) != cudaSuccess) return;
+  cudaFree(e->marks);
+  e->marks = nullptr;
+  e->mark_plane = 0;
+  if (cudaMalloc(&e->marks, 2 * want) != cudaSuccess || cudaMemset(e->marks, 0, 2 * want) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(e->marks);
+    e->marks = nullptr;
+    return;
+  }
+  e->mark_plane = static_cast<unsigned>(want);
 }
 
 int reset_graph(dlp_engine *e, GraphSlot *g, int gid) {
@@ -374,6 +402,13 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
     rh[i].ba = a;
   }
   for (size_t j = 0; j < resumed.size(); ++j) rh[count + j] = e->graphs[resumed[j]]->inflight_rec;
+  // the launch's vertices one graph after the other, for the owned passes
+  size_t vertices = 0;
+  for (int i = 0; i < total; ++i) {
+    rh[i].ba.flat = static_cast<unsigned>(vertices);
+    vertices += owned_room(rh[i].st.n);
+  }
+  const bool owned = vertices <= e->mark_plane;
   GraphRec *recs = e->recs_dev + (p ? e->max_graphs : 0);
   DLP_CUDA_TRY(cudaMemcpyAsync(recs, rh, sizeof(GraphRec) * total, cudaMemcpyHostToDevice, e->stream));
   DLP_CUDA_TRY(cudaEventRecord(e->recs_free[p], e->stream));
@@ -394,10 +429,14 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
   args.slice_ns = opts.slice_ns;
   args.tag = e->steps + 1;
   args.delta = e->cfg.delta;
+  args.tiles = owned ? static_cast<int>(vertices / 64) : 0;
+  args.smem_bytes = static_cast<int>(owned ? e->smem_all : e->smem);
+  args.marks = e->marks;
+  args.mark_plane = e->mark_plane;
   args.progress = sliced ? e->progress_dev : nullptr;
   DLP_CUDA_TRY(cudaEventRecord(e->ev[slot][0], e->stream));
   void *kargs[] = {&args};
-  DLP_TRY(dlp::launch_cooperative(e->kernel, e->grid, dlp::session::kBlock, kargs, e->smem, e->stream));
+  DLP_TRY(dlp::launch_cooperative(e->kernel, e->grid, dlp::session::kBlock, kargs, args.smem_bytes, e->stream));
   DLP_CUDA_TRY(cudaEventRecord(e->ev[slot][1], e->stream));
   for (int i = 0; i < count; ++i) {
     GraphSlot *g = e->graphs[gids[i]];
@@ -614,7 +653,13 @@ int dlp_engine_create(const dlp_config *cfg_in, int max_graphs, size_t memory_bu
   int sms = 0, per_sm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device);
   e->smem = dlp::engine::engine_dynamic_smem();
-  if (cudaFuncSetAttribute(e->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(e->smem)) !=
+  int smem_max = 0;
+  cudaFuncAttributes fa{};
+  if (cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, cfg.device) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa, e->kernel) != cudaSuccess)
+    return bail(dlp::fail(DLP_ERR_CUDA, "attribute query failed for the engine kernel"));
+  e->smem_all = std::max(e->smem, (static_cast<size_t>(smem_max) - fa.sharedSizeBytes) & ~static_cast<size_t>(15));
+  if (cudaFuncSetAttribute(e->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(e->smem_all)) !=
       cudaSuccess)
     return bail(dlp::fail(DLP_ERR_CUDA, "could not reserve the engine kernel's shared memory"));
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, e->kernel, dlp::session::kBlock, e->smem) !=
@@ -729,6 +774,7 @@ int dlp_engine_add_graph(dlp_engine *e, int n, int64_t m, const int *row_ptr, co
   if ((st = reset_graph(e, g, gid))) return bail(st);
   e->graphs[gid] = g;
   e->used += g->bytes;
+  grow_marks(e);
   *graph_id = gid;
   return DLP_OK;
 }
@@ -885,6 +931,7 @@ int restore_graph(dlp_engine *e, const void *snapshot, size_t bytes, int want, i
   e->graphs[gid] = g;
   e->held[gid] = 0;
   e->used += g->bytes;
+  grow_marks(e);
   *graph_id = gid;
   return DLP_OK;
 }
@@ -928,6 +975,8 @@ int dlp_engine_reset_graph(dlp_engine *e, int graph_id) {
   GraphSlot *g = slot_of(e, graph_id);
   if (!g) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "unknown graph id");
   DLP_CUDA_TRY(cudaSetDevice(e->device));
+  // a step that failed may have left frontier marks behind
+  if (e->marks) DLP_CUDA_TRY(cudaMemsetAsync(e->marks, 0, 2 * static_cast<size_t>(e->mark_plane), e->stream));
   DLP_TRY(reset_graph(e, g, graph_id));
   int zero = 0;
   DLP_CUDA_TRY(cudaMemcpy(&e->ectl->err, &zero, sizeof(int), cudaMemcpyHostToDevice));

@@ -77,6 +77,13 @@ struct EngineArgs {
   unsigned long long slice_ns;    // propagation time after which the launch stops (0: no limit)
   int tag;                        // unique per launch (stop requests)
   float delta;                    // convergence threshold (the engine's, the same for every graph)
+  // Owned passes (owner_pass.cuh): tiles of 64 vertices of all graphs of the
+  // launch (0: passes over frontier lists), and the two mark planes, all zero
+  // between stints.
+  int tiles;
+  int smem_bytes;                 // dynamic shared memory of the launch
+  unsigned char *marks;
+  unsigned mark_plane;            // bytes of a plane
   int2 *progress;                 // per graph: {1 batch finished / 0 continues, passes so far}
 };
 
@@ -85,8 +92,11 @@ struct EngineArgs {
 void launch_zero_counters(const GraphRec *recs, int ng_new, EngineCtl *ectl, cudaStream_t stream);
 
 const void *engine_kernel_ptr(int lanes);
-// Dynamic shared memory per block of the engine kernel (the solo-mode cache).
+// Dynamic shared memory per block that every launch of the engine kernel needs
+// (the one-block mode's); launches with owned passes take all there is.
 size_t engine_dynamic_smem();
+// Vertices (a multiple of 64) of a launch up to which a grid can own them.
+unsigned owned_limit(int grid);
 
 }  // namespace engine
 }  // namespace dlp

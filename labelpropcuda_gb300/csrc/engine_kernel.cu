@@ -15,6 +15,7 @@
 //     built with -fmad=false.
 //   * supernode weights are exact 32.32 fixed-point sums (order independent).
 #include "engine.cuh"
+#include "owner_pass.cuh"
 #include "row_stint.cuh"
 
 namespace dlp {
@@ -1091,9 +1092,7 @@ __device__ __noinline__ void solo_passes(const EngineArgs &e, int k0, int slot) 
   __syncthreads();
   // Labels written during the stint go back to HBM; the marks of pass k are
   // the frontier; vertices that were or are in a frontier join the touched
-  // list the first time in this batch. Their stamp is the graph's own last
-  // pass (below the next grid pass's stamp of a running graph and below the
-  // next batch's first stamp).
+  // list the first time in this batch, with the batch's first stamp.
   const int jp = (k - k0) & 1;
   for (int i = tid; i < stint::kSlots; i += kBlock) {
     const unsigned long long key = c.key[i];
@@ -1117,7 +1116,7 @@ __device__ __noinline__ void solo_passes(const EngineArgs &e, int k0, int slot) 
       else list[atomicAdd(&s.bc->front_count[set][0], 1)] = v;
     }
     const unsigned g0 = s.ctl->stamp_base + 1u;
-    if (atomicMax(&s.front_stamp[v], g0 + static_cast<unsigned>(s.bc->passes)) < g0) {
+    if (atomicMax(&s.front_stamp[v], g0) < g0) {
       const int t = r.ba.seq & 1;
       s.touched[static_cast<size_t>(t) * s.n + atomicAdd(&s.ctl->touched_count[t], 1)] = v;
     }
@@ -1459,12 +1458,202 @@ __device__ __forceinline__ void pass_sizes(const EngineArgs &e, int k, int *pref
   tw = pref2[ng];
 }
 
+// The engine's graphs as owned passes read them.
+struct OwnedGraphs {
+  const EngineArgs &e;
+  __device__ int nodes(int g) const { return e.recs[g].st.n; }
+  __device__ int2 row(int g, int v) const { return e.recs[g].st.rowinfo[v]; }
+  __device__ bool markable(int g, int v) const { return (e.recs[g].st.nmeta[v] & 1u) != 0; }
+  __device__ void entry(int g, int at, int &v, float &w) const {
+    const int2 ent = e.recs[g].st.act_adj[at];
+    v = ent.x;
+    w = __int_as_float(ent.y);
+  }
+};
+
+// Recorded frontier sizes of pass k back to zero, by one block.
+__device__ __forceinline__ void clear_record(const EngineArgs &e, int k) {
+  for (int g = threadIdx.x; g < e.ng; g += kBlock) {
+    const GraphRec &r = e.recs[g];
+    const int kg = k + r.ba.pass0;
+    if (r.ba.record && kg < kRecordIters && kg < r.ba.max_iter) r.st.rec_fsizes[kg] = 0;
+  }
+}
+
+// The passes of a stint on owned rows, from k on; returns the first pass not
+// run, or -1 when the launch has to end. Not inlined, so that its registers
+// are its own.
+__device__ __noinline__ int owned_loop(const EngineArgs &e, int k, owner::Store s, bool rec_any) {
+  const OwnedGraphs gr{e};
+  owner::Head &h = s.head();
+  unsigned before = 0xffffffffu;  // rows of the pass before the last
+  for (;;) {
+    if (s.tiles > 0) {
+      unsigned char *own = h.marks + (k & 1 ? h.plane : 0u) + h.flat;
+      unsigned char *next = h.marks + (k & 1 ? 0u : h.plane);
+      owner::pass(s, gr, own, next, k, h.delta, h.fast != 0, [&](int i) {
+        if (!rec_any) return;
+        const GraphRec &r = e.recs[h.first_graph + owner::graph_of(s.meta(i))];
+        const int kg = k + r.ba.pass0;
+        if (r.ba.record && kg < kRecordIters) atomicAdd(&r.st.rec_fsizes[kg], 1);
+      });
+    } else if (rec_any && blockIdx.x == 0) {
+      clear_record(e, k + 1);
+    }
+    unsigned long long sum;
+    const bool ok = sum_sync(&e.ectl->bar, s_bar, &e.ectl->err, e.timeout_ns, [&]() -> unsigned long long {
+      if (s.tiles == 0) {
+        if (blockIdx.x != 0 || !slice_over(e)) return 0ull;
+        e.ectl->slice_stop = stop_code(e, k + 1);
+        return kSumStop;
+      }
+      const unsigned long long mine =
+          static_cast<unsigned>((h.count & 0xffff) + (h.count >> 16) + h.wide) | (h.moved ? kSumMoved : 0ull);
+      h.count = h.wide = 0;
+      h.moved = 0;
+      return mine;
+    }, sum);
+    if (!ok) return -1;
+    ++k;
+    const unsigned rows = static_cast<unsigned>(sum);
+    const bool moved = (sum & (0xffull * kSumMoved)) != 0, stop = (sum & (0xffull * kSumStop)) != 0;
+    if (!moved || stop || k >= h.budget || k >= h.stint_end) return k;
+    // small in two passes running: the next one is small too, as a rule
+    if (max(rows, before) <= h.solo_entry && k >= h.solo_from) return k;
+    before = rows;
+  }
+}
+
+// Passes from k0 on by the blocks that own the rows (owner_pass.cuh). The
+// frontier of pass k0 is in the lists (pref, pref2: its sizes), that of the
+// pass returned in k_out is in them again. Ends when the frontier empties,
+// fits the one-block mode, at a pass or time limit. `loaded`: this block holds
+// its rows already.
+__device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_from, const int *pref,
+                                          const int *pref2, int tn, int tw, bool loaded, int *k_out) {
+  const int ng = e.ng, tid = threadIdx.x;
+  const OwnedGraphs gr{e};
+  auto marks = [&](int k) { return e.marks + (k & 1 ? e.mark_plane : 0u); };
+  // frontier lists -> marks
+  for (int item = blockIdx.x * kBlock + tid; item < tn + tw; item += gridDim.x * kBlock) {
+    const bool wide = item >= tn;
+    const int at = wide ? item - tn : item;
+    const int g = locate(wide ? pref2 : pref, ng, at);
+    const GraphRec &r = e.recs[g];
+    const int i = at - (wide ? pref2 : pref)[g];
+    const int v = r.st.flist[static_cast<size_t>((k0 + r.ba.pass0) % 3) * r.st.n + (wide ? r.st.n - 1 - i : i)];
+    marks(k0)[r.ba.flat + v] = 1;
+  }
+  int first, end;
+  owner::range(e.tiles, blockIdx.x, gridDim.x, first, end);
+  const owner::Store s = owner::store(e.smem_bytes, end - first);
+  owner::Head &h = s.head();
+  const bool owns = end > first;
+  if (owns && !loaded) {
+    auto graph_of_tile = [&](int t) {  // the last graph that starts at or before tile t
+      int lo = 0, hi = ng - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (e.recs[mid].ba.flat <= static_cast<unsigned>(t) * owner::kTile) lo = mid;
+        else hi = mid - 1;
+      }
+      return lo;
+    };
+    const int g0 = graph_of_tile(first);
+    if (tid < end - first) s.of_tile(tid) = static_cast<unsigned char>(graph_of_tile(first + tid) - g0);
+    if (tid == 0) {
+      h.first_graph = g0;
+      h.num_graphs = graph_of_tile(end - 1) - g0 + 1;
+      h.flat = static_cast<unsigned>(first) * owner::kTile;
+      h.pool_used = 0;
+      h.first_limit = 0x7fffffff;
+      h.count = h.wide = 0;
+      h.moved = 0;
+    }
+    __syncthreads();
+    if (tid < h.num_graphs) {
+      const GraphRec &r = e.recs[g0 + tid];
+      const bool swapped = ((r.st.ctl->cur_buf ^ r.ba.pass0) & 1) != 0;
+      owner::Local &l = s.graph(tid);
+      l.lab[0] = swapped ? r.st.lab1 : r.st.lab0;
+      l.lab[1] = swapped ? r.st.lab0 : r.st.lab1;
+      l.flat = r.ba.flat;
+      l.limit = r.ba.max_iter - r.ba.pass0;
+      atomicMin(&h.first_limit, l.limit);
+    }
+    __syncthreads();
+    owner::load(s, gr);
+  }
+  if (tid == 0) {
+    h.marks = e.marks;
+    h.plane = e.mark_plane;
+    h.delta = e.delta;
+    h.fast = e.fast_div;
+    h.budget = e.pass_budget > 0 ? e.pass_budget : 0x7fffffff;
+    h.solo_entry = (e.solo & 1) ? static_cast<unsigned>(e.solo_entry) : 0u;
+    h.solo_from = solo_from;
+    h.stint_end = k0 + owner::kMaxStint;
+  }
+  if (owns && tid < h.num_graphs) {
+    s.graph(tid).last = -1;
+    s.graph(tid).edges = s.graph(tid).visits = 0;
+  }
+  bool rec_any = false;
+  for (int g = tid; g < ng; g += kBlock) rec_any |= e.recs[g].ba.record != 0;
+  rec_any = __syncthreads_or(rec_any) != 0;
+  if (rec_any && blockIdx.x == 0) clear_record(e, k0);
+  if (!launch_sync(e)) return false;
+  if (blockIdx.x == 0)  // the lists are filled again at the end
+    for (int i = tid; i < 6 * ng; i += kBlock) (&e.recs[i / 6].st.bc->front_count[0][0])[i % 6] = 0;
+  const int k = owned_loop(e, k0, s, rec_any);
+  if (k < 0) return false;
+  // marks -> frontier lists; visits -> counters; vertices that were or are in a
+  // frontier join the touched list the first time in this batch
+  if (owns) {
+    for (int i = tid; i < s.n(); i += kBlock) {
+      const unsigned vis = s.visits(i);
+      const int lg = owner::graph_of(s.meta(i));
+      const GraphRec &r = e.recs[h.first_graph + lg];
+      const DevState &d = r.st;
+      const int v = static_cast<int>(h.flat + i - s.graph(lg).flat);
+      unsigned char *mark = marks(k) + h.flat + i;
+      const bool marked = __ldcg(mark) != 0;
+      if (marked) *mark = 0;
+      s.visits(i) = 0;
+      const bool front = marked && k < s.graph(lg).limit;
+      const int len = vis || front ? d.act_len[v] : 0;
+      const int set = (k + r.ba.pass0) % 3;
+      int *list = d.flist + static_cast<size_t>(set) * d.n;
+      append_keyed(front && len <= kNarrowMax, v, list, &d.bc->front_count[set][0]);
+      append_back_keyed(front && len > kNarrowMax, v, list, d.n, &d.bc->front_count[set][1]);
+      if (vis) {
+        atomicAdd(&s.graph(lg).edges, static_cast<unsigned long long>(vis) * len);
+        atomicAdd(&s.graph(lg).visits, static_cast<unsigned long long>(vis));
+      }
+      const unsigned g0 = d.ctl->stamp_base + 1u;
+      const bool fresh = (vis || front) && atomicMax(&d.front_stamp[v], g0) < g0;
+      append_keyed(fresh, v, d.touched + static_cast<size_t>(r.ba.seq & 1) * d.n,
+                   &d.ctl->touched_count[r.ba.seq & 1]);
+    }
+    __syncthreads();
+    if (tid < h.num_graphs && s.graph(tid).last >= 0) {
+      const GraphRec &r = e.recs[h.first_graph + tid];
+      atomicAdd(&r.st.bc->aff_edges, s.graph(tid).edges);
+      atomicAdd(&r.st.bc->front_visits, s.graph(tid).visits);
+      atomicMax(&r.st.bc->passes, s.graph(tid).last + r.ba.pass0 + 1);
+    }
+  }
+  *k_out = k;
+  return launch_sync(e);
+}
+
 // The propagation passes of the launch; k_end is the first pass not run (the
 // graphs whose frontier is live at k_end continue in a later launch).
 template <int G>
 __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2, int &k_end) {
   int no_small_at = -1;  // a pass the one-block mode declined goes to the full grid
   int solo_from = 0;     // the one-block mode declined: not tried again before this pass
+  bool owned = false;    // the block holds its rows (owned_passes)
   int stint_no = 0;
   int k = 0;
   // thread 0 of block 0: passes and device time per mode in this launch
@@ -1496,6 +1685,17 @@ __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2
       continue;
     }
     const uint64_t tp = c.gtid == 0 ? global_timer_ns() : 0;
+    if (e.tiles > 0) {
+      int kk = k;
+      if (!owned_passes(e, k, solo_from, pref, pref2, tn, tw, owned, &kk)) return false;
+      owned = true;
+      if (c.gtid == 0) {
+        mp[1] += kk - k;
+        mns[1] += global_timer_ns() - tp;
+      }
+      k = kk - 1;  // the loop increment resumes at pass kk
+      continue;
+    }
     run_pass<G>(e, k, pref, tn, pref2, tw, c.lane, c.gwarp, c.nwarps, c.gtid, c.nthreads);
     if (c.gtid == 0 && slice_over(e)) e.ectl->slice_stop = stop_code(e, k + 1);
     if (!launch_sync(e)) return false;
@@ -1702,6 +1902,10 @@ void launch_zero_counters(const GraphRec *recs, int ng_new, EngineCtl *ectl, cud
 }
 
 size_t engine_dynamic_smem() { return sizeof(SoloCache); }
+
+unsigned owned_limit(int grid) {
+  return grid > 1 ? static_cast<unsigned>(grid - 1) * (owner::kMaxVertices - owner::kTile) : 0u;
+}
 
 const void *engine_kernel_ptr(int lanes) {
   switch (lanes) {

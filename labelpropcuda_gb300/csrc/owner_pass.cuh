@@ -1,0 +1,428 @@
+// Full-grid propagation passes over owned rows.
+//
+// Every block but the first owns a contiguous range of the launch's vertices
+// (tiles of 64, all graphs one after the other) and keeps their live rows in
+// shared memory for the whole launch. A frontier is a byte per vertex in
+// global memory, one plane per pass parity. A pass is: read and clear the own
+// range's bytes, list the set ones in shared memory, run their rows with one
+// lane per row of at most 8 entries, four lanes up to 32 and a warp beyond,
+// store a byte for every neighbour that a moved label marks, barrier. The first
+// block owns nothing: it runs the one-block passes and the clock.
+//
+// What bounds a pass: four trips to L2 in a row (own bytes, neighbour labels,
+// acknowledged stores, barrier). A pass over frontier lists takes twice as
+// many (counts, list entry, row start, row, labels, mark atomic, reservation,
+// list store, barrier). Static ownership is what saves them: a row needs no
+// lookup, a mark no answer, and the list of a block no global counter. Range
+// scans cost a byte per owned vertex and pass, which is why launches beyond
+// kMaxVertices per block use frontier lists instead.
+//
+// Measured, microseconds a pass, owned rows against lists: 5,000 vertices of
+// degree 5 4.0 against 5.1, 20,000 of degree 7 4.2 against 6.2, 50,000 of degree
+// 5 4.3 against 7.5 to 8.0, 500,000 of degree 7 6.0 against 16.2.
+#pragma once
+
+#include "common.cuh"
+
+namespace dlp {
+namespace owner {
+
+constexpr int kTile = 64;
+constexpr int kMaxVertices = 16384;             // per block
+constexpr int kMaxTiles = kMaxVertices / kTile; // and so at most this many graphs
+constexpr int kLaneEntries = 8;
+constexpr int kLongLanes = 4;
+constexpr int kMaxRow = kLaneEntries * kLongLanes;
+constexpr unsigned kNoPool = (1u << 18) - 1;    // the row did not fit the pool: read from global memory
+constexpr unsigned kUnmarkable = 0x80000000u;   // pool entry: a neighbour that is never marked
+constexpr unsigned kNoEntry = 0xffffffffu;      // pool entry: soft-deleted
+
+struct Local {           // a graph of the block's range
+  float *lab[2];         // [k & 1] is read by launch pass k
+  unsigned flat;         // its first vertex among the launch's
+  int limit;             // first launch pass its pass limit forbids
+  int last;              // last launch pass it took part in, -1 none
+  unsigned long long edges, visits;  // of the stint
+};
+
+struct Head {
+  int num_graphs, first_graph;
+  unsigned flat;         // first owned vertex among the launch's
+  int pool_used;
+  int first_limit;       // the smallest limit of the block's graphs
+  int count;             // rows of the pass: short | long << 16
+  int wide;              // its rows of more than 32 entries
+  int moved;
+  // what every pass reads
+  unsigned char *marks;
+  unsigned plane;
+  float delta;
+  int fast;
+  int budget, solo_from, stint_end;
+  unsigned solo_entry;
+};
+
+// The block's dynamic shared memory: Head, then with T = V / 64 owned tiles
+// graph[T], of_tile[T], meta[V], visits[V], list[V], pool[cap]. Named by 32-bit
+// offsets from its start, so that a pass keeps no pointers in registers: a
+// register spilled there is a trip to L2 in every pass, because the barrier's
+// acquire empties L1.
+extern __shared__ __align__(16) unsigned char g_smem[];
+constexpr int kHeadBytes = (sizeof(Head) + 15) & ~15;
+constexpr int kTileBytes = sizeof(Local) + 1 + kTile * (4 + 2 + 2);  // per tile, without the pool
+constexpr int kMaxStint = 32000;  // passes of a stint (visits counts 15 bits)
+constexpr unsigned short kWideRow = 0x8000;
+
+struct Store {
+  int tiles;
+  int pool_cap;
+  __device__ int n() const { return tiles * kTile; }  // owned vertices
+  __device__ Head &head() const { return *reinterpret_cast<Head *>(g_smem); }
+  __device__ Local &graph(int i) const { return reinterpret_cast<Local *>(g_smem + kHeadBytes)[i]; }
+  // pool offset (18 bits) | length (6 bits, 63: longer than 32) | local graph (8 bits)
+  __device__ unsigned &meta(int i) const {
+    return reinterpret_cast<unsigned *>(g_smem + kHeadBytes + tiles * static_cast<int>(sizeof(Local)))[i];
+  }
+  // passes that updated the row; kWideRow: the pass has listed it as a wide row
+  __device__ unsigned short &visits(int i) const {
+    return reinterpret_cast<unsigned short *>(g_smem + kHeadBytes +
+                                              tiles * static_cast<int>(sizeof(Local) + 4 * kTile))[i];
+  }
+  // rows of the pass: short from the front, long from the back
+  __device__ unsigned short &list(int i) const { return (&visits(0) + tiles * kTile)[i]; }
+  // {neighbour | kUnmarkable, weight}
+  __device__ int2 &pool(int i) const {
+    return reinterpret_cast<int2 *>(g_smem + kHeadBytes + tiles * static_cast<int>(sizeof(Local) + 8 * kTile))[i];
+  }
+  // graph of an owned tile (behind the pool)
+  __device__ unsigned char &of_tile(int i) const { return reinterpret_cast<unsigned char *>(&pool(pool_cap))[i]; }
+};
+static_assert(sizeof(Local) % 8 == 0 && kTile % 16 == 0, "the pool is 8-byte aligned");
+
+__device__ __forceinline__ Store store(int bytes, int tiles) {
+  const int room = (bytes - kHeadBytes - kTileBytes * tiles) / static_cast<int>(sizeof(int2));
+  return Store{tiles, min(room, static_cast<int>(kNoPool) - kMaxRow)};
+}
+
+__device__ __forceinline__ unsigned pack(unsigned off, int len, int g) {
+  return off | (static_cast<unsigned>(len > kMaxRow ? 63 : len) << 18) | (static_cast<unsigned>(g) << 24);
+}
+__device__ __forceinline__ unsigned pool_of(unsigned m) { return m & kNoPool; }
+__device__ __forceinline__ int len_of(unsigned m) { return static_cast<int>((m >> 18) & 63u); }
+__device__ __forceinline__ int graph_of(unsigned m) { return static_cast<int>(m >> 24); }
+
+// tiles: all tiles of the launch; the range of block b in [1, blocks).
+__device__ __forceinline__ void range(int tiles, int b, int blocks, int &first, int &end) {
+  first = end = 0;
+  if (b == 0) return;
+  first = static_cast<int>(static_cast<long long>(tiles) * (b - 1) / (blocks - 1));
+  end = static_cast<int>(static_cast<long long>(tiles) * b / (blocks - 1));
+}
+
+// Rows of the block's range into shared memory (head filled by the caller).
+// Graph: row(g, v) {start, length}; markable(g, v); entry(g, at, v, w), v = -1
+// for an entry that does not count; nodes(g).
+template <class Graph>
+__device__ void load(const Store &s, const Graph &gr) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  Head &h = s.head();
+  for (int i = tid; i < s.n(); i += blockDim.x) {
+    const int lg = s.of_tile(i / kTile), g = h.first_graph + lg;
+    const int v = static_cast<int>(h.flat + i - s.graph(lg).flat);
+    int2 ri = make_int2(0, 0);
+    if (v < gr.nodes(g) && gr.markable(g, v)) ri = gr.row(g, v);
+    const int len = ri.y;
+    // pool room for the warp's rows, one reservation
+    const int want = len <= kMaxRow ? len : 0;
+    int incl = want;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    int base = 0;
+    if (lane == 31 && incl) base = atomicAdd(&h.pool_used, incl);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    const int off = base + incl - want;
+    const bool fits = off + want <= s.pool_cap;
+    s.meta(i) = pack(fits ? static_cast<unsigned>(off) : kNoPool, len, lg);
+    s.visits(i) = 0;
+    if (!fits) continue;  // lanes of the next round reconverge at its first shuffle
+    for (int b = 0; b < want; b += kLaneEntries) {
+      int u[kLaneEntries];
+      float w[kLaneEntries];
+#pragma unroll
+      for (int r = 0; r < kLaneEntries; ++r) {
+        u[r] = -1;
+        w[r] = 0.0f;
+        if (b + r < want) gr.entry(g, ri.x + b + r, u[r], w[r]);
+      }
+      unsigned mk = 0;
+#pragma unroll
+      for (int r = 0; r < kLaneEntries; ++r)
+        if (u[r] >= 0 && gr.markable(g, u[r])) mk |= 1u << r;
+#pragma unroll
+      for (int r = 0; r < kLaneEntries; ++r)
+        if (b + r < want) {
+          const bool live = u[r] >= 0;
+          const unsigned x = static_cast<unsigned>(u[r]) | ((mk >> r) & 1u ? 0u : kUnmarkable);
+          s.pool(off + b + r) = make_int2(static_cast<int>(live ? x : kNoEntry), __float_as_int(live ? w[r] : 0.0f));
+        }
+    }
+  }
+}
+
+// A label from L2, 0 without `take`; predicated, because a load in a branch is
+// waited for before the next one is issued (and a stand-in address that all
+// idle lanes share queues up in its L2 slice: it cost 3,000 cycles a pass).
+__device__ __forceinline__ float gather(const float *at, bool take) {
+  float x;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.s32 p, %2, 0;\n\t"
+      "mov.f32 %0, 0f00000000;\n\t"
+      "@p ld.global.cg.f32 %0, [%1];\n\t"
+      "}" : "=f"(x) : "l"(at), "r"(static_cast<int>(take)));
+  return x;
+}
+
+// A mark, predicated instead of branched around.
+__device__ __forceinline__ void mark(unsigned char *at, bool set) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.s32 p, %1, 0;\n\t"
+      "@p st.global.u8 [%0], %2;\n\t"
+      "}" ::"l"(at), "r"(static_cast<int>(set)), "r"(1) : "memory");
+}
+
+// The row of owned vertex i by LANES lanes (1: up to 8 entries, 4: up to 32).
+// All lanes of the warp call; returns whether the label moved (on every lane of
+// the row).
+template <int LANES, class Graph>
+__device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid, int i, int k, float delta, bool fast,
+                                    unsigned char *next) {
+  const int sub = threadIdx.x & (LANES - 1);
+  const unsigned m = valid ? s.meta(i) : 0;
+  const int len = valid ? len_of(m) : 0, lg = graph_of(m);
+  const unsigned off = pool_of(m);
+  const Local &l = s.graph(lg);
+  const float *src = l.lab[k & 1];
+  const int v = static_cast<int>(s.head().flat + i - l.flat);
+  const float old = gather(src + v, valid);
+  unsigned u[kLaneEntries];
+  float w[kLaneEntries], x[kLaneEntries];
+  if (off != kNoPool) {
+#pragma unroll
+    for (int r = 0; r < kLaneEntries; ++r) {
+      const int e = LANES == 1 ? r : sub + LANES * r;
+      const int2 ent = s.pool(e < len ? static_cast<int>(off) + e : 0);
+      u[r] = e < len ? static_cast<unsigned>(ent.x) : kNoEntry;
+      w[r] = e < len ? __int_as_float(ent.y) : 0.0f;
+    }
+  } else {
+    const int g = s.head().first_graph + lg;
+    const int start = gr.row(g, v).x;
+#pragma unroll
+    for (int r = 0; r < kLaneEntries; ++r) {
+      const int e = LANES == 1 ? r : sub + LANES * r;
+      int c = -1;
+      w[r] = 0.0f;
+      if (e < len) gr.entry(g, start + e, c, w[r]);
+      if (c < 0) w[r] = 0.0f;
+      u[r] = c < 0 ? kNoEntry : static_cast<unsigned>(c);
+    }
+#pragma unroll
+    for (int r = 0; r < kLaneEntries; ++r)
+      if (!(u[r] & kUnmarkable) && !gr.markable(g, static_cast<int>(u[r]))) u[r] |= kUnmarkable;
+  }
+#pragma unroll
+  for (int r = 0; r < kLaneEntries; ++r) x[r] = gather(src + (u[r] & ~kUnmarkable), u[r] != kNoEntry);
+#pragma unroll
+  for (int r = 0; r < kLaneEntries; ++r) x[r] = u[r] == kNoEntry ? 0.0f : __fmaf_rn(w[r], x[r], 0.0f);
+  // the reference's tree (row_sums.cuh): strides 16 to 4 within a lane of a
+  // long row, 2 and 1 across its lanes; strides 4 to 1 within that of a short
+#pragma unroll
+  for (int h = kLaneEntries / 2; h >= 1; h >>= 1)
+#pragma unroll
+    for (int r = 0; r < h; ++r) {
+      x[r] = x[r] + x[r + h];
+      w[r] = w[r] + w[r + h];
+    }
+  float tl = x[0], tw = w[0];
+#pragma unroll
+  for (int o = LANES / 2; o >= 1; o >>= 1) {
+    tl = tl + __shfl_xor_sync(0xffffffffu, tl, o);
+    tw = tw + __shfl_xor_sync(0xffffffffu, tw, o);
+  }
+  if (!valid) return false;
+  const float nl = updated_label(tw, tl, old, fast);
+  if (sub == 0) {
+    l.lab[(k & 1) ^ 1][v] = nl;
+    ++s.visits(i);
+    s.graph(lg).last = k;
+  }
+  const bool moved = fabsf(nl - old) > delta;
+  unsigned char *const marks = next + l.flat;
+#pragma unroll
+  for (int r = 0; r < kLaneEntries; ++r) mark(marks + u[r], moved && !(u[r] & kUnmarkable));
+  mark(marks + v, moved && sub == 0);
+  return moved;
+}
+
+// A row of more than 32 entries by a warp, from global memory: slots lane + 32 j
+// of 256, then the tree.
+template <class Graph>
+__device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i, int k, float delta, bool fast,
+                                         unsigned char *next) {
+  const int lane = threadIdx.x & 31;
+  const int lg = graph_of(s.meta(i)), g = s.head().first_graph + lg;
+  const Local &l = s.graph(lg);
+  const float *src = l.lab[k & 1];
+  const int v = static_cast<int>(s.head().flat + i - l.flat);
+  const int2 ri = gr.row(g, v);
+  float sw[8], sl[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sw[j] = sl[j] = 0.0f;
+  for (int p = 0; p < ri.y; p += 256) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int e = p + j * 32 + lane;
+      int u = -1;
+      float w = 0.0f;
+      if (e < ri.y) gr.entry(g, ri.x + e, u, w);
+      if (u >= 0) {
+        sw[j] = sw[j] + w;
+        sl[j] = __fmaf_rn(w, __ldcg(src + u), sl[j]);
+      }
+    }
+  }
+#pragma unroll
+  for (int half = 4; half >= 1; half >>= 1)
+#pragma unroll
+    for (int j = 0; j < half; ++j) {
+      sw[j] = sw[j] + sw[j + half];
+      sl[j] = sl[j] + sl[j + half];
+    }
+  float tw = sw[0], tl = sl[0];
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    tw = tw + __shfl_xor_sync(0xffffffffu, tw, o);
+    tl = tl + __shfl_xor_sync(0xffffffffu, tl, o);
+  }
+  const float old = __ldcg(src + v);
+  const float nl = updated_label(tw, tl, old, fast);
+  if (lane == 0) {
+    l.lab[(k & 1) ^ 1][v] = nl;
+    ++s.visits(i);
+    s.graph(lg).last = k;
+  }
+  if (!(fabsf(nl - old) > delta)) return false;
+  for (int e = lane; e < ri.y; e += 32) {
+    int u = -1;
+    float w;
+    gr.entry(g, ri.x + e, u, w);
+    if (u >= 0 && gr.markable(g, u)) next[l.flat + u] = 1;
+  }
+  if (lane == 0) next[l.flat + v] = 1;
+  return true;
+}
+
+// Pass k of the block's range, up to the barrier. own: the range's bytes of
+// this pass's plane; next: the whole plane of the next pass. The rows are
+// listed for the whole block and dealt out evenly: with every warp on its own
+// part of the range, the warps with the most marked rows took two to four
+// steps where most took one, and every block waits for the slowest.
+template <class Graph, class Each>
+__device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned char *own, unsigned char *next, int k,
+                                     float delta, bool fast, Each each) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+  Head &h = s.head();
+  const int n = s.n();
+  // A byte per lane, four loads in flight; the set ones are listed with one
+  // reservation per warp.
+  constexpr int kAhead = 4;
+  for (int base = warp * 32; base < n; base += kAhead * nwarps * 32) {
+    unsigned char b[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const int i = base + j * nwarps * 32 + lane;
+      b[j] = i < n ? __ldcg(own + i) : 0;
+    }
+    unsigned shorts[kAhead], longs[kAhead];
+    int add = 0;
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      shorts[j] = longs[j] = 0;
+      if (!__any_sync(0xffffffffu, b[j] != 0)) continue;
+      const int i = base + j * nwarps * 32 + lane;
+      int kind = 3;
+      if (b[j]) {
+        own[i] = 0;
+        const unsigned m = s.meta(i);
+        const int len = len_of(m);
+        kind = len <= kLaneEntries ? 0 : len <= kMaxRow ? 1 : 2;
+        if (k >= h.first_limit && k >= s.graph(graph_of(m)).limit) kind = 3;
+        else each(i);
+      }
+      shorts[j] = __ballot_sync(0xffffffffu, kind == 0);
+      longs[j] = __ballot_sync(0xffffffffu, kind == 1);
+      add += __popc(shorts[j]) + (__popc(longs[j]) << 16);
+      if (kind == 2) {  // a warp's work each: found again below
+        atomicAdd(&h.wide, 1);
+        s.visits(i) |= kWideRow;
+      }
+    }
+    if (add == 0) continue;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&h.count, add);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    int at_short = at & 0xffff, at_long = n - 1 - (at >> 16);
+    const unsigned bit = 1u << lane, below = bit - 1u;
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const unsigned short i = static_cast<unsigned short>(base + j * nwarps * 32 + lane);
+      if (shorts[j] & bit) s.list(at_short + __popc(shorts[j] & below)) = i;
+      if (longs[j] & bit) s.list(at_long - __popc(longs[j] & below)) = i;
+      at_short += __popc(shorts[j]);
+      at_long -= __popc(longs[j]);
+    }
+  }
+  __syncthreads();
+  const int ns = h.count & 0xffff, nl = h.count >> 16, nw = h.wide;
+  bool moved = false;
+  constexpr int kPer = 32 / kLongLanes;
+  const int sub = lane / kLongLanes;
+  if (ns + nl <= kPer * nwarps) {  // one step of 4-lane groups, spread over all warps
+    if (warp < ns + nl) {
+      const int r = warp + sub * nwarps;
+      const bool valid = r < ns + nl;
+      moved = row<kLongLanes>(s, gr, valid, valid ? s.list(r < ns ? r : n - 1 - (r - ns)) : 0, k, delta, fast, next);
+    }
+  } else {
+    // short rows from the first warp up, long ones from the last down
+    for (int b = warp * 32; b < ns; b += nwarps * 32) {
+      const bool valid = b + lane < ns;
+      moved |= row<1>(s, gr, valid, valid ? s.list(b + lane) : 0, k, delta, fast, next);
+    }
+    for (int b = (nwarps - 1 - warp) * kPer; b < nl; b += nwarps * kPer) {
+      const bool valid = b + sub < nl;
+      moved |= row<kLongLanes>(s, gr, valid, valid ? s.list(n - 1 - (b + sub)) : 0, k, delta, fast, next);
+    }
+  }
+  if (nw)
+    for (int b = warp * 32; b < n; b += nwarps * 32) {
+      unsigned todo = __ballot_sync(0xffffffffu, (s.visits(b + lane) & kWideRow) != 0);
+      for (; todo; todo &= todo - 1) {
+        const int i = b + __ffs(todo) - 1;
+        if (lane == 0) s.visits(i) &= static_cast<unsigned short>(~kWideRow);
+        __syncwarp();
+        moved |= wide_row(s, gr, i, k, delta, fast, next);
+      }
+    }
+  if (__any_sync(0xffffffffu, moved) && lane == 0) h.moved = 1;
+}
+
+}  // namespace owner
+}  // namespace dlp

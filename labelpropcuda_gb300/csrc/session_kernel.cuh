@@ -122,6 +122,7 @@ struct BatchArgs {
   int spec;
   int record;
   int solo;                 // small frontiers run on one block (see phase G)
+  unsigned flat;            // the graph's first vertex among the launch's (owned passes)
   int pass0;                // propagation passes run by earlier launches (0: batch starts here)
   unsigned long long timeout_ns;
 };

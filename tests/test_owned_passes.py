@@ -1,0 +1,62 @@
+"""Full-grid passes on owned rows (csrc/owner_pass.cuh), bit-exact against the
+oracle with the one-block mode off: graphs of one tile, of a tile and a vertex,
+rows of 8, 9, 32 and 33 entries, several graphs in one launch (with pass limits
+that end at different launch passes), and blocks whose rows do not fit their
+shared memory."""
+from __future__ import annotations
+
+import pytest
+
+import labelpropcuda_gb300 as dlp
+from parity_checks import EXACT_STATS, check_batch
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,degree,sem", [(63, 4, dlp.SEMANTICS_REF), (64, 4, dlp.SEMANTICS_SPEC),
+                                          (65, 9, dlp.SEMANTICS_REF), (400, 33, dlp.SEMANTICS_SPEC),
+                                          (9700, 8, dlp.SEMANTICS_REF)])
+def test_owned_passes_match_oracle(gpu, oracle, n, degree, sem):
+    p = dlp.Problem(n, degree, 5, 3, cache_dir="")
+    cap = 120
+    orc = oracle.OracleRun.from_problem(p, semantics=sem, record=True, threads=4, max_iterations=cap)
+    sess = dlp.Session.from_problem(p, semantics=sem, record=True, max_iterations=cap, small_frontier_solo=0)
+    for b, batch in enumerate(p.batches):
+        check_batch(b, sess.apply(b, batch), orc.apply(b, batch), sess, orc, oracle)
+
+
+@pytest.mark.gpu
+def test_owned_passes_rows_beyond_shared_memory(gpu, oracle):
+    p = dlp.Problem(160000, 30, 3, 5, cache_dir="")  # 1,060 vertices, 32,000 entries per block
+    cap = 25
+    orc = oracle.OracleRun.from_problem(p, threads=0, max_iterations=cap)
+    sess = dlp.Session.from_problem(p, max_iterations=cap, small_frontier_solo=0)
+    for b, batch in enumerate(p.batches):
+        got, want = sess.apply(b, batch), orc.apply(b, batch)
+        for k in EXACT_STATS:
+            assert got[k] == want[k], (b, k)
+        assert sess.labels().tobytes() == orc.labels().tobytes(), b
+
+
+@pytest.mark.gpu
+def test_owned_passes_of_continued_batches(gpu, oracle):
+    """Graphs that continue a batch beside graphs that start one: their pass
+    numbers, buffers and pass limits differ within a launch."""
+    probs = [dlp.Problem(n, d, 4, s, cache_dir="") for n, d, s in ((1500, 5, 1), (64, 3, 2), (3000, 7, 3))]
+    cap = 90
+    orcs = [oracle.OracleRun.from_problem(p, threads=4, max_iterations=cap) for p in probs]
+    eng = dlp.Engine(len(probs), max_iterations=cap, small_frontier_solo=0)
+    ids = [eng.add_problem(p) for p in probs]
+    dev = [[dlp.DeviceBatch(b) for b in p.batches] for p in probs]
+    nxt, step = [0] * len(probs), 0
+    while any(x < 4 for x in nxt) or any(eng.in_progress(g) for g in ids):
+        start = [i for i, g in enumerate(ids) if nxt[i] < 4 and not eng.in_progress(g) and (step + i) % 2 == 0]
+        done, _ = eng.step_sliced([(ids[i], nxt[i], dev[i][nxt[i]]) for i in start], pass_budget=37)
+        for i in start:
+            nxt[i] += 1
+        for g in done:
+            i = ids.index(g)
+            want, got = orcs[i].apply(nxt[i] - 1, probs[i].batches[nxt[i] - 1]), eng.stats(g, nxt[i] - 1)
+            for k in EXACT_STATS:
+                assert got[k] == want[k], (i, nxt[i] - 1, k)
+            assert eng.labels(g).tobytes() == orcs[i].labels().tobytes(), (i, nxt[i] - 1)
+        step += 1
