@@ -157,8 +157,8 @@ struct dlp_engine {
   bool ev_made = false;
   int2 *progress_dev = nullptr;     // per launch position: {finished, passes}
   int2 *progress_host = nullptr;    // pinned copy
-  unsigned char *marks = nullptr;   // two planes of frontier marks (owned passes), all zero between stints
-  unsigned mark_plane = 0;          // bytes of a plane
+  unsigned *marks = nullptr;   // two planes of frontier marks (owned passes), all zero between stints
+  unsigned mark_plane = 0;          // words of a plane
   int inflight = 0;                 // graphs whose batch continues in a later step
   std::vector<int> last_finished;   // graphs whose batch ended in the last sliced step
 
@@ -243,7 +243,10 @@ int grow_graph_scratch(dlp_engine *e, GraphSlot *g, int E, int D) {
 }
 
 // A graph's vertices among those of a launch: whole tiles.
-size_t owned_room(int n) { return (static_cast<size_t>(n) + 63) & ~static_cast<size_t>(63); }
+size_t owned_room(int n) {
+  constexpr size_t t = dlp::engine::kOwnedTile;
+  return (static_cast<size_t>(n) + t - 1) / t * t;
+}
 
 // Mark planes for a launch over all resident graphs, as far as a grid can own
 // their vertices; sized when graphs are added, so that steps allocate nothing.
@@ -257,7 +260,7 @@ void grow_marks(dlp_engine *e) {
   cudaFree(e->marks);
   e->marks = nullptr;
   e->mark_plane = 0;
-  if (cudaMalloc(&e->marks, 2 * want) != cudaSuccess || cudaMemset(e->marks, 0, 2 * want) != cudaSuccess) {
+  if (cudaMalloc(&e->marks, 8 * want) != cudaSuccess || cudaMemset(e->marks, 0, 8 * want) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(e->marks);
     e->marks = nullptr;
@@ -429,7 +432,7 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
   args.slice_ns = opts.slice_ns;
   args.tag = e->steps + 1;
   args.delta = e->cfg.delta;
-  args.tiles = owned ? static_cast<int>(vertices / 64) : 0;
+  args.tiles = owned ? static_cast<int>(vertices / dlp::engine::kOwnedTile) : 0;
   args.smem_bytes = static_cast<int>(owned ? e->smem_all : e->smem);
   args.marks = e->marks;
   args.mark_plane = e->mark_plane;
@@ -976,7 +979,7 @@ int dlp_engine_reset_graph(dlp_engine *e, int graph_id) {
   if (!g) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "unknown graph id");
   DLP_CUDA_TRY(cudaSetDevice(e->device));
   // a step that failed may have left frontier marks behind
-  if (e->marks) DLP_CUDA_TRY(cudaMemsetAsync(e->marks, 0, 2 * static_cast<size_t>(e->mark_plane), e->stream));
+  if (e->marks) DLP_CUDA_TRY(cudaMemsetAsync(e->marks, 0, 8 * static_cast<size_t>(e->mark_plane), e->stream));
   DLP_TRY(reset_graph(e, g, graph_id));
   int zero = 0;
   DLP_CUDA_TRY(cudaMemcpy(&e->ectl->err, &zero, sizeof(int), cudaMemcpyHostToDevice));

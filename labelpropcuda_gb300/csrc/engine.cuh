@@ -34,6 +34,8 @@ constexpr int kSoloEntryDefault = 512;
 constexpr int kSoloEntryMax = 1024;
 constexpr int kSubEntryMax = 4096;  // dlp_config.subgrid_entry, accepted and without effect
 
+constexpr int kOwnedTile = 32;  // a graph's vertices count in whole tiles (owner_pass.cuh)
+
 struct GraphRec {
   session::DevState st;
   session::BatchArgs ba;
@@ -77,13 +79,13 @@ struct EngineArgs {
   unsigned long long slice_ns;    // propagation time after which the launch stops (0: no limit)
   int tag;                        // unique per launch (stop requests)
   float delta;                    // convergence threshold (the engine's, the same for every graph)
-  // Owned passes (owner_pass.cuh): tiles of 64 vertices of all graphs of the
+  // Owned passes (owner_pass.cuh): tiles of kOwnedTile vertices of all graphs of the
   // launch (0: passes over frontier lists), and the two mark planes, all zero
   // between stints.
   int tiles;
   int smem_bytes;                 // dynamic shared memory of the launch
-  unsigned char *marks;
-  unsigned mark_plane;            // bytes of a plane
+  unsigned *marks;
+  unsigned mark_plane;            // words of a plane
   int2 *progress;                 // per graph: {1 batch finished / 0 continues, passes so far}
 };
 
@@ -95,7 +97,7 @@ const void *engine_kernel_ptr(int lanes);
 // Dynamic shared memory per block that every launch of the engine kernel needs
 // (the one-block mode's); launches with owned passes take all there is.
 size_t engine_dynamic_smem();
-// Vertices (a multiple of 64) of a launch up to which a grid can own them.
+// Vertices (in whole tiles) of a launch up to which a grid can own them.
 unsigned owned_limit(int grid);
 
 }  // namespace engine

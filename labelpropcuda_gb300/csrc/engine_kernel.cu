@@ -940,6 +940,7 @@ __device__ __forceinline__ unsigned long long stop_code(const EngineArgs &e, int
 // mark atomics and a reservation.
 static_assert(kBlock == stint::kThreads, "block 0 runs a stint with all its threads");
 static_assert(kSoloEntryMax <= stint::kSlotsUse, "a stint starts by putting the whole frontier into the vertex table");
+static_assert(kOwnedTile == owner::kTile && kMaxGraphs <= 1024, "what owner_pass.cuh packs");
 static_assert(kNarrowMax == stint::kMaxRow, "rows the frontier calls narrow are rows a stint can hold");
 constexpr unsigned long long kSoloBudgetNs = 100000000ull;
 constexpr int kTeamWarps = 16;  // a pass by at most this many warps counts as a team pass
@@ -1461,6 +1462,7 @@ __device__ __forceinline__ void pass_sizes(const EngineArgs &e, int k, int *pref
 // The engine's graphs as owned passes read them.
 struct OwnedGraphs {
   const EngineArgs &e;
+  __device__ int graphs() const { return e.ng; }
   __device__ int nodes(int g) const { return e.recs[g].st.n; }
   __device__ int2 row(int g, int v) const { return e.recs[g].st.rowinfo[v]; }
   __device__ bool markable(int g, int v) const { return (e.recs[g].st.nmeta[v] & 1u) != 0; }
@@ -1489,11 +1491,11 @@ __device__ __noinline__ int owned_loop(const EngineArgs &e, int k, owner::Store 
   unsigned before = 0xffffffffu;  // rows of the pass before the last
   for (;;) {
     if (s.tiles > 0) {
-      unsigned char *own = h.marks + (k & 1 ? h.plane : 0u) + h.flat;
-      unsigned char *next = h.marks + (k & 1 ? 0u : h.plane);
+      unsigned *own = h.marks + (k & 1 ? h.plane : 0u);
+      unsigned *next = h.marks + (k & 1 ? 0u : h.plane);
       owner::pass(s, gr, own, next, k, h.delta, h.fast != 0, [&](int i) {
         if (!rec_any) return;
-        const GraphRec &r = e.recs[h.first_graph + owner::graph_of(s.meta(i))];
+        const GraphRec &r = e.recs[owner::graph_of(s.meta(i))];
         const int kg = k + r.ba.pass0;
         if (r.ba.record && kg < kRecordIters) atomicAdd(&r.st.rec_fsizes[kg], 1);
       });
@@ -1544,37 +1546,21 @@ __device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_
     const int v = r.st.flist[static_cast<size_t>((k0 + r.ba.pass0) % 3) * r.st.n + (wide ? r.st.n - 1 - i : i)];
     marks(k0)[r.ba.flat + v] = 1;
   }
-  int first, end;
-  owner::range(e.tiles, blockIdx.x, gridDim.x, first, end);
-  const owner::Store s = owner::store(e.smem_bytes, end - first);
+  const owner::Store s = owner::store(e.smem_bytes, ng, owner::owned_tiles(e.tiles));
   owner::Head &h = s.head();
-  const bool owns = end > first;
+  const bool owns = s.tiles > 0;
   if (owns && !loaded) {
-    auto graph_of_tile = [&](int t) {  // the last graph that starts at or before tile t
-      int lo = 0, hi = ng - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (e.recs[mid].ba.flat <= static_cast<unsigned>(t) * owner::kTile) lo = mid;
-        else hi = mid - 1;
-      }
-      return lo;
-    };
-    const int g0 = graph_of_tile(first);
-    if (tid < end - first) s.of_tile(tid) = static_cast<unsigned char>(graph_of_tile(first + tid) - g0);
     if (tid == 0) {
-      h.first_graph = g0;
-      h.num_graphs = graph_of_tile(end - 1) - g0 + 1;
-      h.flat = static_cast<unsigned>(first) * owner::kTile;
       h.pool_used = 0;
       h.first_limit = 0x7fffffff;
       h.count = h.wide = 0;
       h.moved = 0;
     }
     __syncthreads();
-    if (tid < h.num_graphs) {
-      const GraphRec &r = e.recs[g0 + tid];
+    for (int g = tid; g < ng; g += kBlock) {
+      const GraphRec &r = e.recs[g];
       const bool swapped = ((r.st.ctl->cur_buf ^ r.ba.pass0) & 1) != 0;
-      owner::Local &l = s.graph(tid);
+      owner::Local &l = s.graph(g);
       l.lab[0] = swapped ? r.st.lab1 : r.st.lab0;
       l.lab[1] = swapped ? r.st.lab0 : r.st.lab1;
       l.flat = r.ba.flat;
@@ -1594,10 +1580,11 @@ __device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_
     h.solo_from = solo_from;
     h.stint_end = k0 + owner::kMaxStint;
   }
-  if (owns && tid < h.num_graphs) {
-    s.graph(tid).last = -1;
-    s.graph(tid).edges = s.graph(tid).visits = 0;
-  }
+  if (owns)
+    for (int g = tid; g < ng; g += kBlock) {
+      s.graph(g).last = -1;
+      s.graph(g).edges = s.graph(g).visits = 0;
+    }
   bool rec_any = false;
   for (int g = tid; g < ng; g += kBlock) rec_any |= e.recs[g].ba.record != 0;
   rec_any = __syncthreads_or(rec_any) != 0;
@@ -1613,10 +1600,10 @@ __device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_
     for (int i = tid; i < s.n(); i += kBlock) {
       const unsigned vis = s.visits(i);
       const int lg = owner::graph_of(s.meta(i));
-      const GraphRec &r = e.recs[h.first_graph + lg];
+      const GraphRec &r = e.recs[lg];
       const DevState &d = r.st;
-      const int v = static_cast<int>(h.flat + i - s.graph(lg).flat);
-      unsigned char *mark = marks(k) + h.flat + i;
+      const int v = static_cast<int>(owner::flat_of(i) - s.graph(lg).flat);
+      unsigned *mark = marks(k) + owner::flat_of(i);
       const bool marked = __ldcg(mark) != 0;
       if (marked) *mark = 0;
       s.visits(i) = 0;
@@ -1636,11 +1623,13 @@ __device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_
                    &d.ctl->touched_count[r.ba.seq & 1]);
     }
     __syncthreads();
-    if (tid < h.num_graphs && s.graph(tid).last >= 0) {
-      const GraphRec &r = e.recs[h.first_graph + tid];
-      atomicAdd(&r.st.bc->aff_edges, s.graph(tid).edges);
-      atomicAdd(&r.st.bc->front_visits, s.graph(tid).visits);
-      atomicMax(&r.st.bc->passes, s.graph(tid).last + r.ba.pass0 + 1);
+    for (int g = tid; g < ng; g += kBlock) {
+      const owner::Local &l = s.graph(g);
+      if (l.last < 0) continue;
+      const GraphRec &r = e.recs[g];
+      atomicAdd(&r.st.bc->aff_edges, l.edges);
+      atomicAdd(&r.st.bc->front_visits, l.visits);
+      atomicMax(&r.st.bc->passes, l.last + r.ba.pass0 + 1);
     }
   }
   *k_out = k;

@@ -1,21 +1,24 @@
 // Full-grid propagation passes over owned rows.
 //
-// Every block but the first owns a contiguous range of the launch's vertices
-// (tiles of 64, all graphs one after the other) and keeps their live rows in
-// shared memory for the whole launch. A frontier is a byte per vertex in
+// Every block but the first owns a share of the launch's vertices (tiles of 32,
+// dealt out in turn, all graphs one after the other) and keeps their live rows
+// in shared memory for the whole launch. A frontier is a word per vertex in
 // global memory, one plane per pass parity. A pass is: read and clear the own
-// range's bytes, list the set ones in shared memory, run their rows with one
+// words, list the set ones in shared memory, run their rows with one
 // lane per row of at most 8 entries, four lanes up to 32 and a warp beyond,
-// store a byte for every neighbour that a moved label marks, barrier. The first
+// store a word for every neighbour that a moved label marks, barrier. The first
 // block owns nothing: it runs the one-block passes and the clock.
 //
-// What bounds a pass: four trips to L2 in a row (own bytes, neighbour labels,
+// What bounds a pass: four trips to L2 in a row (own words, neighbour labels,
 // acknowledged stores, barrier). A pass over frontier lists takes twice as
 // many (counts, list entry, row start, row, labels, mark atomic, reservation,
 // list store, barrier). Static ownership is what saves them: a row needs no
-// lookup, a mark no answer, and the list of a block no global counter. Range
-// scans cost a byte per owned vertex and pass, which is why launches beyond
-// kMaxVertices per block use frontier lists instead.
+// lookup, a mark no answer, and the list of a block no global counter. Scans
+// cost a word per owned vertex and pass, which is why launches beyond
+// kMaxVertices per block use frontier lists instead. On large frontiers the
+// scattered stores bound a pass: the GPU takes 173 G a second of 4-byte ones
+// over 690,000 vertices and 83 G over 50,000, but 107 G and 47 G of single bytes
+// (and 298 G loads), hence words.
 //
 // Measured, microseconds a pass, owned rows against lists: 5,000 vertices of
 // degree 5 4.0 against 5.1, 20,000 of degree 7 4.2 against 6.2, 50,000 of degree
@@ -27,34 +30,33 @@
 namespace dlp {
 namespace owner {
 
-constexpr int kTile = 64;
+constexpr int kTile = 32;                       // vertices of a warp's scan step
 constexpr int kMaxVertices = 16384;             // per block
-constexpr int kMaxTiles = kMaxVertices / kTile; // and so at most this many graphs
 constexpr int kLaneEntries = 8;
 constexpr int kLongLanes = 4;
 constexpr int kMaxRow = kLaneEntries * kLongLanes;
-constexpr unsigned kNoPool = (1u << 18) - 1;    // the row did not fit the pool: read from global memory
+constexpr unsigned kNoPool = (1u << 15) - 1;    // the row did not fit the pool: read from global memory
 constexpr unsigned kUnmarkable = 0x80000000u;   // pool entry: a neighbour that is never marked
 constexpr unsigned kNoEntry = 0xffffffffu;      // pool entry: soft-deleted
+constexpr int kMaxStint = 32000;                // passes of a stint (visits counts 15 bits)
+constexpr unsigned short kWideRow = 0x8000;
 
-struct Local {           // a graph of the block's range
+struct Local {           // a graph of the launch
   float *lab[2];         // [k & 1] is read by launch pass k
   unsigned flat;         // its first vertex among the launch's
   int limit;             // first launch pass its pass limit forbids
-  int last;              // last launch pass it took part in, -1 none
+  int last;              // last launch pass the block ran a row of it in, -1 none
   unsigned long long edges, visits;  // of the stint
 };
 
 struct Head {
-  int num_graphs, first_graph;
-  unsigned flat;         // first owned vertex among the launch's
   int pool_used;
-  int first_limit;       // the smallest limit of the block's graphs
+  int first_limit;       // the smallest limit of the graphs
   int count;             // rows of the pass: short | long << 16
   int wide;              // its rows of more than 32 entries
   int moved;
   // what every pass reads
-  unsigned char *marks;
+  unsigned *marks;
   unsigned plane;
   float delta;
   int fast;
@@ -62,73 +64,81 @@ struct Head {
   unsigned solo_entry;
 };
 
-// The block's dynamic shared memory: Head, then with T = V / 64 owned tiles
-// graph[T], of_tile[T], meta[V], visits[V], list[V], pool[cap]. Named by 32-bit
-// offsets from its start, so that a pass keeps no pointers in registers: a
-// register spilled there is a trip to L2 in every pass, because the barrier's
-// acquire empties L1.
+// The block's dynamic shared memory: Head, then graph[graphs], and with V =
+// 32 tiles meta[V], visits[V], list[V], pool[cap]. Named by 32-bit offsets
+// from its start, so that a pass keeps no pointers in registers: a register
+// spilled there is a trip to L2 in every pass, because the barrier's acquire
+// empties L1.
 extern __shared__ __align__(16) unsigned char g_smem[];
 constexpr int kHeadBytes = (sizeof(Head) + 15) & ~15;
-constexpr int kTileBytes = sizeof(Local) + 1 + kTile * (4 + 2 + 2);  // per tile, without the pool
-constexpr int kMaxStint = 32000;  // passes of a stint (visits counts 15 bits)
-constexpr unsigned short kWideRow = 0x8000;
+static_assert(sizeof(Local) % 16 == 0, "what follows the graphs stays aligned");
 
 struct Store {
-  int tiles;
+  int tiles;     // owned
+  int meta_at;   // byte offset of meta[]
   int pool_cap;
   __device__ int n() const { return tiles * kTile; }  // owned vertices
   __device__ Head &head() const { return *reinterpret_cast<Head *>(g_smem); }
   __device__ Local &graph(int i) const { return reinterpret_cast<Local *>(g_smem + kHeadBytes)[i]; }
-  // pool offset (18 bits) | length (6 bits, 63: longer than 32) | local graph (8 bits)
-  __device__ unsigned &meta(int i) const {
-    return reinterpret_cast<unsigned *>(g_smem + kHeadBytes + tiles * static_cast<int>(sizeof(Local)))[i];
-  }
+  // pool offset (15 bits) | length (6 bits, 63: longer than 32) | graph (10 bits)
+  __device__ unsigned &meta(int i) const { return reinterpret_cast<unsigned *>(g_smem + meta_at)[i]; }
   // passes that updated the row; kWideRow: the pass has listed it as a wide row
   __device__ unsigned short &visits(int i) const {
-    return reinterpret_cast<unsigned short *>(g_smem + kHeadBytes +
-                                              tiles * static_cast<int>(sizeof(Local) + 4 * kTile))[i];
+    return reinterpret_cast<unsigned short *>(g_smem + meta_at + 4 * kTile * tiles)[i];
   }
   // rows of the pass: short from the front, long from the back
-  __device__ unsigned short &list(int i) const { return (&visits(0) + tiles * kTile)[i]; }
-  // {neighbour | kUnmarkable, weight}
-  __device__ int2 &pool(int i) const {
-    return reinterpret_cast<int2 *>(g_smem + kHeadBytes + tiles * static_cast<int>(sizeof(Local) + 8 * kTile))[i];
+  __device__ unsigned short &list(int i) const {
+    return reinterpret_cast<unsigned short *>(g_smem + meta_at + 6 * kTile * tiles)[i];
   }
-  // graph of an owned tile (behind the pool)
-  __device__ unsigned char &of_tile(int i) const { return reinterpret_cast<unsigned char *>(&pool(pool_cap))[i]; }
+  // {neighbour | kUnmarkable, weight}
+  __device__ int2 &pool(int i) const { return reinterpret_cast<int2 *>(g_smem + meta_at + 8 * kTile * tiles)[i]; }
 };
-static_assert(sizeof(Local) % 8 == 0 && kTile % 16 == 0, "the pool is 8-byte aligned");
 
-__device__ __forceinline__ Store store(int bytes, int tiles) {
-  const int room = (bytes - kHeadBytes - kTileBytes * tiles) / static_cast<int>(sizeof(int2));
-  return Store{tiles, min(room, static_cast<int>(kNoPool) - kMaxRow)};
+__device__ __forceinline__ Store store(int bytes, int graphs, int tiles) {
+  const int at = kHeadBytes + graphs * static_cast<int>(sizeof(Local));
+  const int room = (bytes - at - 8 * kTile * tiles) / static_cast<int>(sizeof(int2));
+  return Store{tiles, at, min(room, static_cast<int>(kNoPool) - kMaxRow)};
 }
 
 __device__ __forceinline__ unsigned pack(unsigned off, int len, int g) {
-  return off | (static_cast<unsigned>(len > kMaxRow ? 63 : len) << 18) | (static_cast<unsigned>(g) << 24);
+  return off | (static_cast<unsigned>(len > kMaxRow ? 63 : len) << 15) | (static_cast<unsigned>(g) << 21);
 }
 __device__ __forceinline__ unsigned pool_of(unsigned m) { return m & kNoPool; }
-__device__ __forceinline__ int len_of(unsigned m) { return static_cast<int>((m >> 18) & 63u); }
-__device__ __forceinline__ int graph_of(unsigned m) { return static_cast<int>(m >> 24); }
+__device__ __forceinline__ int len_of(unsigned m) { return static_cast<int>((m >> 15) & 63u); }
+__device__ __forceinline__ int graph_of(unsigned m) { return static_cast<int>(m >> 21); }
 
-// tiles: all tiles of the launch; the range of block b in [1, blocks).
-__device__ __forceinline__ void range(int tiles, int b, int blocks, int &first, int &end) {
-  first = end = 0;
-  if (b == 0) return;
-  first = static_cast<int>(static_cast<long long>(tiles) * (b - 1) / (blocks - 1));
-  end = static_cast<int>(static_cast<long long>(tiles) * b / (blocks - 1));
+// The tiles of the launch are dealt out to the blocks but the first in turn. A
+// contiguous range per block would follow the graphs and the vertex ids, and so
+// do frontiers: some graphs have converged while others have a quarter of
+// their vertices in the frontier, and the first frontier of a batch is at low
+// ids. The slowest blocks then ran 1,800 rows a pass where others ran none.
+__device__ __forceinline__ int owned_tiles(int tiles) {
+  const int b = static_cast<int>(blockIdx.x) - 1, blocks = static_cast<int>(gridDim.x) - 1;
+  return b < 0 || b >= tiles ? 0 : (tiles - b - 1) / blocks + 1;
+}
+// Owned vertex i among the launch's vertices.
+__device__ __forceinline__ unsigned flat_of(int i) {
+  return (blockIdx.x - 1u + static_cast<unsigned>(i / kTile) * (gridDim.x - 1u)) * kTile +
+         static_cast<unsigned>(i % kTile);
 }
 
-// Rows of the block's range into shared memory (head filled by the caller).
-// Graph: row(g, v) {start, length}; markable(g, v); entry(g, at, v, w), v = -1
-// for an entry that does not count; nodes(g).
+// Rows of the block's vertices into shared memory (head and graphs filled by
+// the caller).
+// Graph: graphs(); nodes(g); row(g, v) {start, length}; markable(g, v);
+// entry(g, at, v, w), v = -1 for an entry that does not count.
 template <class Graph>
 __device__ void load(const Store &s, const Graph &gr) {
   const int tid = threadIdx.x, lane = tid & 31;
   Head &h = s.head();
   for (int i = tid; i < s.n(); i += blockDim.x) {
-    const int lg = s.of_tile(i / kTile), g = h.first_graph + lg;
-    const int v = static_cast<int>(h.flat + i - s.graph(lg).flat);
+    const unsigned flat = flat_of(i);
+    int g = 0;  // the last graph that starts at or before the vertex
+    for (int hi = gr.graphs() - 1; g < hi;) {
+      const int mid = (g + hi + 1) >> 1;
+      if (s.graph(mid).flat <= flat) g = mid;
+      else hi = mid - 1;
+    }
+    const int v = static_cast<int>(flat - s.graph(g).flat);
     int2 ri = make_int2(0, 0);
     if (v < gr.nodes(g) && gr.markable(g, v)) ri = gr.row(g, v);
     const int len = ri.y;
@@ -145,7 +155,7 @@ __device__ void load(const Store &s, const Graph &gr) {
     base = __shfl_sync(0xffffffffu, base, 31);
     const int off = base + incl - want;
     const bool fits = off + want <= s.pool_cap;
-    s.meta(i) = pack(fits ? static_cast<unsigned>(off) : kNoPool, len, lg);
+    s.meta(i) = pack(fits ? static_cast<unsigned>(off) : kNoPool, len, g);
     s.visits(i) = 0;
     if (!fits) continue;  // lanes of the next round reconverge at its first shuffle
     for (int b = 0; b < want; b += kLaneEntries) {
@@ -188,12 +198,12 @@ __device__ __forceinline__ float gather(const float *at, bool take) {
 }
 
 // A mark, predicated instead of branched around.
-__device__ __forceinline__ void mark(unsigned char *at, bool set) {
+__device__ __forceinline__ void mark(unsigned *at, bool set) {
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
       "setp.ne.s32 p, %1, 0;\n\t"
-      "@p st.global.u8 [%0], %2;\n\t"
+      "@p st.global.u32 [%0], %2;\n\t"
       "}" ::"l"(at), "r"(static_cast<int>(set)), "r"(1) : "memory");
 }
 
@@ -202,14 +212,14 @@ __device__ __forceinline__ void mark(unsigned char *at, bool set) {
 // the row).
 template <int LANES, class Graph>
 __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid, int i, int k, float delta, bool fast,
-                                    unsigned char *next) {
+                                    unsigned *next) {
   const int sub = threadIdx.x & (LANES - 1);
   const unsigned m = valid ? s.meta(i) : 0;
   const int len = valid ? len_of(m) : 0, lg = graph_of(m);
   const unsigned off = pool_of(m);
   const Local &l = s.graph(lg);
   const float *src = l.lab[k & 1];
-  const int v = static_cast<int>(s.head().flat + i - l.flat);
+  const int v = static_cast<int>(flat_of(i) - l.flat);
   const float old = gather(src + v, valid);
   unsigned u[kLaneEntries];
   float w[kLaneEntries], x[kLaneEntries];
@@ -222,7 +232,7 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
       w[r] = e < len ? __int_as_float(ent.y) : 0.0f;
     }
   } else {
-    const int g = s.head().first_graph + lg;
+    const int g = lg;
     const int start = gr.row(g, v).x;
 #pragma unroll
     for (int r = 0; r < kLaneEntries; ++r) {
@@ -264,7 +274,7 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
     s.graph(lg).last = k;
   }
   const bool moved = fabsf(nl - old) > delta;
-  unsigned char *const marks = next + l.flat;
+  unsigned *const marks = next + l.flat;
 #pragma unroll
   for (int r = 0; r < kLaneEntries; ++r) mark(marks + u[r], moved && !(u[r] & kUnmarkable));
   mark(marks + v, moved && sub == 0);
@@ -275,12 +285,12 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
 // of 256, then the tree.
 template <class Graph>
 __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i, int k, float delta, bool fast,
-                                         unsigned char *next) {
+                                         unsigned *next) {
   const int lane = threadIdx.x & 31;
-  const int lg = graph_of(s.meta(i)), g = s.head().first_graph + lg;
+  const int lg = graph_of(s.meta(i)), g = lg;
   const Local &l = s.graph(lg);
   const float *src = l.lab[k & 1];
-  const int v = static_cast<int>(s.head().flat + i - l.flat);
+  const int v = static_cast<int>(flat_of(i) - l.flat);
   const int2 ri = gr.row(g, v);
   float sw[8], sl[8];
 #pragma unroll
@@ -329,26 +339,26 @@ __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i,
   return true;
 }
 
-// Pass k of the block's range, up to the barrier. own: the range's bytes of
-// this pass's plane; next: the whole plane of the next pass. The rows are
+// Pass k of the block's vertices, up to the barrier. own: this pass's plane;
+// next: the plane of the next pass. The rows are
 // listed for the whole block and dealt out evenly: with every warp on its own
-// part of the range, the warps with the most marked rows took two to four
+// part of them, the warps with the most marked rows took two to four
 // steps where most took one, and every block waits for the slowest.
 template <class Graph, class Each>
-__device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned char *own, unsigned char *next, int k,
+__device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned *own, unsigned *next, int k,
                                      float delta, bool fast, Each each) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
   Head &h = s.head();
   const int n = s.n();
-  // A byte per lane, four loads in flight; the set ones are listed with one
+  // A word per lane, four loads in flight; the set ones are listed with one
   // reservation per warp.
   constexpr int kAhead = 4;
   for (int base = warp * 32; base < n; base += kAhead * nwarps * 32) {
-    unsigned char b[kAhead];
+    unsigned b[kAhead];
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) {
       const int i = base + j * nwarps * 32 + lane;
-      b[j] = i < n ? __ldcg(own + i) : 0;
+      b[j] = i < n ? __ldcg(own + flat_of(i)) : 0;
     }
     unsigned shorts[kAhead], longs[kAhead];
     int add = 0;
@@ -359,7 +369,7 @@ __device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned c
       const int i = base + j * nwarps * 32 + lane;
       int kind = 3;
       if (b[j]) {
-        own[i] = 0;
+        own[flat_of(i)] = 0;
         const unsigned m = s.meta(i);
         const int len = len_of(m);
         kind = len <= kLaneEntries ? 0 : len <= kMaxRow ? 1 : 2;

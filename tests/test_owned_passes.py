@@ -1,5 +1,5 @@
 """Full-grid passes on owned rows (csrc/owner_pass.cuh), bit-exact against the
-oracle with the one-block mode off: graphs of one tile, of a tile and a vertex,
+oracle with the one-block mode off: graphs of two tiles, of two tiles and a vertex,
 rows of 8, 9, 32 and 33 entries, several graphs in one launch (with pass limits
 that end at different launch passes), and blocks whose rows do not fit their
 shared memory."""
