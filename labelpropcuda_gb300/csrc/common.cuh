@@ -267,6 +267,33 @@ __device__ __forceinline__ float updated_label(float w_all, float w_label, float
   return fminf(fmaxf(nl, 0.0f), 1.0f);
 }
 
+// a / b, correctly rounded, from y = RN(1 / b): q1 is a/b to within an ulp, its
+// remainder is exact, and one more correction by y rounds correctly (P.
+// Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34(1), 1990). 1e-10 < b <= kDivHi, and a is 0
+// or in [kDivLo, kDivHi], so that nothing here underflows or overflows. The
+// reciprocal can be known before the numerator, which leaves five dependent
+// multiply-adds of the division; and a zero numerator, which is common where all
+// neighbours have label 0, takes no other path.
+constexpr float kDivLo = 0x1p-40f, kDivHi = 0x1p40f;
+__device__ __forceinline__ float divide(float a, float b, float y) {
+  const float q0 = __fmul_rn(a, y);
+  const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
+  return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
+}
+
+// updated_label from the reciprocal of the weight sum: label_recip is 0, and
+// recip_serves false, where updated_label has to be called instead.
+__device__ __forceinline__ float label_recip(float w_all, bool fast) {
+  return !fast && w_all > 1e-10f && w_all <= kDivHi ? __frcp_rn(w_all) : 0.0f;
+}
+__device__ __forceinline__ bool recip_serves(float recip, float w_label) {
+  return (recip != 0.0f) & ((w_label == 0.0f) | ((w_label >= kDivLo) & (w_label <= kDivHi)));
+}
+__device__ __forceinline__ float label_by_recip(float w_all, float recip, float w_label) {
+  return fminf(fmaxf(divide(w_label, w_all, recip), 0.0f), 1.0f);
+}
+
 // Launch helper: cooperative launch of `kernel` with `args` on `stream`.
 int launch_cooperative(const void *kernel, int grid, int block, void **args, size_t smem,
                        cudaStream_t stream);

@@ -1493,12 +1493,15 @@ __device__ __noinline__ int owned_loop(const EngineArgs &e, int k, owner::Store 
     if (s.tiles > 0) {
       unsigned *own = h.marks + (k & 1 ? h.plane : 0u);
       unsigned *next = h.marks + (k & 1 ? 0u : h.plane);
-      owner::pass(s, gr, own, next, k, h.delta, h.fast != 0, [&](int i) {
+      auto each = [&](int i) {
         if (!rec_any) return;
         const GraphRec &r = e.recs[owner::graph_of(s.meta(i))];
         const int kg = k + r.ba.pass0;
         if (r.ba.record && kg < kRecordIters) atomicAdd(&r.st.rec_fsizes[kg], 1);
-      });
+      };
+      // Up to 1,024 owned vertices a block: 151 x 1,024 in the launch.
+      if (s.n() <= kBlock) owner::tile_pass(s, gr, own, next, k, h.delta, h.fast != 0, each);
+      else owner::pass(s, gr, own, next, k, h.delta, h.fast != 0, each);
     } else if (rec_any && blockIdx.x == 0) {
       clear_record(e, k + 1);
     }

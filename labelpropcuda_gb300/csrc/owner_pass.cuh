@@ -182,29 +182,52 @@ __device__ void load(const Store &s, const Graph &gr) {
   }
 }
 
-// A label from L2, 0 without `take`; predicated, because a load in a branch is
-// waited for before the next one is issued (and a stand-in address that all
-// idle lanes share queues up in its L2 slice: it cost 3,000 cycles a pass).
-__device__ __forceinline__ float gather(const float *at, bool take) {
+// The accesses of a row step are predicated, not branched around: a load in a
+// branch is waited for before the next one is issued. (A stand-in address that
+// all idle lanes share is no way out: its L2 slice cost 3,000 cycles a pass.)
+// Pool entry at byte address `at` + OFF of shared memory, kNoEntry with weight 0
+// unless `e` < `len`.
+template <int OFF>
+__device__ __forceinline__ void pool_entry(unsigned at, int e, int len, unsigned &u, float &w) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.lt.s32 p, %3, %4;\n\t"
+      "mov.b32 %0, -1;\n\t"
+      "mov.f32 %1, 0f00000000;\n\t"
+      "@p ld.shared.v2.b32 {%0, %1}, [%2+%5];\n\t"
+      "}" : "=&r"(u), "=&f"(w) : "r"(at), "r"(e), "r"(len), "n"(OFF));
+}
+// The label of entry u from L2, 0 for kNoEntry.
+__device__ __forceinline__ float gather(const float *src, unsigned u) {
   float x;
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
-      "setp.ne.s32 p, %2, 0;\n\t"
+      "setp.ne.u32 p, %2, -1;\n\t"
       "mov.f32 %0, 0f00000000;\n\t"
       "@p ld.global.cg.f32 %0, [%1];\n\t"
-      "}" : "=f"(x) : "l"(at), "r"(static_cast<int>(take)));
+      "}" : "=&f"(x) : "l"(src + (u & ~kUnmarkable)), "r"(u));
   return x;
 }
-
-// A mark, predicated instead of branched around.
-__device__ __forceinline__ void mark(unsigned *at, bool set) {
+// Marks entry u if it can be and `moved`.
+__device__ __forceinline__ void mark(unsigned *marks, unsigned u, int moved) {
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.s32 p, %1, 0;\n\t"
-      "@p st.global.u32 [%0], %2;\n\t"
-      "}" ::"l"(at), "r"(static_cast<int>(set)), "r"(1) : "memory");
+      ".reg .pred p, q;\n\t"
+      "setp.ne.s32 q, %2, 0;\n\t"
+      "setp.ge.and.s32 p, %1, 0, q;\n\t"
+      "@p st.global.u32 [%0], %3;\n\t"
+      "}" ::"l"(marks + (u & ~kUnmarkable)), "r"(u), "r"(moved), "r"(1) : "memory");
+}
+
+template <int LANES, int R = 0>
+__device__ __forceinline__ void pool_row(unsigned at, int sub, int len, unsigned (&u)[kLaneEntries],
+                                         float (&w)[kLaneEntries]) {
+  if constexpr (R < kLaneEntries) {
+    pool_entry<8 * LANES * R>(at, sub + LANES * R, len, u[R], w[R]);
+    pool_row<LANES, R + 1>(at, sub, len, u, w);
+  }
 }
 
 // The row of owned vertex i by LANES lanes (1: up to 8 entries, 4: up to 32).
@@ -214,31 +237,24 @@ template <int LANES, class Graph>
 __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid, int i, int k, float delta, bool fast,
                                     unsigned *next) {
   const int sub = threadIdx.x & (LANES - 1);
-  const unsigned m = valid ? s.meta(i) : 0;
-  const int len = valid ? len_of(m) : 0, lg = graph_of(m);
+  const unsigned m = s.meta(i);
+  const int len = valid ? len_of(m) : 0, g = graph_of(m);
   const unsigned off = pool_of(m);
-  const Local &l = s.graph(lg);
+  const Local &l = s.graph(g);
   const float *src = l.lab[k & 1];
-  const int v = static_cast<int>(flat_of(i) - l.flat);
-  const float old = gather(src + v, valid);
+  const unsigned first = l.flat;
+  const unsigned v = flat_of(i) - first;
+  const float old = gather(src, valid ? v : kNoEntry);
   unsigned u[kLaneEntries];
   float w[kLaneEntries], x[kLaneEntries];
-  if (off != kNoPool) {
+  pool_row<LANES>(static_cast<unsigned>(__cvta_generic_to_shared(&s.pool(0))) + 8 * (off + sub), sub,
+                  off != kNoPool ? len : 0, u, w);
+  if (off == kNoPool) {
+    const int start = gr.row(g, static_cast<int>(v)).x;
 #pragma unroll
     for (int r = 0; r < kLaneEntries; ++r) {
-      const int e = LANES == 1 ? r : sub + LANES * r;
-      const int2 ent = s.pool(e < len ? static_cast<int>(off) + e : 0);
-      u[r] = e < len ? static_cast<unsigned>(ent.x) : kNoEntry;
-      w[r] = e < len ? __int_as_float(ent.y) : 0.0f;
-    }
-  } else {
-    const int g = lg;
-    const int start = gr.row(g, v).x;
-#pragma unroll
-    for (int r = 0; r < kLaneEntries; ++r) {
-      const int e = LANES == 1 ? r : sub + LANES * r;
+      const int e = sub + LANES * r;
       int c = -1;
-      w[r] = 0.0f;
       if (e < len) gr.entry(g, start + e, c, w[r]);
       if (c < 0) w[r] = 0.0f;
       u[r] = c < 0 ? kNoEntry : static_cast<unsigned>(c);
@@ -248,9 +264,9 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
       if (!(u[r] & kUnmarkable) && !gr.markable(g, static_cast<int>(u[r]))) u[r] |= kUnmarkable;
   }
 #pragma unroll
-  for (int r = 0; r < kLaneEntries; ++r) x[r] = gather(src + (u[r] & ~kUnmarkable), u[r] != kNoEntry);
+  for (int r = 0; r < kLaneEntries; ++r) x[r] = gather(src, u[r]);
 #pragma unroll
-  for (int r = 0; r < kLaneEntries; ++r) x[r] = u[r] == kNoEntry ? 0.0f : __fmaf_rn(w[r], x[r], 0.0f);
+  for (int r = 0; r < kLaneEntries; ++r) x[r] = __fmaf_rn(w[r], x[r], 0.0f);  // an empty slot: 0 * 0 + 0
   // the reference's tree (row_sums.cuh): strides 16 to 4 within a lane of a
   // long row, 2 and 1 across its lanes; strides 4 to 1 within that of a short
 #pragma unroll
@@ -266,18 +282,19 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
     tl = tl + __shfl_xor_sync(0xffffffffu, tl, o);
     tw = tw + __shfl_xor_sync(0xffffffffu, tw, o);
   }
-  if (!valid) return false;
-  const float nl = updated_label(tw, tl, old, fast);
-  if (sub == 0) {
+  const float recip = label_recip(tw, fast);
+  float nl = label_by_recip(tw, recip, tl);
+  if (valid & !recip_serves(recip, tl)) nl = updated_label(tw, tl, old, fast);
+  const bool moved = valid & (fabsf(nl - old) > delta);
+  unsigned *const marks = next + first;
+#pragma unroll
+  for (int r = 0; r < kLaneEntries; ++r) mark(marks, u[r], moved);
+  if (valid && sub == 0) {
     l.lab[(k & 1) ^ 1][v] = nl;
     ++s.visits(i);
-    s.graph(lg).last = k;
+    s.graph(g).last = k;
+    mark(marks, v, moved);
   }
-  const bool moved = fabsf(nl - old) > delta;
-  unsigned *const marks = next + l.flat;
-#pragma unroll
-  for (int r = 0; r < kLaneEntries; ++r) mark(marks + u[r], moved && !(u[r] & kUnmarkable));
-  mark(marks + v, moved && sub == 0);
   return moved;
 }
 
@@ -339,6 +356,50 @@ __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i,
   return true;
 }
 
+// Kind of the row of marked vertex i in pass k: 0 short, 1 long, 2 wide, 3 past
+// its graph's pass limit.
+__device__ __forceinline__ int kind_of(const Store &s, int i, int k) {
+  const unsigned m = s.meta(i);
+  const int len = len_of(m);
+  if (k >= s.head().first_limit && k >= s.graph(graph_of(m)).limit) return 3;
+  return len <= kLaneEntries ? 0 : len <= kMaxRow ? 1 : 2;
+}
+
+// A pass of a block that owns at most 32 vertices per warp: every warp runs the
+// marked rows of its own tile, without a list and without waiting for the
+// others.
+template <class Graph, class Each>
+__device__ __forceinline__ void tile_pass(const Store &s, const Graph &gr, unsigned *own, unsigned *next, int k,
+                                          float delta, bool fast, Each each) {
+  const int lane = threadIdx.x & 31, i = threadIdx.x;
+  const bool marked = i < s.n() && __ldcg(own + flat_of(i)) != 0;
+  if (!__any_sync(0xffffffffu, marked)) return;
+  int kind = 3;
+  if (marked) {
+    own[flat_of(i)] = 0;
+    kind = kind_of(s, i, k);
+    if (kind != 3) each(i);
+  }
+  bool moved = false;
+  if (__any_sync(0xffffffffu, kind == 0)) moved = row<1>(s, gr, kind == 0, i, k, delta, fast, next);
+  unsigned longs = __ballot_sync(0xffffffffu, kind == 1), wides = __ballot_sync(0xffffffffu, kind == 2);
+  const int rows = __popc(__ballot_sync(0xffffffffu, kind != 3));
+  while (longs) {  // 8 at a time, the q-th remaining one to the q-th lanes
+    unsigned m = longs;
+    for (int q = lane / kLongLanes; q > 0 && m; --q) m &= m - 1;
+    const int at = (i - lane) + __ffs(m ? m : longs) - 1;
+    moved |= row<kLongLanes>(s, gr, m != 0, at, k, delta, fast, next);
+    for (int q = 32 / kLongLanes; q > 0 && longs; --q) longs &= longs - 1;
+  }
+  for (; wides; wides &= wides - 1)
+    moved |= wide_row(s, gr, (i - lane) + __ffs(wides) - 1, k, delta, fast, next);
+  moved = __any_sync(0xffffffffu, moved);
+  if (lane == 0) {
+    atomicAdd(&s.head().count, rows);
+    if (moved) s.head().moved = 1;
+  }
+}
+
 // Pass k of the block's vertices, up to the barrier. own: this pass's plane;
 // next: the plane of the next pass. The rows are
 // listed for the whole block and dealt out evenly: with every warp on its own
@@ -370,11 +431,8 @@ __device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned *
       int kind = 3;
       if (b[j]) {
         own[flat_of(i)] = 0;
-        const unsigned m = s.meta(i);
-        const int len = len_of(m);
-        kind = len <= kLaneEntries ? 0 : len <= kMaxRow ? 1 : 2;
-        if (k >= h.first_limit && k >= s.graph(graph_of(m)).limit) kind = 3;
-        else each(i);
+        kind = kind_of(s, i, k);
+        if (kind != 3) each(i);
       }
       shorts[j] = __ballot_sync(0xffffffffu, kind == 0);
       longs[j] = __ballot_sync(0xffffffffu, kind == 1);
@@ -404,22 +462,16 @@ __device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned *
   bool moved = false;
   constexpr int kPer = 32 / kLongLanes;
   const int sub = lane / kLongLanes;
-  if (ns + nl <= kPer * nwarps) {  // one step of 4-lane groups, spread over all warps
-    if (warp < ns + nl) {
-      const int r = warp + sub * nwarps;
-      const bool valid = r < ns + nl;
-      moved = row<kLongLanes>(s, gr, valid, valid ? s.list(r < ns ? r : n - 1 - (r - ns)) : 0, k, delta, fast, next);
-    }
-  } else {
-    // short rows from the first warp up, long ones from the last down
-    for (int b = warp * 32; b < ns; b += nwarps * 32) {
-      const bool valid = b + lane < ns;
-      moved |= row<1>(s, gr, valid, valid ? s.list(b + lane) : 0, k, delta, fast, next);
-    }
-    for (int b = (nwarps - 1 - warp) * kPer; b < nl; b += nwarps * kPer) {
-      const bool valid = b + sub < nl;
-      moved |= row<kLongLanes>(s, gr, valid, valid ? s.list(n - 1 - (b + sub)) : 0, k, delta, fast, next);
-    }
+  // Short rows from the first warp up, 32 to a warp, long ones from the last
+  // down, 8 to a warp: a step is some 300 instructions however many rows it
+  // holds, and few full warps issue them sooner than many with a row each.
+  for (int b = warp * 32; b < ns; b += nwarps * 32) {
+    const bool valid = b + lane < ns;
+    moved |= row<1>(s, gr, valid, s.list(valid ? b + lane : b), k, delta, fast, next);
+  }
+  for (int b = (nwarps - 1 - warp) * kPer; b < nl; b += nwarps * kPer) {
+    const bool valid = b + sub < nl;
+    moved |= row<kLongLanes>(s, gr, valid, s.list(n - 1 - (valid ? b + sub : b)), k, delta, fast, next);
   }
   if (nw)
     for (int b = warp * 32; b < n; b += nwarps * 32) {

@@ -173,20 +173,6 @@ __device__ __forceinline__ int long_warps(const Cache &c) {
   return (c.num_long + 32 / kLongLanes - 1) / (32 / kLongLanes);
 }
 
-// a / b, correctly rounded, from y = RN(1 / b): q1 is a/b to within an ulp, its
-// remainder is exact, and one more correction by y rounds correctly (P.
-// Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", IBM J. Res. Dev. 34(1), 1990). 1e-10 < b <= kDivHi, and a is 0
-// or in [kDivLo, kDivHi], so that nothing here underflows or overflows. The
-// reciprocal is known when a row is loaded, which leaves five dependent
-// multiply-adds of the division in a pass.
-constexpr float kDivLo = 0x1p-40f, kDivHi = 0x1p40f;
-__device__ __forceinline__ float divide(float a, float b, float y) {
-  const float q0 = __fmul_rn(a, y);
-  const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
-  return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
-}
-
 // Gives every marked vertex of pass parity p without a row a place and loads
 // its row. Short rows fill the lanes from warp 0 up, long rows those from the
 // last warp down, so a warp holds one kind. All threads of the block call;
@@ -284,7 +270,7 @@ __device__ bool load_rows(Cache &c, const Graph &gr, Row &row, int p, int q, boo
     }
     if (mine) {
       row.total = tw;
-      row.recip = !fast && tw > 1e-10f && tw <= kDivHi ? __frcp_rn(tw) : 0.0f;
+      row.recip = label_recip(tw, fast);
     }
   }
   __syncthreads();
@@ -362,10 +348,8 @@ __device__ __forceinline__ bool pass(Row &row, unsigned now, unsigned next, unsi
 #pragma unroll
     for (int o = kLongLanes / 2; o >= 1; o >>= 1) tl = tl + __shfl_xor_sync(0xffffffffu, tl, o);
   }
-  // updated_label (common.cuh) with the quotient from the row's reciprocal
-  float nl = fminf(fmaxf(divide(tl, row.total, row.recip), 0.0f), 1.0f);
-  const bool plain = (row.recip != 0.0f) & ((tl == 0.0f) | ((tl >= kDivLo) & (tl <= kDivHi)));
-  if (act & !plain) nl = updated_label(row.total, tl, old, fast);
+  float nl = label_by_recip(row.total, row.recip, tl);
+  if (act & !recip_serves(row.recip, tl)) nl = updated_label(row.total, tl, old, fast);
   const bool moved = act & (fabsf(nl - old) > delta);
   row.visits += act ? 1u : 0u;
   row.last = act ? k : row.last;
