@@ -1094,13 +1094,12 @@ __device__ __noinline__ void solo_passes(const EngineArgs &e, int k0, int slot) 
   // Labels written during the stint go back to HBM; the marks of pass k are
   // the frontier; vertices that were or are in a frontier join the touched
   // list the first time in this batch, with the batch's first stamp.
-  const int jp = (k - k0) & 1;
   for (int i = tid; i < stint::kSlots; i += kBlock) {
     const unsigned long long key = c.key[i];
     if (key == stint::kEmptyKey) continue;
     const unsigned meta = c.meta[i];
     const bool visited = (meta & stint::kVisited) != 0;
-    const bool front = c.mark[jp][i] != 0 && (meta & stint::kMarkable) != 0;
+    const bool front = stint::marked(c, i, k - k0) && (meta & stint::kMarkable) != 0;
     if (!visited && !front) continue;
     const GraphRec &r = e.recs[key >> 32];
     const DevState &s = r.st;
@@ -1465,6 +1464,7 @@ struct OwnedGraphs {
   __device__ int graphs() const { return e.ng; }
   __device__ int nodes(int g) const { return e.recs[g].st.n; }
   __device__ int2 row(int g, int v) const { return e.recs[g].st.rowinfo[v]; }
+  __device__ bool active(int g, int v) const { return markable(g, v); }
   __device__ bool markable(int g, int v) const { return (e.recs[g].st.nmeta[v] & 1u) != 0; }
   __device__ void entry(int g, int at, int &v, float &w) const {
     const int2 ent = e.recs[g].st.act_adj[at];

@@ -17,6 +17,8 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "owner_pass.cuh"
+#include "row_stint.cuh"
 #include "row_sums.cuh"
 
 namespace dlp {
@@ -531,6 +533,329 @@ __global__ void __launch_bounds__(kBlock) prop_kernel(PropArgs a) {
   if (t == 0) a.out[0] = k;
 }
 
+// -------------------------------------- propagation and IrLP on owned rows --
+// Graphs whose vertices the blocks can own (owner_pass.cuh) propagate as the
+// resident engine does: full-grid passes on rows in shared memory, frontiers of
+// up to kSmallFront vertices on one block with rows in registers
+// (row_stint.cuh). Larger graphs take prop_kernel above.
+//
+// Measured against prop_kernel and irlp_kernel: propagation from 1,000 affected
+// vertices of 50,000 (degree 5, 2,000 passes at most) 1.13 against 2.64 ms, from
+// 50,000 of a million (degree 7, 300 passes at most) 4.1 against 8.7 ms; recompute
+// of 100,000 vertices 0.82 against 2.43 ms.
+constexpr int kOwnBlock = stint::kThreads;
+constexpr int kSmallFront = 512;
+constexpr unsigned long long kStintNs = 100000000ull;  // the other blocks wait in a barrier with a 2 s limit
+
+// The caller's arrays as owned passes and stints read them.
+struct CsrGraph {
+  const int *row_ptr, *col;
+  const float *val;
+  const int *status, *gt;
+  int n;
+  __device__ int graphs() const { return 1; }
+  __device__ int nodes(int) const { return n; }
+  __device__ int2 row(int, int v) const { return make_int2(row_ptr[v], row_ptr[v + 1] - row_ptr[v]); }
+  __device__ bool active(int, int v) const { return gt[v] < 0 && status[v] == kActive; }
+  __device__ bool markable(int, int v) const { return gt[v] < 0; }
+  __device__ void entry(int, int at, int &v, float &w) const {
+    v = col[at];
+    w = val[at];
+    if (v >= 0 && status[v] == kDeleted) v = -1;
+  }
+};
+
+struct OwnedArgs {
+  CsrGraph g;
+  float *labels, *buffer;
+  int *affected;
+  float delta;
+  int max_iter;
+  unsigned *marks;        // 2 planes, zeroed
+  int plane;              // words of a plane: whole tiles
+  int *list;              // a small frontier on its way to the first block
+  int *small;             // zeroed: see kOut
+  SumBarrier *bar;        // zeroed
+  unsigned long long timeout_ns;
+  int fast_div;
+  int smem_bytes;
+};
+// Words of OwnedArgs::small.
+enum { kOutPasses = 0, kOutError = 1, kOutListed = 2, kOutPass = 3, kOutFull = 4, kOutFront = 5, kOutWords = 16 };
+
+__shared__ SumState s_bar;
+
+template <class Mine>
+__device__ __forceinline__ bool all_sync(const OwnedArgs &a, Mine mine, unsigned long long &sum) {
+  return sum_sync(a.bar, s_bar, &a.small[kOutError], a.timeout_ns, mine, sum);
+}
+__device__ __forceinline__ bool all_sync(const OwnedArgs &a) {
+  unsigned long long sum;
+  return all_sync(a, [] { return 0ull; }, sum);
+}
+
+// The block's rows; both kernels start with it.
+__device__ __forceinline__ owner::Store own_rows(const OwnedArgs &a) {
+  const int tid = threadIdx.x;
+  const owner::Store s = owner::store(a.smem_bytes, 1, owner::owned_tiles((a.g.n + owner::kTile - 1) / owner::kTile));
+  if (tid == 0) s_bar.gen = 0;
+  if (s.tiles > 0) {
+    owner::Head &h = s.head();
+    if (tid == 0) {
+      h.pool_used = 0;
+      h.first_limit = a.max_iter;
+      h.count = h.wide = h.moved = 0;
+      owner::Local &l = s.graph(0);
+      l.lab[0] = a.labels;
+      l.lab[1] = a.buffer;
+      l.flat = 0;
+      l.limit = a.max_iter;
+      l.last = -1;
+    }
+    __syncthreads();
+    owner::load(s, a.g);
+  }
+  return s;
+}
+
+// Vertices of the graph as the one-block passes from pass k0 on see them.
+struct CsrStint {
+  const OwnedArgs &a;
+  int k0;
+  __device__ void vertex(int, int v, float &even, float &odd, unsigned &meta) const {
+    const float l0 = a.labels[v], l1 = a.buffer[v];
+    even = k0 & 1 ? l1 : l0;
+    odd = k0 & 1 ? l0 : l1;
+    const bool active = a.g.active(0, v);
+    meta = (active ? stint::kMarkable : 0u) | (a.g.markable(0, v) ? stint::kShown : 0u);
+    if (active && a.g.row(0, v).y > kNarrowMax) meta |= stint::kWide;
+  }
+  __device__ int2 row(int g, int v) const { return a.g.row(g, v); }
+  __device__ void entry(int g, int at, int &v, float &w) const { a.g.entry(g, at, v, w); }
+};
+
+struct StintShared {
+  stint::Cache c;
+  unsigned long long start;
+};
+
+// Passes from k0 on by the first block alone, over the frontier in a.list;
+// leaves the next pass, its frontier's marks and what became of the labels in
+// global memory.
+__device__ __noinline__ void small_passes(const OwnedArgs &a, int k0, int listed) {
+  StintShared &sh = *reinterpret_cast<StintShared *>(owner::g_smem);
+  stint::Cache &c = sh.c;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const CsrStint gr{a, k0};
+  stint::clear(c);
+  if (tid == 0) sh.start = global_timer_ns();
+  __syncthreads();
+  for (int i = tid; i < listed; i += kOwnBlock) stint::seed(c, gr, 0, a.list[i]);
+  __syncthreads();
+  stint::Row row;
+  int k = k0, full = 0;
+  for (;;) {
+    const int j = k - k0, q = j % 3;
+    const int4 ctl = c.ctl[q];
+    if (ctl.x == 0 || ctl.z != 0 || k >= a.max_iter) break;
+    if (ctl.y && !stint::load_rows(c, gr, row, j & 1, q, a.fast_div != 0)) {
+      full = 1;
+      break;
+    }
+    const int ns = stint::short_warps(c), nl = stint::long_warps(c);
+    const bool is_long = warp >= stint::kWarps - nl;
+    if (warp < ns || is_long) {
+      const bool leader = tid == (ns > 0 ? 0 : kOwnBlock - 32);
+      auto tick = [&](int) { return global_timer_ns() - sh.start > kStintNs; };
+      const int kk = stint::run(c, row, k, j, a.max_iter, a.delta, a.fast_div != 0, ns + nl, is_long, leader, tick,
+                                false, [](int, int, const stint::Row &) {});
+      if (leader) c.end = kk;
+    }
+    __syncthreads();  // the warps without rows wait here
+    k = c.end;
+  }
+  __syncthreads();
+  if (row.visits != 0 && row.lead) c.meta[row.slot] |= stint::kVisited;
+  __syncthreads();
+  unsigned *plane = a.marks + (k & 1 ? a.plane : 0);
+  int front = 0;
+  for (int i = tid; i < stint::kSlots; i += kOwnBlock) {
+    if (c.key[i] == stint::kEmptyKey) continue;
+    const unsigned meta = c.meta[i];
+    const int v = static_cast<int>(c.key[i]);
+    if (meta & stint::kVisited) {
+      a.labels[v] = c.lab[k0 & 1][i];
+      a.buffer[v] = c.lab[(k0 & 1) ^ 1][i];
+    }
+    if (stint::marked(c, i, k - k0) && (meta & stint::kShown)) {
+      plane[v] = 1;
+      if (meta & stint::kMarkable) front = 1;
+    }
+  }
+  front = __syncthreads_or(front);
+  if (tid == 0) {
+    a.small[kOutPass] = k;
+    a.small[kOutFull] = full && k - k0 < 256;
+    a.small[kOutFront] = front;
+    a.small[kOutListed] = 0;
+  }
+}
+
+// The passes on owned rows from k on until the frontier empties, is small or a
+// limit is reached; not inlined, for its registers. -1: the launch has to end.
+__device__ __noinline__ int large_passes(const OwnedArgs &a, owner::Store s, int k, int small_from, bool &empty) {
+  owner::Head &h = s.head();
+  // in registers: the launch's arguments are memory here
+  unsigned *const even = a.marks, *const odd = a.marks + a.plane;
+  SumBarrier *const bar = a.bar;
+  int *const err = &a.small[kOutError];
+  const uint64_t timeout = a.timeout_ns;
+  const float delta = a.delta;
+  const bool fast = a.fast_div != 0;
+  const int end = min(a.max_iter, k + owner::kMaxStint);
+  unsigned before = 0xffffffffu;
+  for (;;) {
+    if (s.tiles > 0) {
+      unsigned *own = k & 1 ? odd : even, *next = k & 1 ? even : odd;
+      auto each = [](int) {};
+      if (s.n() <= kOwnBlock) owner::tile_pass(s, a.g, own, next, k, delta, fast, each);
+      else owner::pass(s, a.g, own, next, k, delta, fast, each);
+    }
+    unsigned long long sum;
+    const bool ok = sum_sync(bar, s_bar, err, timeout, [&]() -> unsigned long long {
+      if (s.tiles == 0) return 0ull;
+      const unsigned long long mine =
+          static_cast<unsigned>((h.count & 0xffff) + (h.count >> 16) + h.wide) | (h.moved ? kSumMoved : 0ull);
+      h.count = h.wide = 0;
+      h.moved = 0;
+      return mine;
+    }, sum);
+    if (!ok) return -1;
+    ++k;
+    const unsigned rows = static_cast<unsigned>(sum);
+    empty = (sum & (0xffull * kSumMoved)) == 0;
+    if (empty || k >= end) return k;
+    if (max(rows, before) <= kSmallFront && k >= small_from) return k;
+    before = rows;
+  }
+}
+
+// src/iterativePropagation.cu:241-346 in one cooperative launch of a block per
+// SM. The marks of the last pass run stay in the plane of the pass after it:
+// they are the final isAffected.
+__global__ void __launch_bounds__(kOwnBlock, 1) prop_owned_kernel(const __grid_constant__ OwnedArgs a) {
+  const int tid = threadIdx.x, n = a.g.n;
+  const int t = blockIdx.x * kOwnBlock + tid, nt = gridDim.x * kOwnBlock;
+  const owner::Store s = own_rows(a);
+  // both buffers start at the current labels (src/iterativePropagation.cu:268-270);
+  // the first frontier (:63-78)
+  int seeds = 0;
+  for (int v = t; v < n; v += nt) {
+    a.buffer[v] = a.labels[v];
+    if (a.affected[v] == 1 && a.g.active(0, v)) {
+      a.marks[v] = 1;
+      ++seeds;
+    }
+  }
+  __shared__ int s_seeds;
+  if (tid == 0) s_seeds = 0;
+  __syncthreads();
+  if (seeds) atomicAdd(&s_seeds, seeds);
+  unsigned long long sum;
+  if (!all_sync(a, [&] { return static_cast<unsigned long long>(s_seeds); }, sum)) return;
+  int k = 0, small_from = 0;
+  unsigned rows = static_cast<unsigned>(sum);
+  bool empty = rows == 0, try_small = rows <= kSmallFront;
+  while (!empty && k < a.max_iter) {
+    if (try_small) {
+      // the marks of pass k become a list (bounded: a frontier larger than
+      // thought goes back to the owned rows), the first block runs it
+      unsigned *own = a.marks + (k & 1 ? a.plane : 0);
+      for (int i = tid; i < s.n(); i += kOwnBlock) {
+        const unsigned v = owner::flat_of(i);
+        const bool marked = v < static_cast<unsigned>(n) && __ldcg(own + v) != 0;
+        const bool front = marked && owner::kind_of(s, i, k) != 3;
+        warp_append(front, static_cast<int>(v), a.list, &a.small[kOutListed]);
+      }
+      if (!all_sync(a)) return;
+      const int listed = ld_relaxed_i32(&a.small[kOutListed]);
+      if (listed <= kSmallFront) {
+        // pass k is the first block's: its marks go
+        for (int i = tid; i < s.n(); i += kOwnBlock) {
+          const unsigned v = owner::flat_of(i);
+          if (v < static_cast<unsigned>(n) && __ldcg(own + v) != 0) own[v] = 0;
+        }
+        if (!all_sync(a)) return;  // before it leaves marks of its own
+        if (blockIdx.x == 0) small_passes(a, k, listed);
+        if (!all_sync(a)) return;
+        k = ld_relaxed_i32(&a.small[kOutPass]);
+        empty = ld_relaxed_i32(&a.small[kOutFront]) == 0;
+        if (ld_relaxed_i32(&a.small[kOutFull])) small_from = k + 256;
+      } else {
+        if (!all_sync(a)) return;  // every block has read the count
+        if (t == 0) a.small[kOutListed] = 0;
+      }
+      try_small = false;  // at least one pass on the owned rows
+      continue;
+    }
+    k = large_passes(a, s, k, small_from, empty);
+    if (k < 0) return;
+    try_small = true;
+  }
+  // final labels in the primary array, ground truth enforced
+  // (src/iterativePropagation.cu:330-339); isAffected holds the last pass's marks
+  const float *lab = (k & 1) ? a.buffer : a.labels;
+  const unsigned *plane = a.marks + (k & 1 ? a.plane : 0);
+  for (int v = t; v < n; v += nt) {
+    float l = lab[v];
+    const int g = a.g.gt[v];
+    if (g == 0) l = 0.0f;
+    else if (g == 1) l = 1.0f;
+    a.labels[v] = l;
+    if (k > 0) a.affected[v] = __ldcg(plane + v) != 0;
+  }
+  if (t == 0) a.small[kOutPasses] = k;
+}
+
+// src/validation.cu:47-139 and :169-197 on owned rows: every active vertex
+// takes its neighbours' average per pass, until no label moves by more than
+// delta. The others are copied through by the reference, ground truth as 0 / 1:
+// pass 0 reads the caller's labels as they are and its result has the copies, so
+// these are written into the buffer before pass 0 and, ground truth, into the
+// primary array during pass 1.
+__global__ void __launch_bounds__(kOwnBlock, 1) irlp_owned_kernel(const __grid_constant__ OwnedArgs a) {
+  const int n = a.g.n;
+  const int t = blockIdx.x * kOwnBlock + threadIdx.x, nt = gridDim.x * kOwnBlock;
+  const owner::Store s = own_rows(a);
+  auto fixed = [&](int v) {
+    const int g = a.g.gt[v];
+    return g == 0 ? 0.0f : (g == 1 ? 1.0f : a.labels[v]);
+  };
+  for (int v = t; v < n; v += nt)
+    if (!a.g.active(0, v)) a.buffer[v] = fixed(v);
+  int k = 0;
+  while (k < a.max_iter) {
+    if (k == 1)
+      for (int v = t; v < n; v += nt)
+        if (a.g.gt[v] == 0 || a.g.gt[v] == 1) a.labels[v] = fixed(v);
+    if (s.tiles > 0) owner::dense_pass(s, a.g, k, a.delta);
+    unsigned long long sum;
+    if (!all_sync(a, [&]() -> unsigned long long {
+          if (s.tiles == 0) return 0ull;
+          const unsigned long long mine = s.head().moved ? kSumMoved : 0ull;
+          s.head().moved = 0;
+          return mine;
+        }, sum))
+      return;
+    ++k;
+    if ((sum & (0xffull * kSumMoved)) == 0) break;
+  }
+  // the result is the buffer written last; make it the primary array
+  if (k & 1)
+    for (int v = t; v < n; v += nt) a.labels[v] = __ldcg(a.buffer + v);
+  if (t == 0) a.small[kOutPasses] = k;
+}
+
 // ------------------------------------------------------------------ IrLP ---
 struct IrlpArgs {
   const int *row_ptr, *col;
@@ -643,6 +968,84 @@ const void *prop_kernel_ptr(int lanes) {
   }
 }
 
+// Bytes of an owned launch's counters, and of counters and barrier, in scratch.
+constexpr size_t kOwnedSmall = 256, kOwnedFixed = 256 + sizeof(SumBarrier);
+static_assert(sizeof(int) * kOutWords <= kOwnedSmall && kOwnedFixed % 16 == 0, "scratch layout");
+
+// Facts about a device that the owned kernels' launches need, queried once.
+struct OwnedShape {
+  int grid = 0, smem = 0;  // grid 0: the kernels do not fit this device
+};
+
+OwnedShape owned_shape() {
+  constexpr int kMaxDevices = 64;
+  static std::mutex mu;
+  static OwnedShape known[kMaxDevices];
+  static bool asked[kMaxDevices];
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return OwnedShape();
+  std::lock_guard<std::mutex> lock(mu);
+  if (asked[dev]) return known[dev];
+  OwnedShape s;
+  int sms = 0, most = 0;
+  bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+            cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess;
+  s.smem = (most - 1024) & ~15;
+  for (const void *kernel : {reinterpret_cast<const void *>(&prop_owned_kernel),
+                             reinterpret_cast<const void *>(&irlp_owned_kernel)}) {
+    int per_sm = 0;
+    ok = ok && s.smem >= static_cast<int>(sizeof(StintShared)) &&
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kOwnBlock, s.smem) == cudaSuccess && per_sm > 0;
+  }
+  s.grid = ok ? std::min(sms, kSumBlocks) : 0;
+  cudaGetLastError();
+  asked[dev] = true;
+  known[dev] = s;
+  return s;
+}
+
+// Blocks that own a graph of n vertices, 0 when they cannot.
+int owned_grid(int n) {
+  const OwnedShape s = owned_shape();
+  return s.grid > 1 && n <= (s.grid - 1) * (owner::kMaxVertices - owner::kTile) ? s.grid : 0;
+}
+
+// Words of a mark plane of n vertices: whole tiles.
+int owned_plane(int n) { return (n + owner::kTile - 1) / owner::kTile * owner::kTile; }
+
+OwnedArgs owned_args(const int *row_ptr, const int *col, const float *val, float *labels, float *buffer,
+                     const int *status, const int *gt, int n, float delta, int max_iterations) {
+  OwnedArgs a{};
+  a.g = CsrGraph{row_ptr, col, val, status, gt, n};
+  a.labels = labels;
+  a.buffer = buffer;
+  a.delta = delta;
+  a.max_iter = max_iterations;
+  a.plane = owned_plane(n);
+  a.timeout_ns = 2000000000ull;
+  a.smem_bytes = owned_shape().smem;
+  return a;
+}
+
+int clear_scratch(void *p, size_t bytes, cudaStream_t s) {
+  DLP_CUDA_TRY(cudaMemsetAsync(p, 0, bytes, s));
+  return DLP_OK;
+}
+
+// Launches an owned kernel, waits for it and returns its pass count.
+int launch_owned(const void *kernel, const OwnedArgs &a, int *passes, cudaStream_t s) {
+  OwnedArgs args = a;
+  void *list[] = {&args};
+  DLP_TRY(launch_cooperative(kernel, owned_shape().grid, kOwnBlock, list, a.smem_bytes, s));
+  int host[2] = {0, 0};  // kOutPasses, kOutError
+  DLP_CUDA_TRY(cudaMemcpyAsync(host, a.small, sizeof(host), cudaMemcpyDeviceToHost, s));
+  DLP_CUDA_TRY(cudaStreamSynchronize(s));
+  if (host[kOutError]) return fail(host[kOutError], "propagation failed on the device");
+  *passes = host[kOutPasses];
+  return DLP_OK;
+}
+
 int coop_grid(const void *kernel) {
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return -1;
@@ -661,20 +1064,21 @@ int coop_grid(const void *kernel) {
 using namespace dlp::ref_layout;
 
 // ---------------------------------------------------------------------------
-// Scratch of dlp_iterative_propagation_noalloc: the frontier stamps, the three
-// frontier lists, the counters and the grid barrier of one propagation call on
-// a graph of at most kNoAllocMaxNodes vertices (16 MiB + 1 KiB). It is a
+// Scratch of dlp_iterative_propagation_noalloc: the counters, the barrier, the
+// frontier marks and the frontier list of one propagation call on a graph of at
+// most kNoAllocMaxNodes vertices (16 MiB + 1 KiB at most). It is a
 // file-scope device array, so it exists on every GPU that loads this library,
 // from module load until the process exits, whether or not the entry point is
 // ever called.
 namespace {
 constexpr int kNoAllocMaxNodes = 1 << 20;
 struct NoAllocScratch {
-  unsigned stamp[kNoAllocMaxNodes];
-  int lists[3 * kNoAllocMaxNodes];
-  int small[16];
-  dlp::GridBarrier bar;
+  char fixed[kOwnedFixed];  // counters and barrier, directly before the marks: cleared with them
+  unsigned marks[2 * kNoAllocMaxNodes];
+  int list[kNoAllocMaxNodes];
+  int unused[kNoAllocMaxNodes];
 };
+static_assert(kNoAllocMaxNodes <= 150 * dlp::owner::kMaxVertices, "such graphs run on owned rows");
 }  // namespace
 
 static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
@@ -883,6 +1287,25 @@ int dlp_iterative_propagation(const int *d_row_ptr, const int *d_col_ind, const 
     return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "invalid arguments to dlp_iterative_propagation");
   DLP_TRY(dlp::require_device());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (owned_grid(num_nodes) > 0) {
+    // one block of scratch: counters, barrier, marks (zeroed), list
+    const size_t n = static_cast<size_t>(num_nodes);
+    char *scratch = nullptr;
+    const size_t zeroed = kOwnedFixed + 2 * sizeof(unsigned) * owned_plane(num_nodes);
+    DLP_TRY(tmp_alloc(&scratch, zeroed + sizeof(int) * n, s));
+    OwnedArgs a = owned_args(d_row_ptr, d_col_ind, d_values, d_labels, d_labels_buffer, d_vertex_status, d_gt_class,
+                             num_nodes, delta, max_iterations);
+    a.affected = d_is_affected;
+    a.fast_div = g_launcher_arith.load();
+    a.small = reinterpret_cast<int *>(scratch);
+    a.bar = reinterpret_cast<dlp::SumBarrier *>(scratch + kOwnedSmall);
+    a.marks = reinterpret_cast<unsigned *>(scratch + kOwnedFixed);
+    a.list = reinterpret_cast<int *>(scratch + zeroed);
+    int st = clear_scratch(scratch, zeroed, s);
+    if (st == DLP_OK) st = launch_owned(reinterpret_cast<const void *>(&prop_owned_kernel), a, iterations_used, s);
+    cudaFreeAsync(scratch, s);
+    return st;
+  }
   const size_t n = static_cast<size_t>(num_nodes);
   // both buffers start at the current labels (src/iterativePropagation.cu:268-270)
   DLP_CUDA_TRY(cudaMemcpyAsync(d_labels_buffer, d_labels, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
@@ -960,44 +1383,19 @@ int dlp_iterative_propagation_noalloc(const int *d_row_ptr, const int *d_col_ind
   NoAllocScratch *sc = nullptr;
   DLP_TRY(noalloc_scratch(&sc));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const size_t n = static_cast<size_t>(num_nodes);
-  DLP_CUDA_TRY(cudaMemcpyAsync(d_labels_buffer, d_labels, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
-  // what must start at zero: the stamps in use, the counters, the barrier
-  DLP_CUDA_TRY(cudaMemsetAsync(sc->stamp, 0, sizeof(unsigned) * n, s));
-  DLP_CUDA_TRY(cudaMemsetAsync(sc->small, 0, sizeof(sc->small), s));
-  DLP_CUDA_TRY(cudaMemsetAsync(&sc->bar, 0, sizeof(sc->bar), s));
-  PropArgs a{};
-  a.row_ptr = d_row_ptr;
-  a.col = d_col_ind;
-  a.val = d_values;
-  a.labels = d_labels;
-  a.buffer = d_labels_buffer;
-  a.status = d_vertex_status;
-  a.gt = d_gt_class;
+  if (owned_grid(num_nodes) <= 0) return dlp::fail(DLP_ERR_CUDA, "no room for the propagation kernel's blocks");
+  OwnedArgs a = owned_args(d_row_ptr, d_col_ind, d_values, d_labels, d_labels_buffer, d_vertex_status, d_gt_class,
+                           num_nodes, delta, max_iterations);
   a.affected = d_is_affected;
-  a.n = num_nodes;
-  a.delta = delta;
-  a.max_iter = max_iterations;
-  a.stamp = sc->stamp;
-  a.lists = sc->lists;
-  a.counts = sc->small;
-  a.out = sc->small + 8;
-  a.err = sc->small + 12;
-  a.bar = &sc->bar;
-  a.timeout_ns = 2000000000ull;
   a.fast_div = g_launcher_arith.load();
-  const void *kern = prop_kernel_ptr(8);
-  const int grid = coop_grid(kern);
-  if (grid <= 0) return dlp::fail(DLP_ERR_CUDA, "occupancy query failed");
-  void *args[] = {&a};
-  DLP_TRY(dlp::launch_cooperative(kern, grid, kBlock, args, 0, s));
-  int host[2] = {0, 0};
-  DLP_CUDA_TRY(cudaMemcpyAsync(&host[0], a.out, sizeof(int), cudaMemcpyDeviceToHost, s));
-  DLP_CUDA_TRY(cudaMemcpyAsync(&host[1], a.err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  DLP_CUDA_TRY(cudaStreamSynchronize(s));
-  if (host[1]) return dlp::fail(host[1], "propagation failed on the device");
-  *iterations_used = host[0];
-  return DLP_OK;
+  char *scratch = reinterpret_cast<char *>(sc);
+  a.small = reinterpret_cast<int *>(scratch);
+  a.bar = reinterpret_cast<dlp::SumBarrier *>(scratch + kOwnedSmall);
+  a.marks = sc->marks;
+  a.list = sc->list;
+  // what must start at zero: the counters, the barrier and the marks in use
+  DLP_TRY(clear_scratch(scratch, kOwnedFixed + 2 * sizeof(unsigned) * owned_plane(num_nodes), s));
+  return launch_owned(reinterpret_cast<const void *>(&prop_owned_kernel), a, iterations_used, s);
 }
 
 int dlp_irlp(const int *d_row_ptr, const int *d_col_ind, const float *d_values, float *d_labels,
@@ -1011,6 +1409,18 @@ int dlp_irlp(const int *d_row_ptr, const int *d_col_ind, const float *d_values, 
   DLP_TRY(dlp::require_device());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t n = static_cast<size_t>(num_nodes);
+  if (owned_grid(num_nodes) > 0) {
+    char *scratch = nullptr;
+    DLP_TRY(tmp_alloc(&scratch, kOwnedFixed + sizeof(float) * n, s));
+    OwnedArgs a = owned_args(d_row_ptr, d_col_ind, d_values, d_labels, reinterpret_cast<float *>(scratch + kOwnedFixed),
+                             d_vertex_status, d_gt_class, num_nodes, delta, max_iterations);
+    a.small = reinterpret_cast<int *>(scratch);
+    a.bar = reinterpret_cast<dlp::SumBarrier *>(scratch + kOwnedSmall);
+    int st = clear_scratch(scratch, kOwnedFixed, s);
+    if (st == DLP_OK) st = launch_owned(reinterpret_cast<const void *>(&irlp_owned_kernel), a, iterations_used, s);
+    cudaFreeAsync(scratch, s);
+    return st;
+  }
   float *buffer = nullptr;
   int *small = nullptr;
   dlp::GridBarrier *bar = nullptr;

@@ -38,6 +38,7 @@ constexpr int kMaxRow = kLaneEntries * kLongLanes;
 constexpr unsigned kNoPool = (1u << 15) - 1;    // the row did not fit the pool: read from global memory
 constexpr unsigned kUnmarkable = 0x80000000u;   // pool entry: a neighbour that is never marked
 constexpr unsigned kNoEntry = 0xffffffffu;      // pool entry: soft-deleted
+constexpr int kWideLen = 63, kNoRowLen = 62;    // length codes: longer than 32, not active
 constexpr int kMaxStint = 32000;                // passes of a stint (visits counts 15 bits)
 constexpr unsigned short kWideRow = 0x8000;
 
@@ -80,7 +81,7 @@ struct Store {
   __device__ int n() const { return tiles * kTile; }  // owned vertices
   __device__ Head &head() const { return *reinterpret_cast<Head *>(g_smem); }
   __device__ Local &graph(int i) const { return reinterpret_cast<Local *>(g_smem + kHeadBytes)[i]; }
-  // pool offset (15 bits) | length (6 bits, 63: longer than 32) | graph (10 bits)
+  // pool offset (15 bits) | length (6 bits: kWideLen, kNoRowLen) | graph (10 bits)
   __device__ unsigned &meta(int i) const { return reinterpret_cast<unsigned *>(g_smem + meta_at)[i]; }
   // passes that updated the row; kWideRow: the pass has listed it as a wide row
   __device__ unsigned short &visits(int i) const {
@@ -101,7 +102,7 @@ __device__ __forceinline__ Store store(int bytes, int graphs, int tiles) {
 }
 
 __device__ __forceinline__ unsigned pack(unsigned off, int len, int g) {
-  return off | (static_cast<unsigned>(len > kMaxRow ? 63 : len) << 15) | (static_cast<unsigned>(g) << 21);
+  return off | (static_cast<unsigned>(len) << 15) | (static_cast<unsigned>(g) << 21);
 }
 __device__ __forceinline__ unsigned pool_of(unsigned m) { return m & kNoPool; }
 __device__ __forceinline__ int len_of(unsigned m) { return static_cast<int>((m >> 15) & 63u); }
@@ -124,8 +125,9 @@ __device__ __forceinline__ unsigned flat_of(int i) {
 
 // Rows of the block's vertices into shared memory (head and graphs filled by
 // the caller).
-// Graph: graphs(); nodes(g); row(g, v) {start, length}; markable(g, v);
-// entry(g, at, v, w), v = -1 for an entry that does not count.
+// Graph: graphs(); nodes(g); row(g, v) {start, length}; active(g, v): v can be in
+// a frontier; markable(g, v): v is marked as a neighbour (every active vertex
+// is); entry(g, at, v, w), v = -1 for an entry that does not count.
 template <class Graph>
 __device__ void load(const Store &s, const Graph &gr) {
   const int tid = threadIdx.x, lane = tid & 31;
@@ -140,7 +142,8 @@ __device__ void load(const Store &s, const Graph &gr) {
     }
     const int v = static_cast<int>(flat - s.graph(g).flat);
     int2 ri = make_int2(0, 0);
-    if (v < gr.nodes(g) && gr.markable(g, v)) ri = gr.row(g, v);
+    const bool active = v < gr.nodes(g) && gr.active(g, v);
+    if (active) ri = gr.row(g, v);
     const int len = ri.y;
     // pool room for the warp's rows, one reservation
     const int want = len <= kMaxRow ? len : 0;
@@ -155,7 +158,7 @@ __device__ void load(const Store &s, const Graph &gr) {
     base = __shfl_sync(0xffffffffu, base, 31);
     const int off = base + incl - want;
     const bool fits = off + want <= s.pool_cap;
-    s.meta(i) = pack(fits ? static_cast<unsigned>(off) : kNoPool, len, g);
+    s.meta(i) = pack(fits ? static_cast<unsigned>(off) : kNoPool, active ? (len > kMaxRow ? kWideLen : len) : kNoRowLen, g);
     s.visits(i) = 0;
     if (!fits) continue;  // lanes of the next round reconverge at its first shuffle
     for (int b = 0; b < want; b += kLaneEntries) {
@@ -232,8 +235,8 @@ __device__ __forceinline__ void pool_row(unsigned at, int sub, int len, unsigned
 
 // The row of owned vertex i by LANES lanes (1: up to 8 entries, 4: up to 32).
 // All lanes of the warp call; returns whether the label moved (on every lane of
-// the row).
-template <int LANES, class Graph>
+// the row). MARK: a moved label marks, and the row's visits are counted.
+template <int LANES, bool MARK = true, class Graph>
 __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid, int i, int k, float delta, bool fast,
                                     unsigned *next) {
   const int sub = threadIdx.x & (LANES - 1);
@@ -287,20 +290,24 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
   if (valid & !recip_serves(recip, tl)) nl = updated_label(tw, tl, old, fast);
   const bool moved = valid & (fabsf(nl - old) > delta);
   unsigned *const marks = next + first;
+  if (MARK) {
 #pragma unroll
-  for (int r = 0; r < kLaneEntries; ++r) mark(marks, u[r], moved);
+    for (int r = 0; r < kLaneEntries; ++r) mark(marks, u[r], moved);
+  }
   if (valid && sub == 0) {
     l.lab[(k & 1) ^ 1][v] = nl;
-    ++s.visits(i);
-    s.graph(g).last = k;
-    mark(marks, v, moved);
+    if (MARK) {
+      ++s.visits(i);
+      s.graph(g).last = k;
+      mark(marks, v, moved);
+    }
   }
   return moved;
 }
 
 // A row of more than 32 entries by a warp, from global memory: slots lane + 32 j
 // of 256, then the tree.
-template <class Graph>
+template <bool MARK = true, class Graph>
 __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i, int k, float delta, bool fast,
                                          unsigned *next) {
   const int lane = threadIdx.x & 31;
@@ -342,27 +349,52 @@ __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i,
   const float nl = updated_label(tw, tl, old, fast);
   if (lane == 0) {
     l.lab[(k & 1) ^ 1][v] = nl;
-    ++s.visits(i);
-    s.graph(lg).last = k;
+    if (MARK) {
+      ++s.visits(i);
+      s.graph(lg).last = k;
+    }
   }
   if (!(fabsf(nl - old) > delta)) return false;
-  for (int e = lane; e < ri.y; e += 32) {
-    int u = -1;
-    float w;
-    gr.entry(g, ri.x + e, u, w);
-    if (u >= 0 && gr.markable(g, u)) next[l.flat + u] = 1;
+  if constexpr (MARK) {
+    for (int e = lane; e < ri.y; e += 32) {
+      int u = -1;
+      float w;
+      gr.entry(g, ri.x + e, u, w);
+      if (u >= 0 && gr.markable(g, u)) next[l.flat + u] = 1;
+    }
+    if (lane == 0) next[l.flat + v] = 1;
   }
-  if (lane == 0) next[l.flat + v] = 1;
   return true;
 }
 
-// Kind of the row of marked vertex i in pass k: 0 short, 1 long, 2 wide, 3 past
-// its graph's pass limit.
+// Kind of the row of marked vertex i in pass k: 0 short, 1 long, 2 wide, 3 none
+// (not active, or past its graph's pass limit).
 __device__ __forceinline__ int kind_of(const Store &s, int i, int k) {
   const unsigned m = s.meta(i);
   const int len = len_of(m);
-  if (k >= s.head().first_limit && k >= s.graph(graph_of(m)).limit) return 3;
+  if (len == kNoRowLen || (k >= s.head().first_limit && k >= s.graph(graph_of(m)).limit)) return 3;
   return len <= kLaneEntries ? 0 : len <= kMaxRow ? 1 : 2;
+}
+
+// The rows of a warp's tile, vertices first .. first + 31, each lane with the
+// kind of its own. Returns whether a label moved, on all lanes.
+template <bool MARK, class Graph>
+__device__ __forceinline__ bool tile_rows(const Store &s, const Graph &gr, int first, int kind, int k, float delta,
+                                          bool fast, unsigned *next) {
+  const int lane = threadIdx.x & 31;
+  bool moved = false;
+  if (__any_sync(0xffffffffu, kind == 0))
+    moved = row<1, MARK>(s, gr, kind == 0, first + lane, k, delta, fast, next);
+  unsigned longs = __ballot_sync(0xffffffffu, kind == 1), wides = __ballot_sync(0xffffffffu, kind == 2);
+  while (longs) {  // 8 at a time, the q-th remaining one to the q-th lanes
+    unsigned m = longs;
+    for (int q = lane / kLongLanes; q > 0 && m; --q) m &= m - 1;
+    moved |= row<kLongLanes, MARK>(s, gr, m != 0, first + __ffs(m ? m : longs) - 1, k, delta, fast, next);
+    for (int q = 32 / kLongLanes; q > 0 && longs; --q) longs &= longs - 1;
+  }
+  for (; wides; wides &= wides - 1)
+    moved |= wide_row<MARK>(s, gr, first + __ffs(wides) - 1, k, delta, fast, next);
+  return __any_sync(0xffffffffu, moved);
 }
 
 // A pass of a block that owns at most 32 vertices per warp: every warp runs the
@@ -380,24 +412,23 @@ __device__ __forceinline__ void tile_pass(const Store &s, const Graph &gr, unsig
     kind = kind_of(s, i, k);
     if (kind != 3) each(i);
   }
-  bool moved = false;
-  if (__any_sync(0xffffffffu, kind == 0)) moved = row<1>(s, gr, kind == 0, i, k, delta, fast, next);
-  unsigned longs = __ballot_sync(0xffffffffu, kind == 1), wides = __ballot_sync(0xffffffffu, kind == 2);
+  const bool moved = tile_rows<true>(s, gr, i - lane, kind, k, delta, fast, next);
   const int rows = __popc(__ballot_sync(0xffffffffu, kind != 3));
-  while (longs) {  // 8 at a time, the q-th remaining one to the q-th lanes
-    unsigned m = longs;
-    for (int q = lane / kLongLanes; q > 0 && m; --q) m &= m - 1;
-    const int at = (i - lane) + __ffs(m ? m : longs) - 1;
-    moved |= row<kLongLanes>(s, gr, m != 0, at, k, delta, fast, next);
-    for (int q = 32 / kLongLanes; q > 0 && longs; --q) longs &= longs - 1;
-  }
-  for (; wides; wides &= wides - 1)
-    moved |= wide_row(s, gr, (i - lane) + __ffs(wides) - 1, k, delta, fast, next);
-  moved = __any_sync(0xffffffffu, moved);
-  if (lane == 0) {
+  if (lane == 0 && rows) {
     atomicAdd(&s.head().count, rows);
     if (moved) s.head().moved = 1;
   }
+}
+
+// A pass over all rows of the block (no marks): every active vertex takes the
+// average of its neighbours.
+template <class Graph>
+__device__ __forceinline__ void dense_pass(const Store &s, const Graph &gr, int k, float delta) {
+  const int lane = threadIdx.x & 31;
+  bool moved = false;
+  for (int i = threadIdx.x; i < s.n(); i += blockDim.x)
+    moved |= tile_rows<false>(s, gr, i - lane, kind_of(s, i, k), k, delta, false, nullptr);
+  if (moved && lane == 0) s.head().moved = 1;
 }
 
 // Pass k of the block's vertices, up to the barrier. own: this pass's plane;

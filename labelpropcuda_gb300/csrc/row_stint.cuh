@@ -51,12 +51,14 @@ constexpr int kRepack = 512;               // passes between two looks at the ro
 constexpr int kEager = 8;                  // up to this many warps, every lane gathers before its mark is known
 constexpr unsigned short kNoRow = 0xffff;
 constexpr unsigned long long kEmptyKey = ~0ull;
-constexpr unsigned kMarkable = 1, kWide = 2, kOwned = 4, kVisited = 8, kSwapped = 16;  // Cache::meta bits
+// Cache::meta bits. kMarkable: can be in the frontier. kShown: not read here
+// (what else the caller wants to know about a marked vertex).
+constexpr unsigned kMarkable = 1, kWide = 2, kOwned = 4, kVisited = 8, kSwapped = 16, kShown = 32;
 
 struct Cache {
   unsigned long long key[kSlots];  // (graph << 32) | vertex, kEmptyKey = free
   float lab[2][kSlots + 4];        // [j & 1] is read by stint pass j
-  int mark[2][kSlots + 4];         // [j & 1] is the frontier of stint pass j
+  int mark[2][kSlots + 4];         // [j & 1]: j + 1 where a vertex is marked for stint pass j (see marked())
   unsigned char meta[kSlots + 4];
   unsigned short place[kThreads];  // slot of the row of each thread, kNoRow = none
   unsigned short list[kThreads];   // rows to load
@@ -155,6 +157,11 @@ __device__ __forceinline__ void clear(Cache &c) {
     c.recent = 0;
   }
 }
+
+// Whether slot h is marked for stint pass j. The marks of rows that are held
+// are cleared when the row runs; those of other vertices stay, so their value
+// says for which pass they are.
+__device__ __forceinline__ bool marked(const Cache &c, int h, int j) { return c.mark[j & 1][h] == j + 1; }
 
 // A vertex of the stint's first frontier (pass 0), by one thread.
 template <class Graph>
@@ -310,7 +317,7 @@ __device__ __forceinline__ int4 ld4(unsigned a) {
 // warps per scheduler a branch costs as much as four dependent additions.
 template <int P, bool EAGER>
 __device__ __forceinline__ bool pass(Row &row, unsigned now, unsigned next, unsigned after, bool is_long, bool leader,
-                                     bool in_limit, float delta, bool fast, int k) {
+                                     bool in_limit, float delta, bool fast, int k, int stamp) {
   const int4 ctl = ld4(now);
   const float mark = ld<2 + P>(row.own);
   float x[kEntries], old = 0.0f;
@@ -380,7 +387,7 @@ __device__ __forceinline__ bool pass(Row &row, unsigned now, unsigned next, unsi
       "@pl st.shared.v4.b32 [%20], {%6, %6, %6, %6};\n\t"
       "}" ::"r"(static_cast<int>(act)),
       "r"(static_cast<int>(moved)), "r"(static_cast<int>(row.open)), "r"(static_cast<int>(leader)), "r"(row.own),
-      "f"(nl), "r"(0), "r"(1), "r"(row.at[0]), "r"(row.at[1]), "r"(row.at[2]), "r"(row.at[3]), "r"(row.at[4]),
+      "f"(nl), "r"(0), "r"(stamp), "r"(row.at[0]), "r"(row.at[1]), "r"(row.at[2]), "r"(row.at[3]), "r"(row.at[4]),
       "r"(row.at[5]), "r"(row.at[6]), "r"(row.at[7]), "n"((2 + P) * kPlane), "n"((2 + (P ^ 1)) * kPlane),
       "n"((P ^ 1) * kPlane), "r"(next), "r"(after)
       : "memory");
@@ -405,7 +412,7 @@ __device__ __noinline__ int run_as(Cache &c, Row &kept, int k, int j, int last, 
   auto step = [&](auto parity) {
     constexpr int P = decltype(parity)::value;
     if (RECORD) record(k, k + j_of_k, row);
-    if (!pass<P, EAGER>(row, now, next, after, is_long, leader, k < last, delta, fast, k)) return false;
+    if (!pass<P, EAGER>(row, now, next, after, is_long, leader, k < last, delta, fast, k, k + j_of_k + 2)) return false;
     if (P == 1 && ((k + j_of_k) & 63) == 63) {
       const int jj = (k + j_of_k) & (kRepack - 1);
       if (leader) {
