@@ -1,5 +1,6 @@
 // C ABI plumbing: error reporting, device checks, the problem (input
 // generation) object and small device helpers for bindings.
+#include <atomic>
 #include <cerrno>
 #include <cstdio>
 #include <cstring>
@@ -32,7 +33,14 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
 }
 
 int require_device() {
+  // a device that has passed is not asked again: what it is does not change
+  constexpr int kMaxDevices = 64;
+  static std::atomic<bool> passed[kMaxDevices];
   int dev = 0, count = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices &&
+      passed[dev].load(std::memory_order_relaxed))
+    return DLP_OK;
+  cudaGetLastError();
   cudaError_t e = cudaGetDeviceCount(&count);
   if (e != cudaSuccess || count == 0) {
     cudaGetLastError();
@@ -46,6 +54,7 @@ int require_device() {
     return fail(DLP_ERR_NO_DEVICE, "this build targets sm_103a (GB300); device " +
                                        std::to_string(dev) + " is sm_" + std::to_string(major) +
                                        std::to_string(minor));
+  if (dev >= 0 && dev < kMaxDevices) passed[dev].store(true, std::memory_order_relaxed);
   return DLP_OK;
 }
 

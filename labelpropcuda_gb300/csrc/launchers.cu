@@ -42,9 +42,59 @@ int grid_for(long long items, int per_block) {
   return static_cast<int>(std::max<long long>(1, std::min<long long>(g, 152LL * 32)));
 }
 
+// The launchers' temporaries come from a stream-ordered pool of the library's
+// own, one per device, that holds on to at most kPoolBytes between calls. (The
+// default pool gives everything back to the system at each device
+// synchronisation, and the next call maps it again: 200 us a call for a caller
+// that synchronises the device between calls.) The driver orders its blocks
+// between streams and threads; what a call allocates beyond the limit goes back
+// at the next synchronisation, the rest when the library is unloaded.
+constexpr unsigned long long kPoolBytes = 32ull << 20;
+
+class TmpPools {
+ public:
+  // The current device's pool, or null where there is none (the default pool
+  // serves then).
+  cudaMemPool_t current() {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!asked_[dev]) {
+      asked_[dev] = true;
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      unsigned long long keep = kPoolBytes;
+      if (cudaMemPoolCreate(&pool_[dev], &props) != cudaSuccess) pool_[dev] = nullptr;
+      else cudaMemPoolSetAttribute(pool_[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+      cudaGetLastError();
+    }
+    return pool_[dev];
+  }
+  ~TmpPools() {
+    for (cudaMemPool_t p : pool_)
+      if (p) cudaMemPoolDestroy(p);
+  }
+
+ private:
+  static constexpr int kDevices = 64;
+  std::mutex mu_;
+  bool asked_[kDevices] = {};
+  cudaMemPool_t pool_[kDevices] = {};
+};
+
+TmpPools &tmp_pools() {
+  static TmpPools pools;
+  return pools;
+}
+
 template <class T>
 int tmp_alloc(T **p, size_t count, cudaStream_t s) {
-  DLP_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(p), std::max<size_t>(count, 1) * sizeof(T), s));
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  cudaMemPool_t pool = tmp_pools().current();
+  if (pool) DLP_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), bytes, pool, s));
+  else DLP_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(p), bytes, s));
   return DLP_OK;
 }
 
@@ -128,7 +178,7 @@ __device__ __forceinline__ bool kept_edge(const SparsifyArgs &a, int i, int &u, 
 // between their phases (SumBarrier: @@ us) instead of a launch. A few thousand
 // items per block; small steps take one block, whose barrier is __syncthreads.
 constexpr int kStepBlock = 1024;
-struct StepScratch {       // zeroed before the launch
+struct StepScratch {       // zeroed before the launch of more than one block
   SumBarrier bar;
   int out[16];             // kStep*
   int count[kSumBlocks + 1];  // per block
@@ -137,6 +187,12 @@ enum { kStepError = 0, kStepTotal = 1 };
 
 __shared__ SumState s_step;
 
+// Every step kernel's first statement.
+__device__ __forceinline__ void step_begin(StepScratch *sc) {
+  if (threadIdx.x != 0) return;
+  s_step.gen = 0;
+  if (gridDim.x == 1) sc->out[kStepError] = sc->out[kStepTotal] = 0;
+}
 __device__ __forceinline__ bool step_sync(StepScratch *sc, unsigned long long mine, unsigned long long &sum) {
   return sum_sync(&sc->bar, s_step, &sc->out[kStepError], 2000000000ull, [&] { return mine; }, sum);
 }
@@ -181,7 +237,7 @@ __device__ __forceinline__ int blocks_before(const int *count) {
 // numInserted, :259-263). Nothing is written when an endpoint is invalid.
 __global__ void __launch_bounds__(kStepBlock, 1)
     sparsify_kernel(SparsifyArgs a, StepScratch *sc, int *affected, int mark_limit, int *sub_col, float *sub_val) {
-  if (threadIdx.x == 0) s_step.gen = 0;
+  step_begin(sc);
   const int per = (a.m + gridDim.x - 1) / gridDim.x;
   const int lo = min(static_cast<int>(blockIdx.x) * per, a.m), hi = min(lo + per, a.m);
   bool bad = false;
@@ -243,7 +299,7 @@ struct CcArgs {
 // of 2 million and 700,000 edges: @@ us, against 142 us with five kernels, whose
 // scan of the root bits ran on one block.
 __global__ void __launch_bounds__(kStepBlock, 1) cc_kernel(CcArgs a) {
-  if (threadIdx.x == 0) s_step.gen = 0;
+  step_begin(a.sc);
   const int t = blockIdx.x * kStepBlock + threadIdx.x, nt = gridDim.x * kStepBlock;
   const int words = (a.n + 31) / 32;
   bool bad = false;
@@ -334,7 +390,7 @@ struct InitArgs {
 // src/labelInitialization.cu:59-142 in one launch: supernode weights per
 // component in exact fixed-point sums, then the labels.
 __global__ void __launch_bounds__(kStepBlock, 1) init_kernel(InitArgs a) {
-  if (threadIdx.x == 0) s_step.gen = 0;
+  step_begin(a.sc);
   const int t = blockIdx.x * kStepBlock + threadIdx.x, nt = gridDim.x * kStepBlock;
   for (int i = t; i < 2 * max(a.num_comp, 1); i += nt) a.acc[i] = 0;
   if (!step_sync(a.sc)) return;
@@ -1044,15 +1100,20 @@ int step_blocks() {
   return sms;
 }
 
-// One step kernel over `items`: clears its scratch and launches it; with
+// One step kernel over `items`: clears its scratch (one block does it itself,
+// step_begin) and launches it; with
 // `total` waits and returns kStepTotal.
 int run_step(const void *kernel, long long items, void **args, StepScratch *sc, int *total, cudaStream_t s) {
   constexpr long long kPerBlock = 2048;
   const int most = step_blocks();
   if (most <= 0) return fail(DLP_ERR_CUDA, "device query failed");
   const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>((items + kPerBlock - 1) / kPerBlock, most)));
-  DLP_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(StepScratch), s));
-  DLP_TRY(launch_cooperative(kernel, grid, kStepBlock, args, 0, s));
+  if (grid == 1) {  // no barrier to clear and nothing to be resident with
+    DLP_CUDA_TRY(cudaLaunchKernel(kernel, dim3(1), dim3(kStepBlock), args, 0, s));
+  } else {
+    DLP_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(StepScratch), s));
+    DLP_TRY(launch_cooperative(kernel, grid, kStepBlock, args, 0, s));
+  }
   if (!total) return DLP_OK;
   int host[2] = {0, 0};  // kStepError, kStepTotal
   DLP_CUDA_TRY(cudaMemcpyAsync(host, sc->out, sizeof(host), cudaMemcpyDeviceToHost, s));
