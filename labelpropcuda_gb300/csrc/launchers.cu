@@ -818,27 +818,35 @@ __device__ __noinline__ void small_passes(const OwnedArgs &a, int k0, int listed
 }
 
 // The passes on owned rows from k on until the frontier empties, is small or a
-// limit is reached; not inlined, for its registers. -1: the launch has to end.
+// limit is reached; not inlined, for its registers. TILES: see owned passes of
+// the engine. -1: the launch has to end.
+template <bool TILES>
 __device__ __noinline__ int large_passes(const OwnedArgs &a, owner::Store s, int k, int small_from, bool &empty) {
   owner::Head &h = s.head();
-  // in registers: the launch's arguments are memory here
-  unsigned *const even = a.marks, *const odd = a.marks + a.plane;
-  SumBarrier *const bar = a.bar;
-  int *const err = &a.small[kOutError];
-  const uint64_t timeout = a.timeout_ns;
-  const float delta = a.delta;
-  const bool fast = a.fast_div != 0;
-  const int end = min(a.max_iter, k + owner::kMaxStint);
+  // in shared memory: the launch's arguments are memory here
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    h.marks = a.marks;
+    h.plane = a.plane;
+    h.delta = a.delta;
+    h.fast = a.fast_div;
+    h.budget = min(a.max_iter, k + owner::kMaxStint);
+    h.solo_from = small_from;
+    h.bar = a.bar;
+    h.err = &a.small[kOutError];
+    h.timeout_ns = a.timeout_ns;
+  }
+  __syncthreads();
   unsigned before = 0xffffffffu;
   for (;;) {
     if (s.tiles > 0) {
-      unsigned *own = k & 1 ? odd : even, *next = k & 1 ? even : odd;
+      unsigned *own = h.marks + (k & 1 ? h.plane : 0u), *next = h.marks + (k & 1 ? 0u : h.plane);
       auto each = [](int) {};
-      if (s.n() <= kOwnBlock) owner::tile_pass(s, a.g, own, next, k, delta, fast, each);
-      else owner::pass(s, a.g, own, next, k, delta, fast, each);
+      if (TILES) owner::tile_pass(s, a.g, own, next, k, h.delta, h.fast != 0, each);
+      else owner::pass(s, a.g, own, next, k, h.delta, h.fast != 0, each);
     }
     unsigned long long sum;
-    const bool ok = sum_sync(bar, s_bar, err, timeout, [&]() -> unsigned long long {
+    const bool ok = sum_sync(h.bar, s_bar, h.err, h.timeout_ns, [&]() -> unsigned long long {
       if (s.tiles == 0) return 0ull;
       const unsigned long long mine =
           static_cast<unsigned>((h.count & 0xffff) + (h.count >> 16) + h.wide) | (h.moved ? kSumMoved : 0ull);
@@ -850,8 +858,8 @@ __device__ __noinline__ int large_passes(const OwnedArgs &a, owner::Store s, int
     ++k;
     const unsigned rows = static_cast<unsigned>(sum);
     empty = (sum & (0xffull * kSumMoved)) == 0;
-    if (empty || k >= end) return k;
-    if (max(rows, before) <= kSmallFront && k >= small_from) return k;
+    if (empty || k >= h.budget) return k;
+    if (max(rows, before) <= kSmallFront && k >= h.solo_from) return k;
     before = rows;
   }
 }
@@ -914,7 +922,8 @@ __global__ void __launch_bounds__(kOwnBlock, 1) prop_owned_kernel(const __grid_c
       try_small = false;  // at least one pass on the owned rows
       continue;
     }
-    k = large_passes(a, s, k, small_from, empty);
+    k = s.n() <= kOwnBlock ? large_passes<true>(a, s, k, small_from, empty)
+                           : large_passes<false>(a, s, k, small_from, empty);
     if (k < 0) return;
     try_small = true;
   }

@@ -63,6 +63,9 @@ struct Head {
   int fast;
   int budget, solo_from, stint_end;
   unsigned solo_entry;
+  SumBarrier *bar;
+  int *err;
+  unsigned long long timeout_ns;
 };
 
 // The block's dynamic shared memory: Head, then graph[graphs], and with V =
