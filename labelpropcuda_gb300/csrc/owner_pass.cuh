@@ -68,14 +68,19 @@ struct Head {
   unsigned long long timeout_ns;
 };
 
-// The block's dynamic shared memory: Head, then graph[graphs], and with V =
-// 32 tiles meta[V], visits[V], list[V], pool[cap]. Named by 32-bit offsets
+// The block's dynamic shared memory: Head, then graph[graphs], kinds[tiles], and
+// with V = 32 tiles meta[V], visits[V], list[V], pool[cap]. Named by 32-bit offsets
 // from its start, so that a pass keeps no pointers in registers: a register
 // spilled there is a trip to L2 in every pass, because the barrier's acquire
 // empties L1.
 extern __shared__ __align__(16) unsigned char g_smem[];
 constexpr int kHeadBytes = (sizeof(Head) + 15) & ~15;
 static_assert(sizeof(Local) % 16 == 0, "what follows the graphs stays aligned");
+
+// The active vertices of a tile by the kind of their row, a bit per vertex.
+struct alignas(16) Kinds {
+  unsigned shorts, longs, wides;
+};
 
 struct Store {
   int tiles;     // owned
@@ -84,6 +89,9 @@ struct Store {
   __device__ int n() const { return tiles * kTile; }  // owned vertices
   __device__ Head &head() const { return *reinterpret_cast<Head *>(g_smem); }
   __device__ Local &graph(int i) const { return reinterpret_cast<Local *>(g_smem + kHeadBytes)[i]; }
+  __device__ Kinds &kinds(int tile) const {
+    return reinterpret_cast<Kinds *>(g_smem + meta_at - static_cast<int>(sizeof(Kinds)) * tiles)[tile];
+  }
   // pool offset (15 bits) | length (6 bits: kWideLen, kNoRowLen) | graph (10 bits)
   __device__ unsigned &meta(int i) const { return reinterpret_cast<unsigned *>(g_smem + meta_at)[i]; }
   // passes that updated the row; kWideRow: the pass has listed it as a wide row
@@ -99,7 +107,7 @@ struct Store {
 };
 
 __device__ __forceinline__ Store store(int bytes, int graphs, int tiles) {
-  const int at = kHeadBytes + graphs * static_cast<int>(sizeof(Local));
+  const int at = kHeadBytes + graphs * static_cast<int>(sizeof(Local)) + tiles * static_cast<int>(sizeof(Kinds));
   const int room = (bytes - at - 8 * kTile * tiles) / static_cast<int>(sizeof(int2));
   return Store{tiles, at, min(room, static_cast<int>(kNoPool) - kMaxRow)};
 }
@@ -163,6 +171,11 @@ __device__ void load(const Store &s, const Graph &gr) {
     const bool fits = off + want <= s.pool_cap;
     s.meta(i) = pack(fits ? static_cast<unsigned>(off) : kNoPool, active ? (len > kMaxRow ? kWideLen : len) : kNoRowLen, g);
     s.visits(i) = 0;
+    Kinds kinds;
+    kinds.shorts = __ballot_sync(0xffffffffu, active && len <= kLaneEntries);
+    kinds.longs = __ballot_sync(0xffffffffu, active && len > kLaneEntries && len <= kMaxRow);
+    kinds.wides = __ballot_sync(0xffffffffu, active && len > kMaxRow);
+    if (lane == 0) s.kinds(i / kTile) = kinds;
     if (!fits) continue;  // lanes of the next round reconverge at its first shuffle
     for (int b = 0; b < want; b += kLaneEntries) {
       int u[kLaneEntries];
@@ -379,6 +392,20 @@ __device__ __forceinline__ int kind_of(const Store &s, int i, int k) {
   return len <= kLaneEntries ? 0 : len <= kMaxRow ? 1 : 2;
 }
 
+// The rows that a warp's tile runs in pass k of its marked vertices (a bit
+// each): all but those past their graph's pass limit. All lanes call.
+__device__ __forceinline__ Kinds kinds_of(const Store &s, int tile, unsigned marked, int k) {
+  if (k >= s.head().first_limit) {
+    const bool past = k >= s.graph(graph_of(s.meta(tile * kTile + (threadIdx.x & 31)))).limit;
+    marked &= ~__ballot_sync(0xffffffffu, past);
+  }
+  Kinds c = s.kinds(tile);
+  c.shorts &= marked;
+  c.longs &= marked;
+  c.wides &= marked;
+  return c;
+}
+
 // The rows of a warp's tile, vertices first .. first + 31, each lane with the
 // kind of its own. Returns whether a label moved, on all lanes.
 template <bool MARK, class Graph>
@@ -460,18 +487,16 @@ __device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned *
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) {
       shorts[j] = longs[j] = 0;
-      if (!__any_sync(0xffffffffu, b[j] != 0)) continue;
+      const unsigned marked = __ballot_sync(0xffffffffu, b[j] != 0);
+      if (!marked) continue;
       const int i = base + j * nwarps * 32 + lane;
-      int kind = 3;
-      if (b[j]) {
-        own[flat_of(i)] = 0;
-        kind = kind_of(s, i, k);
-        if (kind != 3) each(i);
-      }
-      shorts[j] = __ballot_sync(0xffffffffu, kind == 0);
-      longs[j] = __ballot_sync(0xffffffffu, kind == 1);
-      add += __popc(shorts[j]) + (__popc(longs[j]) << 16);
-      if (kind == 2) {  // a warp's work each: found again below
+      if (b[j]) own[flat_of(i)] = 0;
+      const Kinds c = kinds_of(s, i / kTile, marked, k);
+      if (((c.shorts | c.longs | c.wides) >> lane) & 1u) each(i);
+      shorts[j] = c.shorts;
+      longs[j] = c.longs;
+      add += __popc(c.shorts) + (__popc(c.longs) << 16);
+      if ((c.wides >> lane) & 1u) {  // a warp's work each: found again below
         atomicAdd(&h.wide, 1);
         s.visits(i) |= kWideRow;
       }
