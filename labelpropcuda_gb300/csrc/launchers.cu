@@ -958,6 +958,10 @@ __global__ void __launch_bounds__(kOwnBlock, 1) irlp_owned_kernel(const __grid_c
   };
   for (int v = t; v < n; v += nt)
     if (!a.g.active(0, v)) a.buffer[v] = fixed(v);
+  if (s.tiles > 0) {
+    __syncthreads();
+    owner::list_all(s);
+  }
   int k = 0;
   while (k < a.max_iter) {
     if (k == 1)

@@ -408,22 +408,22 @@ __device__ __forceinline__ Kinds kinds_of(const Store &s, int tile, unsigned mar
 
 // The rows of a warp's tile, vertices first .. first + 31, each lane with the
 // kind of its own. Returns whether a label moved, on all lanes.
-template <bool MARK, class Graph>
+template <class Graph>
 __device__ __forceinline__ bool tile_rows(const Store &s, const Graph &gr, int first, int kind, int k, float delta,
                                           bool fast, unsigned *next) {
   const int lane = threadIdx.x & 31;
   bool moved = false;
   if (__any_sync(0xffffffffu, kind == 0))
-    moved = row<1, MARK>(s, gr, kind == 0, first + lane, k, delta, fast, next);
+    moved = row<1>(s, gr, kind == 0, first + lane, k, delta, fast, next);
   unsigned longs = __ballot_sync(0xffffffffu, kind == 1), wides = __ballot_sync(0xffffffffu, kind == 2);
   while (longs) {  // 8 at a time, the q-th remaining one to the q-th lanes
     unsigned m = longs;
     for (int q = lane / kLongLanes; q > 0 && m; --q) m &= m - 1;
-    moved |= row<kLongLanes, MARK>(s, gr, m != 0, first + __ffs(m ? m : longs) - 1, k, delta, fast, next);
+    moved |= row<kLongLanes>(s, gr, m != 0, first + __ffs(m ? m : longs) - 1, k, delta, fast, next);
     for (int q = 32 / kLongLanes; q > 0 && longs; --q) longs &= longs - 1;
   }
   for (; wides; wides &= wides - 1)
-    moved |= wide_row<MARK>(s, gr, first + __ffs(wides) - 1, k, delta, fast, next);
+    moved |= wide_row(s, gr, first + __ffs(wides) - 1, k, delta, fast, next);
   return __any_sync(0xffffffffu, moved);
 }
 
@@ -442,7 +442,7 @@ __device__ __forceinline__ void tile_pass(const Store &s, const Graph &gr, unsig
     kind = kind_of(s, i, k);
     if (kind != 3) each(i);
   }
-  const bool moved = tile_rows<true>(s, gr, i - lane, kind, k, delta, fast, next);
+  const bool moved = tile_rows(s, gr, i - lane, kind, k, delta, fast, next);
   const int rows = __popc(__ballot_sync(0xffffffffu, kind != 3));
   if (lane == 0 && rows) {
     atomicAdd(&s.head().count, rows);
@@ -450,15 +450,26 @@ __device__ __forceinline__ void tile_pass(const Store &s, const Graph &gr, unsig
   }
 }
 
-// A pass over all rows of the block (no marks): every active vertex takes the
-// average of its neighbours.
-template <class Graph>
-__device__ __forceinline__ void dense_pass(const Store &s, const Graph &gr, int k, float delta) {
-  const int lane = threadIdx.x & 31;
+// The listed rows, dealt out evenly: ns short ones from the first warp up, 32 to
+// a warp, nl long ones from the last down, 8 to a warp. A step is some 300
+// instructions however many rows it holds, and few full warps issue them sooner
+// than many with a row each. Returns whether one of the lane's labels moved.
+template <bool MARK, class Graph>
+__device__ __forceinline__ bool listed_rows(const Store &s, const Graph &gr, int ns, int nl, int k, float delta,
+                                            bool fast, unsigned *next) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  constexpr int kPer = 32 / kLongLanes;
+  const int n = s.n(), sub = lane / kLongLanes;
   bool moved = false;
-  for (int i = threadIdx.x; i < s.n(); i += blockDim.x)
-    moved |= tile_rows<false>(s, gr, i - lane, kind_of(s, i, k), k, delta, false, nullptr);
-  if (moved && lane == 0) s.head().moved = 1;
+  for (int b = warp * 32; b < ns; b += nwarps * 32) {
+    const bool valid = b + lane < ns;
+    moved |= row<1, MARK>(s, gr, valid, s.list(valid ? b + lane : b), k, delta, fast, next);
+  }
+  for (int b = (nwarps - 1 - warp) * kPer; b < nl; b += nwarps * kPer) {
+    const bool valid = b + sub < nl;
+    moved |= row<kLongLanes, MARK>(s, gr, valid, s.list(n - 1 - (valid ? b + sub : b)), k, delta, fast, next);
+  }
+  return moved;
 }
 
 // Pass k of the block's vertices, up to the barrier. own: this pass's plane;
@@ -517,21 +528,8 @@ __device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned *
     }
   }
   __syncthreads();
-  const int ns = h.count & 0xffff, nl = h.count >> 16, nw = h.wide;
-  bool moved = false;
-  constexpr int kPer = 32 / kLongLanes;
-  const int sub = lane / kLongLanes;
-  // Short rows from the first warp up, 32 to a warp, long ones from the last
-  // down, 8 to a warp: a step is some 300 instructions however many rows it
-  // holds, and few full warps issue them sooner than many with a row each.
-  for (int b = warp * 32; b < ns; b += nwarps * 32) {
-    const bool valid = b + lane < ns;
-    moved |= row<1>(s, gr, valid, s.list(valid ? b + lane : b), k, delta, fast, next);
-  }
-  for (int b = (nwarps - 1 - warp) * kPer; b < nl; b += nwarps * kPer) {
-    const bool valid = b + sub < nl;
-    moved |= row<kLongLanes>(s, gr, valid, s.list(n - 1 - (valid ? b + sub : b)), k, delta, fast, next);
-  }
+  const int nw = h.wide;
+  bool moved = listed_rows<true>(s, gr, h.count & 0xffff, h.count >> 16, k, delta, fast, next);
   if (nw)
     for (int b = warp * 32; b < n; b += nwarps * 32) {
       unsigned todo = __ballot_sync(0xffffffffu, (s.visits(b + lane) & kWideRow) != 0);
@@ -542,6 +540,39 @@ __device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned *
         moved |= wide_row(s, gr, i, k, delta, fast, next);
       }
     }
+  if (__any_sync(0xffffffffu, moved) && lane == 0) h.moved = 1;
+}
+
+// All active rows of the block into the list, once; then dense_pass runs them
+// (no marks): every active vertex takes the average of its neighbours.
+__device__ __forceinline__ void list_all(const Store &s) {
+  const int lane = threadIdx.x & 31, n = s.n();
+  Head &h = s.head();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const Kinds c = s.kinds(i / kTile);
+    const int add = __popc(c.shorts) + (__popc(c.longs) << 16);
+    int at = 0;
+    if (lane == 0) {
+      if (add) at = atomicAdd(&h.count, add);
+      if (c.wides) atomicAdd(&h.wide, 1);
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    const unsigned bit = 1u << lane, below = bit - 1u;
+    if (c.shorts & bit) s.list((at & 0xffff) + __popc(c.shorts & below)) = static_cast<unsigned short>(i);
+    if (c.longs & bit) s.list(n - 1 - (at >> 16) - __popc(c.longs & below)) = static_cast<unsigned short>(i);
+  }
+  __syncthreads();
+}
+
+template <class Graph>
+__device__ __forceinline__ void dense_pass(const Store &s, const Graph &gr, int k, float delta) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  Head &h = s.head();
+  bool moved = listed_rows<false>(s, gr, h.count & 0xffff, h.count >> 16, k, delta, false, nullptr);
+  if (h.wide)
+    for (int tile = warp; tile < s.tiles; tile += nwarps)
+      for (unsigned w = s.kinds(tile).wides; w; w &= w - 1)
+        moved |= wide_row<false>(s, gr, tile * kTile + __ffs(w) - 1, k, delta, false, nullptr);
   if (__any_sync(0xffffffffu, moved) && lane == 0) h.moved = 1;
 }
 
