@@ -1028,12 +1028,11 @@ __device__ __noinline__ void solo_passes(const EngineArgs &e, int k0, int slot) 
     __syncthreads();
   }
   stint::Row row;
-  int k = k0;
+  int j = 0;  // stint pass: launch pass k0 + j
   for (;;) {
-    const int j = k - k0, q = j % 3;
-    const int4 ctl = c.ctl[q];
-    if (ctl.x == 0 || ctl.z != 0 || k >= last) break;
-    if (ctl.y && !stint::load_rows(c, gr, row, j & 1, q, e.fast_div)) {
+    const int4 ctl = c.ctl;
+    if (!stint::goes_on(ctl, j) || j >= last - k0) break;
+    if (stint::needs_rows(ctl, j) && !stint::load_rows(c, gr, row, j, e.fast_div)) {
       if (tid == 0) sc.full = 1;
       break;
     }
@@ -1042,30 +1041,31 @@ __device__ __noinline__ void solo_passes(const EngineArgs &e, int k0, int slot) 
     const int warps = (e.solo & 4) ? ns + nl : stint::kWarps;
     if (!(e.solo & 4) || warp < ns || is_long) {
       const bool leader = tid == (ns > 0 || !(e.solo & 4) ? 0 : kBlock - 32);
-      auto tick = [&](int) {  // time budgets
+      auto tick = [&] {  // time budgets
         const uint64_t now = global_timer_ns();
         const bool slice = e.slice_ns != 0 && now - sc.launch > e.slice_ns;
         if (slice) sc.stop_slice = 1;
         return slice || now - sc.start > kSoloBudgetNs;
       };
-      auto record = [&](int kk, int jj, const stint::Row &r) {
-        const int4 now = c.ctl[jj % 3];
-        if (now.x == 0 || now.y != 0 || now.z != 0 || kk >= last) return;  // the pass will not run
-        if (r.lead && c.mark[jj & 1][r.slot]) {
+      auto record = [&](int jj, const stint::Row &r) {
+        const int4 now = c.ctl;
+        if (!stint::goes_on(now, jj) || stint::needs_rows(now, jj) || jj >= last - k0) return;  // it will not run
+        if (r.lead && stint::marked(c, r.slot, jj)) {
           const GraphRec &gr2 = e.recs[c.key[r.slot] >> 32];
-          const int kg = kk + gr2.ba.pass0;
+          const int kg = k0 + jj + gr2.ba.pass0;
           if (gr2.ba.record && kg < kRecordIters) atomicAdd(&gr2.st.rec_fsizes[kg], 1);
         }
-        if (leader) clear_record(kk + 1, 0, 1);
+        if (leader) clear_record(k0 + jj + 1, 0, 1);
       };
-      const int kk =
-          stint::run(c, row, k, j, last, e.delta, e.fast_div, warps, is_long, leader, tick, rec_any, record);
-      if (leader) c.end = kk;
+      const int end =
+          stint::run(c, row, j, last - k0, e.delta, e.fast_div, warps, is_long, leader, tick, rec_any, record);
+      if (leader) c.end = end;
     }
     __syncthreads();  // the warps without rows wait here
-    if (tid == 0 && warps <= kTeamWarps) sc.team += c.end - k;
-    k = c.end;
+    if (tid == 0 && warps <= kTeamWarps) sc.team += c.end - j;
+    j = c.end;
   }
+  const int k = k0 + j;
   __syncthreads();
   if (tid == 0 && sc.stop_slice) e.ectl->slice_stop = stop_code(e, k);  // the grid resumes at pass k and stops
   // rows that took part: their visit counts and the last pass of their graph
@@ -1075,7 +1075,7 @@ __device__ __noinline__ void solo_passes(const EngineArgs &e, int k0, int slot) 
     BatchCounters *bc = e.recs[g].st.bc;
     if (own) {
       c.meta[row.slot] |= stint::kVisited;
-      atomicMax(&sc.lastpass[g], row.last);
+      atomicMax(&sc.lastpass[g], k0 + row.last);
     }
     add_keyed(own, row.visits * static_cast<unsigned>(row.len), &bc->aff_edges);
     add_keyed(own, row.visits, &bc->front_visits);
@@ -1099,7 +1099,7 @@ __device__ __noinline__ void solo_passes(const EngineArgs &e, int k0, int slot) 
     if (key == stint::kEmptyKey) continue;
     const unsigned meta = c.meta[i];
     const bool visited = (meta & stint::kVisited) != 0;
-    const bool front = stint::marked(c, i, k - k0) && (meta & stint::kMarkable) != 0;
+    const bool front = stint::marked(c, i, j) && (meta & stint::kMarkable) != 0;
     if (!visited && !front) continue;
     const GraphRec &r = e.recs[key >> 32];
     const DevState &s = r.st;

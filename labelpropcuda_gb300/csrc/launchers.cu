@@ -769,12 +769,12 @@ __device__ __noinline__ void small_passes(const OwnedArgs &a, int k0, int listed
   for (int i = tid; i < listed; i += kOwnBlock) stint::seed(c, gr, 0, a.list[i]);
   __syncthreads();
   stint::Row row;
-  int k = k0, full = 0;
+  int j = 0, full = 0;  // stint pass: pass k0 + j
+  const int last = a.max_iter - k0;
   for (;;) {
-    const int j = k - k0, q = j % 3;
-    const int4 ctl = c.ctl[q];
-    if (ctl.x == 0 || ctl.z != 0 || k >= a.max_iter) break;
-    if (ctl.y && !stint::load_rows(c, gr, row, j & 1, q, a.fast_div != 0)) {
+    const int4 ctl = c.ctl;
+    if (!stint::goes_on(ctl, j) || j >= last) break;
+    if (stint::needs_rows(ctl, j) && !stint::load_rows(c, gr, row, j, a.fast_div != 0)) {
       full = 1;
       break;
     }
@@ -782,14 +782,15 @@ __device__ __noinline__ void small_passes(const OwnedArgs &a, int k0, int listed
     const bool is_long = warp >= stint::kWarps - nl;
     if (warp < ns || is_long) {
       const bool leader = tid == (ns > 0 ? 0 : kOwnBlock - 32);
-      auto tick = [&](int) { return global_timer_ns() - sh.start > kStintNs; };
-      const int kk = stint::run(c, row, k, j, a.max_iter, a.delta, a.fast_div != 0, ns + nl, is_long, leader, tick,
-                                false, [](int, int, const stint::Row &) {});
-      if (leader) c.end = kk;
+      auto tick = [&] { return global_timer_ns() - sh.start > kStintNs; };
+      const int end = stint::run(c, row, j, last, a.delta, a.fast_div != 0, ns + nl, is_long, leader, tick, false,
+                                 [](int, const stint::Row &) {});
+      if (leader) c.end = end;
     }
     __syncthreads();  // the warps without rows wait here
-    k = c.end;
+    j = c.end;
   }
+  const int k = k0 + j;
   __syncthreads();
   if (row.visits != 0 && row.lead) c.meta[row.slot] |= stint::kVisited;
   __syncthreads();
@@ -803,7 +804,7 @@ __device__ __noinline__ void small_passes(const OwnedArgs &a, int k0, int listed
       a.labels[v] = c.lab[k0 & 1][i];
       a.buffer[v] = c.lab[(k0 & 1) ^ 1][i];
     }
-    if (stint::marked(c, i, k - k0) && (meta & stint::kShown)) {
+    if (stint::marked(c, i, j) && (meta & stint::kShown)) {
       plane[v] = 1;
       if (meta & stint::kMarkable) front = 1;
     }
@@ -811,7 +812,7 @@ __device__ __noinline__ void small_passes(const OwnedArgs &a, int k0, int listed
   front = __syncthreads_or(front);
   if (tid == 0) {
     a.small[kOutPass] = k;
-    a.small[kOutFull] = full && k - k0 < 256;
+    a.small[kOutFull] = full && j < 256;
     a.small[kOutFront] = front;
     a.small[kOutListed] = 0;
   }

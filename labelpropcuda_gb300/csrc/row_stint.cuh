@@ -15,10 +15,11 @@
 //
 // What bounds a pass: the dependent chain labels -> sum -> division -> stores
 // -> barrier on one or two warps per scheduler, and the issue slots and bank
-// conflicts beyond. Measured with every row marked: 333 cycles for 32 rows of 5
-// entries (1 warp), 396 for 128 (4 warps), 606 for 256 (8), 1,046 for 500 (16),
-// 1,994 for 1,000 (32); with four rows of 12 entries among 32, 398. One lane
-// per short row is the shortest chain, because its sum needs no shuffles.
+// conflicts beyond. Measured with every row marked: 324 cycles for 32 rows of 5
+// entries (1 warp, 81 instructions: 148 cycles of arithmetic latency, 47 of
+// branches, 22 of barrier), 389 for 128 (4 warps), 565 for 256 (8), 1,001 for 500
+// (16); with four rows of 12 entries among 32, 389. One lane per short row is
+// the shortest chain, because its sum needs no shuffles.
 //
 // The stint ends when the frontier empties, when a row longer than 32 entries
 // is marked, when the rows no longer fit the block's lanes or the vertices the
@@ -62,17 +63,18 @@ struct Cache {
   unsigned char meta[kSlots + 4];
   unsigned short place[kThreads];  // slot of the row of each thread, kNoRow = none
   unsigned short list[kThreads];   // rows to load
-  // Indexed by stint pass % 3: {the frontier of the pass is not empty, it
-  // holds a vertex whose row is not held yet (or is too long), the stint has to
-  // end}. The words read by pass j are written during pass j - 1 and cleared
-  // during pass j + 1, so a thread at the top of pass j never races a writer.
-  int4 ctl[3];
+  // Stamps, stint pass + 1: {the last pass with a frontier, the last one whose
+  // frontier holds a vertex without a row here (or with one too long), the first
+  // one that must not run}. They only grow (the third only shrinks), so a thread
+  // still at the top of pass j reads the same verdict from what pass j writes for
+  // pass j + 1, and nothing has to be cleared.
+  alignas(16) int4 ctl;
   int used;                        // vertex-table slots in use
   int overflow;                    // a load found no room
   int num_short, num_long;         // rows held, by kind
   int pending;                     // entries of list
   int recent;                      // lanes whose row took part in the last kRepack passes
-  int end;                         // first pass the last run did not take
+  int end;                         // first stint pass the last run did not take
 };
 
 // A lane's share of a row. Slots are shared-memory addresses of their lab[0]
@@ -88,7 +90,7 @@ struct Row {
   bool open = false;     // a neighbour it can mark has no row here
   bool lead = false;     // the lane that reports the row
   unsigned visits = 0;   // passes that updated the row
-  int last = -1;         // the last of them
+  int last = -1;         // the last of them (stint pass)
 };
 
 __device__ __forceinline__ unsigned shared_address(const void *p) {
@@ -141,7 +143,7 @@ __device__ __forceinline__ void clear(Cache &c) {
   const int tid = threadIdx.x;
   for (int i = tid; i < kSlots; i += kThreads) c.key[i] = kEmptyKey;
   c.place[tid] = kNoRow;
-  if (tid < 3) c.ctl[tid] = make_int4(0, 0, 0, 0);
+  if (tid == 0) c.ctl = make_int4(0, 0, 0x7fffffff, 0);
   if (tid < 2) {
     for (int p = 0; p < 2; ++p) {
       c.lab[p][kPad + tid] = 0.0f;
@@ -158,8 +160,7 @@ __device__ __forceinline__ void clear(Cache &c) {
   }
 }
 
-// Whether slot h is marked for stint pass j. The marks of rows that are held
-// are cleared when the row runs; those of other vertices stay, so their value
+// Whether slot h is marked for stint pass j; marks are not cleared, their value
 // says for which pass they are.
 __device__ __forceinline__ bool marked(const Cache &c, int h, int j) { return c.mark[j & 1][h] == j + 1; }
 
@@ -171,8 +172,8 @@ __device__ __forceinline__ void seed(Cache &c, const Graph &gr, int g, int v) {
   if (h < 0) return;
   if (fresh) fill(c, gr, h, g, v);
   c.mark[0][h] = 1;
-  c.ctl[0].x = 1;
-  c.ctl[0].y = 1;
+  c.ctl.x = 1;
+  c.ctl.y = 1;
 }
 
 __device__ __forceinline__ int short_warps(const Cache &c) { return (c.num_short + 31) / 32; }
@@ -180,20 +181,25 @@ __device__ __forceinline__ int long_warps(const Cache &c) {
   return (c.num_long + 32 / kLongLanes - 1) / (32 / kLongLanes);
 }
 
-// Gives every marked vertex of pass parity p without a row a place and loads
+// What the control words say about stint pass j: its frontier is not empty and
+// no request ends the stint; and whether rows have to be loaded first.
+__device__ __forceinline__ bool goes_on(const int4 &ctl, int j) { return ctl.x > j && ctl.z > j + 1; }
+__device__ __forceinline__ bool needs_rows(const int4 &ctl, int j) { return ctl.y == j + 1; }
+
+// Gives every marked vertex of stint pass j without a row a place and loads
 // its row. Short rows fill the lanes from warp 0 up, long rows those from the
 // last warp down, so a warp holds one kind. All threads of the block call;
 // false: a row is too long or there is no room (the stint has to end here; the
 // marks are unchanged).
 template <class Graph>
-__device__ bool load_rows(Cache &c, const Graph &gr, Row &row, int p, int q, bool fast) {
+__device__ bool load_rows(Cache &c, const Graph &gr, Row &row, int j, bool fast) {
   const unsigned lab0 = shared_address(c.lab[0]);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) c.pending = 0;
-  __syncthreads();  // the need word has been read by every thread
-  if (tid == 0) c.ctl[q].y = 0;
+  __syncthreads();  // the control words have been read by every thread
+  if (tid == 0) c.ctl.y = 0;
   for (int i = tid; i < kSlots; i += kThreads) {
-    if (c.key[i] == kEmptyKey || !c.mark[p][i] || (c.meta[i] & (kMarkable | kOwned)) != kMarkable) continue;
+    if (c.key[i] == kEmptyKey || !marked(c, i, j) || (c.meta[i] & (kMarkable | kOwned)) != kMarkable) continue;
     const int at = atomicAdd(&c.pending, 1);
     if (at < kThreads) c.list[at] = static_cast<unsigned short>(i);
   }
@@ -308,17 +314,17 @@ __device__ __forceinline__ int4 ld4(unsigned a) {
   return x;
 }
 
-// One pass of parity P by a warp that holds rows; false, with nothing done,
+// Stint pass j of parity P by a warp that holds rows; false, with nothing done,
 // when the pass must not run. Eager: all lanes gather at once, whether or not
 // their row is marked, so that the mark, the labels and the control words are
-// one shared-memory latency and nothing branches; the other form reads the
-// marks first, which costs a latency and saves the gathers of warps without a
-// marked row. Stores are predicated, not branched around: with one or two
-// warps per scheduler a branch costs as much as four dependent additions.
+// one shared-memory latency and nothing branches; the other form reads the marks
+// first, which costs a latency and saves the gathers of warps without a marked
+// row. Stores are predicated, not branched around: with one or two warps per
+// scheduler a branch costs as much as four dependent additions.
 template <int P, bool EAGER>
-__device__ __forceinline__ bool pass(Row &row, unsigned now, unsigned next, unsigned after, bool is_long, bool leader,
-                                     bool in_limit, float delta, bool fast, int k, int stamp) {
-  const int4 ctl = ld4(now);
+__device__ __forceinline__ bool pass(Row &row, unsigned control, bool is_long, int last, float delta, bool fast,
+                                     int j) {
+  const int4 ctl = ld4(control);
   const float mark = ld<2 + P>(row.own);
   float x[kEntries], old = 0.0f;
   if (EAGER) {
@@ -326,20 +332,16 @@ __device__ __forceinline__ bool pass(Row &row, unsigned now, unsigned next, unsi
 #pragma unroll
     for (int r = 0; r < kEntries; ++r) x[r] = ld<P>(row.at[r]);
   }
-  const bool go = (ctl.x != 0) & ((ctl.y | ctl.z) == 0) & in_limit;
-  const bool act = go & (__float_as_int(mark) != 0);
+  const bool go = goes_on(ctl, j) & !needs_rows(ctl, j) & (j < last);
+  const bool act = go & (__float_as_int(mark) == j + 1);
   if (!EAGER) {
+    if (!__any_sync(0xffffffffu, act)) return go;
 #pragma unroll
     for (int r = 0; r < kEntries; ++r) x[r] = 0.0f;
-    if (__any_sync(0xffffffffu, act)) {
-      if (act) {
-        old = ld<P>(row.own);
+    if (act) {
+      old = ld<P>(row.own);
 #pragma unroll
-        for (int r = 0; r < kEntries; ++r) x[r] = ld<P>(row.at[r]);
-      }
-    } else {
-      if (leader) asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(after), "r"(0) : "memory");
-      return go;
+      for (int r = 0; r < kEntries; ++r) x[r] = ld<P>(row.at[r]);
     }
   }
 #pragma unroll
@@ -359,79 +361,69 @@ __device__ __forceinline__ bool pass(Row &row, unsigned now, unsigned next, unsi
   if (act & !recip_serves(row.recip, tl)) nl = updated_label(row.total, tl, old, fast);
   const bool moved = act & (fabsf(nl - old) > delta);
   row.visits += act ? 1u : 0u;
-  row.last = act ? k : row.last;
-  // Own mark cleared and label stored; where the label moved, marks for the
-  // row and its neighbours (ground-truth neighbours and empty entries too:
-  // nothing owns them, and a load or the end of the stint leaves them out)
-  // and the words of the next pass. The leader clears those of the pass after.
+  row.last = act ? j : row.last;
+  // The label; and where it moved, marks of pass j + 1 for the row and its
+  // neighbours (ground-truth neighbours and empty entries too: nothing owns
+  // them, and a load or the end of the stint leaves them out) and the control
+  // words.
   asm volatile(
       "{\n\t"
-      ".reg .pred pa, pm, po, pl;\n\t"
+      ".reg .pred pa, pm, po;\n\t"
       "setp.ne.s32 pa, %0, 0;\n\t"
       "setp.ne.s32 pm, %1, 0;\n\t"
       "setp.ne.and.s32 po, %2, 0, pm;\n\t"
-      "setp.ne.s32 pl, %3, 0;\n\t"
-      "@pa st.shared.f32 [%4+%18], %5;\n\t"
-      "@pa st.shared.b32 [%4+%16], %6;\n\t"
-      "@pm st.shared.b32 [%8+%17], %7;\n\t"
-      "@pm st.shared.b32 [%9+%17], %7;\n\t"
-      "@pm st.shared.b32 [%10+%17], %7;\n\t"
-      "@pm st.shared.b32 [%11+%17], %7;\n\t"
-      "@pm st.shared.b32 [%12+%17], %7;\n\t"
-      "@pm st.shared.b32 [%13+%17], %7;\n\t"
-      "@pm st.shared.b32 [%14+%17], %7;\n\t"
-      "@pm st.shared.b32 [%15+%17], %7;\n\t"
-      "@pm st.shared.b32 [%4+%17], %7;\n\t"
-      "@pm st.shared.b32 [%19], %7;\n\t"
-      "@po st.shared.b32 [%19+4], %7;\n\t"
-      "@pl st.shared.v4.b32 [%20], {%6, %6, %6, %6};\n\t"
+      "@pa st.shared.f32 [%3+%15], %4;\n\t"
+      "@pm st.shared.b32 [%6+%14], %5;\n\t"
+      "@pm st.shared.b32 [%7+%14], %5;\n\t"
+      "@pm st.shared.b32 [%8+%14], %5;\n\t"
+      "@pm st.shared.b32 [%9+%14], %5;\n\t"
+      "@pm st.shared.b32 [%10+%14], %5;\n\t"
+      "@pm st.shared.b32 [%11+%14], %5;\n\t"
+      "@pm st.shared.b32 [%12+%14], %5;\n\t"
+      "@pm st.shared.b32 [%13+%14], %5;\n\t"
+      "@pm st.shared.b32 [%3+%14], %5;\n\t"
+      "@pm st.shared.b32 [%16], %5;\n\t"
+      "@po st.shared.b32 [%16+4], %5;\n\t"
       "}" ::"r"(static_cast<int>(act)),
-      "r"(static_cast<int>(moved)), "r"(static_cast<int>(row.open)), "r"(static_cast<int>(leader)), "r"(row.own),
-      "f"(nl), "r"(0), "r"(stamp), "r"(row.at[0]), "r"(row.at[1]), "r"(row.at[2]), "r"(row.at[3]), "r"(row.at[4]),
-      "r"(row.at[5]), "r"(row.at[6]), "r"(row.at[7]), "n"((2 + P) * kPlane), "n"((2 + (P ^ 1)) * kPlane),
-      "n"((P ^ 1) * kPlane), "r"(next), "r"(after)
+      "r"(static_cast<int>(moved)), "r"(static_cast<int>(row.open)), "r"(row.own), "f"(nl), "r"(j + 2),
+      "r"(row.at[0]), "r"(row.at[1]), "r"(row.at[2]), "r"(row.at[3]), "r"(row.at[4]), "r"(row.at[5]),
+      "r"(row.at[6]), "r"(row.at[7]), "n"((2 + (P ^ 1)) * kPlane), "n"((P ^ 1) * kPlane), "r"(control)
       : "memory");
   return go;
 }
 
-// Passes from k (stint pass j) on, by the warps that hold rows; returns the
-// first pass not run. Every exit reads words written before the last barrier,
-// so all warps leave together. tick(k) is called by the leader every 64
-// passes and returns whether the stint has to end; record(k, j, row), when
-// RECORD, by every thread in every pass.
+// Stint passes from j to last - 1 at most, by the warps that hold rows; returns
+// the first one not run. Every exit reads words written before the last
+// barrier, so all warps leave together. tick() is called by the leader every 64
+// passes and returns whether the stint has to end; record(j, row), when RECORD,
+// by every thread in every pass.
 //
 // Not inlined, on a copy of the row: the loop then has the thread's registers
 // to itself (inlined, it spilled).
 template <bool EAGER, bool RECORD, class Tick, class Record>
-__device__ __noinline__ int run_as(Cache &c, Row &kept, int k, int j, int last, float delta, bool fast, int warps,
+__device__ __noinline__ int run_as(Cache &c, Row &kept, int j, int last, float delta, bool fast, int warps,
                                    bool is_long, bool leader, Tick tick, Record record) {
   Row row = kept;
-  const unsigned ctl = shared_address(c.ctl);
-  unsigned now = ctl + 16 * (j % 3), next = ctl + 16 * ((j + 1) % 3), after = ctl + 16 * ((j + 2) % 3);
-  const int j_of_k = j - k;  // stint pass = launch pass + j_of_k
+  const unsigned control = shared_address(&c.ctl);
   auto step = [&](auto parity) {
     constexpr int P = decltype(parity)::value;
-    if (RECORD) record(k, k + j_of_k, row);
-    if (!pass<P, EAGER>(row, now, next, after, is_long, leader, k < last, delta, fast, k, k + j_of_k + 2)) return false;
-    if (P == 1 && ((k + j_of_k) & 63) == 63) {
-      const int jj = (k + j_of_k) & (kRepack - 1);
+    if (RECORD) record(j, row);
+    if (!pass<P, EAGER>(row, control, is_long, last, delta, fast, j)) return false;
+    if (P == 1 && (j & 63) == 63) {
+      const int at = j & (kRepack - 1);
       if (leader) {
         // lanes in use during the kRepack passes up to 64 passes ago
-        const bool repack = jj == 63 && k + j_of_k > kRepack && 2 * (c.recent / 32 + 2) <= warps;
-        if (jj == 63) c.recent = 0;
-        if (tick(k) || repack) asm volatile("st.shared.b32 [%0+8], %1;" ::"r"(next), "r"(1) : "memory");
+        const bool repack = at == 63 && j > kRepack && 2 * (c.recent / 32 + 2) <= warps;
+        if (at == 63) c.recent = 0;
+        if (tick() || repack) asm volatile("st.shared.b32 [%0+8], %1;" ::"r"(control), "r"(j + 2) : "memory");
       }
-      if (jj == kRepack - 1) {
-        const int used = __popc(__ballot_sync(0xffffffffu, row.slot != kIdle && row.last > k - kRepack));
+      if (at == kRepack - 1) {
+        const int used = __popc(__ballot_sync(0xffffffffu, row.slot != kIdle && row.last > j - kRepack));
         if ((threadIdx.x & 31) == 0 && used) atomicAdd(&c.recent, used);
       }
     }
     asm volatile("bar.sync 1, %0;" ::"r"(warps * 32) : "memory");
-    ++k;
-    const unsigned z = now;
-    now = next;
-    next = after;
-    after = z;
+    ++j;
     return true;
   };
   using Even = std::integral_constant<int, 0>;
@@ -441,11 +433,11 @@ __device__ __noinline__ int run_as(Cache &c, Row &kept, int k, int j, int last, 
     }
   kept.visits = row.visits;
   kept.last = row.last;
-  return k;
+  return j;
 }
 
 template <class Tick, class Record>
-__device__ __forceinline__ int run(Cache &c, Row &row, int k, int j, int last, float delta, bool fast, int warps,
+__device__ __forceinline__ int run(Cache &c, Row &row, int j, int last, float delta, bool fast, int warps,
                                    bool is_long, bool leader, Tick tick, bool recorded, Record record) {
   if (row.slot == kIdle) {  // a lane without a row gathers from the pad and is never marked
     const unsigned lab0 = shared_address(c.lab[0]);
@@ -456,9 +448,9 @@ __device__ __forceinline__ int run(Cache &c, Row &row, int k, int j, int last, f
       row.w[r] = 0.0f;
     }
   }
-  if (recorded) return run_as<false, true>(c, row, k, j, last, delta, fast, warps, is_long, leader, tick, record);
-  if (warps <= kEager) return run_as<true, false>(c, row, k, j, last, delta, fast, warps, is_long, leader, tick, record);
-  return run_as<false, false>(c, row, k, j, last, delta, fast, warps, is_long, leader, tick, record);
+  if (recorded) return run_as<false, true>(c, row, j, last, delta, fast, warps, is_long, leader, tick, record);
+  if (warps <= kEager) return run_as<true, false>(c, row, j, last, delta, fast, warps, is_long, leader, tick, record);
+  return run_as<false, false>(c, row, j, last, delta, fast, warps, is_long, leader, tick, record);
 }
 
 }  // namespace stint
