@@ -411,7 +411,7 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
     rh[i].ba.flat = static_cast<unsigned>(vertices);
     vertices += owned_room(rh[i].st.n);
   }
-  const bool owned = vertices <= e->mark_plane;
+  const bool owned = vertices <= e->mark_plane && dlp::engine::owned_fits(e->grid, total, vertices, e->smem_all);
   GraphRec *recs = e->recs_dev + (p ? e->max_graphs : 0);
   DLP_CUDA_TRY(cudaMemcpyAsync(recs, rh, sizeof(GraphRec) * total, cudaMemcpyHostToDevice, e->stream));
   DLP_CUDA_TRY(cudaEventRecord(e->recs_free[p], e->stream));

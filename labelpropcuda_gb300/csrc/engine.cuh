@@ -99,6 +99,8 @@ const void *engine_kernel_ptr(int lanes);
 size_t engine_dynamic_smem();
 // Vertices (in whole tiles) of a launch up to which a grid can own them.
 unsigned owned_limit(int grid);
+// Whether that many graphs with that many vertices fit `smem` bytes of each block.
+bool owned_fits(int grid, int graphs, size_t vertices, size_t smem);
 
 }  // namespace engine
 }  // namespace dlp

@@ -1643,13 +1643,16 @@ __device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_
 // graphs whose frontier is live at k_end continue in a later launch).
 template <int G>
 __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2, int &k_end) {
-  int no_small_at = -1;  // a pass the one-block mode declined goes to the full grid
   int solo_from = 0;     // the one-block mode declined: not tried again before this pass
   bool owned = false;    // the block holds its rows (owned_passes)
   int stint_no = 0;
   int k = 0;
-  // thread 0 of block 0: passes and device time per mode in this launch
-  unsigned long long mp[2] = {0, 0}, mns[2] = {0, 0};  // one block, full grid
+  // passes and device time per mode in this launch (one block, full grid), by
+  // thread 0 of block 0; in shared memory, because in registers they cost the
+  // list passes (launches beyond owned rows) 104 bytes of spills and 3%: 62.8
+  // against 60.7 ms for 14 batches of 4.2 million vertices
+  __shared__ unsigned long long mp[2], mns[2], t_mode;
+  if (c.gtid == 0) mp[0] = mp[1] = mns[0] = mns[1] = 0;
   for (;; ++k) {
     int tn, tw;
     pass_sizes(e, k, pref, pref2, tn, tw);
@@ -1657,9 +1660,9 @@ __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2
     if (e.pass_budget > 0 && k >= e.pass_budget) break;
     if (ld_relaxed_u64(&e.ectl->slice_stop) == stop_code(e, k)) break;
     if (c.gtid == 0) e.ectl->where_pass = k;
-    const bool solo_ok = (e.solo & 1) && tn + tw <= e.solo_entry && k != no_small_at && k >= solo_from;
+    const bool solo_ok = (e.solo & 1) && tn + tw <= e.solo_entry && k >= solo_from;
     if (solo_ok) {
-      const uint64_t ts = c.gtid == 0 ? global_timer_ns() : 0;
+      if (c.gtid == 0) t_mode = global_timer_ns();
       if (blockIdx.x == 0) solo_passes(e, k, stint_no & 1);
       if (!launch_sync(e)) return false;
       const int done = ld_relaxed_i32(&e.ectl->solo_passes[stint_no & 1]);
@@ -1667,23 +1670,23 @@ __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2
       ++stint_no;
       if (c.gtid == 0) {
         mp[0] += done;
-        mns[0] += global_timer_ns() - ts;
+        mns[0] += global_timer_ns() - t_mode;
       }
-      if (done == 0) no_small_at = k;
+      if (done == 0) solo_from = k + 1;  // declined: the full grid's
       // A stint that ran out of room soon would run out again: a load costs
       // several passes, so the frontier stays with the grid for a while.
       if (done < 256 && ld_relaxed_i32(&e.ectl->solo_full[(stint_no - 1) & 1])) solo_from = kk + 256;
       k = kk - 1;  // the loop increment resumes at pass kk
       continue;
     }
-    const uint64_t tp = c.gtid == 0 ? global_timer_ns() : 0;
+    if (c.gtid == 0) t_mode = global_timer_ns();
     if (e.tiles > 0) {
       int kk = k;
       if (!owned_passes(e, k, solo_from, pref, pref2, tn, tw, owned, &kk)) return false;
       owned = true;
       if (c.gtid == 0) {
         mp[1] += kk - k;
-        mns[1] += global_timer_ns() - tp;
+        mns[1] += global_timer_ns() - t_mode;
       }
       k = kk - 1;  // the loop increment resumes at pass kk
       continue;
@@ -1693,7 +1696,7 @@ __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2
     if (!launch_sync(e)) return false;
     if (c.gtid == 0) {
       ++mp[1];
-      mns[1] += global_timer_ns() - tp;
+      mns[1] += global_timer_ns() - t_mode;
     }
   }
   k_end = k;
@@ -1897,6 +1900,11 @@ size_t engine_dynamic_smem() { return sizeof(SoloCache); }
 
 unsigned owned_limit(int grid) {
   return grid > 1 ? static_cast<unsigned>(grid - 1) * (owner::kMaxVertices - owner::kTile) : 0u;
+}
+
+bool owned_fits(int grid, int graphs, size_t vertices, size_t smem) {
+  const size_t tiles = vertices / owner::kTile, blocks = static_cast<size_t>(grid - 1);
+  return vertices <= owned_limit(grid) && owner::bytes_of(graphs, (tiles + blocks - 1) / blocks) <= smem;
 }
 
 const void *engine_kernel_ptr(int lanes) {

@@ -13,16 +13,20 @@
 // acknowledged stores, barrier). A pass over frontier lists takes twice as
 // many (counts, list entry, row start, row, labels, mark atomic, reservation,
 // list store, barrier). Static ownership is what saves them: a row needs no
-// lookup, a mark no answer, and the list of a block no global counter. Scans
-// cost a word per owned vertex and pass, which is why launches beyond
-// kMaxVertices per block use frontier lists instead. On large frontiers the
-// scattered stores bound a pass: the GPU takes 173 G a second of 4-byte ones
-// over 690,000 vertices and 83 G over 50,000, but 107 G and 47 G of single bytes
-// (and 298 G loads), hence words.
+// lookup, a mark no answer, and the list of a block no global counter. On large
+// frontiers the scattered stores bound a pass: the GPU takes 173 G a second of
+// 4-byte ones over 690,000 vertices and 83 G over 50,000, but 107 G and 47 G of
+// single bytes (and 298 G loads), hence words.
 //
 // Measured, microseconds a pass, owned rows against lists: 5,000 vertices of
-// degree 5 4.0 against 5.1, 20,000 of degree 7 4.2 against 6.2, 50,000 of degree
-// 5 4.3 against 7.5 to 8.0, 500,000 of degree 7 6.0 against 16.2.
+// degree 5 3.2 against 5.1, 20,000 of degree 7 3.4 against 6.2, 50,000 of degree
+// 5 3.3 against 7.5 to 8.0, 500,000 of degree 7 5.9 against 16.2.
+//
+// Shared memory ends at 24,576 vertices per block (3.7 million on 151), beyond
+// which launches use frontier lists. Most rows then stay in global memory and a
+// scan reads all words of the graph, yet owned rows are the faster ones: 14
+// batches of 2.6 million vertices of degree 7 take 58.7 against 96.7 ms, and of
+// 3.6 million, mostly with small frontiers, 49.2 against 51.8 ms.
 #pragma once
 
 #include "common.cuh"
@@ -31,7 +35,7 @@ namespace dlp {
 namespace owner {
 
 constexpr int kTile = 32;                       // vertices of a warp's scan step
-constexpr int kMaxVertices = 16384;             // per block
+constexpr int kMaxVertices = 24576;             // per block
 constexpr int kLaneEntries = 8;
 constexpr int kLongLanes = 4;
 constexpr int kMaxRow = kLaneEntries * kLongLanes;
@@ -110,6 +114,12 @@ __device__ __forceinline__ Store store(int bytes, int graphs, int tiles) {
   const int at = kHeadBytes + graphs * static_cast<int>(sizeof(Local)) + tiles * static_cast<int>(sizeof(Kinds));
   const int room = (bytes - at - 8 * kTile * tiles) / static_cast<int>(sizeof(int2));
   return Store{tiles, at, min(room, static_cast<int>(kNoPool) - kMaxRow)};
+}
+
+// Shared memory of a block that owns `tiles` of a launch of `graphs` graphs, less
+// the pool.
+constexpr size_t bytes_of(size_t graphs, size_t tiles) {
+  return kHeadBytes + graphs * sizeof(Local) + tiles * (sizeof(Kinds) + 8 * kTile);
 }
 
 __device__ __forceinline__ unsigned pack(unsigned off, int len, int g) {

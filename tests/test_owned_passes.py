@@ -60,3 +60,33 @@ def test_owned_passes_of_continued_batches(gpu, oracle):
                 assert got[k] == want[k], (i, nxt[i] - 1, k)
             assert eng.labels(g).tobytes() == orcs[i].labels().tobytes(), (i, nxt[i] - 1)
         step += 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3706144, 3706145])  # the most that 151 blocks own, and one more
+def test_owned_passes_up_to_the_limit(gpu, oracle, n):
+    p = dlp.Problem(n, 3, 200, 5, cache_dir="")
+    orc = oracle.OracleRun.from_problem(p, threads=0, max_iterations=6)
+    sess = dlp.Session.from_problem(p, max_iterations=6, small_frontier_solo=0)
+    for b, batch in enumerate(p.batches[:3]):
+        got, want = sess.apply(b, batch), orc.apply(b, batch)
+        for k in EXACT_STATS:
+            assert got[k] == want[k], (b, k)
+        assert sess.labels().tobytes() == orc.labels().tobytes(), b
+
+
+@pytest.mark.gpu
+def test_more_graphs_than_a_block_has_room_for(gpu, oracle):
+    """As many vertices as the blocks own for one graph, but the 600 graphs' own
+    records do not fit beside them."""
+    p = dlp.Problem(6000, 3, 4, 9, cache_dir="")
+    orc = oracle.OracleRun.from_problem(p, threads=4, max_iterations=8)
+    eng = dlp.Engine(600, max_iterations=8, small_frontier_solo=0)
+    ids = [eng.add_problem(p) for _ in range(600)]
+    for b, batch in enumerate(p.batches):
+        want, got = orc.apply(b, batch), eng.step([(g, b, batch) for g in ids])
+        for g, st in zip(ids, got):
+            for k in EXACT_STATS:
+                assert st[k] == want[k], (g, b, k)
+        for g in (ids[0], ids[299], ids[599]):
+            assert eng.labels(g).tobytes() == orc.labels().tobytes(), (g, b)
