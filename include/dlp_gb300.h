@@ -301,14 +301,14 @@ int dlp_engine_stats(dlp_engine *e, int graph_id, int batch_index, dlp_batch_sta
 int dlp_engine_steps(const dlp_engine *e);
 /* Device-side diagnostics after a failed step: out[0] error code, out[1] last
  * phase reached (1..10), out[2] last propagation pass started, out[3] passes
- * of the last one-block / sub-grid stint. */
+ * of the last one-block stint. */
 int dlp_engine_debug(dlp_engine *e, int *out4);
 int dlp_engine_elapsed_ms(dlp_engine *e, int first_step, int last_step, float *ms);
 /* Propagation passes the engine's launches have run so far, by mode, and the
  * device time they took: [0] one block (including [1]), [1] those of
- * them run by at most 16 warps (passes only; their time is counted in [0]), [2] always 0 (the
- * sub-grid mode of earlier versions), [3] the full grid. Diagnostics of where a workload's propagation time goes;
- * cumulative since the engine was made. */
+ * them run by at most 16 warps (passes only; their time is counted in [0]),
+ * [2] always 0 (a mode of earlier versions), [3] the full grid. Diagnostics of
+ * where a workload's propagation time goes; cumulative since the engine was made. */
 int dlp_engine_pass_modes(dlp_engine *e, unsigned long long *passes4, double *seconds4);
 int dlp_session_pass_modes(dlp_session *s, unsigned long long *passes4, double *seconds4);
 int dlp_engine_read_labels(dlp_engine *e, int graph_id, float *host_labels);
@@ -316,13 +316,13 @@ int dlp_engine_artefact(dlp_engine *e, int graph_id, int which, void *host_out, 
                         int64_t *count);
 
 /* Autotuner (no counterpart in the reference, whose launch shapes are fixed).
- * Propagation sends rows of at most 32 live entries to groups of
- * narrow_lanes lanes and longer rows to whole warps, and runs each pass on one
- * block, a 16-block sub-grid or the whole grid by the size of the frontier.
- * The lane width of the short-row bucket, the two frontier thresholds
- * (solo_entry, subgrid_entry) and the persistent grid's blocks per SM are
- * chosen by timing every candidate (lanes 1/4/8 x one-block entry
- * 256/512/1024 x sub-grid entry 1024/2048/4096 x the blocks per SM the build
+ * Propagation runs each pass on one block or the whole grid by the size of the
+ * frontier; in launches of more than 3.7 million vertices it sends rows of at
+ * most 32 live entries to groups of narrow_lanes lanes and longer rows to whole
+ * warps. The lane width of the short-row bucket, the frontier threshold
+ * (solo_entry; subgrid_entry has no effect) and the persistent grid's blocks per
+ * SM are chosen by timing every candidate (lanes 1/4/8 x one-block entry
+ * 256/512/1024 x subgrid_entry 1024/2048/4096 x the blocks per SM the build
  * allows) on a sample the library generates with the reference generator:
  * num_graphs graphs of sizes[i] vertices and average degree degrees[i],
  * `batches` batches each, propagation capped at max_iterations passes per

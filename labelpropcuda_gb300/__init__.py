@@ -495,7 +495,7 @@ class Engine:
 def autotune(sizes: list[int], degrees: list[int], batches: int = 10, max_iterations: int = 2000,
              **config) -> dict:
     """Times every launch-shape candidate (lanes per short row x one-block
-    and sub-grid frontier thresholds x blocks per SM) on a generated sample of
+    frontier threshold x subgrid_entry, which has no effect, x blocks per SM) on a generated sample of
     the given graph sizes and degrees and returns the fastest as
     {"narrow_lanes", "blocks_per_sm", "engine_kw": {solo_entry, subgrid_entry},
     "candidates"}; every candidate gave the same statistics (checked by the

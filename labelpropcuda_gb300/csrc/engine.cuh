@@ -29,7 +29,8 @@ constexpr int kMaxGraphs = 1024;
 // Frontier size below which propagation passes leave the full grid for one
 // block (default 512, at most kSoloEntryMax). Tunable per engine. There is no
 // mode on fewer blocks than all of them in between: with SumBarrier a pass over
-// 600 to 2,000 rows takes 5.1 to 6.2 us on 152 blocks and 7 to 8 us on 16.
+// 600 to 2,000 rows takes 5.1 to 6.2 us on 152 blocks (3.2 to 3.4 on owned rows)
+// and 7 to 8 us on 16.
 constexpr int kSoloEntryDefault = 512;
 constexpr int kSoloEntryMax = 1024;
 constexpr int kSubEntryMax = 4096;  // dlp_config.subgrid_entry, accepted and without effect
@@ -44,7 +45,7 @@ struct GraphRec {
 struct EngineCtl {
   SumBarrier bar;       // all blocks of the launch; zeroed before each launch
   int err;
-  // Hand-back of a solo / sub-grid stint: the pass at which it stopped and the
+  // Hand-back of a one-block stint: the pass at which it stopped and the
   // passes it ran, in slot (stint number & 1), so that the next stint cannot
   // overwrite a value a slow block has yet to read.
   int solo_k[2];

@@ -4,12 +4,14 @@
 //
 // The engine's propagation splits rows into two degree buckets: rows of at
 // most 32 live entries go to groups of `narrow_lanes` lanes (4, 8, 16 or 32;
-// or 1: a lane per row of at most 8 entries), longer rows to whole warps. Each pass also picks its launch mode by the
-// total frontier: one block (up to solo_entry vertices), a 16-block sub-grid
-// (up to subgrid_entry) or the whole grid. The tunables are the lane width of
-// the short-row bucket, the two frontier thresholds and the persistent grid's
-// blocks per SM (one for the 1,024-thread build): the best choice depends on
-// the row lengths and frontier sizes of the workload. The tuner builds a
+// or 1: a lane per row of at most 8 entries), longer rows to whole warps (in
+// launches beyond owned rows; those have a fixed split, owner_pass.cuh). Each
+// pass also picks its launch mode by the total frontier: one block (up to
+// solo_entry vertices) or the whole grid. The tunables are the lane width of the
+// short-row bucket, the frontier threshold and the persistent grid's blocks per
+// SM (one for the 1,024-thread build); subgrid_entry is still a field of every
+// candidate, without effect. The best choice depends on the row lengths and
+// frontier sizes of the workload. The tuner builds a
 // sample workload with the reference generator (graph sizes and degrees given
 // by the caller), times every candidate on it with CUDA events (the engine's
 // own step events), checks that every candidate produced the same statistics
