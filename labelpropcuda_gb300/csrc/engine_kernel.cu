@@ -1691,7 +1691,13 @@ __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2
       k = kk - 1;  // the loop increment resumes at pass kk
       continue;
     }
-    run_pass<G>(e, k, pref, tn, pref2, tw, c.lane, c.gwarp, c.nwarps, c.gtid, c.nthreads);
+    // The thread's place is read again, not kept from before the loop (88 instead
+    // of 156 bytes of spill loads): 48 graphs of 100,000 vertices, 276.4 against
+    // 279.3 ms for 10 batches.
+    int tid;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    const int gtid = blockIdx.x * kBlock + tid, nthreads = gridDim.x * kBlock;
+    run_pass<G>(e, k, pref, tn, pref2, tw, tid & 31, gtid >> 5, nthreads >> 5, gtid, nthreads);
     if (c.gtid == 0 && slice_over(e)) e.ectl->slice_stop = stop_code(e, k + 1);
     if (!launch_sync(e)) return false;
     if (c.gtid == 0) {
