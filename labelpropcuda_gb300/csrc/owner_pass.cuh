@@ -278,7 +278,9 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
   float w[kLaneEntries], x[kLaneEntries];
   pool_row<LANES>(static_cast<unsigned>(__cvta_generic_to_shared(&s.pool(0))) + 8 * (off + sub), sub,
                   off != kNoPool ? len : 0, u, w);
-  if (off == kNoPool) {
+  // Lanes without a row have none to look up either: their vertex may lie after
+  // the graph's last one.
+  if (valid && off == kNoPool) {
     const int start = gr.row(g, static_cast<int>(v)).x;
 #pragma unroll
     for (int r = 0; r < kLaneEntries; ++r) {

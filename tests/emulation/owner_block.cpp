@@ -1,0 +1,106 @@
+// One block's owned passes (csrc/owner_pass.cuh) on the CPU, over a graph that
+// checks every vertex and entry it is asked for.
+//   owner_block remainder   a partial last tile whose rows do not fit the pool
+#include "owner_pass.cuh"
+
+#include <cstdio>
+#include <string>
+
+alignas(16) unsigned char dlp::owner::g_smem[1 << 17];
+
+using namespace dlp::owner;
+
+struct Checked {
+  int n;
+  std::vector<int> start, col;
+  std::vector<float> val;
+  mutable int bad = 0;  // lookups outside the graph
+  int graphs() const { return 1; }
+  int nodes(int) const { return n; }
+  bool vertex(int v) const {
+    const bool ok = v >= 0 && v < n;
+    if (!ok) __atomic_fetch_add(&bad, 1, __ATOMIC_SEQ_CST);
+    return ok;
+  }
+  int2 row(int, int v) const { return vertex(v) ? make_int2(start[v], start[v + 1] - start[v]) : make_int2(0, 0); }
+  bool active(int, int v) const { return vertex(v); }
+  bool markable(int, int v) const { return vertex(v); }
+  void entry(int, int at, int &v, float &w) const {
+    if (at < 0 || at >= start[n]) {
+      __atomic_fetch_add(&bad, 1, __ATOMIC_SEQ_CST);
+      return;
+    }
+    v = col[at];
+    w = val[at];
+  }
+};
+
+// Rows of `len(v)` entries at the vertices after v, weights by position.
+template <class Len>
+Checked graph(int n, Len len) {
+  Checked g;
+  g.n = n;
+  g.start.assign(1, 0);
+  for (int v = 0; v < n; ++v) {
+    for (int e = 0; e < len(v); ++e) {
+      g.col.push_back((v + 1 + e) % n);
+      g.val.push_back(0.25f + 0.5f * static_cast<float>((v + e) % 7));
+    }
+    g.start.push_back(static_cast<int>(g.col.size()));
+  }
+  return g;
+}
+
+struct Run {
+  Checked g;
+  Store s;
+  std::vector<float> lab[2];
+  std::vector<unsigned> marks[2];
+
+  Run(Checked graph_, int pool) : g(std::move(graph_)) {
+    gridDim.x = 2;
+    const int tiles = (g.n + kTile - 1) / kTile;
+    s = store(static_cast<int>(bytes_of(1, tiles) + 8 * pool), 1, tiles);
+    for (int p = 0; p < 2; ++p) {
+      marks[p].assign(tiles * kTile, 0);
+      for (int v = 0; v < g.n; ++v) lab[p].push_back(static_cast<float>(v % 5) / 4.0f);
+    }
+    Head &h = s.head();
+    std::memset(&h, 0, sizeof h);
+    h.first_limit = 0x7fffffff;
+    Local &l = s.graph(0);
+    l.lab[0] = lab[0].data();
+    l.lab[1] = lab[1].data();
+    l.flat = 0;
+    l.limit = 0x7fffffff;
+  }
+  // The average that the pass has to give vertex v from buffer `src`.
+  float average(int src, int v) const {
+    double w = 0, l = 0;
+    for (int e = g.start[v]; e < g.start[v + 1]; ++e) {
+      w += g.val[e];
+      l += static_cast<double>(g.val[e]) * lab[src][g.col[e]];
+    }
+    return static_cast<float>(l / w);
+  }
+};
+
+int main(int argc, char **argv) {
+  const std::string what = argc > 1 ? argv[1] : "";
+  int wrong = 0;
+  if (what == "remainder") {
+    Run r(graph(40, [](int v) { return v % 4 ? 30 : 5; }), 100);
+    for (int v = 0; v < r.g.n; ++v) r.marks[0][v] = 1;
+    run_block(1, 64, [&] {
+      load(r.s, r.g);
+      __syncthreads();
+      tile_pass(r.s, r.g, r.marks[0].data(), r.marks[1].data(), 0, 1e-4f, false, [](int) {});
+    });
+    for (int v = 0; v < r.g.n; ++v) wrong += std::fabs(r.lab[1][v] - r.average(0, v)) > 1e-5f;
+    for (int v = r.g.n; v < 64; ++v) wrong += r.marks[1][v] != 0;
+    std::printf("outside %d wrong %d\n", r.g.bad, wrong);
+  } else {
+    return 2;
+  }
+  return 0;
+}

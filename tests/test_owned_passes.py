@@ -90,3 +90,18 @@ def test_more_graphs_than_a_block_has_room_for(gpu, oracle):
                 assert st[k] == want[k], (g, b, k)
         for g in (ids[0], ids[299], ids[599]):
             assert eng.labels(g).tobytes() == orc.labels().tobytes(), (g, b)
+
+
+@pytest.mark.gpu
+def test_owned_passes_partial_tile_beyond_shared_memory(gpu, oracle):
+    """At most 1,024 vertices per block (a tile per warp), a last tile of 17
+    vertices, and about 30 entries per row, more than the blocks have room for."""
+    p = dlp.Problem(150001, 30, 3, 6, cache_dir="")
+    cap = 25
+    orc = oracle.OracleRun.from_problem(p, threads=0, max_iterations=cap)
+    sess = dlp.Session.from_problem(p, max_iterations=cap, small_frontier_solo=0)
+    for b, batch in enumerate(p.batches):
+        got, want = sess.apply(b, batch), orc.apply(b, batch)
+        for k in EXACT_STATS:
+            assert got[k] == want[k], (b, k)
+        assert sess.labels().tobytes() == orc.labels().tobytes(), b
