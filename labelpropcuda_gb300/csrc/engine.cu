@@ -233,12 +233,25 @@ int grow_graph_scratch(dlp_engine *e, GraphSlot *g, int E, int D) {
     int *nk = nullptr;
     DLP_CUDA_TRY(cudaStreamSynchronize(e->stream));
     DLP_CUDA_TRY(cudaMalloc(&nk, sizeof(int) * cap));
-    if (g->del_keep && g->prev_d > 0)
-      DLP_CUDA_TRY(cudaMemcpy(nk, g->del_keep, sizeof(int) * g->prev_d, cudaMemcpyDeviceToDevice));
+    if (g->del_keep && g->prev_d > 0) {
+      DLP_CUDA_TRY(
+          cudaMemcpyAsync(nk, g->del_keep, sizeof(int) * g->prev_d, cudaMemcpyDeviceToDevice, e->stream));
+      DLP_CUDA_TRY(cudaStreamSynchronize(e->stream));
+    }
     cudaFree(g->del_keep);
     g->del_keep = nk;
     g->keep_cap = cap;
   }
+  return DLP_OK;
+}
+
+// Everything that writes device memory does so on the engine's stream, which does
+// not wait for the default stream: a clear or a copy issued there may come after
+// the step that relies on it. Returns when `src` can be reused.
+int copy_in(dlp_engine *e, void *dst, const void *src, size_t bytes) {
+  if (bytes == 0) return DLP_OK;
+  DLP_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, e->stream));
+  DLP_CUDA_TRY(cudaStreamSynchronize(e->stream));
   return DLP_OK;
 }
 
@@ -260,7 +273,8 @@ void grow_marks(dlp_engine *e) {
   cudaFree(e->marks);
   e->marks = nullptr;
   e->mark_plane = 0;
-  if (cudaMalloc(&e->marks, 8 * want) != cudaSuccess || cudaMemset(e->marks, 0, 8 * want) != cudaSuccess) {
+  if (cudaMalloc(&e->marks, 8 * want) != cudaSuccess ||
+      cudaMemsetAsync(e->marks, 0, 8 * want, e->stream) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(e->marks);
     e->marks = nullptr;
@@ -287,6 +301,7 @@ int reset_graph(dlp_engine *e, GraphSlot *g, int gid) {
   fill_f32_kernel<<<1024, 256, 0, q>>>(d.lab1, 0.5f, n);
   DLP_CUDA_TRY(cudaGetLastError());
   DLP_CUDA_TRY(cudaMemsetAsync(e->ctl_all + gid, 0, sizeof(SessionCtl), q));
+  DLP_CUDA_TRY(cudaMemsetAsync(e->bc_all + gid, 0, sizeof(BatchCounters), q));
   DLP_CUDA_TRY(cudaStreamSynchronize(q));
   g->seq = 0;
   g->prev_d = 0;
@@ -295,7 +310,6 @@ int reset_graph(dlp_engine *e, GraphSlot *g, int gid) {
     g->inflight = false;
     --e->inflight;
   }
-  DLP_CUDA_TRY(cudaMemset(e->bc_all + gid, 0, sizeof(BatchCounters)));
   g->seq_batch.clear();
   g->seq_step.clear();
   return DLP_OK;
@@ -680,9 +694,9 @@ int dlp_engine_create(const dlp_config *cfg_in, int max_graphs, size_t memory_bu
     return bail(st);
   if (cudaMallocHost(&e->progress_host, sizeof(int2) * max_graphs) != cudaSuccess)
     return bail(dlp::fail(DLP_ERR_OUT_OF_MEMORY, "pinned host allocation failed"));
-  if (cudaMemset(e->ectl, 0, sizeof(EngineCtl)) != cudaSuccess ||
-      cudaMemset(e->ctl_all, 0, sizeof(SessionCtl) * max_graphs) != cudaSuccess ||
-      cudaMemset(e->bc_all, 0, sizeof(BatchCounters) * max_graphs) != cudaSuccess)
+  if (cudaMemsetAsync(e->ectl, 0, sizeof(EngineCtl), e->stream) != cudaSuccess ||
+      cudaMemsetAsync(e->ctl_all, 0, sizeof(SessionCtl) * max_graphs, e->stream) != cudaSuccess ||
+      cudaMemsetAsync(e->bc_all, 0, sizeof(BatchCounters) * max_graphs, e->stream) != cudaSuccess)
     return bail(dlp::fail(DLP_ERR_CUDA, "initialisation failed"));
   e->graphs.assign(max_graphs, nullptr);
   e->held.assign(max_graphs, 0);
@@ -742,11 +756,7 @@ int dlp_engine_add_graph(dlp_engine *e, int n, int64_t m, const int *row_ptr, co
   uint8_t *truth = const_cast<uint8_t *>(d.truth);
   int *bmap = const_cast<int *>(d.batch_map);
   int st = DLP_OK;
-  auto up = [&](void *dst, const void *src, size_t bytes) -> int {
-    if (bytes == 0) return DLP_OK;
-    DLP_CUDA_TRY(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
-    return DLP_OK;
-  };
+  auto up = [&](void *dst, const void *src, size_t bytes) { return copy_in(e, dst, src, bytes); };
   if ((st = up(full_row, row_ptr, sizeof(int) * (n + 1)))) return bail(st);
   if (m > 0) {
     int *col_tmp = nullptr;
@@ -914,10 +924,7 @@ int restore_graph(dlp_engine *e, const void *snapshot, size_t bytes, int want, i
   g->prev_d = h.prev_d;  // del_keep is still null, so growing it below copies nothing
   if (bytes < snapshot_bytes(g)) return bail(dlp::fail(DLP_ERR_INVALID_ARGUMENT, "snapshot too short"));
   int st = DLP_OK;
-  auto up = [&](void *dst, const void *src, size_t n) -> int {
-    DLP_CUDA_TRY(cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice));
-    return DLP_OK;
-  };
+  auto up = [&](void *dst, const void *src, size_t n) { return copy_in(e, dst, src, n); };
   if ((st = up(e->ctl_all + gid, p, sizeof(SessionCtl)))) return bail(st);
   p += sizeof(SessionCtl);
   if ((st = up(e->bc_all + gid, p, sizeof(BatchCounters)))) return bail(st);
@@ -982,8 +989,7 @@ int dlp_engine_reset_graph(dlp_engine *e, int graph_id) {
   if (e->marks) DLP_CUDA_TRY(cudaMemsetAsync(e->marks, 0, 8 * static_cast<size_t>(e->mark_plane), e->stream));
   DLP_TRY(reset_graph(e, g, graph_id));
   int zero = 0;
-  DLP_CUDA_TRY(cudaMemcpy(&e->ectl->err, &zero, sizeof(int), cudaMemcpyHostToDevice));
-  return DLP_OK;
+  return copy_in(e, &e->ectl->err, &zero, sizeof(int));
 }
 
 float dlp_engine_tau(const dlp_engine *e, int graph_id) {
