@@ -1460,6 +1460,7 @@ __device__ __forceinline__ void pass_sizes(const EngineArgs &e, int k, int *pref
 
 // The engine's graphs as owned passes read them.
 struct OwnedGraphs {
+  static constexpr bool kCounts = true;
   const EngineArgs &e;
   __device__ int graphs() const { return e.ng; }
   __device__ int nodes(int g) const { return e.recs[g].st.n; }

@@ -665,6 +665,7 @@ constexpr unsigned long long kStintNs = 100000000ull;  // the other blocks wait 
 
 // The caller's arrays as owned passes and stints read them.
 struct CsrGraph {
+  static constexpr bool kCounts = false;  // nothing here reads visits, nor clears them
   const int *row_ptr, *col;
   const float *val;
   const int *status, *gt;
@@ -831,7 +832,7 @@ __device__ __noinline__ int large_passes(const OwnedArgs &a, owner::Store s, int
     h.plane = a.plane;
     h.delta = a.delta;
     h.fast = a.fast_div;
-    h.budget = min(a.max_iter, k + owner::kMaxStint);
+    h.budget = a.max_iter;
     h.solo_from = small_from;
     h.bar = a.bar;
     h.err = &a.small[kOutError];

@@ -43,7 +43,7 @@ constexpr unsigned kNoPool = (1u << 15) - 1;    // the row did not fit the pool:
 constexpr unsigned kUnmarkable = 0x80000000u;   // pool entry: a neighbour that is never marked
 constexpr unsigned kNoEntry = 0xffffffffu;      // pool entry: soft-deleted
 constexpr int kWideLen = 63, kNoRowLen = 62;    // length codes: longer than 32, not active
-constexpr int kMaxStint = 32000;                // passes of a stint (visits counts 15 bits)
+constexpr int kMaxStint = 32000;                // passes between two clears of visits (15 bits)
 constexpr unsigned short kWideRow = 0x8000;
 
 struct Local {           // a graph of the launch
@@ -98,7 +98,8 @@ struct Store {
   }
   // pool offset (15 bits) | length (6 bits: kWideLen, kNoRowLen) | graph (10 bits)
   __device__ unsigned &meta(int i) const { return reinterpret_cast<unsigned *>(g_smem + meta_at)[i]; }
-  // passes that updated the row; kWideRow: the pass has listed it as a wide row
+  // passes that updated the row (Graph::kCounts); kWideRow: the pass has listed it
+  // as a wide row
   __device__ unsigned short &visits(int i) const {
     return reinterpret_cast<unsigned short *>(g_smem + meta_at + 4 * kTile * tiles)[i];
   }
@@ -146,7 +147,8 @@ __device__ __forceinline__ unsigned flat_of(int i) {
 
 // Rows of the block's vertices into shared memory (head and graphs filled by
 // the caller).
-// Graph: graphs(); nodes(g); row(g, v) {start, length}; active(g, v): v can be in
+// Graph: kCounts, whether visits and last passes of the rows are kept (their
+// reader has to clear them every kMaxStint passes); graphs(); nodes(g); row(g, v) {start, length}; active(g, v): v can be in
 // a frontier; markable(g, v): v is marked as a neighbour (every active vertex
 // is); entry(g, at, v, w), v = -1 for an entry that does not count.
 template <class Graph>
@@ -261,7 +263,8 @@ __device__ __forceinline__ void pool_row(unsigned at, int sub, int len, unsigned
 
 // The row of owned vertex i by LANES lanes (1: up to 8 entries, 4: up to 32).
 // All lanes of the warp call; returns whether the label moved (on every lane of
-// the row). MARK: a moved label marks, and the row's visits are counted.
+// the row). MARK: a moved label marks, and (Graph::kCounts) the row's visits are
+// counted.
 template <int LANES, bool MARK = true, class Graph>
 __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid, int i, int k, float delta, bool fast,
                                     unsigned *next) {
@@ -325,8 +328,10 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
   if (valid && sub == 0) {
     l.lab[(k & 1) ^ 1][v] = nl;
     if (MARK) {
-      ++s.visits(i);
-      s.graph(g).last = k;
+      if constexpr (Graph::kCounts) {
+        ++s.visits(i);
+        s.graph(g).last = k;
+      }
       mark(marks, v, moved);
     }
   }
@@ -377,7 +382,7 @@ __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i,
   const float nl = updated_label(tw, tl, old, fast);
   if (lane == 0) {
     l.lab[(k & 1) ^ 1][v] = nl;
-    if (MARK) {
+    if constexpr (MARK && Graph::kCounts) {
       ++s.visits(i);
       s.graph(lg).last = k;
     }

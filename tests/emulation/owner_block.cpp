@@ -1,6 +1,7 @@
 // One block's owned passes (csrc/owner_pass.cuh) on the CPU, over a graph that
 // checks every vertex and entry it is asked for.
 //   owner_block remainder   a partial last tile whose rows do not fit the pool
+//   owner_block counter     rows at the end of their visit counters beside a wide row
 #include "owner_pass.cuh"
 
 #include <cstdio>
@@ -11,6 +12,7 @@ alignas(16) unsigned char dlp::owner::g_smem[1 << 17];
 using namespace dlp::owner;
 
 struct Checked {
+  static constexpr bool kCounts = false;
   int n;
   std::vector<int> start, col;
   std::vector<float> val;
@@ -99,6 +101,29 @@ int main(int argc, char **argv) {
     for (int v = 0; v < r.g.n; ++v) wrong += std::fabs(r.lab[1][v] - r.average(0, v)) > 1e-5f;
     for (int v = r.g.n; v < 64; ++v) wrong += r.marks[1][v] != 0;
     std::printf("outside %d wrong %d\n", r.g.bad, wrong);
+  } else if (what == "counter") {
+    // Vertex 3 runs in pass 0, vertex 0 (40 entries) in pass 1. A reader of the
+    // counters that has not cleared them for 32,767 passes would see this:
+    Run r(graph(96, [](int v) { return v == 0 ? 40 : 5; }), 1000);
+    r.marks[0][3] = 1;
+    run_block(1, 32, [&] {
+      load(r.s, r.g);
+      __syncthreads();
+      if (threadIdx.x == 0) r.s.visits(3) = 0x7fff;
+      __syncthreads();
+      auto each = [](int) {};
+      pass(r.s, r.g, r.marks[0].data(), r.marks[1].data(), 0, 2.0f, false, each);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        r.s.head().count = r.s.head().wide = 0;
+        r.marks[1][0] = 1;
+        r.lab[0][3] = 7.0f;  // what pass 1 must not touch
+      }
+      __syncthreads();
+      pass(r.s, r.g, r.marks[1].data(), r.marks[0].data(), 1, 2.0f, false, each);
+    });
+    wrong += std::fabs(r.lab[0][0] - r.average(1, 0)) > 1e-5f;
+    std::printf("outside %d wrong %d label %.1f\n", r.g.bad, wrong, r.lab[0][3]);
   } else {
     return 2;
   }

@@ -54,3 +54,9 @@ def test_partial_tile_beyond_the_pool(block):
     """40 rows of 5 and of 30 entries, room for 100 entries: the lanes after the last
     vertex look nothing up."""
     assert block("remainder") == "outside 0 wrong 0\n"
+
+
+def test_rows_keep_no_count_that_can_run_over(block):
+    """A row whose visit counter would run over is not taken for one listed as a
+    row of more than 32 entries."""
+    assert block("counter") == "outside 0 wrong 0 label 7.0\n"
