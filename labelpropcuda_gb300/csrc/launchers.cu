@@ -384,20 +384,14 @@ struct InitArgs {
   int I, n;
   long long *acc;  // 2 per component
   int fast_div;
-  StepScratch *sc;
 };
 
-// src/labelInitialization.cu:59-142 in one launch: supernode weights per
-// component in exact fixed-point sums, then the labels.
-__global__ void __launch_bounds__(kStepBlock, 1) init_kernel(InitArgs a) {
-  step_begin(a.sc);
-  const int t = blockIdx.x * kStepBlock + threadIdx.x, nt = gridDim.x * kStepBlock;
-  for (int i = t; i < 2 * max(a.num_comp, 1); i += nt) a.acc[i] = 0;
-  if (!step_sync(a.sc)) return;
-  // A lane per row: 155,000 rows in flight instead of 19,000 with eight lanes
-  // each, and the step is bound by the dependent loads of a row (vertex,
-  // component and row start, entries, classes). Rows beyond kLaneRow entries
-  // are shared by the warp.
+// src/labelInitialization.cu:59-88: supernode weights per component in exact
+// fixed-point sums. A lane per row: 155,000 rows in flight instead of 19,000 with
+// eight lanes each, and the step is bound by the dependent loads of a row (vertex,
+// component and row start, entries, classes). Rows beyond kLaneRow entries are
+// shared by the warp.
+__device__ __forceinline__ void init_weights(const InitArgs &a, int t, int nt) {
   constexpr int kLaneRow = 64, kAhead = 4;
   const int lane = threadIdx.x & 31;
   auto add = [&](int c, long long q0, long long q1) {
@@ -452,7 +446,10 @@ __global__ void __launch_bounds__(kStepBlock, 1) init_kernel(InitArgs a) {
       if (lane == 0) add(cq, p0, p1);
     }
   }
-  if (!step_sync(a.sc)) return;
+}
+
+// src/labelInitialization.cu:99-142.
+__device__ __forceinline__ void init_labels(const InitArgs &a, int t, int nt) {
   for (int i = t; i < a.I; i += nt) {
     const int u = a.ins[i];
     if (!in_range(u, a.n)) continue;
@@ -466,6 +463,23 @@ __global__ void __launch_bounds__(kStepBlock, 1) init_kernel(InitArgs a) {
     const float den = w0 + w1;
     a.labels[u] = den > 1e-10f ? quotient(w1, den, a.fast_div) : 0.5f;
   }
+}
+
+// The step returns nothing to the host, so nothing in it may fail on the device:
+// two ordinary launches, no grid barrier whose wait could run out unseen. What
+// one block takes is one launch.
+__global__ void __launch_bounds__(kStepBlock, 1) init_weights_kernel(InitArgs a) {
+  init_weights(a, blockIdx.x * kStepBlock + threadIdx.x, gridDim.x * kStepBlock);
+}
+__global__ void __launch_bounds__(kStepBlock, 1) init_labels_kernel(InitArgs a) {
+  init_labels(a, blockIdx.x * kStepBlock + threadIdx.x, gridDim.x * kStepBlock);
+}
+__global__ void __launch_bounds__(kStepBlock, 1) init_kernel(InitArgs a) {
+  for (int i = threadIdx.x; i < 2 * max(a.num_comp, 1); i += kStepBlock) a.acc[i] = 0;
+  __syncthreads();
+  init_weights(a, threadIdx.x, kStepBlock);
+  __syncthreads();
+  init_labels(a, threadIdx.x, kStepBlock);
 }
 
 // ------------------------------------------------------- propagation -------
@@ -1115,26 +1129,34 @@ int step_blocks() {
   return sms;
 }
 
-// One step kernel over `items`: clears its scratch (one block does it itself,
-// step_begin) and launches it; with
-// `total` waits and returns kStepTotal.
-int run_step(const void *kernel, long long items, void **args, StepScratch *sc, int *total, cudaStream_t s) {
+// Blocks of a step over `items`, 0 with an error.
+int step_grid(long long items) {
   constexpr long long kPerBlock = 2048;
   const int most = step_blocks();
-  if (most <= 0) return fail(DLP_ERR_CUDA, "device query failed");
-  const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>((items + kPerBlock - 1) / kPerBlock, most)));
+  if (most <= 0) fail(DLP_ERR_CUDA, "device query failed");
+  return static_cast<int>(std::min<long long>(std::max<long long>((items + kPerBlock - 1) / kPerBlock, 1), most));
+}
+
+// One step kernel over `items`: clears its scratch (one block does it itself,
+// step_begin), launches it, waits and returns kStepTotal. `invalid`: what
+// DLP_ERR_INVALID_ARGUMENT from the device means.
+int run_step(const void *kernel, const char *what, const char *invalid, long long items, void **args, StepScratch *sc,
+             int *total, cudaStream_t s) {
+  const int grid = step_grid(items);
+  if (grid <= 0) return DLP_ERR_CUDA;
   if (grid == 1) {  // no barrier to clear and nothing to be resident with
     DLP_CUDA_TRY(cudaLaunchKernel(kernel, dim3(1), dim3(kStepBlock), args, 0, s));
   } else {
     DLP_CUDA_TRY(cudaMemsetAsync(sc, 0, sizeof(StepScratch), s));
     DLP_TRY(launch_cooperative(kernel, grid, kStepBlock, args, 0, s));
   }
-  if (!total) return DLP_OK;
   int host[2] = {0, 0};  // kStepError, kStepTotal
   DLP_CUDA_TRY(cudaMemcpyAsync(host, sc->out, sizeof(host), cudaMemcpyDeviceToHost, s));
   DLP_CUDA_TRY(cudaStreamSynchronize(s));
+  if (host[kStepError] == DLP_ERR_INVALID_ARGUMENT) return fail(host[kStepError], invalid);
+  if (host[kStepError]) return fail(host[kStepError], std::string(what) + " failed on the device");
   *total = host[kStepTotal];
-  return host[kStepError];
+  return DLP_OK;
 }
 
 // Bytes of an owned launch's counters, and of counters and barrier, in scratch.
@@ -1335,9 +1357,9 @@ int dlp_build_sparsified_subgraph(int *d_row_ptr, int *d_col_ind, float *d_value
   int mark_limit = num_inserted;
   void *args[] = {&a, &sc, &d_is_affected, &mark_limit, &d_sub_col_ind, &d_sub_values};
   int total = 0;
-  const int st = run_step(reinterpret_cast<const void *>(&sparsify_kernel), num_new_edges, args, sc, &total, s);
+  const int st = run_step(reinterpret_cast<const void *>(&sparsify_kernel), "sparsification",
+                          "edge endpoint out of range", num_new_edges, args, sc, &total, s);
   cudaFreeAsync(sc, s);
-  if (st == DLP_ERR_INVALID_ARGUMENT) return dlp::fail(st, "edge endpoint out of range");
   DLP_TRY(st);
   *num_sub_edges = total;
   return DLP_OK;
@@ -1375,9 +1397,9 @@ int dlp_connected_components(const int *d_edge_src, const int *d_edge_dst, int n
   void *args[] = {&a};
   int total = 0;
   const long long items = std::max<long long>(std::max(num_edges, num_inserted), num_nodes / 4);
-  const int st = run_step(reinterpret_cast<const void *>(&cc_kernel), items, args, sc, &total, s);
+  const int st = run_step(reinterpret_cast<const void *>(&cc_kernel), "connected components",
+                          "connected components failed on the device", items, args, sc, &total, s);
   cudaFreeAsync(scratch, s);
-  if (st == DLP_ERR_INVALID_ARGUMENT) return dlp::fail(st, "connected components failed on the device");
   DLP_TRY(st);
   *num_components = total;
   return DLP_OK;
@@ -1396,17 +1418,27 @@ int dlp_label_initialization(const int *d_row_ptr, const int *d_col_ind, const f
   DLP_TRY(dlp::require_device());
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t nc = static_cast<size_t>(std::max(num_components, 1));
-  char *scratch = nullptr;
-  DLP_TRY(tmp_alloc(&scratch, sizeof(StepScratch) + 2 * sizeof(long long) * nc, s));
-  StepScratch *sc = reinterpret_cast<StepScratch *>(scratch);
-  InitArgs a{d_row_ptr, d_col_ind, d_values, d_labels, d_component_id, num_components, d_gt_class, d_inserted_nodes,
-             num_inserted, num_nodes, reinterpret_cast<long long *>(scratch + sizeof(StepScratch)),
-             g_launcher_arith.load(), sc};
-  void *args[] = {&a};
-  const int st =
-      run_step(reinterpret_cast<const void *>(&init_kernel), std::max<long long>(num_inserted, nc), args, sc, nullptr, s);
-  cudaFreeAsync(scratch, s);
-  return st;
+  const int grid = step_grid(std::max<long long>(num_inserted, nc));
+  if (grid <= 0) return DLP_ERR_CUDA;
+  long long *acc = nullptr;
+  DLP_TRY(tmp_alloc(&acc, 2 * nc, s));
+  const InitArgs a{d_row_ptr,  d_col_ind,        d_values,     d_labels,  d_component_id, num_components,
+                   d_gt_class, d_inserted_nodes, num_inserted, num_nodes, acc,            g_launcher_arith.load()};
+  cudaError_t e = cudaSuccess;
+  if (grid == 1) {
+    init_kernel<<<1, kStepBlock, 0, s>>>(a);
+    e = cudaGetLastError();
+  } else {
+    e = cudaMemsetAsync(acc, 0, 2 * nc * sizeof(long long), s);
+    if (e == cudaSuccess) {
+      init_weights_kernel<<<grid, kStepBlock, 0, s>>>(a);
+      init_labels_kernel<<<grid, kStepBlock, 0, s>>>(a);
+      e = cudaGetLastError();
+    }
+  }
+  cudaFreeAsync(acc, s);
+  DLP_CUDA_TRY(e);
+  return DLP_OK;
 }
 
 int dlp_iterative_propagation(const int *d_row_ptr, const int *d_col_ind, const float *d_values, float *d_labels,

@@ -81,3 +81,37 @@ def test_engine_writes_on_its_own_stream_only(runtime):
     streams = {s for _, s in ops}
     assert len(ops) > 40 and len(streams) == 1 and "default" not in streams, ops
     eng.close()
+
+
+def arrays(*counts):
+    return [dlp.DeviceArray(np.zeros(c, np.int32)) for c in counts]
+
+
+@pytest.mark.parametrize("edges", [10, 10000])  # one block, several
+@pytest.mark.parametrize("status", [N.DLP_ERR_TIMEOUT, N.DLP_ERR_INVALID_ARGUMENT])
+def test_step_launchers_report_what_failed_on_the_device(runtime, edges, status):
+    a = arrays(*[2 * edges] * 8)
+    x, y = ctypes.c_int(0), ctypes.c_int(0)
+    runtime.result(status, 5)
+    with pytest.raises(dlp.DlpError, match="[a-z]{4}") as e:
+        N.check(N.lib().dlp_connected_components(a[0].ptr, a[1].ptr, edges, a[2].ptr, edges, a[3].ptr, ctypes.byref(x),
+                                                 edges, None))
+    assert e.value.status == status
+    runtime.result(status, 5)
+    with pytest.raises(dlp.DlpError, match="[a-z]{4}") as e:
+        N.check(N.lib().dlp_build_sparsified_subgraph(
+            None, None, None, a[0].ptr, None, a[1].ptr, a[2].ptr, a[3].ptr, edges, a[4].ptr, edges, a[5].ptr, 0.5, None,
+            a[6].ptr, a[7].ptr, ctypes.byref(x), ctypes.byref(y), None))
+    assert e.value.status == status
+
+
+@pytest.mark.parametrize("inserted", [10, 10000])
+def test_label_initialisation_cannot_fail_unseen(runtime, inserted):
+    """It returns without waiting for the device, so it may hold no wait of a grid
+    barrier that can run out there."""
+    a = arrays(*[inserted + 1] * 6)
+    runtime.log()
+    N.check(N.lib().dlp_label_initialization(a[0].ptr, a[1].ptr, a[2].ptr, a[3].ptr, None, a[4].ptr, inserted, a[5].ptr,
+                                             inserted, a[0].ptr, inserted, None))
+    ops = [x[0] for x in runtime.log()]
+    assert ops and set(ops) <= {"launch", "clear"}
