@@ -251,6 +251,10 @@ int dlp_engine_create(const dlp_config *cfg, int max_graphs, size_t memory_budge
 int dlp_engine_destroy(dlp_engine *e);
 /* Device bytes a graph of this size occupies once added (admission). */
 size_t dlp_engine_graph_bytes(int num_nodes, int64_t num_edges, int with_truth, int with_batch_map, int record);
+/* Bytes of the resident graphs. Frontier marks (8 bytes a vertex, for up to 3.7
+ * million vertices) come on top: within a budget they take only what it leaves
+ * over, and give way to a graph that needs it. Without them propagation gives the
+ * same results over frontier lists. */
 size_t dlp_engine_bytes_in_use(const dlp_engine *e);
 /* Uploads a graph (same arrays as dlp_session_create); fails with
  * DLP_ERR_OUT_OF_MEMORY when it would exceed the budget. */

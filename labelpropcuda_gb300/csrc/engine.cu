@@ -159,6 +159,7 @@ struct dlp_engine {
   int2 *progress_host = nullptr;    // pinned copy
   unsigned *marks = nullptr;   // two planes of frontier marks (owned passes), all zero between stints
   unsigned mark_plane = 0;          // words of a plane
+  bool marks_off = false;           // a server's budget has no room for them
   int inflight = 0;                 // graphs whose batch continues in a later step
   std::vector<int> last_finished;   // graphs whose batch ended in the last sliced step
 
@@ -261,26 +262,50 @@ size_t owned_room(int n) {
   return (static_cast<size_t>(n) + t - 1) / t * t;
 }
 
+size_t mark_bytes(const dlp_engine *e) { return 8 * static_cast<size_t>(e->mark_plane); }
+
+void drop_marks(dlp_engine *e) {
+  if (e->marks) cudaStreamSynchronize(e->stream);
+  cudaFree(e->marks);
+  e->marks = nullptr;
+  e->mark_plane = 0;
+}
+
 // Mark planes for a launch over all resident graphs, as far as a grid can own
 // their vertices; sized when graphs are added, so that steps allocate nothing.
-// Without them (no memory, or a larger launch) passes run over frontier lists.
+// They take only memory that the budget leaves over, and give way to a graph that
+// needs it (with_room). Without them (no memory, or a larger launch) passes run
+// over frontier lists.
 void grow_marks(dlp_engine *e) {
   size_t want = 0;
   for (GraphSlot *g : e->graphs)
     if (g) want += owned_room(g->n);
   want = std::min<size_t>(want, dlp::engine::owned_limit(e->grid));
-  if (want <= e->mark_plane || cudaStreamSynchronize(e->stream) != cudaSuccess) return;
-  cudaFree(e->marks);
-  e->marks = nullptr;
-  e->mark_plane = 0;
+  if (e->marks_off || want <= e->mark_plane || (e->budget > 0 && e->used + 8 * want > e->budget) ||
+      cudaStreamSynchronize(e->stream) != cudaSuccess)
+    return;
+  drop_marks(e);
   if (cudaMalloc(&e->marks, 8 * want) != cudaSuccess ||
       cudaMemsetAsync(e->marks, 0, 8 * want, e->stream) != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(e->marks);
-    e->marks = nullptr;
+    drop_marks(e);
     return;
   }
   e->mark_plane = static_cast<unsigned>(want);
+}
+
+// place(), which makes a graph of `need` bytes resident; the mark planes give way
+// to it, within the budget and on a full device.
+template <class Place>
+int with_room(dlp_engine *e, size_t need, Place place) {
+  if (e->budget > 0 && e->used + need + mark_bytes(e) > e->budget) drop_marks(e);
+  int st = place();
+  if (st == DLP_ERR_OUT_OF_MEMORY && e->marks) {
+    drop_marks(e);
+    dlp::clear_error();
+    st = place();
+  }
+  return st;
 }
 
 int reset_graph(dlp_engine *e, GraphSlot *g, int gid) {
@@ -610,6 +635,12 @@ int find_seq(GraphSlot *g, int batch) {
 
 }  // namespace
 
+void dlp::engine::fit_marks(dlp_engine *e, size_t room) {
+  if (mark_bytes(e) <= room) return;
+  drop_marks(e);
+  e->marks_off = true;
+}
+
 extern "C" {
 
 void dlp_config_default(dlp_config *cfg) {
@@ -715,33 +746,10 @@ size_t dlp_engine_graph_bytes(int num_nodes, int64_t num_edges, int with_truth, 
 
 size_t dlp_engine_bytes_in_use(const dlp_engine *e) { return e ? e->used : 0; }
 
-int dlp_engine_add_graph(dlp_engine *e, int n, int64_t m, const int *row_ptr, const int *col_ind,
-                         const float *values, const float *true_labels, const int *vertex_batch_map,
-                         int *graph_id) {
-  dlp::clear_error();
-  if (!e || !graph_id) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "null argument");
-  *graph_id = -1;
-  if (n <= 0 || m < 0 || m > 0x7fffffffLL || !row_ptr || (m > 0 && (!col_ind || !values)))
-    return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "invalid graph arrays");
-  if (row_ptr[0] != 0 || row_ptr[n] != m)
-    return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "row_ptr must start at 0 and end at num_edges");
-  for (int i = 0; i < n; ++i)
-    if (row_ptr[i + 1] < row_ptr[i]) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "row_ptr not monotone");
-  for (int64_t k = 0; k < m; ++k)
-    if (col_ind[k] >= n) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "col_ind out of range");
-  const size_t need = graph_bytes(n, m, true_labels != nullptr, vertex_batch_map != nullptr, e->cfg.record != 0);
-  if (e->budget > 0 && e->used + need > e->budget)
-    return dlp::fail(DLP_ERR_OUT_OF_MEMORY, "graph does not fit the engine's device-memory budget (" +
-                                                std::to_string(e->used + need) + " > " + std::to_string(e->budget) +
-                                                " bytes)");
-  int gid = -1;
-  for (int i = 0; i < e->max_graphs; ++i)
-    if (!e->graphs[i] && !e->held[i]) {
-      gid = i;
-      break;
-    }
-  if (gid < 0) return dlp::fail(DLP_ERR_OUT_OF_MEMORY, "the engine holds max_graphs graphs already");
-  DLP_CUDA_TRY(cudaSetDevice(e->device));
+namespace {
+// Makes a graph resident under the free id `gid`.
+int place_graph(dlp_engine *e, int gid, int n, int64_t m, const int *row_ptr, const int *col_ind, const float *values,
+                const float *true_labels, const int *vertex_batch_map) {
   GraphSlot *g = nullptr;
   DLP_TRY(alloc_graph(e, n, m, true_labels != nullptr, vertex_batch_map != nullptr, gid, &g));
   g->tau = e->cfg.tau < 0.0f ? dlp_mean_edge_weight(m, col_ind, values) : e->cfg.tau;
@@ -788,6 +796,40 @@ int dlp_engine_add_graph(dlp_engine *e, int n, int64_t m, const int *row_ptr, co
   e->graphs[gid] = g;
   e->used += g->bytes;
   grow_marks(e);
+  return DLP_OK;
+}
+}  // namespace
+
+int dlp_engine_add_graph(dlp_engine *e, int n, int64_t m, const int *row_ptr, const int *col_ind,
+                         const float *values, const float *true_labels, const int *vertex_batch_map,
+                         int *graph_id) {
+  dlp::clear_error();
+  if (!e || !graph_id) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "null argument");
+  *graph_id = -1;
+  if (n <= 0 || m < 0 || m > 0x7fffffffLL || !row_ptr || (m > 0 && (!col_ind || !values)))
+    return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "invalid graph arrays");
+  if (row_ptr[0] != 0 || row_ptr[n] != m)
+    return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "row_ptr must start at 0 and end at num_edges");
+  for (int i = 0; i < n; ++i)
+    if (row_ptr[i + 1] < row_ptr[i]) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "row_ptr not monotone");
+  for (int64_t k = 0; k < m; ++k)
+    if (col_ind[k] >= n) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "col_ind out of range");
+  const size_t need = graph_bytes(n, m, true_labels != nullptr, vertex_batch_map != nullptr, e->cfg.record != 0);
+  if (e->budget > 0 && e->used + need > e->budget)
+    return dlp::fail(DLP_ERR_OUT_OF_MEMORY, "graph does not fit the engine's device-memory budget (" +
+                                                std::to_string(e->used + need) + " > " + std::to_string(e->budget) +
+                                                " bytes)");
+  int gid = -1;
+  for (int i = 0; i < e->max_graphs; ++i)
+    if (!e->graphs[i] && !e->held[i]) {
+      gid = i;
+      break;
+    }
+  if (gid < 0) return dlp::fail(DLP_ERR_OUT_OF_MEMORY, "the engine holds max_graphs graphs already");
+  DLP_CUDA_TRY(cudaSetDevice(e->device));
+  DLP_TRY(with_room(e, need, [&] {
+    return place_graph(e, gid, n, m, row_ptr, col_ind, values, true_labels, vertex_batch_map);
+  }));
   *graph_id = gid;
   return DLP_OK;
 }
@@ -873,35 +915,8 @@ int dlp_engine_snapshot(dlp_engine *e, int graph_id, void *out, size_t capacity,
 }
 
 namespace {
-// Restores into graph id `want` (a free id), or into the first free id when
-// want < 0.
-int restore_graph(dlp_engine *e, const void *snapshot, size_t bytes, int want, int *graph_id) {
-  *graph_id = -1;
-  SnapHeader h{};
-  if (bytes < sizeof(h)) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "snapshot too short");
-  std::memcpy(&h, snapshot, sizeof(h));
-  if (h.magic != kSnapMagic) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "not a graph snapshot");
-  if (h.record != (e->cfg.record != 0) || h.semantics != e->cfg.semantics)
-    return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "snapshot was taken by an engine with other settings");
-  if (h.n <= 0 || h.m < 0 || h.seq < 0 || h.prev_d < 0 || h.narrays <= 0)
-    return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "corrupt snapshot header");
-  const size_t need = graph_bytes(h.n, h.m, h.truth != 0, h.bmap != 0, h.record != 0);
-  if (e->budget > 0 && e->used + need > e->budget)
-    return dlp::fail(DLP_ERR_OUT_OF_MEMORY, "graph does not fit the engine's device-memory budget");
-  int gid = -1;
-  if (want >= 0) {
-    if (want >= e->max_graphs || e->graphs[want])
-      return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "graph id " + std::to_string(want) + " is not free");
-    gid = want;
-  } else {
-    for (int i = 0; i < e->max_graphs; ++i)
-      if (!e->graphs[i] && !e->held[i]) {
-        gid = i;
-        break;
-      }
-  }
-  if (gid < 0) return dlp::fail(DLP_ERR_OUT_OF_MEMORY, "the engine holds max_graphs graphs already");
-  DLP_CUDA_TRY(cudaSetDevice(e->device));
+// Makes the graph of a snapshot resident under the free id `gid`.
+int place_snapshot(dlp_engine *e, const SnapHeader &h, const void *snapshot, size_t bytes, int gid) {
   GraphSlot *g = nullptr;
   DLP_TRY(alloc_graph(e, h.n, h.m, h.truth != 0, h.bmap != 0, gid, &g));
   auto bail = [&](int st) {
@@ -942,6 +957,39 @@ int restore_graph(dlp_engine *e, const void *snapshot, size_t bytes, int want, i
   e->held[gid] = 0;
   e->used += g->bytes;
   grow_marks(e);
+  return DLP_OK;
+}
+
+// Restores into graph id `want` (a free id), or into the first free id when
+// want < 0.
+int restore_graph(dlp_engine *e, const void *snapshot, size_t bytes, int want, int *graph_id) {
+  *graph_id = -1;
+  SnapHeader h{};
+  if (bytes < sizeof(h)) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "snapshot too short");
+  std::memcpy(&h, snapshot, sizeof(h));
+  if (h.magic != kSnapMagic) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "not a graph snapshot");
+  if (h.record != (e->cfg.record != 0) || h.semantics != e->cfg.semantics)
+    return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "snapshot was taken by an engine with other settings");
+  if (h.n <= 0 || h.m < 0 || h.seq < 0 || h.prev_d < 0 || h.narrays <= 0)
+    return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "corrupt snapshot header");
+  const size_t need = graph_bytes(h.n, h.m, h.truth != 0, h.bmap != 0, h.record != 0);
+  if (e->budget > 0 && e->used + need > e->budget)
+    return dlp::fail(DLP_ERR_OUT_OF_MEMORY, "graph does not fit the engine's device-memory budget");
+  int gid = -1;
+  if (want >= 0) {
+    if (want >= e->max_graphs || e->graphs[want])
+      return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "graph id " + std::to_string(want) + " is not free");
+    gid = want;
+  } else {
+    for (int i = 0; i < e->max_graphs; ++i)
+      if (!e->graphs[i] && !e->held[i]) {
+        gid = i;
+        break;
+      }
+  }
+  if (gid < 0) return dlp::fail(DLP_ERR_OUT_OF_MEMORY, "the engine holds max_graphs graphs already");
+  DLP_CUDA_TRY(cudaSetDevice(e->device));
+  DLP_TRY(with_room(e, need, [&] { return place_snapshot(e, h, snapshot, bytes, gid); }));
   *graph_id = gid;
   return DLP_OK;
 }

@@ -98,6 +98,10 @@ const void *engine_kernel_ptr(int lanes);
 // Dynamic shared memory per block that every launch of the engine kernel needs
 // (the one-block mode's); launches with owned passes take all there is.
 size_t engine_dynamic_smem();
+// Frees the engine's mark planes, for good, when they take more than `room` bytes:
+// what a server's budget leaves beside graphs, staging and scratch. Passes then run
+// over frontier lists.
+void fit_marks(dlp_engine *e, size_t room);
 // Vertices (in whole tiles) of a launch up to which a grid can own them.
 unsigned owned_limit(int grid);
 // Whether that many graphs with that many vertices fit `smem` bytes of each block.

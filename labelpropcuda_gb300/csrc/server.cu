@@ -188,6 +188,7 @@ struct dlp_server {
     b.evicted = false;
     ++restores;
     if (b.res_edges > 0 || b.res_deleted > 0) DLP_TRY(dlp_engine_reserve(eng, gid, b.res_edges, b.res_deleted));
+    fit_marks(0);  // the planes may have grown
     return DLP_OK;
   }
 
@@ -238,7 +239,16 @@ struct dlp_server {
       DLP_TRY(evict(victim));
       *ok = fits(need());
     }
+    if (*ok) fit_marks(need());
     return DLP_OK;
+  }
+
+  // The engine's mark planes are not among the bytes that fits() counts: they may
+  // take what those, and `need` more, leave of the budget.
+  void fit_marks(size_t need) {
+    if (cfg.memory_budget_bytes == 0) return;
+    const size_t taken = dlp_engine_bytes_in_use(eng) + staged_bytes + running_bytes + need;
+    dlp::engine::fit_marks(eng, cfg.memory_budget_bytes - std::min(cfg.memory_budget_bytes, taken));
   }
 
   int enqueue(const dlp_request &r, bool copy, double arrival, int *id) {

@@ -115,3 +115,66 @@ def test_label_initialisation_cannot_fail_unseen(runtime, inserted):
                                              inserted, a[0].ptr, inserted, None))
     ops = [x[0] for x in runtime.log()]
     assert ops and set(ops) <= {"launch", "clear"}
+
+
+def graph_bytes(p):
+    return dlp.Engine.graph_bytes(p.num_nodes, p.num_edges)
+
+
+@pytest.mark.parametrize("spare", [0, 100, 1 << 20])
+def test_engine_keeps_its_budget(runtime, spare):
+    """What the frontier marks take counts: within the budget when there is room
+    (8 bytes a vertex in whole tiles), given back when there is none."""
+    p = dlp.Problem(1001, 3, 2, 1, cache_dir="")
+    eng = dlp.Engine(3, memory_budget_bytes=2 * graph_bytes(p) + spare)
+    base = runtime.lib.fake_used()
+    taken = []
+    for _ in range(2):
+        eng.add_problem(p)
+        taken.append(runtime.lib.fake_used() - base - eng.bytes_in_use)
+        assert taken[-1] + eng.bytes_in_use <= 2 * graph_bytes(p) + spare
+    assert taken == ([8 * 1024, 16 * 1024] if spare >= 16 * 1024 else [8 * 1024, 0])
+    with pytest.raises(dlp.DlpError):
+        eng.add_problem(dlp.Problem(8000, 3, 2, 1, cache_dir=""))
+    eng.close()
+
+
+def test_marks_give_way_to_a_graph_on_a_full_device(runtime):
+    p = dlp.Problem(1001, 3, 2, 1, cache_dir="")
+    eng = dlp.Engine(2)
+    eng.add_problem(p)
+    snap = eng.snapshot(0)
+    # room for the graph and what its upload or its kept deletions take, but not
+    # for the marks of the first one (8 KiB) as well
+    for again, full in ((lambda: eng.restore(snap), 4096), (lambda: eng.add_problem(p), 8 * p.num_edges)):
+        runtime.lib.fake_capacity(runtime.lib.fake_used() + graph_bytes(p) + full - 8192)
+        g = again()
+        runtime.lib.fake_capacity(ctypes.c_size_t(-1).value)
+        eng.remove_graph(g)
+        eng.remove_graph(0)
+        assert eng.add_problem(p) == 0
+    eng.close()
+
+
+def test_server_keeps_its_budget(runtime):
+    p = dlp.Problem(1001, 3, 2, 1, cache_dir="")
+    eng = dlp.Engine(2)
+    g = eng.add_problem(p)
+    batch = p.batches[0]
+    request = 24 * batch.edge_src.size + 8 * batch.deleted.size + batch.nbytes() + 256
+    for room in (request, request + 8 * 1024):
+        srv = dlp.Server(eng, memory_budget_bytes=eng.bytes_in_use + room)
+        runtime.log()
+        srv.submit(g, 0, batch)
+        try:
+            srv.poll()
+        except dlp.DlpError:
+            pass  # nothing ran
+        frees = [x for x in runtime.log() if x == ["free", "8192"]]
+        assert len(frees) == (1 if room == request else 0)
+        srv.close()
+        if room == request:
+            eng.close()
+            eng = dlp.Engine(2)
+            g = eng.add_problem(p)
+    eng.close()
