@@ -133,9 +133,10 @@ struct dlp_engine {
   size_t used = 0;
   int lanes = 8;
   int grid = 0;
-  size_t smem = 0;      // dynamic shared memory of a launch over frontier lists
-  size_t smem_all = 0;  // all there is: launches with owned passes
-  const void *kernel = nullptr;
+  // Launches over frontier lists, and launches with owned passes: kernel and
+  // dynamic shared memory (the latter take all there is).
+  const void *kernel = nullptr, *owned_kernel = nullptr;
+  size_t smem = 0, smem_all = 0;
   cudaStream_t stream = nullptr;
   std::vector<void *> owned;
   size_t owned_bytes = 0;
@@ -450,7 +451,9 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
     rh[i].ba.flat = static_cast<unsigned>(vertices);
     vertices += owned_room(rh[i].st.n);
   }
-  const bool owned = vertices <= e->mark_plane && dlp::engine::owned_fits(e->grid, total, vertices, e->smem_all);
+  const size_t owned_smem =
+      vertices <= e->mark_plane ? dlp::engine::owned_smem(e->grid, total, vertices, e->smem_all) : 0;
+  const bool owned = owned_smem > 0;
   GraphRec *recs = e->recs_dev + (p ? e->max_graphs : 0);
   DLP_CUDA_TRY(cudaMemcpyAsync(recs, rh, sizeof(GraphRec) * total, cudaMemcpyHostToDevice, e->stream));
   DLP_CUDA_TRY(cudaEventRecord(e->recs_free[p], e->stream));
@@ -472,13 +475,14 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
   args.tag = e->steps + 1;
   args.delta = e->cfg.delta;
   args.tiles = owned ? static_cast<int>(vertices / dlp::engine::kOwnedTile) : 0;
-  args.smem_bytes = static_cast<int>(owned ? e->smem_all : e->smem);
+  args.smem_bytes = static_cast<int>(owned ? owned_smem : e->smem);
   args.marks = e->marks;
   args.mark_plane = e->mark_plane;
   args.progress = sliced ? e->progress_dev : nullptr;
   DLP_CUDA_TRY(cudaEventRecord(e->ev[slot][0], e->stream));
   void *kargs[] = {&args};
-  DLP_TRY(dlp::launch_cooperative(e->kernel, e->grid, dlp::session::kBlock, kargs, args.smem_bytes, e->stream));
+  DLP_TRY(dlp::launch_cooperative(owned ? e->owned_kernel : e->kernel, e->grid, dlp::session::kBlock, kargs,
+                                  args.smem_bytes, e->stream));
   DLP_CUDA_TRY(cudaEventRecord(e->ev[slot][1], e->stream));
   for (int i = 0; i < count; ++i) {
     GraphSlot *g = e->graphs[gids[i]];
@@ -681,6 +685,7 @@ int dlp_engine_create(const dlp_config *cfg_in, int max_graphs, size_t memory_bu
   e->budget = memory_budget_bytes;
   e->lanes = lanes;
   e->kernel = dlp::engine::engine_kernel_ptr(lanes);
+  e->owned_kernel = dlp::engine::owned_kernel_ptr();
   auto bail = [&](int st) {
     delete e;
     return st;
@@ -704,11 +709,14 @@ int dlp_engine_create(const dlp_config *cfg_in, int max_graphs, size_t memory_bu
   int smem_max = 0;
   cudaFuncAttributes fa{};
   if (cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, cfg.device) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa, e->kernel) != cudaSuccess)
+      cudaFuncGetAttributes(&fa, e->owned_kernel) != cudaSuccess)
     return bail(dlp::fail(DLP_ERR_CUDA, "attribute query failed for the engine kernel"));
   e->smem_all = std::max(e->smem, (static_cast<size_t>(smem_max) - fa.sharedSizeBytes) & ~static_cast<size_t>(15));
-  if (cudaFuncSetAttribute(e->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(e->smem_all)) !=
-      cudaSuccess)
+  auto reserve = [](const void *kernel, size_t smem) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) ==
+           cudaSuccess;
+  };
+  if (!reserve(e->kernel, e->smem) || !reserve(e->owned_kernel, e->smem_all))
     return bail(dlp::fail(DLP_ERR_CUDA, "could not reserve the engine kernel's shared memory"));
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, e->kernel, dlp::session::kBlock, e->smem) !=
           cudaSuccess ||

@@ -94,7 +94,10 @@ struct EngineArgs {
 // and the launch's barrier.
 void launch_zero_counters(const GraphRec *recs, int ng_new, EngineCtl *ectl, cudaStream_t stream);
 
+// Launches over frontier lists only, by lanes per short row, and launches with
+// owned passes.
 const void *engine_kernel_ptr(int lanes);
+const void *owned_kernel_ptr();
 // Dynamic shared memory per block that every launch of the engine kernel needs
 // (the one-block mode's); launches with owned passes take all there is.
 size_t engine_dynamic_smem();
@@ -104,8 +107,9 @@ size_t engine_dynamic_smem();
 void fit_marks(dlp_engine *e, size_t room);
 // Vertices (in whole tiles) of a launch up to which a grid can own them.
 unsigned owned_limit(int grid);
-// Whether that many graphs with that many vertices fit `smem` bytes of each block.
-bool owned_fits(int grid, int graphs, size_t vertices, size_t smem);
+// Dynamic shared memory of a launch with owned passes over that many graphs and
+// vertices (in whole tiles), at most `most`; 0 when they do not fit.
+size_t owned_smem(int grid, int graphs, size_t vertices, size_t most);
 
 }  // namespace engine
 }  // namespace dlp

@@ -1641,9 +1641,16 @@ __device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_
 }
 
 // The propagation passes of the launch; k_end is the first pass not run (the
-// graphs whose frontier is live at k_end continue in a later launch).
-template <int G>
-__device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2, int &k_end) {
+// graphs whose frontier is live at k_end continue in a later launch). OWNED:
+// passes run on owned rows, otherwise over lists, in a kernel of its own.
+template <int G, bool OWNED>
+__device__ bool phase_g(const EngineArgs &e, int *pref, int *pref2, int &k_end) {
+  auto place = [] {
+    int t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t;
+  };
+  auto lead = [&] { return blockIdx.x == 0 && place() == 0; };
   int solo_from = 0;     // the one-block mode declined: not tried again before this pass
   bool owned = false;    // the block holds its rows (owned_passes)
   int stint_no = 0;
@@ -1653,23 +1660,23 @@ __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2
   // list passes (launches beyond owned rows) 104 bytes of spills and 3%: 62.8
   // against 60.7 ms for 14 batches of 4.2 million vertices
   __shared__ unsigned long long mp[2], mns[2], t_mode;
-  if (c.gtid == 0) mp[0] = mp[1] = mns[0] = mns[1] = 0;
+  if (lead()) mp[0] = mp[1] = mns[0] = mns[1] = 0;
   for (;; ++k) {
     int tn, tw;
     pass_sizes(e, k, pref, pref2, tn, tw);
     if (tn + tw == 0) break;
     if (e.pass_budget > 0 && k >= e.pass_budget) break;
     if (ld_relaxed_u64(&e.ectl->slice_stop) == stop_code(e, k)) break;
-    if (c.gtid == 0) e.ectl->where_pass = k;
+    if (lead()) e.ectl->where_pass = k;
     const bool solo_ok = (e.solo & 1) && tn + tw <= e.solo_entry && k >= solo_from;
     if (solo_ok) {
-      if (c.gtid == 0) t_mode = global_timer_ns();
+      if (lead()) t_mode = global_timer_ns();
       if (blockIdx.x == 0) solo_passes(e, k, stint_no & 1);
       if (!launch_sync(e)) return false;
       const int done = ld_relaxed_i32(&e.ectl->solo_passes[stint_no & 1]);
       const int kk = ld_relaxed_i32(&e.ectl->solo_k[stint_no & 1]);
       ++stint_no;
-      if (c.gtid == 0) {
+      if (lead()) {
         mp[0] += done;
         mns[0] += global_timer_ns() - t_mode;
       }
@@ -1680,34 +1687,34 @@ __device__ bool phase_g(const EngineArgs &e, const Ctx &c, int *pref, int *pref2
       k = kk - 1;  // the loop increment resumes at pass kk
       continue;
     }
-    if (c.gtid == 0) t_mode = global_timer_ns();
-    if (e.tiles > 0) {
+    if (lead()) t_mode = global_timer_ns();
+    if (OWNED) {
       int kk = k;
       if (!owned_passes(e, k, solo_from, pref, pref2, tn, tw, owned, &kk)) return false;
       owned = true;
-      if (c.gtid == 0) {
+      if (lead()) {
         mp[1] += kk - k;
         mns[1] += global_timer_ns() - t_mode;
       }
       k = kk - 1;  // the loop increment resumes at pass kk
       continue;
     }
-    // The thread's place is read again, not kept from before the loop (88 instead
-    // of 156 bytes of spill loads): 48 graphs of 100,000 vertices, 276.4 against
-    // 279.3 ms for 10 batches.
-    int tid;
-    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    // Nothing of the thread's place is kept over the loop: the call of the one-block
+    // mode leaves few registers for it (4 and 16 bytes of spill stores and loads
+    // instead of 40 and 88, with the owned passes in the same kernel). 4.2 million
+    // vertices, frontiers of 210,000 and 340,000 rows: 46 -> 44 and 67 -> 64 us.
+    const int tid = place();
     const int gtid = blockIdx.x * kBlock + tid, nthreads = gridDim.x * kBlock;
     run_pass<G>(e, k, pref, tn, pref2, tw, tid & 31, gtid >> 5, nthreads >> 5, gtid, nthreads);
-    if (c.gtid == 0 && slice_over(e)) e.ectl->slice_stop = stop_code(e, k + 1);
+    if (lead() && slice_over(e)) e.ectl->slice_stop = stop_code(e, k + 1);
     if (!launch_sync(e)) return false;
-    if (c.gtid == 0) {
+    if (lead()) {
       ++mp[1];
       mns[1] += global_timer_ns() - t_mode;
     }
   }
   k_end = k;
-  if (c.gtid == 0) {
+  if (lead()) {
     e.ectl->mode_passes[0] += mp[0];
     e.ectl->mode_ns[0] += mns[0];
     e.ectl->mode_passes[3] += mp[1];
@@ -1784,7 +1791,7 @@ __device__ void phase_h(const EngineArgs &e, const Ctx &c, int *pref, int k_end)
 
 }  // namespace
 
-template <int G>
+template <int G, bool OWNED>
 __global__ void __launch_bounds__(kBlock, 1024 / kBlock) engine_kernel(const __grid_constant__ EngineArgs e) {
   const Ctx c = make_ctx();
   __shared__ int pref[kMaxGraphs + 1];
@@ -1825,7 +1832,7 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) engine_kernel(const __g
   }
   at(8);
   int k_end = 0;
-  if (!phase_g<G>(e, c, pref, pref2, k_end)) return;
+  if (!phase_g<G, OWNED>(e, pref, pref2, k_end)) return;
   at(9);
   phase_h(e, c, pref, k_end);
   if (!launch_sync(e)) return;
@@ -1881,11 +1888,12 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) engine_kernel(const __g
   }
 }
 
-template __global__ void engine_kernel<1>(const __grid_constant__ EngineArgs);
-template __global__ void engine_kernel<4>(const __grid_constant__ EngineArgs);
-template __global__ void engine_kernel<8>(const __grid_constant__ EngineArgs);
-template __global__ void engine_kernel<16>(const __grid_constant__ EngineArgs);
-template __global__ void engine_kernel<32>(const __grid_constant__ EngineArgs);
+template __global__ void engine_kernel<1, false>(const __grid_constant__ EngineArgs);
+template __global__ void engine_kernel<4, false>(const __grid_constant__ EngineArgs);
+template __global__ void engine_kernel<8, false>(const __grid_constant__ EngineArgs);
+template __global__ void engine_kernel<16, false>(const __grid_constant__ EngineArgs);
+template __global__ void engine_kernel<32, false>(const __grid_constant__ EngineArgs);
+template __global__ void engine_kernel<8, true>(const __grid_constant__ EngineArgs);
 
 // One block per graph that starts a batch: its counters back to zero; block 0
 // also clears the launch's barrier.
@@ -1909,18 +1917,22 @@ unsigned owned_limit(int grid) {
   return grid > 1 ? static_cast<unsigned>(grid - 1) * (owner::kMaxVertices - owner::kTile) : 0u;
 }
 
-bool owned_fits(int grid, int graphs, size_t vertices, size_t smem) {
+size_t owned_smem(int grid, int graphs, size_t vertices, size_t most) {
+  if (vertices > owned_limit(grid)) return 0;
   const size_t tiles = vertices / owner::kTile, blocks = static_cast<size_t>(grid - 1);
-  return vertices <= owned_limit(grid) && owner::bytes_of(graphs, (tiles + blocks - 1) / blocks) <= smem;
+  const size_t need = owner::bytes_of(graphs, (tiles + blocks - 1) / blocks);
+  return need > most ? 0 : most;
 }
+
+const void *owned_kernel_ptr() { return reinterpret_cast<const void *>(&engine_kernel<8, true>); }
 
 const void *engine_kernel_ptr(int lanes) {
   switch (lanes) {
-    case 1: return reinterpret_cast<const void *>(&engine_kernel<1>);
-    case 4: return reinterpret_cast<const void *>(&engine_kernel<4>);
-    case 8: return reinterpret_cast<const void *>(&engine_kernel<8>);
-    case 16: return reinterpret_cast<const void *>(&engine_kernel<16>);
-    case 32: return reinterpret_cast<const void *>(&engine_kernel<32>);
+    case 1: return reinterpret_cast<const void *>(&engine_kernel<1, false>);
+    case 4: return reinterpret_cast<const void *>(&engine_kernel<4, false>);
+    case 8: return reinterpret_cast<const void *>(&engine_kernel<8, false>);
+    case 16: return reinterpret_cast<const void *>(&engine_kernel<16, false>);
+    case 32: return reinterpret_cast<const void *>(&engine_kernel<32, false>);
     default: return nullptr;
   }
 }
