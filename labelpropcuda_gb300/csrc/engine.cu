@@ -133,10 +133,10 @@ struct dlp_engine {
   size_t used = 0;
   int lanes = 8;
   int grid = 0;
-  // Launches over frontier lists, and launches with owned passes: kernel and
-  // dynamic shared memory (the latter take all there is).
+  // Launches over frontier lists and launches with owned passes; the dynamic shared
+  // memory of the former, the most of the latter beside their static one.
   const void *kernel = nullptr, *owned_kernel = nullptr;
-  size_t smem = 0, smem_all = 0;
+  size_t smem = 0, smem_all = 0, smem_fixed = 0;
   cudaStream_t stream = nullptr;
   std::vector<void *> owned;
   size_t owned_bytes = 0;
@@ -452,7 +452,7 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
     vertices += owned_room(rh[i].st.n);
   }
   const size_t owned_smem =
-      vertices <= e->mark_plane ? dlp::engine::owned_smem(e->grid, total, vertices, e->smem_all) : 0;
+      vertices <= e->mark_plane ? dlp::engine::owned_smem(e->grid, total, vertices, e->smem_fixed, e->smem_all) : 0;
   const bool owned = owned_smem > 0;
   GraphRec *recs = e->recs_dev + (p ? e->max_graphs : 0);
   DLP_CUDA_TRY(cudaMemcpyAsync(recs, rh, sizeof(GraphRec) * total, cudaMemcpyHostToDevice, e->stream));
@@ -712,6 +712,7 @@ int dlp_engine_create(const dlp_config *cfg_in, int max_graphs, size_t memory_bu
       cudaFuncGetAttributes(&fa, e->owned_kernel) != cudaSuccess)
     return bail(dlp::fail(DLP_ERR_CUDA, "attribute query failed for the engine kernel"));
   e->smem_all = std::max(e->smem, (static_cast<size_t>(smem_max) - fa.sharedSizeBytes) & ~static_cast<size_t>(15));
+  e->smem_fixed = fa.sharedSizeBytes;
   auto reserve = [](const void *kernel, size_t smem) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) ==
            cudaSuccess;

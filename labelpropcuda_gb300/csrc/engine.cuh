@@ -99,7 +99,7 @@ void launch_zero_counters(const GraphRec *recs, int ng_new, EngineCtl *ectl, cud
 const void *engine_kernel_ptr(int lanes);
 const void *owned_kernel_ptr();
 // Dynamic shared memory per block that every launch of the engine kernel needs
-// (the one-block mode's); launches with owned passes take all there is.
+// (the one-block mode's).
 size_t engine_dynamic_smem();
 // Frees the engine's mark planes, for good, when they take more than `room` bytes:
 // what a server's budget leaves beside graphs, staging and scratch. Passes then run
@@ -108,8 +108,9 @@ void fit_marks(dlp_engine *e, size_t room);
 // Vertices (in whole tiles) of a launch up to which a grid can own them.
 unsigned owned_limit(int grid);
 // Dynamic shared memory of a launch with owned passes over that many graphs and
-// vertices (in whole tiles), at most `most`; 0 when they do not fit.
-size_t owned_smem(int grid, int graphs, size_t vertices, size_t most);
+// vertices (in whole tiles), beside `fixed` bytes of static shared memory and at
+// most `most`; 0 when they do not fit.
+size_t owned_smem(int grid, int graphs, size_t vertices, size_t fixed, size_t most);
 
 }  // namespace engine
 }  // namespace dlp

@@ -1913,15 +1913,21 @@ void launch_zero_counters(const GraphRec *recs, int ng_new, EngineCtl *ectl, cud
 
 size_t engine_dynamic_smem() { return sizeof(SoloCache); }
 
+namespace {
+size_t owned_need(int grid, int graphs, size_t tiles) {
+  const size_t blocks = static_cast<size_t>(grid - 1);
+  return owner::bytes_of(graphs, (tiles + blocks - 1) / blocks);
+}
+}  // namespace
+
 unsigned owned_limit(int grid) {
   return grid > 1 ? static_cast<unsigned>(grid - 1) * (owner::kMaxVertices - owner::kTile) : 0u;
 }
 
-size_t owned_smem(int grid, int graphs, size_t vertices, size_t most) {
+size_t owned_smem(int grid, int graphs, size_t vertices, size_t fixed, size_t most) {
   if (vertices > owned_limit(grid)) return 0;
-  const size_t tiles = vertices / owner::kTile, blocks = static_cast<size_t>(grid - 1);
-  const size_t need = owner::bytes_of(graphs, (tiles + blocks - 1) / blocks);
-  return need > most ? 0 : most;
+  const size_t need = owned_need(grid, graphs, vertices / owner::kTile);
+  return need > most ? 0 : owner::smem_of(need, sizeof(SoloCache), fixed, most);
 }
 
 const void *owned_kernel_ptr() { return reinterpret_cast<const void *>(&engine_kernel<8, true>); }

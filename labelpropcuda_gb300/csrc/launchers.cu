@@ -1165,7 +1165,8 @@ static_assert(sizeof(int) * kOutWords <= kOwnedSmall && kOwnedFixed % 16 == 0, "
 
 // Facts about a device that the owned kernels' launches need, queried once.
 struct OwnedShape {
-  int grid = 0, smem = 0;  // grid 0: the kernels do not fit this device
+  int grid = 0;            // 0: the kernels do not fit this device
+  size_t fixed = 0, smem = 0;  // static shared memory, the most of the dynamic one
 };
 
 OwnedShape owned_shape() {
@@ -1181,14 +1182,21 @@ OwnedShape owned_shape() {
   int sms = 0, most = 0;
   bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
             cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess;
-  s.smem = (most - 1024) & ~15;
-  for (const void *kernel : {reinterpret_cast<const void *>(&prop_owned_kernel),
-                             reinterpret_cast<const void *>(&irlp_owned_kernel)}) {
+  const void *const kernels[] = {reinterpret_cast<const void *>(&prop_owned_kernel),
+                                 reinterpret_cast<const void *>(&irlp_owned_kernel)};
+  for (const void *kernel : kernels) {
+    cudaFuncAttributes fa{};
+    ok = ok && cudaFuncGetAttributes(&fa, kernel) == cudaSuccess;
+    s.fixed = std::max(s.fixed, fa.sharedSizeBytes);
+  }
+  s.smem = (static_cast<size_t>(most) - s.fixed) & ~static_cast<size_t>(15);
+  for (const void *kernel : kernels) {
     int per_sm = 0;
-    ok = ok && s.smem >= static_cast<int>(sizeof(StintShared)) &&
-         static_cast<size_t>(s.smem) >= owner::bytes_of(1, owner::kMaxVertices / owner::kTile) &&
-         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, s.smem) == cudaSuccess &&
-         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kOwnBlock, s.smem) == cudaSuccess && per_sm > 0;
+    ok = ok && s.smem >= sizeof(StintShared) && s.smem >= owner::bytes_of(1, owner::kMaxVertices / owner::kTile) &&
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(s.smem)) ==
+             cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kOwnBlock, s.smem) == cudaSuccess &&
+         per_sm > 0;
   }
   s.grid = ok ? std::min(sms, kSumBlocks) : 0;
   cudaGetLastError();
@@ -1201,6 +1209,13 @@ OwnedShape owned_shape() {
 int owned_grid(int n) {
   const OwnedShape s = owned_shape();
   return s.grid > 1 && n <= (s.grid - 1) * (owner::kMaxVertices - owner::kTile) ? s.grid : 0;
+}
+
+// Dynamic shared memory of a launch over n vertices.
+size_t owned_smem(int n) {
+  const OwnedShape s = owned_shape();
+  const size_t tiles = (static_cast<size_t>(n) + owner::kTile - 1) / owner::kTile, blocks = s.grid - 1;
+  return owner::smem_of(owner::bytes_of(1, (tiles + blocks - 1) / blocks), sizeof(StintShared), s.fixed, s.smem);
 }
 
 // Words of a mark plane of n vertices: whole tiles.
@@ -1216,7 +1231,7 @@ OwnedArgs owned_args(const int *row_ptr, const int *col, const float *val, float
   a.max_iter = max_iterations;
   a.plane = owned_plane(n);
   a.timeout_ns = 2000000000ull;
-  a.smem_bytes = owned_shape().smem;
+  a.smem_bytes = static_cast<int>(owned_smem(n));
   return a;
 }
 
