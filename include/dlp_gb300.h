@@ -251,7 +251,7 @@ int dlp_engine_create(const dlp_config *cfg, int max_graphs, size_t memory_budge
 int dlp_engine_destroy(dlp_engine *e);
 /* Device bytes a graph of this size occupies once added (admission). */
 size_t dlp_engine_graph_bytes(int num_nodes, int64_t num_edges, int with_truth, int with_batch_map, int record);
-/* Bytes of the resident graphs. Frontier marks (8 bytes a vertex, for up to 3.7
+/* Bytes of the resident graphs. Frontier marks (8 bytes a vertex, for up to 3.1
  * million vertices) come on top: within a budget they take only what it leaves
  * over, and give way to a graph that needs it. Without them propagation gives the
  * same results over frontier lists. */
@@ -321,7 +321,7 @@ int dlp_engine_artefact(dlp_engine *e, int graph_id, int which, void *host_out, 
 
 /* Autotuner (no counterpart in the reference, whose launch shapes are fixed).
  * Propagation runs each pass on one block or the whole grid by the size of the
- * frontier; in launches of more than 3.7 million vertices it sends rows of at
+ * frontier; in launches of more than 3.1 million vertices it sends rows of at
  * most 32 live entries to groups of narrow_lanes lanes and longer rows to whole
  * warps. The lane width of the short-row bucket, the frontier threshold
  * (solo_entry; subgrid_entry has no effect) and the persistent grid's blocks per

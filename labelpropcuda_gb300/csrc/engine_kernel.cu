@@ -1920,9 +1920,15 @@ size_t owned_need(int grid, int graphs, size_t tiles) {
 }
 }  // namespace
 
-unsigned owned_limit(int grid) {
-  return grid > 1 ? static_cast<unsigned>(grid - 1) * (owner::kMaxVertices - owner::kTile) : 0u;
-}
+// As many as leave L1 more than its last 28 KB (smem_of, owner_pass.cuh). With
+// that little, lists are faster: 14 batches of 300 passes at most, milliseconds
+// over lists and on owned rows: 3.0 million vertices of degree 7 35.2 and 29.8, 3.3
+// million of degree 5 9.6 and 11.6, 3.5 million of degree 5 9.8 and 14.8, 3.6 million of
+// degree 7 43.4 and 46.2.
+constexpr int kOwnedVertices = 20320;
+static_assert(owner::leaves_l1(owner::bytes_of(1, kOwnedVertices / owner::kTile) + owner::kPoolBytes, 10240));
+
+unsigned owned_limit(int grid) { return grid > 1 ? static_cast<unsigned>(grid - 1) * kOwnedVertices : 0u; }
 
 size_t owned_smem(int grid, int graphs, size_t vertices, size_t fixed, size_t most) {
   if (vertices > owned_limit(grid)) return 0;

@@ -22,12 +22,13 @@
 // degree 5 3.2 against 5.1, 20,000 of degree 7 3.4 against 6.2, 50,000 of degree
 // 5 3.3 against 7.5 to 8.0, 500,000 of degree 7 5.9 against 16.2.
 //
-// Shared memory ends at 24,576 vertices per block (3.7 million on 151), beyond
-// which launches use frontier lists. Most rows then stay in global memory and a
-// scan reads all words of the graph, yet owned rows are the faster ones: 14
-// batches of 2.6 million vertices of degree 7 take 58.7 against 96.7 ms, and of
-// 3.6 million, mostly with small frontiers, 49.2 against 51.8 ms.
+// Shared memory ends at 24,576 vertices per block (3.7 million on 151). Most rows
+// then stay in global memory and a scan reads all words of the graph. The engine
+// uses frontier lists beyond 20,320 (engine_kernel.cu), the launchers, whose list
+// passes are the slower ones, beyond 24,544.
 #pragma once
+
+#include <algorithm>
 
 #include "common.cuh"
 
@@ -134,15 +135,18 @@ constexpr size_t bytes_of(size_t graphs, size_t tiles) {
 // most) 6.65 and 5.62, of a million 9.47 and 8.2, of 2 million 14.5 and 13.0, of
 // 2.6 million 16.4 and 15.7; 10 of 2 million with 2 passes 3.34 and 2.8; a
 // recompute of 3.5 million (30 passes) 12.7 and 7.5.
-constexpr size_t kPoolBytes = 16 << 10;
+constexpr size_t kPoolBytes = 16 << 10, kSystemBytes = 1 << 10;
+constexpr size_t kSteps[] = {100 << 10, 132 << 10, 164 << 10, 196 << 10};
+constexpr bool leaves_l1(size_t need, size_t fixed) { return need + fixed + kSystemBytes <= kSteps[3]; }
 inline size_t smem_of(size_t need, size_t least, size_t fixed, size_t most) {
-  constexpr size_t kSteps[] = {100 << 10, 132 << 10, 164 << 10, 196 << 10};
-  fixed += 1024;
-  for (const size_t step : kSteps)
-    if (fixed + (need + kPoolBytes > least ? need + kPoolBytes : least) <= step ||
-        (step == kSteps[3] && fixed + need <= step && fixed + least <= step))
-      return (step - fixed < most ? step - fixed : most) & ~static_cast<size_t>(15);
-  return most & ~static_cast<size_t>(15);
+  const size_t asked = std::max(need + kPoolBytes, least), bound = std::max(need, least);
+  size_t bytes = most;
+  if (leaves_l1(bound, fixed))
+    for (const size_t step : kSteps) {
+      bytes = step - fixed - kSystemBytes;
+      if (asked <= bytes) break;
+    }
+  return std::min(bytes, most) & ~static_cast<size_t>(15);
 }
 
 __device__ __forceinline__ unsigned pack(unsigned off, int len, int g) {
