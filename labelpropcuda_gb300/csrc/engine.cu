@@ -447,12 +447,17 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
   for (size_t j = 0; j < resumed.size(); ++j) rh[count + j] = e->graphs[resumed[j]]->inflight_rec;
   // the launch's vertices one graph after the other, for the owned passes
   size_t vertices = 0;
+  int passes = 0;  // at most, of the launch
   for (int i = 0; i < total; ++i) {
     rh[i].ba.flat = static_cast<unsigned>(vertices);
     vertices += owned_room(rh[i].st.n);
+    passes = std::max(passes, rh[i].ba.max_iter - rh[i].ba.pass0);
   }
+  if (opts.pass_budget > 0) passes = std::min(passes, opts.pass_budget);
   const size_t owned_smem =
-      vertices <= e->mark_plane ? dlp::engine::owned_smem(e->grid, total, vertices, e->smem_fixed, e->smem_all) : 0;
+      passes > dlp::engine::kListOnly && vertices <= e->mark_plane
+          ? dlp::engine::owned_smem(e->grid, total, vertices, e->smem_fixed, e->smem_all)
+          : 0;
   const bool owned = owned_smem > 0;
   GraphRec *recs = e->recs_dev + (p ? e->max_graphs : 0);
   DLP_CUDA_TRY(cudaMemcpyAsync(recs, rh, sizeof(GraphRec) * total, cudaMemcpyHostToDevice, e->stream));
@@ -476,6 +481,7 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
   args.delta = e->cfg.delta;
   args.tiles = owned ? static_cast<int>(vertices / dlp::engine::kOwnedTile) : 0;
   args.smem_bytes = static_cast<int>(owned ? owned_smem : e->smem);
+  args.list_passes = dlp::engine::list_passes(vertices);
   args.marks = e->marks;
   args.mark_plane = e->mark_plane;
   args.progress = sliced ? e->progress_dev : nullptr;

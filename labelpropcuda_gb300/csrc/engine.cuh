@@ -87,6 +87,7 @@ struct EngineArgs {
   int smem_bytes;                 // dynamic shared memory of the launch
   unsigned *marks;
   unsigned mark_plane;            // words of a plane
+  int list_passes;                // full-grid passes over lists before rows are loaded
   int2 *progress;                 // per graph: {1 batch finished / 0 continues, passes so far}
 };
 
@@ -107,6 +108,10 @@ size_t engine_dynamic_smem();
 void fit_marks(dlp_engine *e, size_t room);
 // Vertices (in whole tiles) of a launch up to which a grid can own them.
 unsigned owned_limit(int grid);
+// Full-grid passes over lists before a launch of that many vertices loads rows; and
+// the most passes that a launch may run over lists only.
+int list_passes(size_t vertices);
+constexpr int kListOnly = 3;
 // Dynamic shared memory of a launch with owned passes over that many graphs and
 // vertices (in whole tiles), beside `fixed` bytes of static shared memory and at
 // most `most`; 0 when they do not fit.

@@ -1642,7 +1642,8 @@ __device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_
 
 // The propagation passes of the launch; k_end is the first pass not run (the
 // graphs whose frontier is live at k_end continue in a later launch). OWNED:
-// passes run on owned rows, otherwise over lists, in a kernel of its own.
+// passes run on owned rows after the first e.list_passes, otherwise over lists, in a
+// kernel of its own.
 template <int G, bool OWNED>
 __device__ bool phase_g(const EngineArgs &e, int *pref, int *pref2, int &k_end) {
   auto place = [] {
@@ -1654,6 +1655,7 @@ __device__ bool phase_g(const EngineArgs &e, int *pref, int *pref2, int &k_end) 
   int solo_from = 0;     // the one-block mode declined: not tried again before this pass
   bool owned = false;    // the block holds its rows (owned_passes)
   int stint_no = 0;
+  int listed = 0;        // full-grid passes run over lists
   int k = 0;
   // passes and device time per mode in this launch (one block, full grid), by
   // thread 0 of block 0; in shared memory, because in registers they cost the
@@ -1688,7 +1690,7 @@ __device__ bool phase_g(const EngineArgs &e, int *pref, int *pref2, int &k_end) 
       continue;
     }
     if (lead()) t_mode = global_timer_ns();
-    if (OWNED) {
+    if (OWNED && listed >= e.list_passes) {
       int kk = k;
       if (!owned_passes(e, k, solo_from, pref, pref2, tn, tw, owned, &kk)) return false;
       owned = true;
@@ -1699,6 +1701,7 @@ __device__ bool phase_g(const EngineArgs &e, int *pref, int *pref2, int &k_end) 
       k = kk - 1;  // the loop increment resumes at pass kk
       continue;
     }
+    ++listed;
     // Nothing of the thread's place is kept over the loop: the call of the one-block
     // mode leaves few registers for it (4 and 16 bytes of spill stores and loads
     // instead of 40 and 88, with the owned passes in the same kernel). 4.2 million
@@ -1929,6 +1932,16 @@ constexpr int kOwnedVertices = 20320;
 static_assert(owner::leaves_l1(owner::bytes_of(1, kOwnedVertices / owner::kTile) + owner::kPoolBytes, 10240));
 
 unsigned owned_limit(int grid) { return grid > 1 ? static_cast<unsigned>(grid - 1) * kOwnedVertices : 0u; }
+
+// Rows are loaded for the passes that follow: some 20 us for a million vertices, 60 for
+// 2 and 75 for 3. A launch that may run 3 full-grid passes at most (pass limits, pass
+// budget) runs them over lists: 100 steps of 2 passes over 32 graphs (560,000 vertices)
+// 9.7 and 9.0 ms. From 1.75 million vertices on, a launch starts with 8 passes over
+// lists, which a batch that goes on makes up for. 10 batches of 2, 8, 20 and 60 passes,
+// milliseconds, rows loaded at once and after 8: 1.5 million vertices 2.2, 2.7, 3.3, 5.0
+// and 1.9, 2.4, 3.4, 5.1; 2 million 2.8, 3.3, 4.0, 6.3 and 2.4, 2.8, 4.1, 6.2; 2.6 million
+// 3.5, 4.1, 5.0, 7.7 and 3.0, 3.5, 5.0, 7.5; with 300 passes they differ by less than 1%.
+int list_passes(size_t vertices) { return vertices < 1750000 ? 0 : 8; }
 
 size_t owned_smem(int grid, int graphs, size_t vertices, size_t fixed, size_t most) {
   if (vertices > owned_limit(grid)) return 0;

@@ -105,3 +105,45 @@ def test_owned_passes_partial_tile_beyond_shared_memory(gpu, oracle):
         for k in EXACT_STATS:
             assert got[k] == want[k], (b, k)
         assert sess.labels().tobytes() == orc.labels().tobytes(), b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solo", [0, 7])
+def test_lists_before_owned_rows(gpu, oracle, solo):
+    """From 1.75 million vertices on, a launch runs 8 full-grid passes over lists
+    before it loads rows."""
+    p = dlp.Problem(1800001, 4, 150, 5, cache_dir="")
+    orc = oracle.OracleRun.from_problem(p, threads=0, max_iterations=20)
+    sess = dlp.Session.from_problem(p, max_iterations=20, small_frontier_solo=solo)
+    for b, batch in enumerate(p.batches[:4]):
+        got, want = sess.apply(b, batch), orc.apply(b, batch)
+        for k in EXACT_STATS:
+            assert got[k] == want[k], (b, k)
+        assert sess.labels().tobytes() == orc.labels().tobytes(), b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("solo", [0, 7])
+def test_launches_of_few_passes_among_longer_ones(gpu, oracle, solo):
+    """At most 3 passes run over lists, more on owned rows: batches that go through
+    both, with pass limits that end in either."""
+    probs = [dlp.Problem(n, d, 4, s, cache_dir="") for n, d, s in ((1500, 5, 1), (64, 3, 2), (3000, 34, 3))]
+    cap, budgets = 61, (2, 5, 3, 1, 4)
+    orcs = [oracle.OracleRun.from_problem(p, threads=4, max_iterations=cap) for p in probs]
+    eng = dlp.Engine(len(probs), max_iterations=cap, small_frontier_solo=solo)
+    ids = [eng.add_problem(p) for p in probs]
+    dev = [[dlp.DeviceBatch(b) for b in p.batches] for p in probs]
+    nxt, step = [0] * len(probs), 0
+    while any(x < 4 for x in nxt) or any(eng.in_progress(g) for g in ids):
+        start = [i for i, g in enumerate(ids) if nxt[i] < 4 and not eng.in_progress(g) and (step + i) % 2 == 0]
+        done, _ = eng.step_sliced([(ids[i], nxt[i], dev[i][nxt[i]]) for i in start],
+                                  pass_budget=budgets[step % len(budgets)])
+        for i in start:
+            nxt[i] += 1
+        for g in done:
+            i = ids.index(g)
+            want, got = orcs[i].apply(nxt[i] - 1, probs[i].batches[nxt[i] - 1]), eng.stats(g, nxt[i] - 1)
+            for k in EXACT_STATS:
+                assert got[k] == want[k], (i, nxt[i] - 1, k)
+            assert eng.labels(g).tobytes() == orcs[i].labels().tobytes(), (i, nxt[i] - 1)
+        step += 1
