@@ -214,6 +214,44 @@ __device__ __forceinline__ bool sum_sync(SumBarrier *bar, SumState &f, int *err,
   return (sum & (0xffull * kSumError)) == 0;
 }
 
+// *p if c, else d; the load is predicated, not branched around, so that several are in
+// flight together.
+__device__ __forceinline__ int load_if(bool c, const int *p, int d) {
+  int v;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.s32 p, %2, 0;\n\t"
+      "mov.b32 %0, %3;\n\t"
+      "@p ld.global.b32 %0, [%1];\n\t"
+      "}" : "=&r"(v) : "l"(p), "r"(static_cast<int>(c)), "r"(d));
+  return v;
+}
+__device__ __forceinline__ int2 load_if(bool c, const int2 *p, int d) {
+  int2 v;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.s32 p, %3, 0;\n\t"
+      "mov.b32 %0, %4;\n\t"
+      "mov.b32 %1, %4;\n\t"
+      "@p ld.global.v2.b32 {%0, %1}, [%2];\n\t"
+      "}" : "=&r"(v.x), "=&r"(v.y) : "l"(p), "r"(static_cast<int>(c)), "r"(d));
+  return v;
+}
+
+__device__ __forceinline__ unsigned load_if(bool c, const uint8_t *p, unsigned d) {
+  unsigned v;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.s32 p, %2, 0;\n\t"
+      "mov.b32 %0, %3;\n\t"
+      "@p ld.global.u8 %0, [%1];\n\t"
+      "}" : "=&r"(v) : "l"(p), "r"(static_cast<int>(c)), "r"(d));
+  return v;
+}
+
 // Appends the set lanes' values to list[*count ...] with one atomic per warp.
 // Must be called by all lanes of the warp (convergent).
 __device__ __forceinline__ void warp_append(bool pred, int value, int *list, int *count) {

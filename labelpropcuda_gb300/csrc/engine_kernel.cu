@@ -1472,6 +1472,24 @@ struct OwnedGraphs {
     v = ent.x;
     w = __int_as_float(ent.y);
   }
+  template <int N>
+  __device__ void entries(int g, int start, int first, int step, int len, int (&v)[N], float (&w)[N]) const {
+    const int2 *adj = e.recs[g].st.act_adj + start;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const int2 ent = load_if(first + j * step < len, adj + first + j * step, -1);
+      v[j] = ent.x;
+      w[j] = __int_as_float(ent.y);
+    }
+  }
+  template <int N>
+  __device__ unsigned markables(int g, const int (&v)[N]) const {
+    const uint8_t *meta = e.recs[g].st.nmeta;
+    unsigned can = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) can |= (load_if(v[j] >= 0, meta + v[j], 0) & 1u) << j;
+    return can;
+  }
 };
 
 // Recorded frontier sizes of pass k back to zero, by one block.
@@ -1485,7 +1503,9 @@ __device__ __forceinline__ void clear_record(const EngineArgs &e, int k) {
 
 // The passes of a stint on owned rows, from k on; returns the first pass not
 // run, or -1 when the launch has to end. Not inlined, so that its registers
-// are its own.
+// are its own. TILES: the block's passes are tile_pass (up to 1,024 owned vertices, 151
+// x 1,024 in the launch, in tiles of few steps).
+template <bool TILES>
 __device__ __noinline__ int owned_loop(const EngineArgs &e, int k, owner::Store s, bool rec_any) {
   const OwnedGraphs gr{e};
   owner::Head &h = s.head();
@@ -1500,8 +1520,7 @@ __device__ __noinline__ int owned_loop(const EngineArgs &e, int k, owner::Store 
         const int kg = k + r.ba.pass0;
         if (r.ba.record && kg < kRecordIters) atomicAdd(&r.st.rec_fsizes[kg], 1);
       };
-      // Up to 1,024 owned vertices a block: 151 x 1,024 in the launch.
-      if (s.n() <= kBlock) owner::tile_pass(s, gr, own, next, k, h.delta, h.fast != 0, each);
+      if (TILES) owner::tile_pass(s, gr, own, next, k, h.delta, h.fast != 0, each);
       else owner::pass(s, gr, own, next, k, h.delta, h.fast != 0, each);
     } else if (rec_any && blockIdx.x == 0) {
       clear_record(e, k + 1);
@@ -1515,7 +1534,7 @@ __device__ __noinline__ int owned_loop(const EngineArgs &e, int k, owner::Store 
       }
       const unsigned long long mine =
           static_cast<unsigned>((h.count & 0xffff) + (h.count >> 16) + h.wide) | (h.moved ? kSumMoved : 0ull);
-      h.count = h.wide = 0;
+      h.count = h.wide = h.wide_at = 0;
       h.moved = 0;
       return mine;
     }, sum);
@@ -1557,8 +1576,8 @@ __device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_
     if (tid == 0) {
       h.pool_used = 0;
       h.first_limit = 0x7fffffff;
-      h.count = h.wide = 0;
-      h.moved = 0;
+      h.count = h.wide = h.wide_at = 0;
+      h.moved = h.steps = 0;
     }
     __syncthreads();
     for (int g = tid; g < ng; g += kBlock) {
@@ -1596,7 +1615,8 @@ __device__ __noinline__ bool owned_passes(const EngineArgs &e, int k0, int solo_
   if (!launch_sync(e)) return false;
   if (blockIdx.x == 0)  // the lists are filled again at the end
     for (int i = tid; i < 6 * ng; i += kBlock) (&e.recs[i / 6].st.bc->front_count[0][0])[i % 6] = 0;
-  const int k = owned_loop(e, k0, s, rec_any);
+  const bool tiles = !owns || (s.n() <= kBlock && h.steps <= owner::kTileSteps);
+  const int k = tiles ? owned_loop<true>(e, k0, s, rec_any) : owned_loop<false>(e, k0, s, rec_any);
   if (k < 0) return false;
   // marks -> frontier lists; visits -> counters; vertices that were or are in a
   // frontier join the touched list the first time in this batch

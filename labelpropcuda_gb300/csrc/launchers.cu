@@ -694,6 +694,28 @@ struct CsrGraph {
     w = val[at];
     if (v >= 0 && status[v] == kDeleted) v = -1;
   }
+  template <int N>
+  __device__ void entries(int, int start, int first, int step, int len, int (&v)[N], float (&w)[N]) const {
+    int st[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = load_if(first + j * step < len, col + start + first + j * step, -1);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      w[j] = __int_as_float(
+          load_if(first + j * step < len, reinterpret_cast<const int *>(val) + start + first + j * step, 0));
+#pragma unroll
+    for (int j = 0; j < N; ++j) st[j] = load_if(v[j] >= 0, status + v[j], kDeleted);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (st[j] == kDeleted) v[j] = -1;
+  }
+  template <int N>
+  __device__ unsigned markables(int, const int (&v)[N]) const {
+    unsigned can = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) can |= (load_if(v[j] >= 0, gt + v[j], 0) < 0 ? 1u : 0u) << j;
+    return can;
+  }
 };
 
 struct OwnedArgs {
@@ -735,7 +757,8 @@ __device__ __forceinline__ owner::Store own_rows(const OwnedArgs &a) {
     if (tid == 0) {
       h.pool_used = 0;
       h.first_limit = a.max_iter;
-      h.count = h.wide = h.moved = 0;
+      h.count = h.wide = h.wide_at = 0;
+      h.moved = h.steps = 0;
       owner::Local &l = s.graph(0);
       l.lab[0] = a.labels;
       l.lab[1] = a.buffer;
@@ -866,7 +889,7 @@ __device__ __noinline__ int large_passes(const OwnedArgs &a, owner::Store s, int
       if (s.tiles == 0) return 0ull;
       const unsigned long long mine =
           static_cast<unsigned>((h.count & 0xffff) + (h.count >> 16) + h.wide) | (h.moved ? kSumMoved : 0ull);
-      h.count = h.wide = 0;
+      h.count = h.wide = h.wide_at = 0;
       h.moved = 0;
       return mine;
     }, sum);
@@ -938,8 +961,8 @@ __global__ void __launch_bounds__(kOwnBlock, 1) prop_owned_kernel(const __grid_c
       try_small = false;  // at least one pass on the owned rows
       continue;
     }
-    k = s.n() <= kOwnBlock ? large_passes<true>(a, s, k, small_from, empty)
-                           : large_passes<false>(a, s, k, small_from, empty);
+    const bool tiles = s.n() <= kOwnBlock && s.head().steps <= owner::kTileSteps;
+    k = tiles ? large_passes<true>(a, s, k, small_from, empty) : large_passes<false>(a, s, k, small_from, empty);
     if (k < 0) return;
     try_small = true;
   }

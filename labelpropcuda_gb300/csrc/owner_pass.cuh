@@ -60,7 +60,9 @@ struct Head {
   int first_limit;       // the smallest limit of the graphs
   int count;             // rows of the pass: short | long << 16
   int wide;              // its rows of more than 32 entries
+  int wide_at;           // of them in the list
   int moved;
+  int steps;             // the most steps that a tile's rows take a warp (tile_steps)
   // what every pass reads
   unsigned *marks;
   unsigned plane;
@@ -156,6 +158,19 @@ __device__ __forceinline__ unsigned pool_of(unsigned m) { return m & kNoPool; }
 __device__ __forceinline__ int len_of(unsigned m) { return static_cast<int>((m >> 15) & 63u); }
 __device__ __forceinline__ int graph_of(unsigned m) { return static_cast<int>(m >> 21); }
 
+// Steps of a warp that runs all rows of a tile (tile_rows): 32 short rows, 8 long
+// ones or a wide one each. Beyond kTileSteps a block's rows are listed and dealt out to
+// all its warps, also where it owns at most 32 vertices per warp: 2,000 vertices of
+// degree 100 are a tile a block, whose warp ran 32 rows one after the other while 31
+// waited. Measured, 8 batches in milliseconds over lists, always by tiles, and so:
+// 2,000 vertices of degree 100 5.3, 10.5 and 2.8; 20,000 of degree 100 5.9, 8.6 and 4.3;
+// 5,000 of degree 20 6.9, 3.9 and 3.5; 20,000 of degree 12 13.7, 6.6 and 6.5. (With 4
+// steps the last two take 4.1 and 7.1.)
+constexpr int kTileSteps = 2;
+__device__ __forceinline__ int tile_steps(const Kinds &c) {
+  return (c.shorts != 0) + (__popc(c.longs) + 32 / kLongLanes - 1) / (32 / kLongLanes) + __popc(c.wides);
+}
+
 // The tiles of the launch are dealt out to the blocks but the first in turn. A
 // contiguous range per block would follow the graphs and the vertex ids, and so
 // do frontiers: some graphs have converged while others have a quarter of
@@ -176,7 +191,10 @@ __device__ __forceinline__ unsigned flat_of(int i) {
 // Graph: kCounts, whether visits and last passes of the rows are kept (their
 // reader has to clear them every kMaxStint passes); graphs(); nodes(g); row(g, v) {start, length}; active(g, v): v can be in
 // a frontier; markable(g, v): v is marked as a neighbour (every active vertex
-// is); entry(g, at, v, w), v = -1 for an entry that does not count.
+// is); entry(g, at, v, w), v = -1 for an entry that does not count; entries<N>(g,
+// start, e, step, len, v, w), N of them from start + e on, v = -1 also for those from
+// start + len on, and markables<N>(g, v), a bit for each that is markable, both with
+// the loads of all N in flight together.
 template <class Graph>
 __device__ void load(const Store &s, const Graph &gr) {
   const int tid = threadIdx.x, lane = tid & 31;
@@ -213,7 +231,10 @@ __device__ void load(const Store &s, const Graph &gr) {
     kinds.shorts = __ballot_sync(0xffffffffu, active && len <= kLaneEntries);
     kinds.longs = __ballot_sync(0xffffffffu, active && len > kLaneEntries && len <= kMaxRow);
     kinds.wides = __ballot_sync(0xffffffffu, active && len > kMaxRow);
-    if (lane == 0) s.kinds(i / kTile) = kinds;
+    if (lane == 0) {
+      s.kinds(i / kTile) = kinds;
+      atomicMax(&h.steps, tile_steps(kinds));
+    }
     if (!fits) continue;  // lanes of the next round reconverge at its first shuffle
     for (int b = 0; b < want; b += kLaneEntries) {
       int u[kLaneEntries];
@@ -365,8 +386,10 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
 }
 
 // A row of more than 32 entries by a warp, from global memory: slots lane + 32 j
-// of 256, then the tree.
-template <bool MARK = true, class Graph>
+// of 256, then the tree. AHEAD entries a lane in flight: with four, a step is three
+// trips to L2 (entries, what the caller knows of the neighbours, labels) for 128
+// entries; passes over tiles, which have few such rows, have no registers for that.
+template <bool MARK, int AHEAD, class Graph>
 __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i, int k, float delta, bool fast,
                                          unsigned *next) {
   const int lane = threadIdx.x & 31;
@@ -380,14 +403,18 @@ __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i,
   for (int j = 0; j < 8; ++j) sw[j] = sl[j] = 0.0f;
   for (int p = 0; p < ri.y; p += 256) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int e = p + j * 32 + lane;
-      int u = -1;
-      float w = 0.0f;
-      if (e < ri.y) gr.entry(g, ri.x + e, u, w);
-      if (u >= 0) {
-        sw[j] = sw[j] + w;
-        sl[j] = __fmaf_rn(w, __ldcg(src + u), sl[j]);
+    for (int j0 = 0; j0 < 8; j0 += AHEAD) {
+      const int e = p + j0 * 32 + lane;
+      if (e - lane >= ri.y) break;
+      int u[AHEAD];
+      float w[AHEAD], x[AHEAD];
+      gr.template entries<AHEAD>(g, ri.x, e, 32, ri.y, u, w);
+#pragma unroll
+      for (int j = 0; j < AHEAD; ++j) x[j] = gather(src, static_cast<unsigned>(u[j]));
+#pragma unroll
+      for (int j = 0; j < AHEAD; ++j) {
+        sw[j0 + j] = u[j] >= 0 ? sw[j0 + j] + w[j] : sw[j0 + j];
+        sl[j0 + j] = u[j] >= 0 ? __fmaf_rn(w[j], x[j], sl[j0 + j]) : sl[j0 + j];
       }
     }
   }
@@ -415,11 +442,14 @@ __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i,
   }
   if (!(fabsf(nl - old) > delta)) return false;
   if constexpr (MARK) {
-    for (int e = lane; e < ri.y; e += 32) {
-      int u = -1;
-      float w;
-      gr.entry(g, ri.x + e, u, w);
-      if (u >= 0 && gr.markable(g, u)) next[l.flat + u] = 1;
+    for (int e = lane; e - lane < ri.y; e += AHEAD * 32) {
+      int u[AHEAD];
+      float w[AHEAD];
+      gr.template entries<AHEAD>(g, ri.x, e, 32, ri.y, u, w);
+      const unsigned can = gr.template markables<AHEAD>(g, u);
+#pragma unroll
+      for (int j = 0; j < AHEAD; ++j)
+        if ((can >> j) & 1u) next[l.flat + u[j]] = 1;
     }
     if (lane == 0) next[l.flat + v] = 1;
   }
@@ -466,7 +496,7 @@ __device__ __forceinline__ bool tile_rows(const Store &s, const Graph &gr, int f
     for (int q = 32 / kLongLanes; q > 0 && longs; --q) longs &= longs - 1;
   }
   for (; wides; wides &= wides - 1)
-    moved |= wide_row(s, gr, first + __ffs(wides) - 1, k, delta, fast, next);
+    moved |= wide_row<true, 1>(s, gr, first + __ffs(wides) - 1, k, delta, fast, next);
   return __any_sync(0xffffffffu, moved);
 }
 
@@ -550,7 +580,7 @@ __device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned *
       shorts[j] = c.shorts;
       longs[j] = c.longs;
       add += __popc(c.shorts) + (__popc(c.longs) << 16);
-      if ((c.wides >> lane) & 1u) {  // a warp's work each: found again below
+      if ((c.wides >> lane) & 1u) {  // listed below
         atomicAdd(&h.wide, 1);
         s.visits(i) |= kWideRow;
       }
@@ -571,23 +601,23 @@ __device__ __forceinline__ void pass(const Store &s, const Graph &gr, unsigned *
     }
   }
   __syncthreads();
-  const int nw = h.wide;
-  bool moved = listed_rows<true>(s, gr, h.count & 0xffff, h.count >> 16, k, delta, fast, next);
-  if (nw)
-    for (int b = warp * 32; b < n; b += nwarps * 32) {
-      unsigned todo = __ballot_sync(0xffffffffu, (s.visits(b + lane) & kWideRow) != 0);
-      for (; todo; todo &= todo - 1) {
-        const int i = b + __ffs(todo) - 1;
-        if (lane == 0) s.visits(i) &= static_cast<unsigned short>(~kWideRow);
-        __syncwarp();
-        moved |= wide_row(s, gr, i, k, delta, fast, next);
+  const int nw = h.wide, ns = h.count & 0xffff, nl = h.count >> 16;
+  bool moved = listed_rows<true>(s, gr, ns, nl, k, delta, fast, next);
+  if (nw) {  // the room between the short and the long rows holds them
+    for (int i = tid; i < n; i += blockDim.x)
+      if (s.visits(i) & kWideRow) {
+        s.visits(i) &= static_cast<unsigned short>(~kWideRow);
+        s.list(ns + atomicAdd(&h.wide_at, 1)) = static_cast<unsigned short>(i);
       }
-    }
+    __syncthreads();
+    for (int q = warp; q < nw; q += nwarps) moved |= wide_row<true, 4>(s, gr, s.list(ns + q), k, delta, fast, next);
+  }
   if (__any_sync(0xffffffffu, moved) && lane == 0) h.moved = 1;
 }
 
-// All active rows of the block into the list, once; then dense_pass runs them
-// (no marks): every active vertex takes the average of its neighbours.
+// All active rows of the block into the list, once (the wide ones behind the short
+// ones); then dense_pass runs them (no marks): every active vertex takes the average
+// of its neighbours.
 __device__ __forceinline__ void list_all(const Store &s) {
   const int lane = threadIdx.x & 31, n = s.n();
   Head &h = s.head();
@@ -595,15 +625,16 @@ __device__ __forceinline__ void list_all(const Store &s) {
     const Kinds c = s.kinds(i / kTile);
     const int add = __popc(c.shorts) + (__popc(c.longs) << 16);
     int at = 0;
-    if (lane == 0) {
-      if (add) at = atomicAdd(&h.count, add);
-      if (c.wides) atomicAdd(&h.wide, 1);
-    }
+    if (lane == 0 && add) at = atomicAdd(&h.count, add);
     at = __shfl_sync(0xffffffffu, at, 0);
     const unsigned bit = 1u << lane, below = bit - 1u;
     if (c.shorts & bit) s.list((at & 0xffff) + __popc(c.shorts & below)) = static_cast<unsigned short>(i);
     if (c.longs & bit) s.list(n - 1 - (at >> 16) - __popc(c.longs & below)) = static_cast<unsigned short>(i);
   }
+  __syncthreads();
+  const int ns = h.count & 0xffff;
+  for (int i = threadIdx.x; i < n; i += blockDim.x)
+    if ((s.kinds(i / kTile).wides >> lane) & 1u) s.list(ns + atomicAdd(&h.wide, 1)) = static_cast<unsigned short>(i);
   __syncthreads();
 }
 
@@ -611,11 +642,10 @@ template <class Graph>
 __device__ __forceinline__ void dense_pass(const Store &s, const Graph &gr, int k, float delta) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   Head &h = s.head();
-  bool moved = listed_rows<false>(s, gr, h.count & 0xffff, h.count >> 16, k, delta, false, nullptr);
-  if (h.wide)
-    for (int tile = warp; tile < s.tiles; tile += nwarps)
-      for (unsigned w = s.kinds(tile).wides; w; w &= w - 1)
-        moved |= wide_row<false>(s, gr, tile * kTile + __ffs(w) - 1, k, delta, false, nullptr);
+  const int ns = h.count & 0xffff;
+  bool moved = listed_rows<false>(s, gr, ns, h.count >> 16, k, delta, false, nullptr);
+  for (int q = warp; q < h.wide; q += nwarps)
+    moved |= wide_row<false, 4>(s, gr, s.list(ns + q), k, delta, false, nullptr);
   if (__any_sync(0xffffffffu, moved) && lane == 0) h.moved = 1;
 }
 

@@ -35,6 +35,19 @@ struct Checked {
     v = col[at];
     w = val[at];
   }
+  template <int N>
+  void entries(int g, int first, int e, int step, int len, int (&v)[N], float (&w)[N]) const {
+    for (int j = 0; j < N; ++j) {
+      v[j] = -1;
+      if (e + j * step < len) entry(g, first + e + j * step, v[j], w[j]);
+    }
+  }
+  template <int N>
+  unsigned markables(int g, const int (&v)[N]) const {
+    unsigned can = 0;
+    for (int j = 0; j < N; ++j) can |= (v[j] >= 0 && markable(g, v[j]) ? 1u : 0u) << j;
+    return can;
+  }
 };
 
 // Rows of `len(v)` entries at the vertices after v, weights by position.
@@ -115,7 +128,7 @@ int main(int argc, char **argv) {
       pass(r.s, r.g, r.marks[0].data(), r.marks[1].data(), 0, 2.0f, false, each);
       __syncthreads();
       if (threadIdx.x == 0) {
-        r.s.head().count = r.s.head().wide = 0;
+        r.s.head().count = r.s.head().wide = r.s.head().wide_at = 0;
         r.marks[1][0] = 1;
         r.lab[0][3] = 7.0f;  // what pass 1 must not touch
       }

@@ -116,3 +116,24 @@ def test_recompute_matches_restatement(gpu, n, degree, limit):
     N.check(N.lib().dlp_irlp(*[x.ptr for x in d], n, ctypes.c_float(1e-3), limit, ctypes.byref(used), None))
     assert used.value == want[1]
     assert d[3].get().tobytes() == want[0].tobytes()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,degree,limit", [(70, 60, 3), (600, 100, 6), (5000, 34, 2)])
+def test_long_rows_are_dealt_out(gpu, n, degree, limit):
+    """Most rows of more than 32 entries, in blocks of one tile and of two."""
+    row, col, val, labels, status, gt, aff = inputs(n, degree, 0.6, n + degree)
+    for entry in ("dlp_iterative_propagation", "dlp_irlp"):
+        d = [DeviceArray(x) for x in (row, col, val, labels, labels, status, gt, aff)]
+        used = ctypes.c_int(-1)
+        if entry == "dlp_irlp":
+            want = recompute(row, col, val, labels, status, gt, 1e-3, limit)
+            N.check(N.lib().dlp_irlp(*[d[i].ptr for i in (0, 1, 2, 3, 5, 6)], n, ctypes.c_float(1e-3), limit,
+                                     ctypes.byref(used), None))
+        else:
+            want = propagate(row, col, val, labels, status, gt, aff, 1e-3, limit)
+            N.check(N.lib().dlp_iterative_propagation(*[x.ptr for x in d], n, ctypes.c_float(1e-3), limit,
+                                                      ctypes.byref(used), None))
+            np.testing.assert_array_equal(d[7].get(), want[1])
+        assert used.value == want[-1]
+        assert d[3].get().tobytes() == want[0].tobytes()

@@ -147,3 +147,22 @@ def test_launches_of_few_passes_among_longer_ones(gpu, oracle, solo):
                 assert got[k] == want[k], (i, nxt[i] - 1, k)
             assert eng.labels(g).tobytes() == orcs[i].labels().tobytes(), (i, nxt[i] - 1)
         step += 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,degree,solo", [(2000, 100, 0), (2000, 100, 7), (9700, 17, 0), (12000, 40, 7), (200000, 40, 0)])
+def test_rows_that_take_a_tile_many_steps(gpu, oracle, n, degree, solo):
+    """Rows of more than 8 and of more than 32 entries in most places: dealt out to
+    all warps of a block, whether or not it owns more than 32 vertices per warp."""
+    p = dlp.Problem(n, degree, 4, 7, cache_dir="")
+    cap = 40
+    orc = oracle.OracleRun.from_problem(p, record=n < 10000, threads=8, max_iterations=cap)
+    sess = dlp.Session.from_problem(p, record=n < 10000, max_iterations=cap, small_frontier_solo=solo)
+    for b, batch in enumerate(p.batches):
+        if n < 10000:
+            check_batch(b, sess.apply(b, batch), orc.apply(b, batch), sess, orc, oracle)
+            continue
+        got, want = sess.apply(b, batch), orc.apply(b, batch)
+        for k in EXACT_STATS:
+            assert got[k] == want[k], (b, k)
+        assert sess.labels().tobytes() == orc.labels().tobytes(), b
