@@ -323,15 +323,14 @@ int dlp_engine_artefact(dlp_engine *e, int graph_id, int which, void *host_out, 
  * Propagation runs each pass on one block or the whole grid by the size of the
  * frontier; in launches of more than 3.1 million vertices it sends rows of at
  * most 32 live entries to groups of narrow_lanes lanes and longer rows to whole
- * warps. The lane width of the short-row bucket, the frontier threshold
- * (solo_entry; subgrid_entry has no effect) and the persistent grid's blocks per
- * SM are chosen by timing every candidate (lanes 1/4/8 x one-block entry
- * 256/512/1024 x subgrid_entry 1024/2048/4096 x the blocks per SM the build
- * allows) on a sample the library generates with the reference generator:
- * num_graphs graphs of sizes[i] vertices and average degree degrees[i],
- * `batches` batches each, propagation capped at max_iterations passes per
- * batch for the trial. Every candidate must give identical statistics
- * (checked). The fastest is written into cfg->narrow_lanes,
+ * warps. Candidates are lanes 1/4/8 x one-block entry (solo_entry) 256/512/1024
+ * x subgrid_entry 1024/2048/4096 (without effect) x the blocks per SM the build
+ * allows. A sample that the library generates with the reference generator
+ * (num_graphs graphs of sizes[i] vertices and average degree degrees[i],
+ * `batches` batches each, propagation capped at max_iterations passes per batch)
+ * is timed at every solo_entry as such a launch runs, and at every lane width over
+ * frontier lists; a candidate's time is the sum of its two. All must give identical
+ * statistics (checked). The fastest is written into cfg->narrow_lanes,
  * cfg->blocks_per_sm, cfg->solo_entry and cfg->subgrid_entry; other fields are
  * kept. */
 typedef struct {
@@ -341,7 +340,7 @@ typedef struct {
   int blocks_per_sm[32];
   int solo_entry[32];
   int subgrid_entry[32];
-  double ms[32];          /* summed device time of the sample's steps */
+  double ms[32];          /* device time of the sample's steps, the two runs summed */
 } dlp_tune_report;
 int dlp_autotune(dlp_config *cfg, int num_graphs, const int *sizes, const int *degrees, int batches,
                  int max_iterations, dlp_tune_report *report);

@@ -494,12 +494,12 @@ class Engine:
 
 def autotune(sizes: list[int], degrees: list[int], batches: int = 10, max_iterations: int = 2000,
              **config) -> dict:
-    """Times every launch-shape candidate (lanes per short row x one-block
-    frontier threshold x subgrid_entry, which has no effect, x blocks per SM) on a generated sample of
-    the given graph sizes and degrees and returns the fastest as
-    {"narrow_lanes", "blocks_per_sm", "engine_kw": {solo_entry, subgrid_entry},
-    "candidates"}; every candidate gave the same statistics (checked by the
-    library)."""
+    """Times a generated sample of the given graph sizes and degrees at every
+    one-block frontier threshold and, over frontier lists, at every lane width
+    per short row (x blocks per SM), and returns the candidate with the smallest
+    sum as {"narrow_lanes", "blocks_per_sm", "engine_kw": {solo_entry,
+    subgrid_entry (without effect)}, "candidates"}; every run gave the same
+    statistics (checked by the library)."""
     L = _n.lib()
     cfg = _n.Config()
     L.dlp_config_default(ctypes.byref(cfg))

@@ -2,20 +2,21 @@
 // dlp_gb300.h). No counterpart in the reference, whose launch shapes are
 // fixed (256-thread blocks, one block per row, src/iterativePropagation.cu).
 //
-// The engine's propagation splits rows into two degree buckets: rows of at
-// most 32 live entries go to groups of `narrow_lanes` lanes (4, 8, 16 or 32;
-// or 1: a lane per row of at most 8 entries), longer rows to whole warps (in
-// launches beyond owned rows; those have a fixed split, owner_pass.cuh). Each
-// pass also picks its launch mode by the total frontier: one block (up to
-// solo_entry vertices) or the whole grid. The tunables are the lane width of the
-// short-row bucket, the frontier threshold and the persistent grid's blocks per
-// SM (one for the 1,024-thread build); subgrid_entry is still a field of every
-// candidate, without effect. The best choice depends on the row lengths and
-// frontier sizes of the workload. The tuner builds a
-// sample workload with the reference generator (graph sizes and degrees given
-// by the caller), times every candidate on it with CUDA events (the engine's
-// own step events), checks that every candidate produced the same statistics
-// (the arithmetic does not depend on the launch shape) and keeps the fastest.
+// Each pass of the engine's propagation picks its launch mode by the total
+// frontier: one block (up to solo_entry vertices) or the whole grid. In launches
+// over frontier lists, rows of at most 32 live entries go to groups of
+// `narrow_lanes` lanes (4, 8, 16 or 32; or 1: a lane per row of at most 8 entries),
+// longer rows to whole warps; on owned rows the split is fixed (owner_pass.cuh). The
+// tunables are the frontier threshold, the lane width and the persistent grid's
+// blocks per SM (one for the 1,024-thread build); subgrid_entry is still a field of
+// every candidate, without effect. The best choice depends on the row lengths and
+// frontier sizes of the workload. The tuner builds a sample workload with the
+// reference generator (graph sizes and degrees given by the caller), times it with
+// CUDA events (the engine's own step events) at every threshold on owned rows and at
+// every lane width over lists, whatever the sample's size, checks that all gave the
+// same statistics (the arithmetic does not depend on the launch shape) and keeps the
+// candidate with the smallest sum of the two. (Timed as candidates on owned rows, the
+// lane widths differed by 0.3%, which chose one at random for launches over lists.)
 #include <algorithm>
 #include <cstring>
 #include <memory>
@@ -37,11 +38,17 @@ struct EngineDeleter {
 };
 using EnginePtr = std::unique_ptr<dlp_engine, EngineDeleter>;
 
-// Runs the sample on one candidate; returns device ms and the statistics.
+// Runs the sample with one setting; returns device ms and the statistics. lists: all
+// passes over frontier lists, as in launches beyond owned rows (a budget that holds
+// the graphs has no room for the marks that owned rows need).
 int trial(const dlp_config &cfg, const std::vector<ProblemPtr> &probs, int batches,
-          const std::vector<std::vector<int>> &bmaps, double *ms, std::vector<dlp_batch_stats> *stats) {
+          const std::vector<std::vector<int>> &bmaps, bool lists, double *ms, std::vector<dlp_batch_stats> *stats) {
+  size_t budget = 0;
+  if (lists)
+    for (const ProblemPtr &p : probs)
+      budget += dlp_engine_graph_bytes(dlp_problem_num_nodes(p.get()), dlp_problem_num_edges(p.get()), 1, 1, 0);
   dlp_engine *raw = nullptr;
-  DLP_TRY(dlp_engine_create(&cfg, static_cast<int>(probs.size()), 0, &raw));
+  DLP_TRY(dlp_engine_create(&cfg, static_cast<int>(probs.size()), budget, &raw));
   EnginePtr eng(raw);
   std::vector<int> gids(probs.size());
   for (size_t i = 0; i < probs.size(); ++i) {
@@ -124,36 +131,43 @@ int dlp_autotune(dlp_config *cfg, int num_graphs, const int *sizes, const int *d
   dlp_tune_report rep;
   std::memset(&rep, 0, sizeof(rep));
   std::vector<dlp_batch_stats> ref_stats;
+  auto timed = [&](int blocks, int lanes, int solo, bool lists, double *ms) -> int {
+    dlp_config c = *cfg;
+    c.narrow_lanes = lanes;
+    c.blocks_per_sm = blocks;
+    c.solo_entry = solo;
+    c.max_iterations = max_iterations;
+    c.record = 0;
+    std::vector<dlp_batch_stats> st;
+    DLP_TRY(trial(c, probs, batches, bmaps, lists, ms, &st));
+    if (ref_stats.empty()) ref_stats = st;
+    else if (!same_stats(ref_stats, st))
+      return dlp::fail(DLP_ERR_INTERNAL, "launch shapes disagree on the sample's statistics");
+    return DLP_OK;
+  };
   double best = -1.0;
-  for (int bl : kBlocks)
-    for (int ln : kLanes)
-      for (int se : kSoloEntries)
+  for (int bl : kBlocks) {
+    // Each setting where it has an effect: the threshold on owned rows, the lane width
+    // over lists.
+    double by_solo[3], by_lanes[3];
+    for (int i = 0; i < 3; ++i) DLP_TRY(timed(bl, 0, kSoloEntries[i], false, &by_solo[i]));
+    for (int i = 0; i < 3; ++i) DLP_TRY(timed(bl, kLanes[i], cfg->solo_entry, true, &by_lanes[i]));
+    for (int ln = 0; ln < 3; ++ln)
+      for (int se = 0; se < 3; ++se)
         for (int ge : kSubEntries) {
           if (rep.candidates >= kTuneMaxCandidates) break;
-          dlp_config c = *cfg;
-          c.narrow_lanes = ln;
-          c.blocks_per_sm = bl;
-          c.solo_entry = se;
-          c.subgrid_entry = ge;
-          c.max_iterations = max_iterations;
-          c.record = 0;
-          double ms = 0.0;
-          std::vector<dlp_batch_stats> st;
-          DLP_TRY(trial(c, probs, batches, bmaps, &ms, &st));
-          if (ref_stats.empty()) ref_stats = st;
-          else if (!same_stats(ref_stats, st))
-            return dlp::fail(DLP_ERR_INTERNAL, "launch shapes disagree on the sample's statistics");
           const int k = rep.candidates++;
-          rep.lanes[k] = ln;
+          rep.lanes[k] = kLanes[ln];
           rep.blocks_per_sm[k] = bl;
-          rep.solo_entry[k] = se;
+          rep.solo_entry[k] = kSoloEntries[se];
           rep.subgrid_entry[k] = ge;
-          rep.ms[k] = ms;
-          if (best < 0.0 || ms < best) {
-            best = ms;
+          rep.ms[k] = by_solo[se] + by_lanes[ln];
+          if (best < 0.0 || rep.ms[k] < best) {
+            best = rep.ms[k];
             rep.best = k;
           }
         }
+  }
   cfg->narrow_lanes = rep.lanes[rep.best];
   cfg->blocks_per_sm = rep.blocks_per_sm[rep.best];
   cfg->solo_entry = rep.solo_entry[rep.best];

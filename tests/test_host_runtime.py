@@ -178,3 +178,14 @@ def test_server_keeps_its_budget(runtime):
             eng = dlp.Engine(2)
             g = eng.add_problem(p)
     eng.close()
+
+
+def test_autotuner_times_each_setting_where_it_has_an_effect(runtime):
+    """Three one-block thresholds on owned rows and three lane widths over lists, two
+    batches each, and the choice among all combinations of them."""
+    r = dlp.autotune([500, 300], [3, 5], batches=2, max_iterations=10)
+    kernels = [x[1] for x in runtime.log() if x[0] == "cooperative"]
+    owned, lists = ("engine_kernelILi8ELb1", "engine_kernelILi%dELb0")
+    want = 3 * 2 * [owned] + [lists % lanes for lanes in (1, 4, 8) for _ in range(2)]
+    assert len(kernels) == len(want) and all(w in k for w, k in zip(want, kernels)), kernels
+    assert len({(c["narrow_lanes"], c["solo_entry"], c["subgrid_entry"]) for c in r["candidates"]}) == 27
