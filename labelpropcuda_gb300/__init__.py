@@ -523,15 +523,13 @@ def device_name(device: int = 0) -> str:
 
 
 def _kernel_digest() -> str:
-    """Digest of the engine kernel's sources: a tuned shape is only reused for
-    the kernel it was measured on."""
+    """Digest of the library's device sources and of the tuner: a tuned shape is
+    only reused for the kernels it was measured on."""
     import hashlib
     from pathlib import Path
     h = hashlib.sha256()
-    for name in ("engine_kernel.cu", "engine.cuh", "row_sums.cuh", "session_kernel.cuh", "tune.cu"):
-        f = Path(__file__).resolve().parent / "csrc" / name
-        if f.exists():
-            h.update(f.read_bytes())
+    for f in sorted((Path(__file__).resolve().parent / "csrc").glob("*.cu*")):
+        h.update(f.read_bytes())
     return h.hexdigest()[:16]
 
 

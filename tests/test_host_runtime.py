@@ -189,3 +189,17 @@ def test_autotuner_times_each_setting_where_it_has_an_effect(runtime):
     want = 3 * 2 * [owned] + [lists % lanes for lanes in (1, 4, 8) for _ in range(2)]
     assert len(kernels) == len(want) and all(w in k for w, k in zip(want, kernels)), kernels
     assert len({(c["narrow_lanes"], c["solo_entry"], c["subgrid_entry"]) for c in r["candidates"]}) == 27
+
+
+def test_tuned_shapes_are_kept_for_the_kernels_they_were_measured_on(tmp_path, monkeypatch):
+    """The cache key changes with every source that the engine's kernels include."""
+    import shutil
+    src = Path(dlp.__file__).resolve().parent / "csrc"
+    shutil.copytree(src, tmp_path / "csrc")
+    monkeypatch.setattr(dlp, "__file__", str(tmp_path / "__init__.py"))
+    seen = {dlp._kernel_digest()}
+    for name in ("engine_kernel.cu", "engine.cu", "owner_pass.cuh", "row_stint.cuh", "common.cuh", "tune.cu"):
+        with open(tmp_path / "csrc" / name, "a") as f:
+            f.write("// \n")
+        assert dlp._kernel_digest() not in seen, name
+        seen.add(dlp._kernel_digest())
