@@ -1,5 +1,7 @@
 // C ABI plumbing: error reporting, device checks, the problem (input
 // generation) object and small device helpers for bindings.
+#include <cuda.h>
+
 #include <atomic>
 #include <cerrno>
 #include <cstdio>
@@ -56,6 +58,25 @@ int require_device() {
                                        std::to_string(minor));
   if (dev >= 0 && dev < kMaxDevices) passed[dev].store(true, std::memory_order_relaxed);
   return DLP_OK;
+}
+
+unsigned long long context_id() {
+  using GetId = CUresult (*)(CUcontext, unsigned long long *);
+  static const GetId get = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    cudaGetLastError();
+    return reinterpret_cast<GetId>(p);
+  }();
+  unsigned long long id = 0;
+  if (!get) return 0;
+  if (get(nullptr, &id) == CUDA_SUCCESS) return id;
+  cudaFree(nullptr);  // makes the device's context current where none is
+  cudaGetLastError();
+  return get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
 }
 
 int launch_cooperative(const void *kernel, int grid, int block, void **args, size_t smem,

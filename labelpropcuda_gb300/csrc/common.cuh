@@ -339,6 +339,12 @@ __device__ __forceinline__ float label_by_recip(float w_all, float recip, float 
   return fminf(fmaxf(divide(w_label, w_all, recip), 0.0f), 1.0f);
 }
 
+// The current device's context: an id that no other context of the process has had, 0
+// when there is none to be asked. What a host function keeps for a device (a pool,
+// an address, a kernel's attributes) is lost with the context, which
+// cudaDeviceReset ends, and is kept by this id. 12 ns.
+unsigned long long context_id();
+
 // Launch helper: cooperative launch of `kernel` with `args` on `stream`.
 int launch_cooperative(const void *kernel, int grid, int block, void **args, size_t smem,
                        cudaStream_t stream);

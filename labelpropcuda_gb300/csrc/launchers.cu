@@ -14,7 +14,9 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <utility>
 
 #include "common.cuh"
 #include "owner_pass.cuh"
@@ -48,51 +50,62 @@ int grid_for(long long items, int per_block) {
 // synchronisation, and the next call maps it again: 200 us a call for a caller
 // that synchronises the device between calls.) The driver orders its blocks
 // between streams and threads; what a call allocates beyond the limit goes back
-// at the next synchronisation, the rest when the library is unloaded.
+// at the next synchronisation, the rest with the device's context.
 constexpr unsigned long long kPoolBytes = 32ull << 20;
 
-class TmpPools {
- public:
-  // The current device's pool, or null where there is none (the default pool
-  // serves then).
-  cudaMemPool_t current() {
-    int dev = -1;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return nullptr;
-    std::lock_guard<std::mutex> lock(mu_);
-    if (!asked_[dev]) {
-      asked_[dev] = true;
+// What the launchers keep for a device's context, made when it is first asked for.
+struct ContextFacts {
+  bool pool_asked = false;
+  cudaMemPool_t pool = nullptr;  // null: the default pool serves
+  bool shape_asked = false;
+  int owned_grid = 0;            // blocks of the owned kernels, 0 when they do not fit
+  size_t owned_fixed = 0, owned_smem = 0;  // their static shared memory, the most of the dynamic one
+  void *scratch = nullptr;       // of dlp_iterative_propagation_noalloc
+};
+
+// fn on the facts of the current device's context, one thread at a time; false when
+// the context cannot be told.
+template <class Fn>
+bool with_context(Fn fn) {
+  static std::mutex mu;
+  // not destroyed at the end of the process, when the contexts are gone already
+  static auto &known = *new std::map<std::pair<int, unsigned long long>, ContextFacts>();
+  int dev = -1;
+  const unsigned long long id = context_id();
+  if (id == 0 || cudaGetDevice(&dev) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> lock(mu);
+  fn(known[{dev, id}], dev);
+  return true;
+}
+
+// The current device's pool, null for the default one.
+cudaMemPool_t tmp_pool() {
+  cudaMemPool_t pool = nullptr;
+  with_context([&](ContextFacts &f, int dev) {
+    if (!f.pool_asked) {
+      f.pool_asked = true;
       cudaMemPoolProps props{};
       props.allocType = cudaMemAllocationTypePinned;
       props.location.type = cudaMemLocationTypeDevice;
       props.location.id = dev;
       unsigned long long keep = kPoolBytes;
-      if (cudaMemPoolCreate(&pool_[dev], &props) != cudaSuccess) pool_[dev] = nullptr;
-      else cudaMemPoolSetAttribute(pool_[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+      // in a thread that captures a stream, too: the pool is no part of the graph
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (cudaMemPoolCreate(&f.pool, &props) != cudaSuccess) f.pool = nullptr;
+      else cudaMemPoolSetAttribute(f.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      cudaThreadExchangeStreamCaptureMode(&mode);
       cudaGetLastError();
     }
-    return pool_[dev];
-  }
-  ~TmpPools() {
-    for (cudaMemPool_t p : pool_)
-      if (p) cudaMemPoolDestroy(p);
-  }
-
- private:
-  static constexpr int kDevices = 64;
-  std::mutex mu_;
-  bool asked_[kDevices] = {};
-  cudaMemPool_t pool_[kDevices] = {};
-};
-
-TmpPools &tmp_pools() {
-  static TmpPools pools;
-  return pools;
+    pool = f.pool;
+  });
+  return pool;
 }
 
 template <class T>
 int tmp_alloc(T **p, size_t count, cudaStream_t s) {
   const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-  cudaMemPool_t pool = tmp_pools().current();
+  cudaMemPool_t pool = tmp_pool();
   if (pool) DLP_CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void **>(p), bytes, pool, s));
   else DLP_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void **>(p), bytes, s));
   return DLP_OK;
@@ -1186,21 +1199,14 @@ int run_step(const void *kernel, const char *what, const char *invalid, long lon
 constexpr size_t kOwnedSmall = 256, kOwnedFixed = 256 + sizeof(SumBarrier);
 static_assert(sizeof(int) * kOutWords <= kOwnedSmall && kOwnedFixed % 16 == 0, "scratch layout");
 
-// Facts about a device that the owned kernels' launches need, queried once.
+// What the owned kernels' launches need to know of the device.
 struct OwnedShape {
-  int grid = 0;            // 0: the kernels do not fit this device
+  int grid = 0;                // 0: the kernels do not fit this device
   size_t fixed = 0, smem = 0;  // static shared memory, the most of the dynamic one
 };
 
-OwnedShape owned_shape() {
-  constexpr int kMaxDevices = 64;
-  static std::mutex mu;
-  static OwnedShape known[kMaxDevices];
-  static bool asked[kMaxDevices];
-  int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return OwnedShape();
-  std::lock_guard<std::mutex> lock(mu);
-  if (asked[dev]) return known[dev];
+// Sets the kernels' attributes, which a context loses.
+OwnedShape ask_owned_shape(int dev) {
   OwnedShape s;
   int sms = 0, most = 0;
   bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
@@ -1223,8 +1229,26 @@ OwnedShape owned_shape() {
   }
   s.grid = ok ? std::min(sms, kSumBlocks) : 0;
   cudaGetLastError();
-  asked[dev] = true;
-  known[dev] = s;
+  return s;
+}
+
+OwnedShape owned_shape() {
+  OwnedShape s;
+  if (!with_context([&](ContextFacts &f, int dev) {
+        if (!f.shape_asked) {
+          const OwnedShape asked = ask_owned_shape(dev);
+          f.owned_grid = asked.grid;
+          f.owned_fixed = asked.fixed;
+          f.owned_smem = asked.smem;
+          f.shape_asked = true;
+        }
+        s.grid = f.owned_grid;
+        s.fixed = f.owned_fixed;
+        s.smem = f.owned_smem;
+      })) {
+    int dev = -1;
+    if (cudaGetDevice(&dev) == cudaSuccess) s = ask_owned_shape(dev);
+  }
   return s;
 }
 
@@ -1323,24 +1347,18 @@ static_assert(kNoAllocMaxNodes <= 150 * dlp::owner::kMaxVertices, "such graphs r
 static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
 
 namespace {
-// The array's device address, looked up once per device (the host-side name
-// of a __device__ variable is not a device address). Fixed table: no heap use.
-constexpr int kNoAllocMaxDevices = 64;
-std::mutex g_noalloc_mu;
-NoAllocScratch *g_noalloc_addr[kNoAllocMaxDevices] = {};
-
+// The array's device address, looked up once per context (the host-side name of a
+// __device__ variable is not a device address).
 int noalloc_scratch(NoAllocScratch **out) {
-  int dev = -1;
-  DLP_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= kNoAllocMaxDevices) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "device ordinal too large");
-  std::lock_guard<std::mutex> lock(g_noalloc_mu);
-  if (!g_noalloc_addr[dev]) {
-    void *p = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-    if (e != cudaSuccess) return dlp::cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)", __FILE__, __LINE__);
-    g_noalloc_addr[dev] = static_cast<NoAllocScratch *>(p);
-  }
-  *out = g_noalloc_addr[dev];
+  void *p = nullptr;
+  cudaError_t e = cudaSuccess;
+  if (!with_context([&](ContextFacts &f, int) {
+        if (!f.scratch) e = cudaGetSymbolAddress(&f.scratch, g_noalloc_scratch);
+        p = f.scratch;
+      }))
+    e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+  if (e != cudaSuccess) return dlp::cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)", __FILE__, __LINE__);
+  *out = static_cast<NoAllocScratch *>(p);
   return DLP_OK;
 }
 }  // namespace

@@ -2,6 +2,7 @@
 // memory is host memory that starts as garbage, copies and clears happen at once,
 // kernels are written down and not run, and every operation that touches memory
 // or launches is a line of a log with the stream it was issued on.
+#include <cuda.h>
 #include <cuda_runtime_api.h>
 
 #include <cstdint>
@@ -10,6 +11,7 @@
 #include <map>
 #include <set>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace {
@@ -25,6 +27,8 @@ struct State {
   std::map<const void *, std::pair<std::string, size_t>> variable;
   size_t capacity = SIZE_MAX;
   int streams = 0;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
+  bool capturing = false, spoilt = false;  // some stream; by a call it does not take
   unsigned long long context = 1;
 };
 State &st() {
@@ -81,6 +85,14 @@ void fake_clear_log() { st().log.clear(); }
 // The first `n` words of the next copy to the host.
 void fake_result(const int *words, int n) { st().result.assign(words, words + n); }
 void fake_capacity(size_t bytes) { st().capacity = bytes; }
+void fake_begin_capture() {
+  st().capturing = true;
+  st().spoilt = false;
+}
+int fake_end_capture() {
+  st().capturing = false;
+  return st().spoilt ? 1 : 0;
+}
 size_t fake_used() { return used(); }
 
 // ---- the runtime
@@ -219,6 +231,10 @@ cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t pool, cuda
 }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return give(p); }
 cudaError_t cudaMemPoolCreate(cudaMemPool_t *pool, const cudaMemPoolProps *) {
+  if (st().capturing && st().mode != cudaStreamCaptureModeRelaxed) {
+    st().spoilt = true;
+    return cudaErrorStreamCaptureUnsupported;
+  }
   *pool = reinterpret_cast<cudaMemPool_t>(std::malloc(1));
   st().pools.insert(*pool);
   return cudaSuccess;
@@ -227,6 +243,20 @@ cudaError_t cudaMemPoolDestroy(cudaMemPool_t pool) {
   return st().pools.erase(pool) ? cudaSuccess : cudaErrorInvalidValue;
 }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode *m) {
+  std::swap(*m, st().mode);
+  return cudaSuccess;
+}
+static CUresult fake_context_id(CUcontext, unsigned long long *id) {
+  *id = st().context;
+  return CUDA_SUCCESS;
+}
+cudaError_t cudaGetDriverEntryPointByVersion(const char *, void **p, unsigned, unsigned long long,
+                                             cudaDriverEntryPointQueryResult *found) {
+  *p = reinterpret_cast<void *>(&fake_context_id);
+  *found = cudaDriverEntryPointSuccess;
+  return cudaSuccess;
+}
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
   *p = std::calloc(1, n ? n : 1);
   return cudaSuccess;
@@ -246,6 +276,10 @@ cudaError_t cudaMemset(void *p, int v, size_t n) {
 }
 cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t s) {
   note("clear " + std::to_string(n) + " " + name(s));
+  auto block = st().device.upper_bound(p);  // what a lost context had is no memory
+  if (block == st().device.begin() ||
+      static_cast<char *>(p) + n > static_cast<char *>((--block)->first) + block->second)
+    return cudaErrorIllegalAddress;
   std::memset(p, v, n);
   return cudaSuccess;
 }

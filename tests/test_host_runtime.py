@@ -203,3 +203,38 @@ def test_tuned_shapes_are_kept_for_the_kernels_they_were_measured_on(tmp_path, m
             f.write("// \n")
         assert dlp._kernel_digest() not in seen, name
         seen.add(dlp._kernel_digest())
+
+
+def propagate(entry, a, n):
+    used = ctypes.c_int(0)
+    extra = [a[6].ptr, a[7].ptr] if entry != "dlp_irlp" else []
+    ptrs = [x.ptr for x in a[:6]] if entry != "dlp_irlp" else [a[i].ptr for i in (0, 1, 2, 3, 5, 6)]
+    N.check(getattr(N.lib(), entry)(*ptrs, *extra, n, ctypes.c_float(1e-4), 5, ctypes.byref(used), None))
+
+
+def test_launchers_after_a_device_reset(runtime):
+    """cudaDeviceReset ends the context with its pools, kernel attributes and the
+    addresses of device variables; the launchers work in the next one."""
+    n = 1000
+    for _ in range(3):
+        a = arrays(*[n + 1] * 8)
+        for entry in ("dlp_iterative_propagation", "dlp_irlp", "dlp_iterative_propagation_noalloc"):
+            runtime.result(5, 0)
+            propagate(entry, a, n)
+        N.check(N.lib().dlp_label_initialization(a[0].ptr, a[1].ptr, a[2].ptr, a[3].ptr, None, a[4].ptr, n, a[5].ptr, n,
+                                                 a[0].ptr, n, None))
+        for x in a:
+            x.ptr = ctypes.c_void_p()
+        runtime.lib.cudaDeviceReset()
+
+
+def test_label_initialisation_while_a_stream_captures(runtime):
+    """It waits for nothing and can be part of a graph, also as the first call of a
+    context: making the pool must not spoil the capture."""
+    runtime.lib.cudaDeviceReset()
+    n = 100
+    a = arrays(*[n + 1] * 6)
+    runtime.lib.fake_begin_capture()
+    N.check(N.lib().dlp_label_initialization(a[0].ptr, a[1].ptr, a[2].ptr, a[3].ptr, None, a[4].ptr, n, a[5].ptr, n,
+                                             a[0].ptr, n, None))
+    assert runtime.lib.fake_end_capture() == 0
