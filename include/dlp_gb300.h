@@ -487,7 +487,7 @@ int dlp_iterative_propagation(const int *d_row_ptr, const int *d_col_ind, const 
                               void *stream);
 
 /* Same arguments and results as dlp_iterative_propagation, but allocates no
- * device memory: its scratch is a fixed array inside this library (16 MiB +
+ * device memory: its scratch is a fixed array inside this library (12 MiB +
  * 1 KiB, present on every GPU that loads the library until the process ends).
  * No counterpart in the reference, whose launchers call cudaMalloc/cudaFree on
  * every call. For callers that may not allocate device memory while running:

@@ -51,14 +51,14 @@ struct EngineCtl {
   int solo_k[2];
   int solo_passes[2];
   int solo_full[2];     // a one-block stint ended for lack of room
-  // Stop requests, written by thread 0 of block 0 and read by every block at
-  // the top of a pass: (launch tag << 32) | the pass at which to stop. A read
-  // at the top of pass k takes only a request naming pass k, so a request
-  // written during pass k (for pass k + 1) is never seen early by a block that
-  // is slow to start pass k.
   int where;            // last phase block 0 reached (1..10)
   int where_pass;       // last propagation pass block 0 started
-  unsigned long long slice_stop;  // the launch's time slice ran out
+  // The launch's time slice ran out: a request to stop, written by thread 0 of
+  // block 0 and read by every block at the top of a pass, (launch tag << 32) | the
+  // pass at which to stop. A read at the top of pass k takes only a request naming
+  // pass k, so a request written during pass k (for pass k + 1) is never seen early
+  // by a block that is slow to start pass k.
+  unsigned long long slice_stop;
   unsigned long long t_launch;  // global timer at the start of the launch (thread 0 of block 0)
   // Propagation passes run so far by mode, and the device time they took
   // (global timer): 0 one block, 1 of which by at most 16 warps, 2 unused,

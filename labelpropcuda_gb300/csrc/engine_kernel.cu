@@ -920,7 +920,7 @@ __device__ __forceinline__ bool slice_over(const EngineArgs &e) {
   return e.slice_ns != 0 && global_timer_ns() - e.ectl->t_launch > e.slice_ns;
 }
 
-// A stop request for pass k of this launch (EngineCtl::sub_stop, slice_stop).
+// A stop request for pass k of this launch (EngineCtl::slice_stop).
 __device__ __forceinline__ unsigned long long stop_code(const EngineArgs &e, int k) {
   return (static_cast<unsigned long long>(static_cast<unsigned>(e.tag)) << 32) | static_cast<unsigned>(k);
 }

@@ -518,8 +518,8 @@ struct PropArgs {
 // Frontier loop of src/iterativePropagation.cu:274-327 in one cooperative
 // launch; per pass, the frontier is the set of vertices marked in the previous
 // pass that are ACTIVE and not ground truth.
-template <int G>
 __global__ void __launch_bounds__(kBlock) prop_kernel(PropArgs a) {
+  constexpr int G = kGroup;  // lanes per row of at most kNarrowMax entries
   const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31, gwarp = t >> 5, nwarps = nt >> 5;
   const int n = a.n;
@@ -1140,15 +1140,6 @@ __global__ void __launch_bounds__(kBlock) irlp_kernel(IrlpArgs a) {
   if (t == 0) a.flags[4] = k;
 }
 
-const void *prop_kernel_ptr(int lanes) {
-  switch (lanes) {
-    case 4: return reinterpret_cast<const void *>(&prop_kernel<4>);
-    case 16: return reinterpret_cast<const void *>(&prop_kernel<16>);
-    case 32: return reinterpret_cast<const void *>(&prop_kernel<32>);
-    default: return reinterpret_cast<const void *>(&prop_kernel<8>);
-  }
-}
-
 // Blocks of a step kernel: SMs of the current device at most, queried once per
 // device; 0 when the launch is not possible.
 int step_blocks() {
@@ -1329,7 +1320,7 @@ using namespace dlp::ref_layout;
 // ---------------------------------------------------------------------------
 // Scratch of dlp_iterative_propagation_noalloc: the counters, the barrier, the
 // frontier marks and the frontier list of one propagation call on a graph of at
-// most kNoAllocMaxNodes vertices (16 MiB + 1 KiB at most). It is a
+// most kNoAllocMaxNodes vertices (12 MiB and less than 1 KiB). It is a
 // file-scope device array, so it exists on every GPU that loads this library,
 // from module load until the process exits, whether or not the entry point is
 // ever called.
@@ -1339,7 +1330,6 @@ struct NoAllocScratch {
   char fixed[kOwnedFixed];  // counters and barrier, directly before the marks: cleared with them
   unsigned marks[2 * kNoAllocMaxNodes];
   int list[kNoAllocMaxNodes];
-  int unused[kNoAllocMaxNodes];
 };
 static_assert(kNoAllocMaxNodes <= 150 * dlp::owner::kMaxVertices, "such graphs run on owned rows");
 }  // namespace
@@ -1570,7 +1560,7 @@ int dlp_iterative_propagation(const int *d_row_ptr, const int *d_col_ind, const 
   a.bar = bar;
   a.timeout_ns = 2000000000ull;
   a.fast_div = g_launcher_arith.load();
-  const void *kern = prop_kernel_ptr(8);
+  const void *kern = reinterpret_cast<const void *>(&prop_kernel);
   const int grid = coop_grid(kern);
   if (grid <= 0) return dlp::fail(DLP_ERR_CUDA, "occupancy query failed");
   void *args[] = {&a};

@@ -97,6 +97,7 @@ __device__ __forceinline__ unsigned shared_address(const void *p) {
   return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
 
+// The multiplier is that of the finaliser of MurmurHash3 (A. Appleby, public domain).
 __device__ __forceinline__ unsigned mix64(unsigned long long x) {
   x ^= x >> 33;
   x *= 0xff51afd7ed558ccdull;

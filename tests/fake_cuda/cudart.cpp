@@ -94,6 +94,11 @@ int fake_end_capture() {
   return st().spoilt ? 1 : 0;
 }
 size_t fake_used() { return used(); }
+size_t fake_variable_bytes() {  // of the library's device variables
+  size_t n = 0;
+  for (auto &v : st().variable) n += v.second.second;
+  return n;
+}
 
 // ---- the runtime
 cudaError_t cudaDeviceReset() {  // every allocation, pool and attribute is gone

@@ -21,7 +21,7 @@ class Runtime:
     def __init__(self, lib):
         self.lib = lib
         lib.fake_log.restype = ctypes.c_char_p
-        lib.fake_used.restype = ctypes.c_size_t
+        lib.fake_used.restype = lib.fake_variable_bytes.restype = ctypes.c_size_t
         lib.fake_capacity.argtypes = [ctypes.c_size_t]
 
     def log(self) -> list[list[str]]:
@@ -238,3 +238,9 @@ def test_label_initialisation_while_a_stream_captures(runtime):
     N.check(N.lib().dlp_label_initialization(a[0].ptr, a[1].ptr, a[2].ptr, a[3].ptr, None, a[4].ptr, n, a[5].ptr, n,
                                              a[0].ptr, n, None))
     assert runtime.lib.fake_end_capture() == 0
+
+
+def test_device_memory_held_by_loading_the_library(runtime):
+    """The scratch of the allocation-free propagation: three words for each of 2^20
+    vertices, and less than a KiB."""
+    assert 12 << 20 <= runtime.lib.fake_variable_bytes() <= (12 << 20) + 1024
