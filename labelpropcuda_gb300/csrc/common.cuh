@@ -32,6 +32,13 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line);
     if (s_ != DLP_OK) return s_;     \
   } while (0)
 
+// Threads per block of the persistent kernels (a build setting: 512 or 1024).
+#ifndef DLP_BLOCK
+#define DLP_BLOCK 1024
+#endif
+constexpr int kBlockThreads = DLP_BLOCK;
+static_assert(kBlockThreads == 512 || kBlockThreads == 1024, "the persistent kernels are tuned for 512 or 1024 threads");
+
 // Checks that a GPU of compute capability 10.3 is current.
 int require_device();
 

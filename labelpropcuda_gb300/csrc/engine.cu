@@ -133,6 +133,7 @@ struct dlp_engine {
   size_t used = 0;
   int lanes = 8;
   int grid = 0;
+  int owned_grid = 0;   // of launches with owned passes, a block per SM
   // Launches over frontier lists and launches with owned passes; the dynamic shared
   // memory of the former, the most of the latter beside their static one.
   const void *kernel = nullptr, *owned_kernel = nullptr;
@@ -281,7 +282,7 @@ void grow_marks(dlp_engine *e) {
   size_t want = 0;
   for (GraphSlot *g : e->graphs)
     if (g) want += owned_room(g->n);
-  want = std::min<size_t>(want, dlp::engine::owned_limit(e->grid));
+  want = std::min<size_t>(want, dlp::engine::owned_limit(e->owned_grid));
   if (e->marks_off || want <= e->mark_plane || (e->budget > 0 && e->used + 8 * want > e->budget) ||
       cudaStreamSynchronize(e->stream) != cudaSuccess)
     return;
@@ -456,7 +457,7 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
   if (opts.pass_budget > 0) passes = std::min(passes, opts.pass_budget);
   const size_t owned_smem =
       passes > dlp::engine::kListOnly && vertices <= e->mark_plane
-          ? dlp::engine::owned_smem(e->grid, total, vertices, e->smem_fixed, e->smem_all)
+          ? dlp::engine::owned_smem(e->owned_grid, total, vertices, e->smem_fixed, e->smem_all)
           : 0;
   const bool owned = owned_smem > 0;
   GraphRec *recs = e->recs_dev + (p ? e->max_graphs : 0);
@@ -487,8 +488,8 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
   args.progress = sliced ? e->progress_dev : nullptr;
   DLP_CUDA_TRY(cudaEventRecord(e->ev[slot][0], e->stream));
   void *kargs[] = {&args};
-  DLP_TRY(dlp::launch_cooperative(owned ? e->owned_kernel : e->kernel, e->grid, dlp::session::kBlock, kargs,
-                                  args.smem_bytes, e->stream));
+  DLP_TRY(dlp::launch_cooperative(owned ? e->owned_kernel : e->kernel, owned ? e->owned_grid : e->grid,
+                                  dlp::session::kBlock, kargs, args.smem_bytes, e->stream));
   DLP_CUDA_TRY(cudaEventRecord(e->ev[slot][1], e->stream));
   for (int i = 0; i < count; ++i) {
     GraphSlot *g = e->graphs[gids[i]];
@@ -731,6 +732,7 @@ int dlp_engine_create(const dlp_config *cfg_in, int max_graphs, size_t memory_bu
     return bail(dlp::fail(DLP_ERR_CUDA, "occupancy query failed for the engine kernel"));
   if (cfg.blocks_per_sm > 0) per_sm = std::min(per_sm, cfg.blocks_per_sm);
   e->grid = std::min(sms * per_sm, dlp::kSumBlocks);
+  e->owned_grid = std::min(sms, dlp::kSumBlocks);
   int st = DLP_OK;
   if ((st = dalloc(&e->ectl, 1, e->owned, e->owned_bytes)) ||
       (st = dalloc(&e->ctl_all, max_graphs, e->owned, e->owned_bytes)) ||

@@ -39,7 +39,7 @@
 namespace dlp {
 namespace stint {
 
-constexpr int kThreads = 1024;             // threads of the block that runs a stint
+constexpr int kThreads = kBlockThreads;    // threads of the block that runs a stint
 constexpr int kWarps = kThreads / 32;
 constexpr int kSlots = 4096;               // vertex-table slots (power of two)
 constexpr int kSlotsUse = kSlots * 7 / 8;  // in use at most (linear probing stays short below this)

@@ -244,3 +244,12 @@ def test_device_memory_held_by_loading_the_library(runtime):
     """The scratch of the allocation-free propagation: three words for each of 2^20
     vertices, and less than a KiB."""
     assert 12 << 20 <= runtime.lib.fake_variable_bytes() <= (12 << 20) + 1024
+
+
+@pytest.mark.parametrize("source", ["engine.cu", "engine_kernel.cu", "launchers.cu", "tune.cu"])
+def test_the_build_with_512_threads_compiles(tmp_path, source):
+    """A build setting of the persistent kernels (DLP_NVCC_EXTRA=-DDLP_BLOCK=512)."""
+    res = subprocess.run([b._nvcc(), "-gencode", "arch=compute_103a,code=compute_103a", "-std=c++17", "-Xcicc", "-O0",
+                          f"-I{b.INCLUDE}", f"-I{b.CSRC}", "-DDLP_BLOCK=512", "-cuda", str(b.CSRC / source), "-o",
+                          str(tmp_path / "out.ii")], capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr[-2000:]
