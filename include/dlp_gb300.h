@@ -329,8 +329,9 @@ int dlp_engine_artefact(dlp_engine *e, int graph_id, int which, void *host_out, 
  * (num_graphs graphs of sizes[i] vertices and average degree degrees[i],
  * `batches` batches each, propagation capped at max_iterations passes per batch)
  * is timed at every solo_entry as such a launch runs, and at every lane width over
- * frontier lists; a candidate's time is the sum of its two. All must give identical
- * statistics (checked). The fastest is written into cfg->narrow_lanes,
+ * frontier lists; a candidate's time is the sum of its two, a width within 1% of
+ * the default's (8) counting as equal to it. All must give identical statistics
+ * (checked). The fastest is written into cfg->narrow_lanes,
  * cfg->blocks_per_sm, cfg->solo_entry and cfg->subgrid_entry; other fields are
  * kept. */
 typedef struct {

@@ -186,9 +186,11 @@ def test_autotuner_times_each_setting_where_it_has_an_effect(runtime):
     r = dlp.autotune([500, 300], [3, 5], batches=2, max_iterations=10)
     kernels = [x[1] for x in runtime.log() if x[0] == "cooperative"]
     owned, lists = ("engine_kernelILi8ELb1", "engine_kernelILi%dELb0")
-    want = 3 * 2 * [owned] + [lists % lanes for lanes in (1, 4, 8) for _ in range(2)]
+    want = 3 * 2 * [owned] + [lists % lanes for lanes in (8, 4, 1) for _ in range(2)]
     assert len(kernels) == len(want) and all(w in k for w, k in zip(want, kernels)), kernels
     assert len({(c["narrow_lanes"], c["solo_entry"], c["subgrid_entry"]) for c in r["candidates"]}) == 27
+    # a millisecond each in this runtime: nothing to choose by
+    assert (r["narrow_lanes"], r["engine_kw"]) == (8, {"solo_entry": 512, "subgrid_entry": 2048})
 
 
 def test_tuned_shapes_are_kept_for_the_kernels_they_were_measured_on(tmp_path, monkeypatch):
