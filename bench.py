@@ -531,7 +531,7 @@ def gpu_arm(args, td, rank, world, local_rank):
                 "timing": "wall clock, stream synchronised on both sides"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak if peak else None, "traffic": traffic,
-                     "kernel": f"dlp::engine_kernel<{args.lanes or 8}>", "peak_source": peak_kind,
+                     "kernel": "dlp::engine_kernel", "peak_source": peak_kind,
                      "algorithmic_bytes_per_step": bytes_step},
         "cpu_baseline": {"value": cpu_edges / cpu_t if cpu_t > 0 else 0.0, "unit": UNIT, "cores": 1, "kind": "port",
                          "sample": f"oracle port, 1 thread, first {cpu_done} of {nb} batches of the same workload",

@@ -29,7 +29,7 @@ constexpr int kMaxGraphs = 1024;
 // Frontier size below which propagation passes leave the full grid for one
 // block (default 512, at most kSoloEntryMax). Tunable per engine. There is no
 // mode on fewer blocks than all of them in between: with SumBarrier a pass over
-// 600 to 2,000 rows takes 5.1 to 6.2 us on 152 blocks (3.2 to 3.4 on owned rows)
+// 600 to 2,000 rows takes 5.1 to 6.2 us on 152 blocks (3.2 on owned rows)
 // and 7 to 8 us on 16.
 constexpr int kSoloEntryDefault = 512;
 constexpr int kSoloEntryMax = 1024;

@@ -682,10 +682,10 @@ __global__ void __launch_bounds__(kBlock) prop_kernel(PropArgs a) {
 // up to kSmallFront vertices on one block with rows in registers
 // (row_stint.cuh). Larger graphs take prop_kernel above and irlp_kernel below.
 //
-// Measured against prop_kernel and irlp_kernel: propagation from 1,000 affected
-// vertices of 50,000 (degree 5, 2,000 passes at most) 1.13 against 2.64 ms, from
-// 50,000 of a million (degree 7, 300 passes at most) 4.1 against 8.7 ms; recompute
-// of 100,000 vertices 0.82 against 2.43 ms.
+// Measured against prop_kernel and irlp_kernel, on the same inputs: propagation from
+// 1,000 affected vertices of 50,000 (degree 5, 2,000 passes at most) 1.11 against 3.18
+// ms, from 50,000 of a million (degree 7, 300 passes at most) 3.99 against 10.8 ms;
+// recompute of 100,000 vertices 0.75 against 3.09 ms.
 constexpr int kOwnBlock = stint::kThreads;
 constexpr int kSmallFront = 512;
 constexpr unsigned long long kStintNs = 100000000ull;  // the other blocks wait in a barrier with a 2 s limit

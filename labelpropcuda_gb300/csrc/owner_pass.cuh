@@ -19,8 +19,10 @@
 // single bytes (and 298 G loads), hence words.
 //
 // Measured, microseconds a pass, owned rows against lists: 5,000 vertices of
-// degree 5 3.2 against 5.1, 20,000 of degree 7 3.4 against 6.2, 50,000 of degree
-// 5 3.3 against 7.5 to 8.0, 500,000 of degree 7 5.9 against 16.2.
+// degree 5 3.15 against 5.1, 20,000 of degree 7 3.2 against 6.2, 50,000 of degree
+// 5 3.2 against 7.5 to 8.0, 500,000 of degree 7 5.0 against 16.2. A scheduler issues in
+// a fifth of its cycles, and warps stand at the pass's barriers for three quarters of
+// their time.
 //
 // Shared memory ends at 24,576 vertices per block (3.7 million on 151). Most rows
 // then stay in global memory and a scan reads all words of the graph. The engine
