@@ -506,7 +506,7 @@ struct PropArgs {
   float delta;
   int max_iter;
   unsigned *stamp;     // n, zeroed
-  int *lists;          // 3n
+  int *lists;          // 2n: the list of pass k in half k & 1
   int *counts;         // [3][2]
   int *out;            // [0] passes, [1] last mark stamp, [2] next pass after a block-0 stint
   GridBarrier *bar;
@@ -524,10 +524,10 @@ __global__ void __launch_bounds__(kBlock) prop_kernel(PropArgs a) {
   const int lane = threadIdx.x & 31, gwarp = t >> 5, nwarps = nt >> 5;
   const int n = a.n;
   if (ld_relaxed_i32(a.err) != 0) return;
-  auto append = [&](bool pred, int v, int set) {
+  auto append = [&](bool pred, int v, int set, int half) {
     bool wide = false;
     if (pred) wide = a.row_ptr[v + 1] - a.row_ptr[v] > kNarrowMax;
-    int *list = a.lists + static_cast<size_t>(set) * n;
+    int *list = a.lists + static_cast<size_t>(half) * n;
     warp_append(pred && !wide, v, list, &a.counts[2 * set]);
     warp_append_back(pred && wide, v, list, n, &a.counts[2 * set + 1]);
   };
@@ -535,25 +535,24 @@ __global__ void __launch_bounds__(kBlock) prop_kernel(PropArgs a) {
   for (int base = gwarp * 32; base < n; base += nwarps * 32) {
     const int v = base + lane;
     const bool ok = v < n && a.affected[v] == 1 && a.status[v] == kActive && a.gt[v] < 0;
-    append(ok, v, 0);
+    append(ok, v, 0, 0);
   }
   if (!grid_sync(a.bar, a.err, a.timeout_ns)) return;
 
   constexpr int GPW = 32 / G;
   const int grp = lane / G, gl = lane & (G - 1);
-  // The rows of pass k (nn narrow, nw wide in list k % 3) by the warps
-  // [w0, w0 + nws) of the launch; marks go to list (k + 1) % 3.
+  // The rows of pass k (nn narrow, nw wide) by the warps
+  // [w0, w0 + nws) of the launch; marks go to the list of pass k + 1.
   auto rows = [&](int k, int nn, int nw, int w0, int nws) {
-    const int set = k % 3;
     const float *src = (k & 1) ? a.buffer : a.labels;
     float *dst = (k & 1) ? a.labels : a.buffer;
     const unsigned stamp = static_cast<unsigned>(k) + 1u;
     const int nset = (k + 1) % 3;
-    const int *cur = a.lists + static_cast<size_t>(set) * n;
+    const int *cur = a.lists + static_cast<size_t>(k & 1) * n;
     auto mark = [&](bool cand, int v) {
       bool fresh = false;
       if (cand) fresh = atomicMax(&a.stamp[v], stamp) < stamp;
-      append(fresh && a.status[v] == kActive && a.gt[v] < 0, v, nset);
+      append(fresh && a.status[v] == kActive && a.gt[v] < 0, v, nset, (k + 1) & 1);
     };
     for (int base = w0 * GPW; base < nn; base += nws * GPW) {
       const int item = base + grp;
@@ -1282,6 +1281,24 @@ OwnedArgs owned_args(const int *row_ptr, const int *col, const float *val, float
   return a;
 }
 
+PropArgs prop_args(const int *row_ptr, const int *col, const float *val, float *labels, float *buffer,
+                   const int *status, const int *gt, int *affected, int n, float delta, int max_iterations) {
+  PropArgs a{};
+  a.row_ptr = row_ptr;
+  a.col = col;
+  a.val = val;
+  a.labels = labels;
+  a.buffer = buffer;
+  a.status = status;
+  a.gt = gt;
+  a.affected = affected;
+  a.n = n;
+  a.delta = delta;
+  a.max_iter = max_iterations;
+  a.fast_div = g_launcher_arith.load();
+  return a;
+}
+
 int clear_scratch(void *p, size_t bytes, cudaStream_t s) {
   DLP_CUDA_TRY(cudaMemsetAsync(p, 0, bytes, s));
   return DLP_OK;
@@ -1311,6 +1328,37 @@ int coop_grid(const void *kernel) {
   return sms * per_sm;
 }
 
+// Scratch of prop_kernel: `fixed` (kOwnedFixed bytes) holds counters and barrier,
+// `words` (3n) the stamps and the lists. Launches it, waits and returns its pass count.
+int run_lists(PropArgs a, char *fixed, unsigned *words, int *passes, cudaStream_t s) {
+  constexpr size_t kCounters = 64;  // bytes: 16 words
+  static_assert(kCounters + sizeof(GridBarrier) <= kOwnedFixed, "scratch layout");
+  const size_t n = static_cast<size_t>(a.n);
+  // both buffers start at the current labels (src/iterativePropagation.cu:268-270)
+  DLP_CUDA_TRY(cudaMemcpyAsync(a.buffer, a.labels, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
+  DLP_TRY(clear_scratch(fixed, kOwnedFixed, s));
+  DLP_TRY(clear_scratch(words, sizeof(unsigned) * n, s));
+  int *small = reinterpret_cast<int *>(fixed);
+  a.counts = small;  // [0..5]
+  a.out = small + 8;
+  a.err = small + 12;
+  a.bar = reinterpret_cast<GridBarrier *>(fixed + kCounters);
+  a.stamp = words;
+  a.lists = reinterpret_cast<int *>(words + n);
+  a.timeout_ns = 2000000000ull;
+  const void *kern = reinterpret_cast<const void *>(&prop_kernel);
+  const int grid = coop_grid(kern);
+  if (grid <= 0) return fail(DLP_ERR_CUDA, "occupancy query failed");
+  void *args[] = {&a};
+  DLP_TRY(launch_cooperative(kern, grid, kBlock, args, 0, s));
+  int host[5] = {0, 0, 0, 0, 0};  // out[0] and, four words on, err
+  DLP_CUDA_TRY(cudaMemcpyAsync(host, a.out, sizeof(host), cudaMemcpyDeviceToHost, s));
+  DLP_CUDA_TRY(cudaStreamSynchronize(s));
+  if (host[4]) return fail(host[4], "propagation failed on the device");
+  *passes = host[0];
+  return DLP_OK;
+}
+
 }  // namespace
 }  // namespace ref_layout
 }  // namespace dlp
@@ -1318,9 +1366,9 @@ int coop_grid(const void *kernel) {
 using namespace dlp::ref_layout;
 
 // ---------------------------------------------------------------------------
-// Scratch of dlp_iterative_propagation_noalloc: the counters, the barrier, the
-// frontier marks and the frontier list of one propagation call on a graph of at
-// most kNoAllocMaxNodes vertices (12 MiB and less than 1 KiB). It is a
+// Scratch of dlp_iterative_propagation_noalloc: the counters, the barrier and three
+// words for each of at most kNoAllocMaxNodes vertices (two planes of frontier marks
+// and a list; over lists, stamps and two lists): 12 MiB and less than 1 KiB. It is a
 // file-scope device array, so it exists on every GPU that loads this library,
 // from module load until the process exits, whether or not the entry point is
 // ever called.
@@ -1328,10 +1376,8 @@ namespace {
 constexpr int kNoAllocMaxNodes = 1 << 20;
 struct NoAllocScratch {
   char fixed[kOwnedFixed];  // counters and barrier, directly before the marks: cleared with them
-  unsigned marks[2 * kNoAllocMaxNodes];
-  int list[kNoAllocMaxNodes];
+  unsigned words[3 * kNoAllocMaxNodes];
 };
-static_assert(kNoAllocMaxNodes <= 150 * dlp::owner::kMaxVertices, "such graphs run on owned rows");
 }  // namespace
 
 static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
@@ -1527,54 +1573,13 @@ int dlp_iterative_propagation(const int *d_row_ptr, const int *d_col_ind, const 
     cudaFreeAsync(scratch, s);
     return st;
   }
-  const size_t n = static_cast<size_t>(num_nodes);
-  // both buffers start at the current labels (src/iterativePropagation.cu:268-270)
-  DLP_CUDA_TRY(cudaMemcpyAsync(d_labels_buffer, d_labels, sizeof(float) * n, cudaMemcpyDeviceToDevice, s));
-  unsigned *stamp = nullptr;
-  int *lists = nullptr, *small = nullptr;
-  dlp::GridBarrier *bar = nullptr;
-  DLP_TRY(tmp_alloc(&stamp, n, s));
-  DLP_TRY(tmp_alloc(&lists, 3 * n, s));
-  DLP_TRY(tmp_alloc(&small, 16, s));
-  DLP_TRY(tmp_alloc(&bar, 1, s));
-  DLP_CUDA_TRY(cudaMemsetAsync(stamp, 0, sizeof(unsigned) * n, s));
-  DLP_CUDA_TRY(cudaMemsetAsync(small, 0, sizeof(int) * 16, s));
-  DLP_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(dlp::GridBarrier), s));
-  PropArgs a{};
-  a.row_ptr = d_row_ptr;
-  a.col = d_col_ind;
-  a.val = d_values;
-  a.labels = d_labels;
-  a.buffer = d_labels_buffer;
-  a.status = d_vertex_status;
-  a.gt = d_gt_class;
-  a.affected = d_is_affected;
-  a.n = num_nodes;
-  a.delta = delta;
-  a.max_iter = max_iterations;
-  a.stamp = stamp;
-  a.lists = lists;
-  a.counts = small;         // [0..5]
-  a.out = small + 8;        // [8] passes
-  a.err = small + 12;
-  a.bar = bar;
-  a.timeout_ns = 2000000000ull;
-  a.fast_div = g_launcher_arith.load();
-  const void *kern = reinterpret_cast<const void *>(&prop_kernel);
-  const int grid = coop_grid(kern);
-  if (grid <= 0) return dlp::fail(DLP_ERR_CUDA, "occupancy query failed");
-  void *args[] = {&a};
-  DLP_TRY(dlp::launch_cooperative(kern, grid, kBlock, args, 0, s));
-  int host[2] = {0, 0};
-  DLP_CUDA_TRY(cudaMemcpyAsync(&host[0], a.out, sizeof(int), cudaMemcpyDeviceToHost, s));
-  DLP_CUDA_TRY(cudaMemcpyAsync(&host[1], a.err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  DLP_CUDA_TRY(cudaStreamSynchronize(s));
-  for (void *p : {static_cast<void *>(stamp), static_cast<void *>(lists), static_cast<void *>(small),
-                  static_cast<void *>(bar)})
-    cudaFreeAsync(p, s);
-  if (host[1]) return dlp::fail(host[1], "propagation failed on the device");
-  *iterations_used = host[0];
-  return DLP_OK;
+  char *scratch = nullptr;
+  DLP_TRY(tmp_alloc(&scratch, kOwnedFixed + 3 * sizeof(unsigned) * static_cast<size_t>(num_nodes), s));
+  const int st = run_lists(prop_args(d_row_ptr, d_col_ind, d_values, d_labels, d_labels_buffer, d_vertex_status,
+                                     d_gt_class, d_is_affected, num_nodes, delta, max_iterations),
+                           scratch, reinterpret_cast<unsigned *>(scratch + kOwnedFixed), iterations_used, s);
+  cudaFreeAsync(scratch, s);
+  return st;
 }
 
 // dlp_iterative_propagation without any device allocation: the same kernel and
@@ -1604,7 +1609,10 @@ int dlp_iterative_propagation_noalloc(const int *d_row_ptr, const int *d_col_ind
   NoAllocScratch *sc = nullptr;
   DLP_TRY(noalloc_scratch(&sc));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (owned_grid(num_nodes) <= 0) return dlp::fail(DLP_ERR_CUDA, "no room for the propagation kernel's blocks");
+  if (owned_grid(num_nodes) <= 0)  // a part of a GPU, whose blocks cannot own as many vertices
+    return run_lists(prop_args(d_row_ptr, d_col_ind, d_values, d_labels, d_labels_buffer, d_vertex_status, d_gt_class,
+                               d_is_affected, num_nodes, delta, max_iterations),
+                     sc->fixed, sc->words, iterations_used, s);
   OwnedArgs a = owned_args(d_row_ptr, d_col_ind, d_values, d_labels, d_labels_buffer, d_vertex_status, d_gt_class,
                            num_nodes, delta, max_iterations);
   a.affected = d_is_affected;
@@ -1612,8 +1620,8 @@ int dlp_iterative_propagation_noalloc(const int *d_row_ptr, const int *d_col_ind
   char *scratch = reinterpret_cast<char *>(sc);
   a.small = reinterpret_cast<int *>(scratch);
   a.bar = reinterpret_cast<dlp::SumBarrier *>(scratch + kOwnedSmall);
-  a.marks = sc->marks;
-  a.list = sc->list;
+  a.marks = sc->words;
+  a.list = reinterpret_cast<int *>(sc->words + 2 * static_cast<size_t>(kNoAllocMaxNodes));
   // what must start at zero: the counters, the barrier and the marks in use
   DLP_TRY(clear_scratch(scratch, kOwnedFixed + 2 * sizeof(unsigned) * owned_plane(num_nodes), s));
   return launch_owned(reinterpret_cast<const void *>(&prop_owned_kernel), a, iterations_used, s);

@@ -26,6 +26,7 @@ struct State {
   std::map<std::string, void *> symbol;
   std::map<const void *, std::pair<std::string, size_t>> variable;
   size_t capacity = SIZE_MAX;
+  int sms = 152;
   int streams = 0;
   cudaStreamCaptureMode mode = cudaStreamCaptureModeGlobal;
   bool capturing = false, spoilt = false;  // some stream; by a call it does not take
@@ -85,6 +86,7 @@ void fake_clear_log() { st().log.clear(); }
 // The first `n` words of the next copy to the host.
 void fake_result(const int *words, int n) { st().result.assign(words, words + n); }
 void fake_capacity(size_t bytes) { st().capacity = bytes; }
+void fake_multiprocessors(int n) { st().sms = n; }
 void fake_begin_capture() {
   st().capturing = true;
   st().spoilt = false;
@@ -152,7 +154,7 @@ cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3 g, dim3 b, void **, 
 }
 cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
   switch (a) {
-    case cudaDevAttrMultiProcessorCount: *v = 152; break;
+    case cudaDevAttrMultiProcessorCount: *v = st().sms; break;
     case cudaDevAttrMaxSharedMemoryPerBlockOptin: *v = 232448; break;
     case cudaDevAttrMaxSharedMemoryPerMultiprocessor: *v = 233472; break;
     case cudaDevAttrReservedSharedMemoryPerBlock: *v = 1024; break;

@@ -255,3 +255,25 @@ def test_the_build_with_512_threads_compiles(tmp_path, source):
                           f"-I{b.INCLUDE}", f"-I{b.CSRC}", "-DDLP_BLOCK=512", "-cuda", str(b.CSRC / source), "-o",
                           str(tmp_path / "out.ii")], capture_output=True, text=True)
     assert res.returncode == 0, res.stderr[-2000:]
+
+
+def test_allocation_free_propagation_on_a_part_of_a_gpu(runtime):
+    """20 multiprocessors cannot own a million vertices: lists, in the same scratch."""
+    n = 1 << 20
+    a = arrays(*[n + 1] * 8)
+    try:
+        runtime.lib.fake_multiprocessors(20)
+        runtime.lib.cudaDeviceReset()  # the next context asks the device anew
+        runtime.log()
+        runtime.result(7, 0, 0, 0, 0)
+        used = ctypes.c_int(0)
+        N.check(N.lib().dlp_iterative_propagation_noalloc(*[x.ptr for x in a], n, ctypes.c_float(1e-4), 9,
+                                                          ctypes.byref(used), None))
+        assert used.value == 7
+        launched = [x for x in runtime.log() if x[0] == "cooperative"]
+        assert len(launched) == 1 and "prop_kernel" in launched[0][1] and int(launched[0][2]) % 20 == 0
+    finally:
+        runtime.lib.fake_multiprocessors(152)
+        runtime.lib.cudaDeviceReset()
+        for x in a:
+            x.ptr = ctypes.c_void_p()
