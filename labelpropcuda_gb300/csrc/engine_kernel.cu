@@ -1971,8 +1971,9 @@ int list_passes(size_t vertices) { return vertices < 1750000 ? 0 : 8; }
 
 size_t owned_smem(int grid, int graphs, size_t vertices, size_t fixed, size_t most) {
   if (vertices > owned_limit(grid)) return 0;
+  // the graphs' own records count as well
   const size_t need = owned_need(grid, graphs, vertices / owner::kTile);
-  return need > most ? 0 : owner::smem_of(need, sizeof(SoloCache), fixed, most);
+  return owner::leaves_l1(need + owner::kPoolBytes, fixed) ? owner::smem_of(need, sizeof(SoloCache), fixed, most) : 0;
 }
 
 const void *owned_kernel_ptr() { return reinterpret_cast<const void *>(&engine_kernel<8, true>); }
