@@ -455,8 +455,10 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
     passes = std::max(passes, rh[i].ba.max_iter - rh[i].ba.pass0);
   }
   if (opts.pass_budget > 0) passes = std::min(passes, opts.pass_budget);
+  const bool worth = passes > dlp::engine::kListOnly &&
+                     (opts.slice_ns == 0 || opts.slice_ns >= dlp::engine::least_slice_ns(vertices));
   const size_t owned_smem =
-      passes > dlp::engine::kListOnly && vertices <= e->mark_plane
+      worth && vertices <= e->mark_plane
           ? dlp::engine::owned_smem(e->owned_grid, total, vertices, e->smem_fixed, e->smem_all)
           : 0;
   const bool owned = owned_smem > 0;

@@ -108,10 +108,12 @@ size_t engine_dynamic_smem();
 void fit_marks(dlp_engine *e, size_t room);
 // Vertices (in whole tiles) of a launch up to which a grid can own them.
 unsigned owned_limit(int grid);
-// Full-grid passes over lists before a launch of that many vertices loads rows; and
-// the most passes that a launch may run over lists only.
+// Full-grid passes over lists before a launch of that many vertices loads rows; the
+// most passes that a launch may run over lists only, and the shortest time slice of a
+// launch that loads rows.
 int list_passes(size_t vertices);
 constexpr int kListOnly = 3;
+unsigned long long least_slice_ns(size_t vertices);
 // Dynamic shared memory of a launch with owned passes over that many graphs and
 // vertices (in whole tiles), beside `fixed` bytes of static shared memory and at
 // most `most`; 0 when they do not fit.

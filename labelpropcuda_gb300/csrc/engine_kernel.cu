@@ -1969,6 +1969,15 @@ unsigned owned_limit(int grid) { return grid > 1 ? static_cast<unsigned>(grid - 
 // 3.5, 4.1, 5.0, 7.7 and 3.0, 3.5, 5.0, 7.5; with 300 passes they differ by less than 1%.
 int list_passes(size_t vertices) { return vertices < 1750000 ? 0 : 8; }
 
+// Nor does a time slice that is hardly longer than the load. Four batches each over
+// several graphs from a queue, milliseconds over lists and on owned rows: 80,000 vertices
+// in all, slices of 20 us 19.7 and 15.8; 640,000, 30 us 26.8 and 39.3, 60 us 22.9 and
+// 19.3; 1.6 million, 60 us 40.2 and 46.8, 120 us 35.4 and 30.4; 2.4 million, 200 us 49.1
+// and 52.8, 400 us 46.5 and 48.5.
+unsigned long long least_slice_ns(size_t vertices) {
+  return vertices < 1750000 ? 15000 + vertices * 40 / 1000 : 1000000;
+}
+
 size_t owned_smem(int grid, int graphs, size_t vertices, size_t fixed, size_t most) {
   if (vertices > owned_limit(grid)) return 0;
   // the graphs' own records count as well

@@ -277,3 +277,16 @@ def test_allocation_free_propagation_on_a_part_of_a_gpu(runtime):
         runtime.lib.cudaDeviceReset()
         for x in a:
             x.ptr = ctypes.c_void_p()
+
+
+@pytest.mark.parametrize("passes,slice_us,owned", [(3, 0.0, False), (4, 0.0, True), (0, 14.0, False), (0, 16.0, True),
+                                                   (4, 14.0, False), (0, 0.0, True)])
+def test_rows_are_loaded_for_more_than_a_few_passes(runtime, passes, slice_us, owned):
+    p = dlp.Problem(1001, 3, 2, 1, cache_dir="")
+    eng = dlp.Engine(1, max_iterations=50)
+    g = eng.add_problem(p)
+    runtime.log()
+    eng.step_sliced([(g, 0, dlp.DeviceBatch(p.batches[0]))], pass_budget=passes, slice_us=slice_us)
+    kernel, = [x[1] for x in runtime.log() if x[0] == "cooperative"]
+    assert ("ELb1" in kernel) == owned
+    eng.close()

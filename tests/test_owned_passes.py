@@ -166,3 +166,28 @@ def test_rows_that_take_a_tile_many_steps(gpu, oracle, n, degree, solo):
         for k in EXACT_STATS:
             assert got[k] == want[k], (b, k)
         assert sess.labels().tobytes() == orc.labels().tobytes(), b
+
+
+@pytest.mark.gpu
+def test_short_time_slices_among_longer_ones(gpu, oracle):
+    """Slices of 10 us run over lists, of 40 us on owned rows; the results are those of
+    batches run to their end."""
+    probs = [dlp.Problem(n, d, 3, s, cache_dir="") for n, d, s in ((1500, 5, 1), (20000, 9, 2), (3000, 34, 3))]
+    cap = 150
+    orcs = [oracle.OracleRun.from_problem(p, threads=4, max_iterations=cap) for p in probs]
+    eng = dlp.Engine(len(probs), max_iterations=cap)
+    ids = [eng.add_problem(p) for p in probs]
+    dev = [[dlp.DeviceBatch(b) for b in p.batches] for p in probs]
+    nxt, step = [0] * len(probs), 0
+    while any(x < 3 for x in nxt) or any(eng.in_progress(g) for g in ids):
+        start = [i for i, g in enumerate(ids) if nxt[i] < 3 and not eng.in_progress(g)]
+        done, _ = eng.step_sliced([(ids[i], nxt[i], dev[i][nxt[i]]) for i in start], slice_us=(10.0, 40.0)[step % 2])
+        for i in start:
+            nxt[i] += 1
+        for g in done:
+            i = ids.index(g)
+            want, got = orcs[i].apply(nxt[i] - 1, probs[i].batches[nxt[i] - 1]), eng.stats(g, nxt[i] - 1)
+            for k in EXACT_STATS:
+                assert got[k] == want[k], (i, nxt[i] - 1, k)
+            assert eng.labels(g).tobytes() == orcs[i].labels().tobytes(), (i, nxt[i] - 1)
+        step += 1
