@@ -2,6 +2,9 @@
 // checks every vertex and entry it is asked for.
 //   owner_block remainder   a partial last tile whose rows do not fit the pool
 //   owner_block counter     rows at the end of their visit counters beside a wide row
+//   owner_block mixed       passes over short, long and wide rows, listed and by tiles,
+//                           marked and dense, with and without room in the pool
+//   owner_block shared      the shared memory of a launch, over all sizes
 #include "owner_pass.cuh"
 
 #include <cstdio>
@@ -100,6 +103,65 @@ struct Run {
   }
 };
 
+// What a pass over the marked vertices has to leave: labels, marks, and whether a label
+// moved.
+struct Expected {
+  std::vector<float> lab;
+  std::vector<unsigned> marks;
+  int rows = 0;
+  bool moved = false;
+};
+Expected expected(const Run &r, int k, float delta, bool dense) {
+  Expected x{r.lab[(k & 1) ^ 1], std::vector<unsigned>(r.marks[0].size(), 0)};
+  for (int v = 0; v < r.g.n; ++v) {
+    if (!dense && !r.marks[k & 1][v]) continue;
+    ++x.rows;
+    x.lab[v] = r.g.start[v] == r.g.start[v + 1] ? r.lab[k & 1][v] : r.average(k & 1, v);
+    if (std::fabs(x.lab[v] - r.lab[k & 1][v]) <= delta) continue;
+    x.moved = true;
+    x.marks[v] = 1;
+    for (int e = r.g.start[v]; e < r.g.start[v + 1]; ++e) x.marks[r.g.col[e]] = 1;
+  }
+  return x;
+}
+
+// Passes over 300 vertices (ten tiles, the last partial) of a block of `threads`.
+void mixed(unsigned threads, int pool, bool dense, int &outside, int &wrong) {
+  const auto len = [](int v) { return v % 97 == 5 ? 290 : v % 9 == 0 ? 33 + v % 40 : v % 5 == 0 ? 9 + v % 24 : v % 9; };
+  Run r(graph(300, len), pool);
+  Head &h = r.s.head();
+  const float delta = 1e-3f;
+  for (int v = 0; v < r.g.n; ++v) r.marks[0][v] = v % 3 == 0;
+  run_block(1, threads, [&] {
+    load(r.s, r.g);
+    __syncthreads();
+    if (dense) list_all(r.s);
+  });
+  for (int k = 0; k < 4; ++k) {
+    const Expected x = expected(r, k, delta, dense);
+    unsigned *const own = r.marks[k & 1].data(), *const next = r.marks[(k & 1) ^ 1].data();
+    const bool tiles = threads >= 320;
+    run_block(1, threads, [&] {
+      auto each = [](int) {};
+      if (dense) dense_pass(r.s, r.g, k, delta);
+      else if (tiles) tile_pass(r.s, r.g, own, next, k, delta, false, each);
+      else pass(r.s, r.g, own, next, k, delta, false, each);
+    });
+    for (int v = 0; v < r.g.n; ++v) {
+      wrong += std::fabs(r.lab[(k & 1) ^ 1][v] - x.lab[v]) > 1e-6f;
+      if (!dense) wrong += r.marks[(k & 1) ^ 1][v] != x.marks[v] || own[v] != 0;
+    }
+    for (size_t i = r.g.n; i < r.marks[0].size(); ++i) wrong += r.marks[0][i] != 0 || r.marks[1][i] != 0;
+    wrong += (h.moved != 0) != x.moved;
+    if (!dense) {
+      wrong += (h.count & 0xffff) + (h.count >> 16) + h.wide != x.rows;
+      h.count = h.wide = h.wide_at = 0;
+    }
+    h.moved = 0;
+  }
+  outside += r.g.bad;
+}
+
 int main(int argc, char **argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   int wrong = 0;
@@ -137,6 +199,27 @@ int main(int argc, char **argv) {
     });
     wrong += std::fabs(r.lab[0][0] - r.average(1, 0)) > 1e-5f;
     std::printf("outside %d wrong %d label %.1f\n", r.g.bad, wrong, r.lab[0][3]);
+  } else if (what == "mixed") {
+    int outside = 0;
+    for (int pool : {20, 2000, 12000})
+      for (unsigned threads : {64u, 320u}) {
+        mixed(threads, pool, false, outside, wrong);
+        mixed(threads, pool, true, outside, wrong);
+      }
+    std::printf("outside %d wrong %d\n", outside, wrong);
+  } else if (what == "shared") {
+    constexpr size_t kFixed = 10192, kMost = 222240, kLeast = 110768;
+    for (size_t need = 0; need <= kMost; need += 16) {
+      const size_t bytes = smem_of(need, kLeast, kFixed, kMost);
+      wrong += bytes > kMost || bytes % 16 != 0 || bytes < need || bytes < kLeast;
+      // L1 keeps more than its last 28 KB whenever that can be, and no step is taken
+      // that the vertices and their pool do not ask for
+      wrong += leaves_l1(need, kFixed) && bytes + kFixed + kSystemBytes > kSteps[3];
+      for (size_t step : kSteps)
+        wrong += std::max(need + kPoolBytes, kLeast) + kFixed + kSystemBytes <= step &&
+                 bytes + kFixed + kSystemBytes > step;
+    }
+    std::printf("wrong %d\n", wrong);
   } else {
     return 2;
   }

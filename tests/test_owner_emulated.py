@@ -60,3 +60,13 @@ def test_rows_keep_no_count_that_can_run_over(block):
     """A row whose visit counter would run over is not taken for one listed as a
     row of more than 32 entries."""
     assert block("counter") == "outside 0 wrong 0 label 7.0\n"
+
+
+def test_short_long_and_wide_rows(block):
+    """Labels, marks and row counts of passes over rows of 0 to 290 entries, with room
+    for none, some and all of them, listed and by tiles, marked and dense."""
+    assert block("mixed") == "outside 0 wrong 0\n"
+
+
+def test_shared_memory_of_a_launch(block):
+    assert block("shared") == "wrong 0\n"
