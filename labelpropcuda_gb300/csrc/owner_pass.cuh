@@ -165,7 +165,7 @@ __device__ __forceinline__ int graph_of(unsigned m) { return static_cast<int>(m 
 // all its warps, also where it owns at most 32 vertices per warp: 2,000 vertices of
 // degree 100 are a tile a block, whose warp ran 32 rows one after the other while 31
 // waited. Measured, 8 batches in milliseconds over lists, always by tiles, and so:
-// 2,000 vertices of degree 100 5.3, 10.5 and 2.8; 20,000 of degree 100 5.9, 8.6 and 4.3;
+// 2,000 vertices of degree 100 5.3, 10.5 and 2.8; 20,000 of degree 100 5.9, 8.6 and 3.6;
 // 5,000 of degree 20 6.9, 3.9 and 3.5; 20,000 of degree 12 13.7, 6.6 and 6.5. (With 4
 // steps the last two take 4.1 and 7.1.)
 constexpr int kTileSteps = 2;
@@ -391,6 +391,11 @@ __device__ __forceinline__ bool row(const Store &s, const Graph &gr, bool valid,
 // of 256, then the tree. AHEAD entries a lane in flight: with four, a step is three
 // trips to L2 (entries, what the caller knows of the neighbours, labels) for 128
 // entries; passes over tiles, which have few such rows, have no registers for that.
+// The neighbours' marks are set by a reduction: where rows are wide a vertex is
+// marked by many of them in one pass, and stores of one word from many SMs took
+// longer. 45 passes of a propagation over 20,000 vertices of degree 100 take 1.8 ms
+// and 2.4 with stores, 37 over 100,000 of degree 64 4.1 and 4.5; over 2,000 of degree
+// 100, one warp's rows at a time, 0.75 and 0.68; a million of degree 40 the same.
 template <bool MARK, int AHEAD, class Graph>
 __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i, int k, float delta, bool fast,
                                          unsigned *next) {
@@ -451,7 +456,7 @@ __device__ __forceinline__ bool wide_row(const Store &s, const Graph &gr, int i,
       const unsigned can = gr.template markables<AHEAD>(g, u);
 #pragma unroll
       for (int j = 0; j < AHEAD; ++j)
-        if ((can >> j) & 1u) next[l.flat + u[j]] = 1;
+        if ((can >> j) & 1u) atomicOr(next + l.flat + u[j], 1u);
     }
     if (lane == 0) next[l.flat + v] = 1;
   }
