@@ -296,8 +296,8 @@ void grow_marks(dlp_engine *e) {
   e->mark_plane = static_cast<unsigned>(want);
 }
 
-// place(), which makes a graph of `need` bytes resident; the mark planes give way
-// to it, within the budget and on a full device.
+// place(), which makes a graph of `need` bytes resident, or a batch's room (no part of
+// the budget); the mark planes give way to it, within the budget and on a full device.
 template <class Place>
 int with_room(dlp_engine *e, size_t need, Place place) {
   if (e->budget > 0 && e->used + need + mark_bytes(e) > e->budget) drop_marks(e);
@@ -400,7 +400,7 @@ int launch_step(dlp_engine *e, int count, const int *gids, const int *batch_idx,
     for (int j = 0; j < i; ++j)
       if (gids[j] == gids[i]) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "a graph appears twice in one step");
     DLP_TRY(check_view(&dv[i], g->n));
-    DLP_TRY(grow_graph_scratch(e, g, dv[i].num_edges, dv[i].num_deleted));
+    DLP_TRY(with_room(e, 0, [&] { return grow_graph_scratch(e, g, dv[i].num_edges, dv[i].num_deleted); }));
   }
   const int p = e->steps & 1;
   DLP_CUDA_TRY(cudaEventSynchronize(e->recs_free[p]));
@@ -560,7 +560,10 @@ int stage_step(dlp_engine *e, int count, const int *gids, const dlp_batch_view *
     cudaFree(e->stage_dev[p]);
     e->stage_dev[p] = nullptr;
     e->stage_cap[p] = 0;
-    DLP_CUDA_TRY(cudaMalloc(&e->stage_dev[p], total * 2));
+    DLP_TRY(with_room(e, 0, [&]() -> int {
+      DLP_CUDA_TRY(cudaMalloc(&e->stage_dev[p], total * 2));
+      return DLP_OK;
+    }));
     e->stage_cap[p] = total * 2;
   }
   char *hp = e->pinned[p], *dp = e->stage_dev[p];
@@ -1118,7 +1121,7 @@ int dlp_engine_reserve(dlp_engine *e, int graph_id, int max_edges, int max_delet
   GraphSlot *g = slot_of(e, graph_id);
   if (!g || max_edges < 0 || max_deleted < 0) return dlp::fail(DLP_ERR_INVALID_ARGUMENT, "unknown graph or negative size");
   DLP_CUDA_TRY(cudaSetDevice(e->device));
-  return grow_graph_scratch(e, g, max_edges, max_deleted);
+  return with_room(e, 0, [&] { return grow_graph_scratch(e, g, max_edges, max_deleted); });
 }
 
 int dlp_engine_graph_nodes(const dlp_engine *e, int graph_id) {

@@ -156,6 +156,24 @@ def test_marks_give_way_to_a_graph_on_a_full_device(runtime):
     eng.close()
 
 
+@pytest.mark.parametrize("grow", ["reserve", "step", "stage"])
+def test_marks_give_way_to_a_batch_on_a_full_device(runtime, grow):
+    p = dlp.Problem(8000, 3, 1, 1, cache_dir="")
+    batch = dlp.Batch.make(inserted=[0, 1], edge_src=[0], edge_dst=[1], edge_weight=[0.5])
+    eng = dlp.Engine(1)
+    g = eng.add_problem(p)
+    if grow == "stage":
+        eng.reserve(g, 1, 1)  # leaves the copy of the batch to be allocated
+    runtime.log()
+    runtime.lib.fake_capacity(runtime.lib.fake_used())
+    if grow == "reserve":
+        eng.reserve(g, 1, 1)
+    else:
+        eng.step([(g, 0, batch)])
+    assert ["free", str(8 * 8000)] in runtime.log()
+    eng.close()
+
+
 def test_server_keeps_its_budget(runtime):
     p = dlp.Problem(1001, 3, 2, 1, cache_dir="")
     eng = dlp.Engine(2)
